@@ -46,11 +46,11 @@ struct cvtpm_ctx {
     float4* S[2][2];
     float4* smooth[2];
     float4 *tmp, *tmp2, *pdT;
-    float4* pdP[2];
+    float* pdP[2];                    /* smoother duals (pm_pd_dual_bytes) */
     /* the right view's smoother runs on `side`, beside the next left pass,
      * with scratch of its own */
     float4 *tmpR, *tmp2R, *pdTR;
-    float4* pdPR[2];
+    float* pdPR[2];
     cudaStream_t side = nullptr;
     cudaEvent_t side_fork = nullptr, side_join = nullptr;
     short4* list[2];
@@ -212,6 +212,8 @@ cvtpm_status ensure_buffers(cvtpm_ctx* ctx, int W, int H) {
     }
     const size_t n = (size_t)W * H;
     const size_t nr = (size_t)rec_pitch(W) * H;
+    /* duals: the one-step kernel keeps two float4 per pixel, the blocked one six planes */
+    const size_t pd = std::max(n * 32, pm_pd_dual_bytes(W, H));
     size_t off = 0;
     std::vector<std::pair<void**, size_t>> parts;
     auto add = [&](void** p, size_t bytes) { parts.push_back({p, bytes}); off = align_up(off, 256) + bytes; };
@@ -228,7 +230,7 @@ cvtpm_status ensure_buffers(cvtpm_ctx* ctx, int W, int H) {
         add((void**)&ctx->smooth[v], n * 16);
         add((void**)&ctx->list[v], n * 8);
         add((void**)&ctx->win[v], n);
-        add((void**)&ctx->pdP[v], n * 32);
+        add((void**)&ctx->pdP[v], pd);
     }
     add((void**)&ctx->tmp, n * 16);
     add((void**)&ctx->tmp2, n * 16);
@@ -236,8 +238,8 @@ cvtpm_status ensure_buffers(cvtpm_ctx* ctx, int W, int H) {
     add((void**)&ctx->tmpR, n * 16);
     add((void**)&ctx->tmp2R, n * 16);
     add((void**)&ctx->pdTR, n * 16);
-    add((void**)&ctx->pdPR[0], n * 32);
-    add((void**)&ctx->pdPR[1], n * 32);
+    add((void**)&ctx->pdPR[0], pd);
+    add((void**)&ctx->pdPR[1], pd);
     add((void**)&ctx->valid, n);
     add((void**)&ctx->occ, n * 4);
     const size_t need = align_up(off, 256);
@@ -363,20 +365,20 @@ cvtpm_status prep_views(cvtpm_ctx* ctx, const cvtpm_params& p, const float* img0
  * PDROFInpaint::apply, cvt/gfx/PDROFInpaint.h:50-98 (mask: the occlusion
  * map): u warm-starts from `output`, p from 0;
  * `iters` steps, plus one when `iters` is odd so the result lands in
- * `output` (:83-95).  The steps run PDB_K at a time in the temporally blocked
- * kernel (identical arithmetic); iters == 0 keeps the reference's single
+ * `output` (:83-95).  The steps run pm_pd_block_steps() at a time in the
+ * temporally blocked kernel (identical arithmetic); iters == 0 keeps the reference's single
  * extra step from a copy of the input. */
 cvtpm_status pd_apply(cvtpm_ctx* ctx, float4* output, const float4* input, const float* wgt, float lambda, int iters,
                       int W, int H, cudaStream_t st, const float* mask = nullptr, int scratch = 0) {
     const size_t n = (size_t)W * H;
     float4* const pdT = scratch ? ctx->pdTR : ctx->pdT;
-    float4* const pdP0 = scratch ? ctx->pdPR[0] : ctx->pdP[0];
-    float4* const pdP1 = scratch ? ctx->pdPR[1] : ctx->pdP[1];
+    float* const pdP0 = scratch ? ctx->pdPR[0] : ctx->pdP[0];
+    float* const pdP1 = scratch ? ctx->pdPR[1] : ctx->pdP[1];
     PhaseTimer tm(ctx, st, ctx->ev_pd);
     if (iters == 0) {
         CK(cudaMemcpyAsync(pdT, input, n * 16, cudaMemcpyDeviceToDevice, st), "pd copy");
         CK(cudaMemsetAsync(pdP0, 0, n * 32, st), "pd clear");
-        LK(pm_launch_pd_step(output, pdP1, pdT, pdP0, input, wgt, mask, lambda, W, H, st), "pd step");
+        LK(pm_launch_pd_step(output, (float4*)pdP1, pdT, (const float4*)pdP0, input, wgt, mask, lambda, W, H, st), "pd step");
         ++ctx->stats.pd_launches;
         ++ctx->stats.pd_steps;
         tm.stop();
@@ -385,7 +387,7 @@ cvtpm_status pd_apply(cvtpm_ctx* ctx, float4* output, const float4* input, const
     const int total = iters + (iters & 1);
     const int K = pm_pd_block_steps();
     float4* U[2] = {output, pdT};
-    float4* Pp[2] = {pdP0, pdP1};
+    float* Pp[2] = {pdP0, pdP1};
     int l = 0;
     for (int done = 0; done < total; done += K, ++l) {
         const int steps = total - done < K ? total - done : K;
@@ -1413,7 +1415,7 @@ cvtpm_status phase_pd(PhaseState& S, int v, float lambda) {
                 cvtpm_ctx* c = ctx->bpairs[e];
                 W = S.pairs[e].width; H = S.pairs[e].height;
                 float4* U[2] = {c->smooth[v], c->pdT};
-                float4* Pp[2] = {c->pdP[0], c->pdP[1]};
+                float* Pp[2] = {c->pdP[0], c->pdP[1]};
                 a.uout = U[(l + 1) & 1]; a.pout = Pp[(l + 1) & 1];
                 a.uin = U[l & 1]; a.pin = Pp[l & 1];
                 a.f = c->tmp2; a.wgt = c->wgt[v];
@@ -1869,8 +1871,13 @@ cvtpm_status cvtpm_tool_pd_time(cvtpm_ctx* ctx, int steps, void* stream, float* 
     float best = 1e30f;
     cvtpm_status s = CVTPM_OK;
     for (int rep = 0; rep < 3 && s == CVTPM_OK; ++rep) {
-        /* the left view's smoother input of the last call, smoothed into
-         * scratch that the next call rewrites before reading */
+        /* the left view's smoother input of the last call, warm-started from
+         * its smoothed field as depthMap's own calls are, into scratch that the
+         * next call rewrites before reading */
+        if (cudaMemcpyAsync(ctx->tmpR, ctx->smooth[0], (size_t)W * H * 16, cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
+            s = CVTPM_ERR_CUDA;
+            break;
+        }
         cudaEventRecord(a, st);
         s = pd_apply(ctx, ctx->tmpR, ctx->tmp2, ctx->wgt[0], 5.0f, steps, W, H, st, nullptr, 1);
         cudaEventRecord(b, st);

@@ -993,127 +993,323 @@ k_pd_step(float4* __restrict__ uout, float4* __restrict__ pout, const float4* __
     pout[o * 2 + 1] = hi;
 }
 
-/* PDB_K steps per launch on a PDB_TX x PDB_TY tile with a PDB_K-pixel halo
- * held in shared memory.  Every step recomputes the dual over the whole
- * region (phase 1) and then the primal (phase 2), in place; errors from the
- * region's open edges advance one pixel per step, so after PDB_K steps the
- * tile is exact.  Image borders keep the reference's semantics: u is read
- * clamped to the edge, the dual and the weight are zero outside. */
-#define PDB_TX 32
-#ifndef PDB_TY
-#define PDB_TY 16        /* the plain path's tile height; the batch tuner may choose 8 */
-#endif
-#ifndef PDB_K
-#define PDB_K 4
-#endif
-
-/* (k % w, k / w) without an integer division: the fraction of (k + 0.5) / w
- * is at least 0.5 / w away from an integer, and the product with the
- * rounded reciprocal is off by less than 2.4e-7 (k + 0.5) / w, so its
- * truncation is k / w for every k below 2^21. */
-PM_DEV void split_index(int k, int w, float inv_w, int& x, int& y) {
-    y = (int)(((float)k + 0.5f) * inv_w);
-    x = k - y * w;
+/* The temporally blocked smoother: up to K steps per launch on a region of
+ * 64 x (NW * R) cells, the tile being the region without a halo of K cells.
+ * Every step updates every cell of the region; a cell's error from the
+ * region's open edges advances one cell per step, so after K steps the tile
+ * is exact.
+ *
+ * What bounds it is instruction issue, so the layout avoids instructions: a
+ * lane owns two adjacent columns and R rows and keeps u and both duals in
+ * registers as column pairs (packed FP32 arithmetic); the right and left
+ * neighbours of a pair come from the adjacent lanes by shuffle, the rows above
+ * and below a warp's R rows through shared memory (two barriers per step);
+ * the per-cell constants (lambda f, w and the dual denominator with its
+ * reciprocal) are read from shared memory.  The fourth channel is left out:
+ * u.w is 1 after any step and no other channel reads its duals.  Duals are
+ * kept negated, in registers and in memory, as the quotient below comes out.
+ *
+ * Divisions.  A step divides six dual values by the cell's denominator and
+ * three primal values by 1 + tau lambda; both are constant over the steps, so
+ * each is kept with ny = -RN(1/b) and x / b formed from it:
+ *   Q0 = x ny, r0 = Q0 b + x, Q1 = r0 ny + Q0, r1 = Q1 b + x, Q2 = r1 ny + Q1,
+ * all but the first fused.  Q1 is within an ulp of -x/b, so r1 is exact and
+ * Q2 = -RN(x / b) (Markstein's theorem on division by a correctly rounded
+ * reciprocal, "Computation of elementary functions on the IBM RISC System/6000
+ * processor", 1990), including the sign of a zero x.  The theorem wants no
+ * underflow or overflow: a cell with 0 < |x| < 2^-100 takes IEEE divisions,
+ * and so does a block whose values are not all of moderate size (`tame`).
+ *
+ * Measured at 1242x375, 4 steps per launch (ncu): 29-38 us per launch, where
+ * the form that kept everything in shared memory as float4 and divided with
+ * IEEE divisions took 98 us (4.5 times the instructions); depthMap 504.5 ->
+ * 484.7 ms, 640x480 x 3 iterations 139.6 -> 133.6 ms, 64x48 35.3 -> 32.5 ms.
+ * 8 warps of 3 rows: 8 x 2 and 16 x 2 or 3 rows, and 2 or 6 steps per launch,
+ * are within 1.5 % of it at these sizes.
+ */
+#define PDS_RX 64
+constexpr int pds_rows(int NW, int R) { return NW * R; }
+constexpr size_t pds_smem(bool inpaint, int NW, int R) {
+    return (size_t)((inpaint ? 8 : 6) * NW * R + 6 * NW) * PDS_RX * sizeof(float);
 }
+/* row pitch (floats) of a dual plane: even, so a column pair is aligned */
+__host__ __device__ constexpr int pds_pitch(int W) { return (W + 1) & ~1; }
 
-/* shared memory of a TY-row tile with a K-pixel halo: u, both duals and f
- * (float4), w and the dual denominator (float) for every cell of the region */
-constexpr size_t pd_block_smem(int TY, int K = PDB_K) {
-    return (size_t)(PDB_TX + 2 * K) * (TY + 2 * K) * (4 * 16 + 2 * 4);
+/* -RN(x / b) for both halves, from b and ny = -RN(1 / b) */
+PM_DEV float2 neg_div2(float2 x, float2 b, float2 ny) {
+    const float2 q0 = fmul2(x, ny);
+    float2 r = ffma2(q0, b, x);
+    const float2 q1 = ffma2(r, ny, q0);
+    r = ffma2(q1, b, x);
+    return ffma2(r, ny, q1);
 }
+/* s = RN(sqrt(v)) and ny = -RN(1 / s) for both halves, 1 <= v <= PDS_VMAX:
+ * Newton's iteration for 1 / sqrt(v) from rsqrt.approx and one fused residual
+ * step each for the root and its reciprocal (Markstein, as above).  Compared
+ * with __fsqrt_rn and __frcp_rn for every float in [1, 2^100]: the roots are
+ * all equal, and so are the reciprocals but those of significands of ones.
+ * Those, and they alone, leave a residual of 2^-24 before the last step: the
+ * return value is the larger residual. */
+#define PDS_VMAX 1.2676506e30f                       /* 2^100 */
+#define PDS_RESID 5.9604645e-8f                      /* 2^-24 */
+PM_DEV float norm2(float2 v, float2& s, float2& ny) {
+    float2 y;
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(y.x) : "f"(v.x));
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(y.y) : "f"(v.y));
+    float2 g = fmul2(v, y), h = fmul2(y, f2s(0.5f));
+    const float2 r = ffma2(fmul2(y, f2s(-0.5f)), g, f2s(0.5f));
+    g = ffma2(g, r, g);
+    h = ffma2(h, r, h);
+    s = ffma2(ffma2(fmul2(g, f2s(-1.0f)), g, v), h, g);
+    const float2 sn = fmul2(s, f2s(-1.0f));
+    float2 t = fadd2(h, h);
+    t = ffma2(ffma2(sn, t, f2s(1.0f)), t, t);
+    const float2 e = ffma2(sn, t, f2s(1.0f));
+    ny = fmul2(ffma2(e, t, t), f2s(-1.0f));
+    return fmaxf(e.x, e.y);
+}
+/* x / s for both halves (multiplying by -1 is exact) */
+PM_DEV float2 div_norm2(float2 x, float2 s, float2 ny) { return fmul2(neg_div2(x, s, ny), f2s(-1.0f)); }
+/* 2 bits(x) - 1 as unsigned: 0xffffffff for zeros, small for tiny values */
+PM_DEV unsigned pds_mag(float x) { return 2u * (unsigned)__float_as_int(x) - 1u; }
+#define PDS_TINY (2u * (27u << 23) - 1u)             /* pds_mag(2^-100) */
+PM_DEV unsigned pds_mag2(unsigned m, float2 x) { return min(m, min(pds_mag(x.x), pds_mag(x.y))); }
+PM_DEV float neg_div_ieee(float x, float b) { return x == 0.0f ? -x : -(x / b); }
 
-/* TY rows, at most K steps (K is also the halo width). */
-template <bool INPAINT, int TY, int K = PDB_K>
-PM_DEV void pd_block_tile(float4* __restrict__ uout, float4* __restrict__ pout, const float4* __restrict__ uin,
-                          const float4* __restrict__ pin, int pzero, const float4* __restrict__ f,
-                          const float* __restrict__ wgt, const float* __restrict__ mask, float lambda, int nsteps,
-                          int W, int H, int tbx, int tby) {
-    constexpr int PDB_RX = PDB_TX + 2 * K, PDB_RY = TY + 2 * K, PDB_N = PDB_RX * PDB_RY;
-    extern __shared__ __align__(16) float4 sm4[];
-    float4* su = sm4;
-    float4* slo = su + PDB_N;
-    float4* shi = slo + PDB_N;
-    float4* sf = shi + PDB_N;
-    float* sw = (float*)(sf + PDB_N);
-    float* sden = sw + PDB_N;
-    const int tid = threadIdx.y * PDB_TX + threadIdx.x, nt = PDB_TX * TY;
-    const int rx0 = tbx * PDB_TX - K, ry0 = tby * TY - K;
-    for (int i = tid; i < PDB_N; i += nt) {
-        const int gx = rx0 + i % PDB_RX, gy = ry0 + i / PDB_RX;
-        const bool in = gx >= 0 && gy >= 0 && gx < W && gy < H;
-        const size_t o = (size_t)clampi(gy, 0, H - 1) * W + clampi(gx, 0, W - 1);
-        su[i] = uin[o];
-        const float w = in ? wgt[o] : 0.0f;
-        sw[i] = w;
-        sden[i] = pd_den(w);
-        sf[i] = in ? f[o] : f4s(0.0f);
-        slo[i] = (in && !pzero) ? pin[o * 2] : f4s(0.0f);
-        shi[i] = (in && !pzero) ? pin[o * 2 + 1] : f4s(0.0f);
-    }
-    __syncthreads();
-    const float TAU = 1.0f / pm_sqrt(8.0f);
-    const float den_u = 1.0f + TAU * lambda;
-    /* region index of image position (gx, gy) clamped to the image, then to the region */
-    auto at = [&](int gx, int gy) {
-        const int lx = clampi(clampi(gx, 0, W - 1) - rx0, 0, PDB_RX - 1);
-        const int ly = clampi(clampi(gy, 0, H - 1) - ry0, 0, PDB_RY - 1);
-        return ly * PDB_RX + lx;
-    };
-    /* Step st updates the duals at ring distance >= st from the region edge and
-     * the primal at distance >= st+1: by induction u is exact at distance
-     * >= st+1 afterwards (its left/upper duals at distance >= st are exact), so
-     * after the last step the tile (distance K) is. */
-    for (int st = 0; st < nsteps; ++st) {
-        const int dw = PDB_RX - 2 * st, dh = PDB_RY - 2 * st;
-        const float inv_dw = 1.0f / (float)dw, inv_pw = 1.0f / (float)(dw - 2);
-        for (int k = tid; k < dw * dh; k += nt) {                     /* duals */
-            int lx, ly;
-            split_index(k, dw, inv_dw, lx, ly);
-            lx += st; ly += st;
-            const int i = ly * PDB_RX + lx;
-            const int gx = rx0 + lx, gy = ry0 + ly;
-            float4 lo, hi;
-            pd_dual<INPAINT>(sw[i], sden[i], su[at(gx, gy)], su[at(gx + 1, gy)], su[at(gx, gy + 1)], slo[i], shi[i], lo, hi);
-            slo[i] = lo;
-            shi[i] = hi;
-        }
-        __syncthreads();
-        const int pw = dw - 2, ph = dh - 2;
-        for (int k = tid; k < pw * ph; k += nt) {                     /* primal */
-            int lx, ly;
-            split_index(k, pw, inv_pw, lx, ly);
-            lx += st + 1; ly += st + 1;
-            const int gx = rx0 + lx, gy = ry0 + ly;
-            if (gx < 0 || gy < 0 || gx >= W || gy >= H) continue;
-            const int i = ly * PDB_RX + lx;
-            if (INPAINT) {
-                const float lam = lambda * __ldg(&mask[(size_t)gy * W + gx]);
-                su[i] = pd_primal(su[i], sf[i], sw[i], slo[i], slo[i - 1], shi[i], shi[i - PDB_RX], lam, 1.0f + TAU * lam);
-            } else {
-                su[i] = pd_primal(su[i], sf[i], sw[i], slo[i], slo[i - 1], shi[i], shi[i - PDB_RX], lambda, den_u);
+template <bool INPAINT, int NW, int R, int K>
+PM_DEV void pds_tile(float4* __restrict__ uout, float* __restrict__ pout, const float4* __restrict__ uin,
+                     const float* __restrict__ pin, int pzero, const float4* __restrict__ f,
+                     const float* __restrict__ wgt, const float* __restrict__ mask, float lambda, int nsteps, int W,
+                     int H, int tbx, int tby) {
+    constexpr int RY = NW * R, NC = INPAINT ? 8 : 6;
+    static_assert(K % 2 == 0 && RY > 2 * K, "the tile is made of whole column pairs");
+    extern __shared__ __align__(16) float pds_s[];
+    float2* const cells = reinterpret_cast<float2*>(pds_s);          /* [RY][NC][32] */
+    float2* const uex = cells + NC * RY * 32;                        /* [NW][3][32]: a warp's first row of u */
+    float2* const hex = uex + NW * 3 * 32;                           /* [NW][3][32]: a warp's last row of hi */
+    const int lane = threadIdx.x, w = threadIdx.y;
+    const float SIGMA = 1.0f / pm_sqrt(8.0f), TAU = 1.0f / pm_sqrt(8.0f), THETA = 0.5f;
+    const int gx = tbx * (PDS_RX - 2 * K) - K + 2 * lane, gy0 = tby * (RY - 2 * K) - K + w * R;
+    const int pp = pds_pitch(W);
+    const size_t np = (size_t)pp * H;
+    const bool inx0 = gx >= 0 && gx < W, inx1 = gx + 1 >= 0 && gx + 1 < W;
+    const int cx0 = clampi(gx, 0, W - 1), cx1 = clampi(gx + 1, 0, W - 1);
+    const float den_c = 1.0f + TAU * lambda, ny_c = -(1.0f / den_c);
+    float2 u[R][3], lo[R][3], hi[R][3];
+    bool tame = lambda >= 0.0f && den_c >= 1.0f && den_c <= 1048576.0f;
+    auto small = [](float v) { return fabsf(v) < 1.152921504606847e18f; };   /* 2^60; false for NaN */
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int gy = gy0 + r;
+        const bool iny = gy >= 0 && gy < H;
+        const size_t row = (size_t)clampi(gy, 0, H - 1) * W;
+        const float4 a = uin[row + cx0], b = uin[row + cx1];
+        u[r][0] = make_float2(a.x, b.x);
+        u[r][1] = make_float2(a.y, b.y);
+        u[r][2] = make_float2(a.z, b.z);
+        float2 d[6];
+#pragma unroll
+        for (int c = 0; c < 6; ++c) d[c] = make_float2(-0.0f, -0.0f);
+        if (!pzero && iny && inx0) {
+            const float* p = pin + (size_t)gy * pp + gx;
+#pragma unroll
+            for (int c = 0; c < 6; ++c) {
+                d[c] = *reinterpret_cast<const float2*>(p + c * np);
+                if (!inx1) d[c].y = -0.0f;
             }
         }
-        __syncthreads();
+        float2 fw[8];
+        const bool in0 = iny && inx0, in1 = iny && inx1;
+        const float4 f0 = f[row + cx0], f1 = f[row + cx1];
+        const float w0 = in0 ? wgt[row + cx0] : 0.0f, w1 = in1 ? wgt[row + cx1] : 0.0f;
+        float lam0 = lambda, lam1 = lambda;
+        if (INPAINT) {
+            lam0 = lambda * mask[row + cx0];
+            lam1 = lambda * mask[row + cx1];
+            const float b0 = 1.0f + TAU * lam0, b1 = 1.0f + TAU * lam1;
+            fw[6] = make_float2(b0, b1);
+            fw[7] = make_float2(-(1.0f / b0), -(1.0f / b1));
+            tame = tame && b0 >= 1.0f && b0 <= 1048576.0f && b1 >= 1.0f && b1 <= 1048576.0f;
+        }
+        fw[0] = make_float2(in0 ? lam0 * f0.x : 0.0f, in1 ? lam1 * f1.x : 0.0f);
+        fw[1] = make_float2(in0 ? lam0 * f0.y : 0.0f, in1 ? lam1 * f1.y : 0.0f);
+        fw[2] = make_float2(in0 ? lam0 * f0.z : 0.0f, in1 ? lam1 * f1.z : 0.0f);
+        fw[3] = make_float2(w0, w1);
+        /* outside the image the dual stays 0 whatever divides it */
+        const float d0 = in0 ? pd_den(w0) : 1.0f, d1 = in1 ? pd_den(w1) : 1.0f;
+        fw[4] = make_float2(d0, d1);
+        fw[5] = make_float2(-(1.0f / d0), -(1.0f / d1));
+        tame = tame && w0 >= 0.0f && w0 <= 1048576.0f && w1 >= 0.0f && w1 <= 1048576.0f && d0 >= 1.0f &&
+               d0 <= 1048576.0f && d1 >= 1.0f && d1 <= 1048576.0f;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            lo[r][c] = d[c];
+            hi[r][c] = d[3 + c];
+            tame = tame && small(u[r][c].x) && small(u[r][c].y) && small(fw[c].x) && small(fw[c].y);
+        }
+#pragma unroll
+        for (int c = 0; c < 6; ++c) tame = tame && small(d[c].x) && small(d[c].y);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) cells[((w * R + r) * NC + c) * 32 + lane] = fw[c];
     }
-    for (int i = tid; i < PDB_TX * TY; i += nt) {
-        const int lx = K + i % PDB_TX, ly = K + i / PDB_TX;
-        const int gx = rx0 + lx, gy = ry0 + ly;
-        if (gx >= W || gy >= H) continue;
-        const int r = ly * PDB_RX + lx;
-        const size_t o = (size_t)gy * W + gx;
-        uout[o] = su[r];
-        pout[o * 2] = slo[r];
-        pout[o * 2 + 1] = shi[r];
+    tame = __syncthreads_and(tame);                                  /* block-uniform */
+    /* block-uniform: some cell of the region is outside the image or on its last row or column */
+    const bool edge = tbx == 0 || tby == 0 || (tbx + 1) * (PDS_RX - 2 * K) + K >= W || (tby + 1) * (RY - 2 * K) + K >= H;
+    for (int st = 0; st < nsteps; ++st) {
+#pragma unroll
+        for (int c = 0; c < 3; ++c) uex[(w * 3 + c) * 32 + lane] = u[0][c];
+        __syncthreads();
+        /* duals (PDHuberWeighted.cl:49-68) */
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float2* cell = cells + (w * R + r) * NC * 32 + lane;
+            const float2 cw = cell[3 * 32], cd = cell[4 * 32], cn = cell[5 * 32];
+            float2 nl[3], nh[3];
+            unsigned m = 0xffffffffu;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float2 uq = u[r][c];
+                float2 ux = make_float2(uq.y, __shfl_down_sync(0xffffffffu, uq.x, 1));
+                float2 uy = r + 1 < R ? u[r + 1 < R ? r + 1 : r][c] : uex[(min(w + 1, NW - 1) * 3 + c) * 32 + lane];
+                if (edge) {                                          /* read clamped to the image */
+                    if (gx == W - 1) ux.x = uq.x;
+                    if (gx + 1 == W - 1) ux.y = uq.y;
+                    if (gy0 + r == H - 1) uy = uq;
+                }
+                const float2 dx = fmul2(f2s(SIGMA), fmul2(cw, fsub2(uq, ux)));
+                const float2 dy = fmul2(f2s(SIGMA), fmul2(cw, fsub2(uq, uy)));
+                nl[c] = make_float2(dx.x - lo[r][c].x, dx.y - lo[r][c].y);   /* plo + SIGMA dx, plo = -lo */
+                nh[c] = make_float2(dy.x - hi[r][c].x, dy.y - hi[r][c].y);
+                m = pds_mag2(pds_mag2(m, nl[c]), nh[c]);
+            }
+            if (tame && m >= PDS_TINY) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    nl[c] = neg_div2(nl[c], cd, cn);
+                    nh[c] = neg_div2(nh[c], cd, cn);
+                }
+            } else {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    nl[c] = make_float2(neg_div_ieee(nl[c].x, cd.x), neg_div_ieee(nl[c].y, cd.y));
+                    nh[c] = make_float2(neg_div_ieee(nh[c].x, cd.x), neg_div_ieee(nh[c].y, cd.y));
+                }
+            }
+            float2 pt[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float2 a = fmul2(nl[c], nl[c]), b = fmul2(nh[c], nh[c]);
+                pt[c] = make_float2(a.x + b.x, a.y + b.y);
+            }
+            /* the projection divides by max(1, sqrt(v)) = sqrt(max(v, 1)), v the
+             * squared norm (x and y jointly, z apart; INPAINT: each channel) */
+            float2 v[3];
+            if (INPAINT) {
+                v[0] = pt[0];
+                v[1] = pt[1];
+            } else {
+                v[0] = v[1] = make_float2(pt[0].x + pt[1].x, pt[0].y + pt[1].y);
+            }
+            v[2] = pt[2];
+            const float vmax = fmaxf(fmaxf(fmaxf(v[0].x, v[0].y), fmaxf(v[1].x, v[1].y)), fmaxf(v[2].x, v[2].y));
+            if (__any_sync(0xffffffffu, !(vmax <= 1.0f) || !tame)) {
+                float2 s[3], ny[3];
+                float e = 0.0f;
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    if (c == 1 && !INPAINT) { s[c] = s[0]; ny[c] = ny[0]; }
+                    else e = fmaxf(e, norm2(make_float2(fmaxf(v[c].x, 1.0f), fmaxf(v[c].y, 1.0f)), s[c], ny[c]));
+                }
+                if (tame && vmax <= PDS_VMAX && e < PDS_RESID) {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        nl[c] = div_norm2(nl[c], s[c], ny[c]);
+                        nh[c] = div_norm2(nh[c], s[c], ny[c]);
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        const float sx = fmaxf(1.0f, pm_sqrt(v[c].x)), sy = fmaxf(1.0f, pm_sqrt(v[c].y));
+                        nl[c] = make_float2(div_ge1(nl[c].x, sx), div_ge1(nl[c].y, sy));
+                        nh[c] = make_float2(div_ge1(nh[c].x, sx), div_ge1(nh[c].y, sy));
+                    }
+                }
+            }
+#pragma unroll
+            for (int c = 0; c < 3; ++c) { lo[r][c] = nl[c]; hi[r][c] = nh[c]; }
+        }
+#pragma unroll
+        for (int c = 0; c < 3; ++c) hex[(w * 3 + c) * 32 + lane] = hi[R - 1][c];
+        __syncthreads();
+        /* primal (:70-78) */
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const float2* cell = cells + (w * R + r) * NC * 32 + lane;
+            const float2 cw = cell[3 * 32];
+            const float2 bu = INPAINT ? cell[6 % NC * 32] : f2s(den_c), nu = INPAINT ? cell[7 % NC * 32] : f2s(ny_c);
+            float2 num[3];
+            unsigned m = 0xffffffffu;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float2 lc = lo[r][c];
+                const float2 ll = make_float2(__shfl_up_sync(0xffffffffu, lc.y, 1), lc.x);
+                const float2 hu = r > 0 ? hi[r > 0 ? r - 1 : 0][c] : hex[(max(w - 1, 0) * 3 + c) * 32 + lane];
+                const float2 div = fadd2(fsub2(fsub2(ll, lc), hi[r][c]), hu);    /* lo_c - lo_l + hi_c - hi_u */
+                const float2 wd = fmul2(cw, div), fl = cell[c * 32];
+                const float2 t = fmul2(f2s(TAU), make_float2(fl.x - wd.x, fl.y - wd.y));
+                num[c] = make_float2(u[r][c].x + t.x, u[r][c].y + t.y);
+                m = pds_mag2(m, num[c]);
+            }
+            if (tame && m >= PDS_TINY) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) num[c] = neg_div2(num[c], bu, nu);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                    num[c] = make_float2(-(num[c].x / bu.x), -(num[c].y / bu.y));
+            }
+            const bool iny = gy0 + r >= 0 && gy0 + r < H;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float ax = -num[c].x, ay = -num[c].y;
+                float2 v = make_float2(ax + THETA * (ax - u[r][c].x), ay + THETA * (ay - u[r][c].y));
+                if (edge) {                                          /* u is kept outside the image */
+                    if (!(iny && inx0)) v.x = u[r][c].x;
+                    if (!(iny && inx1)) v.y = u[r][c].y;
+                }
+                u[r][c] = v;
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int ry = w * R + r, gy = gy0 + r;
+        if (ry < K || ry >= RY - K || gy >= H || 2 * lane < K || 2 * lane >= PDS_RX - K || !inx0) continue;
+        float4* o = uout + (size_t)gy * W + gx;
+        o[0] = f4(u[r][0].x, u[r][1].x, u[r][2].x, 1.0f);
+        if (inx1) o[1] = f4(u[r][0].y, u[r][1].y, u[r][2].y, 1.0f);
+        float* p = pout + (size_t)gy * pp + gx;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            *reinterpret_cast<float2*>(p + c * np) = lo[r][c];
+            *reinterpret_cast<float2*>(p + (3 + c) * np) = hi[r][c];
+        }
     }
 }
 
+/* The plain path's region: 8 warps of 3 rows, 4 steps (a 56 x 16 tile), two
+ * blocks per SM (108 registers). */
+#define PDS_NW 8
+#define PDS_R 3
+#define PDS_K 4
+
 template <bool INPAINT>
-__global__ void __launch_bounds__(PDB_TX * PDB_TY)
-k_pd_block(float4* __restrict__ uout, float4* __restrict__ pout, const float4* __restrict__ uin,
-           const float4* __restrict__ pin, int pzero, const float4* __restrict__ f, const float* __restrict__ wgt,
+__global__ void __launch_bounds__(32 * PDS_NW, 2)
+k_pd_block(float4* __restrict__ uout, float* __restrict__ pout, const float4* __restrict__ uin,
+           const float* __restrict__ pin, int pzero, const float4* __restrict__ f, const float* __restrict__ wgt,
            const float* __restrict__ mask, float lambda, int nsteps, int W, int H) {
-    pd_block_tile<INPAINT, PDB_TY>(uout, pout, uin, pin, pzero, f, wgt, mask, lambda, nsteps, W, H, blockIdx.x,
-                                   blockIdx.y);
+    pds_tile<INPAINT, PDS_NW, PDS_R, PDS_K>(uout, pout, uin, pin, pzero, f, wgt, mask, lambda, nsteps, W, H, blockIdx.x,
+                                            blockIdx.y);
 }
 
 /* ------------------------------------------------------ batched phases -- */
@@ -1214,14 +1410,15 @@ __global__ void __launch_bounds__(32) kb_fill_output(const __grid_constant__ PmB
     }
 }
 
-template <int TY, int K>
-__global__ void __launch_bounds__(PDB_TX * TY) kb_pd_block(const __grid_constant__ PmBatch<PmPdArgs> b) {
+/* tiles of NW * R - 2K rows */
+template <int NW, int R, int K>
+__global__ void __launch_bounds__(32 * NW) kb_pd_block(const __grid_constant__ PmBatch<PmPdArgs> b) {
     for (int item = blockIdx.x; item < b.first[b.n]; item += gridDim.x) {
         const int p = batch_pair(b, item), t = item - b.first[p];
         const PmPdArgs& a = b.a[p];
         __syncthreads();                                 /* the region in shared memory is reused */
-        pd_block_tile<false, TY, K>(a.uout, a.pout, a.uin, a.pin, a.pzero, a.f, a.wgt, nullptr, a.lambda, a.nsteps, a.W,
-                                 a.H, t % b.tx[p], t / b.tx[p]);
+        pds_tile<false, NW, R, K>(a.uout, a.pout, a.uin, a.pin, a.pzero, a.f, a.wgt, nullptr, a.lambda, a.nsteps, a.W, a.H,
+                                  t % b.tx[p], t / b.tx[p]);
     }
 }
 
@@ -1329,23 +1526,26 @@ cudaError_t pm_launch_fill_output(const float4* in, int W, int H, float scale, f
     return cudaSuccess;
 }
 
-int pm_pd_block_steps() { return PDB_K; }
+int pm_pd_block_steps() { return PDS_K; }
 
-static const size_t kPdBlockSmem = pd_block_smem(PDB_TY);
+size_t pm_pd_dual_bytes(int W, int H) { return (size_t)pds_pitch(W) * H * 6 * sizeof(float); }
+
+static size_t pd_block_smem(bool inpaint) { return pds_smem(inpaint, PDS_NW, PDS_R); }
 
 cudaError_t pm_prepare_kernels() {
-    cudaError_t e = cudaFuncSetAttribute(k_pd_block<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPdBlockSmem);
+    cudaError_t e = cudaFuncSetAttribute(k_pd_block<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pd_block_smem(false));
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_pd_block<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPdBlockSmem);
+    e = cudaFuncSetAttribute(k_pd_block<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pd_block_smem(true));
     if (e != cudaSuccess) return e;
     return pm_batch_prepare_kernels();
 }
 
-cudaError_t pm_launch_pd_block(float4* uout, float4* pout, const float4* uin, const float4* pin, int pzero,
+cudaError_t pm_launch_pd_block(float4* uout, float* pout, const float4* uin, const float* pin, int pzero,
                                const float4* f, const float* wgt, const float* mask, float lambda, int nsteps, int W,
                                int H, cudaStream_t st) {
-    const size_t smem = kPdBlockSmem;
-    dim3 b(PDB_TX, PDB_TY), g((W + PDB_TX - 1) / PDB_TX, (H + PDB_TY - 1) / PDB_TY);
+    constexpr int TX = PDS_RX - 2 * PDS_K, TY = PDS_NW * PDS_R - 2 * PDS_K;
+    const size_t smem = pd_block_smem(mask != nullptr);
+    dim3 b(32, PDS_NW), g((W + TX - 1) / TX, (H + TY - 1) / TY);
     if (mask) k_pd_block<true><<<g, b, smem, st>>>(uout, pout, uin, pin, pzero, f, wgt, mask, lambda, nsteps, W, H);
     else k_pd_block<false><<<g, b, smem, st>>>(uout, pout, uin, pin, pzero, f, wgt, nullptr, lambda, nsteps, W, H);
     PM_LAUNCH_CHECK();
@@ -1406,7 +1606,8 @@ void pm_batch_tiles(PmBatchKernel k, int W, int H, const PmBatchKnobs& kn, int* 
     case PMB_ROW: x = 1; y = H; break;
     case PMB_PD: {
         const int rows = kn.pd_rows == 8 ? 8 : 16;
-        x = (W + PDB_TX - 1) / PDB_TX;
+        const int cols = PDS_RX - 2 * (kn.pd_halo == 2 ? 2 : 4);
+        x = (W + cols - 1) / cols;
         y = (H + rows - 1) / rows;
         break;
     }
@@ -1507,10 +1708,10 @@ cudaError_t pm_batch_fill_output(const PmBatch<PmOutArgs>& b, int maxW, const Pm
 }
 /* b.tx / b.first describe tiles of kn.pd_rows rows (pm_batch_tiles). */
 cudaError_t pm_batch_pd(const PmBatch<PmPdArgs>& b, const PmBatchKnobs& kn, cudaStream_t st) {
-    if (kn.pd_rows == 8 && kn.pd_halo == 2) PM_BATCH_LAUNCH((kb_pd_block<8, 2>), dim3(PDB_TX, 8), pd_block_smem(8, 2));
-    if (kn.pd_rows == 8) PM_BATCH_LAUNCH((kb_pd_block<8, 4>), dim3(PDB_TX, 8), pd_block_smem(8, 4));
-    if (kn.pd_halo == 2) PM_BATCH_LAUNCH((kb_pd_block<16, 2>), dim3(PDB_TX, 16), pd_block_smem(16, 2));
-    PM_BATCH_LAUNCH((kb_pd_block<16, 4>), dim3(PDB_TX, 16), pd_block_smem(16, 4));
+    if (kn.pd_rows == 8 && kn.pd_halo == 2) PM_BATCH_LAUNCH((kb_pd_block<6, 2, 2>), dim3(32, 6), pds_smem(false, 6, 2));
+    if (kn.pd_rows == 8) PM_BATCH_LAUNCH((kb_pd_block<8, 2, 4>), dim3(32, 8), pds_smem(false, 8, 2));
+    if (kn.pd_halo == 2) PM_BATCH_LAUNCH((kb_pd_block<10, 2, 2>), dim3(32, 10), pds_smem(false, 10, 2));
+    PM_BATCH_LAUNCH((kb_pd_block<8, 3, 4>), dim3(32, 8), pds_smem(false, 8, 3));
 }
 cudaError_t pm_batch_prepare_kernels() {
     cudaError_t e;
@@ -1519,11 +1720,11 @@ cudaError_t pm_batch_prepare_kernels() {
     if ((e = cudaFuncSetAttribute(k_nbcost<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, nbmax)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(kb_nbcost<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, nbmax)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(kb_nbcost<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, nbmax)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(kb_pd_block<16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)pd_block_smem(16, 4))) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(kb_pd_block<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)pd_block_smem(8, 4))) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(kb_pd_block<16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)pd_block_smem(16, 2))) != cudaSuccess) return e;
-    return cudaFuncSetAttribute(kb_pd_block<8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pd_block_smem(8, 2));
+    if ((e = cudaFuncSetAttribute(kb_pd_block<8, 3, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)pds_smem(false, 8, 3))) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(kb_pd_block<8, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)pds_smem(false, 8, 2))) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(kb_pd_block<10, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)pds_smem(false, 10, 2))) != cudaSuccess) return e;
+    return cudaFuncSetAttribute(kb_pd_block<6, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pds_smem(false, 6, 2));
 }

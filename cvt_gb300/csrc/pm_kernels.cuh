@@ -55,9 +55,10 @@ struct PmConsArgs { const float4 *L, *R; int W, H; float maxdisp, athr; int lr; 
 struct PmFillArgs { const float4* in; int W, H; float depthmax; int lr; float4* out; };
 struct PmOutArgs { const float4* in; int W, H; float scale; float* dmap; size_t dpitch; float4* nmap; size_t npitch; };
 struct PmPdArgs {
-    float4 *uout, *pout;
-    const float4 *uin, *pin, *f;
-    const float* wgt;
+    float4* uout;
+    float* pout;
+    const float4 *uin, *f;
+    const float *pin, *wgt;
     int pzero, nsteps, W, H;
     float lambda;
 };
@@ -117,7 +118,9 @@ cudaError_t pm_launch_normal_depth(const float4* in, int W, int H, float depthma
 cudaError_t pm_prepare_kernels();
 
 int pm_pd_block_steps();
-cudaError_t pm_launch_pd_block(float4* uout, float4* pout, const float4* uin, const float4* pin, int pzero,
+/* Bytes of a dual buffer of pm_launch_pd_block: six planes of floats. */
+size_t pm_pd_dual_bytes(int W, int H);
+cudaError_t pm_launch_pd_block(float4* uout, float* pout, const float4* uin, const float* pin, int pzero,
                                const float4* f, const float* wgt, const float* mask, float lambda, int nsteps, int W,
                                int H, cudaStream_t st);
 cudaError_t pm_launch_ffma_peak(float* out, int blocks, int iters, cudaStream_t st);
