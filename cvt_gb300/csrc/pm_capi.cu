@@ -62,6 +62,9 @@ struct cvtpm_ctx {
     float* nbcost = nullptr;
     size_t nb_bytes = 0;
     size_t nb_budget = SIZE_MAX;
+    /* tap-parallel passes of small images: the candidates' states and costs */
+    float4* cand = nullptr;
+    size_t cand_bytes = 0;
     bool nb_on = false;
     /* set while a launch sequence is being captured into a graph: scratch
      * must already be sized, nothing may be allocated */
@@ -350,6 +353,31 @@ cvtpm_status ensure_nbcost(cvtpm_ctx* ctx, int W, int H) {
     return CVTPM_OK;
 }
 
+/* The candidate buffer of the tap-parallel passes (320 bytes per pixel of a
+ * small image), under the same budget; without it the passes take the other
+ * path (same results). */
+cvtpm_status ensure_cand(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H, float4** cand) {
+    *cand = nullptr;
+    if (p.schedule != CVTPM_SCHEDULE_JACOBI || !pm_tap_parallel(base_args(ctx, p, W, H, 0).k)) return CVTPM_OK;
+    const size_t need = pm_tap_parallel_bytes(W, H);
+    if (need > ctx->nb_budget) return CVTPM_OK;
+    if (ctx->cand_bytes < need) {
+        if (ctx->no_alloc) return CVTPM_OK;
+        if (ctx->cand) { CK(cudaFree(ctx->cand), "free candidates"); ctx->cand = nullptr; ctx->cand_bytes = 0; }
+        size_t fr = 0, tot = 0;
+        CK(cudaMemGetInfo(&fr, &tot), "memory info");
+        if ((double)need > 0.6 * (double)fr) return CVTPM_OK;
+        if (cudaMalloc(&ctx->cand, need) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->cand = nullptr;
+            return CVTPM_OK;
+        }
+        ctx->cand_bytes = need;
+    }
+    *cand = ctx->cand;
+    return CVTPM_OK;
+}
+
 cvtpm_status prep_views(cvtpm_ctx* ctx, const cvtpm_params& p, const float* img0, const float* img1, int W, int H,
                         size_t pitch, cudaStream_t st, bool records = false) {
     const float* im[2] = {img0, img1};
@@ -460,8 +488,12 @@ cvtpm_status run_depthmap(cvtpm_ctx* ctx, const cvtpm_params& p, float* dmap, si
     const float dscale = p.dscale <= 0.0f ? 1.0f / dmax : p.dscale;
     const int N = p.iterations;
     PmPassArgs aL = base_args(ctx, p, W, H, 0), aR = base_args(ctx, p, W, H, 1);
-    if ((s = ensure_nbcost(ctx, W, H)) != CVTPM_OK) return s;
-    if (ctx->nb_on) aL.nbcost = aR.nbcost = ctx->nbcost;
+    if ((s = ensure_cand(ctx, p, W, H, &aL.cand)) != CVTPM_OK) return s;
+    aR.cand = aL.cand;
+    if (!aL.cand) {
+        if ((s = ensure_nbcost(ctx, W, H)) != CVTPM_OK) return s;
+        if (ctx->nb_on) aL.nbcost = aR.nbcost = ctx->nbcost;
+    }
     if (!ctx->dcount) {
         if (ctx->no_alloc) return fail(ctx, CVTPM_ERR_ALLOC, "counters not allocated before capture");
         CK(cudaMalloc(&ctx->dcount, 2 * sizeof(unsigned long long)), "counters");
@@ -597,8 +629,12 @@ cvtpm_status run_depthmap_inpaint(cvtpm_ctx* ctx, const cvtpm_params& p, float* 
     const float dmax = p.depthmax;
     const int N = p.iterations;
     PmPassArgs aL = base_args(ctx, p, W, H, 0), aR = base_args(ctx, p, W, H, 1);
-    if ((s = ensure_nbcost(ctx, W, H)) != CVTPM_OK) return s;
-    if (ctx->nb_on) aL.nbcost = aR.nbcost = ctx->nbcost;
+    if ((s = ensure_cand(ctx, p, W, H, &aL.cand)) != CVTPM_OK) return s;
+    aR.cand = aL.cand;
+    if (!aL.cand) {
+        if ((s = ensure_nbcost(ctx, W, H)) != CVTPM_OK) return s;
+        if (ctx->nb_on) aL.nbcost = aR.nbcost = ctx->nbcost;
+    }
     if (!ctx->dcount) {
         if (ctx->no_alloc) return fail(ctx, CVTPM_ERR_ALLOC, "counters not allocated before capture");
         CK(cudaMalloc(&ctx->dcount, 2 * sizeof(unsigned long long)), "counters");
@@ -772,6 +808,7 @@ cvtpm_status cvtpm_destroy(cvtpm_ctx* ctx) {
     if (ctx->bjoin) cudaEventDestroy(ctx->bjoin);
     if (ctx->stage) cudaFree(ctx->stage);
     if (ctx->nbcost) cudaFree(ctx->nbcost);
+    if (ctx->cand) cudaFree(ctx->cand);
     if (ctx->istage) cudaFree(ctx->istage);
     if (ctx->dcount) cudaFree(ctx->dcount);
     for (auto& pr : ctx->ev_prop) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
@@ -955,6 +992,12 @@ cvtpm_status cvtpm_set_memory_budget(cvtpm_ctx* ctx, size_t bytes) {
         ctx->nbcost = nullptr;
         ctx->nb_bytes = 0;
     }
+    if (ctx->cand && ctx->cand_bytes > bytes) {
+        CK(cudaSetDevice(ctx->device), "cudaSetDevice");
+        CK(cudaFree(ctx->cand), "free candidates");
+        ctx->cand = nullptr;
+        ctx->cand_bytes = 0;
+    }
     return CVTPM_OK;
 }
 
@@ -1132,7 +1175,9 @@ cvtpm_status capture_batch(cvtpm_ctx* ctx, const cvtpm_pair* pairs, int npairs, 
         c->timing = false;
         for (int i : plan[j]) {
             if ((s = ensure_buffers(c, pairs[i].width, pairs[i].height)) != CVTPM_OK) return fail(ctx, s, c->err);
-            if ((s = ensure_nbcost(c, pairs[i].width, pairs[i].height)) != CVTPM_OK) return fail(ctx, s, c->err);
+            float4* cand = nullptr;
+            if ((s = ensure_cand(c, p, pairs[i].width, pairs[i].height, &cand)) != CVTPM_OK) return fail(ctx, s, c->err);
+            if (!cand && (s = ensure_nbcost(c, pairs[i].width, pairs[i].height)) != CVTPM_OK) return fail(ctx, s, c->err);
         }
     }
     if (k > 0 && (s = ensure_tables(ctx->lanes[0].c, p, ctx->bstream)) != CVTPM_OK) return fail(ctx, s, ctx->lanes[0].c->err);
@@ -1623,16 +1668,18 @@ cvtpm_status tune_mode(PhaseState& full, float ms[2]) {
     PhaseState S = full;
     long long px = 0;
     int maxW = 1, maxH = 1;
+    cvtpm_ctx* ctx = S.ctx;
+    cvtpm_ctx* lane = ctx->lanes[0].c;
+    cvtpm_status s = cvtpm_set_memory_budget(lane, ctx->nb_budget);
     S.n = 0;
     while (S.n < full.n && (S.n == 0 || px < 4000000)) {
+        float4* cand = nullptr;
+        if (s == CVTPM_OK) s = ensure_cand(lane, S.p, full.pairs[S.n].width, full.pairs[S.n].height, &cand);
         px += (long long)full.pairs[S.n].width * full.pairs[S.n].height;
         maxW = std::max(maxW, full.pairs[S.n].width);
         maxH = std::max(maxH, full.pairs[S.n].height);
         ++S.n;
     }
-    cvtpm_ctx* ctx = S.ctx;
-    cvtpm_ctx* lane = ctx->lanes[0].c;
-    cvtpm_status s = cvtpm_set_memory_budget(lane, ctx->nb_budget);
     if (s == CVTPM_OK) s = ensure_buffers(lane, maxW, maxH);
     if (s == CVTPM_OK) s = ensure_nbcost(lane, maxW, maxH);
     if (s != CVTPM_OK) return fail(ctx, s, lane->err);

@@ -6,6 +6,7 @@
  *  k_records            (fast arithmetic only) value/forward-difference records of a view
  *  k_init<EXACT>        pmhstereo_init (:230-248)
  *  k_propagate<EXACT>   pmhstereo_propagate_view (:286-404) without the scatter
+ *  k_taps_*<EXACT>      init and propagate for small images, the taps of a window in parallel
  *  k_nbcost<EXACT>      its candidates 1-8 (:330-342), plane by plane over shared windows
  *  k_view_list          the scatter of :391-400, made deterministic (smallest source x first)
  *  k_consistency        pmhstereo_consistency (:428-464)
@@ -17,6 +18,7 @@
 #define PM_KERNELS_TU 1
 #include "pm_kernels.cuh"
 
+#include <cmath>
 #include <type_traits>
 
 /* Blocks of 256 threads per SM the FAST propagation and the neighbour
@@ -698,6 +700,378 @@ PM_DEV void nbcost_tile(const PmPassArgs& a, int tbx, int tby) {
 template <bool EXACT>
 __global__ void __launch_bounds__(32 * NB_WARPS, PM_NB_MINB) k_nbcost(PmPassArgs a) {
     nbcost_tile<EXACT>(a, blockIdx.x, blockIdx.y);
+}
+
+/* ------------------------------------------------- tap-parallel passes -- */
+/* The propagation of images too small to fill the GPU with one thread per
+ * pixel.  There every launch of the kernels above lasts as long as one
+ * thread's chain of (2P+1)^2 taps, a few hundred cycles each, for up to 16
+ * candidates: 2.0 ms for stage 1 of a 64x48 pass that is 0.1 ms of issue
+ * slots.  Here a block takes 32 pixels of a row and its warps share their
+ * window: producer warp w forms the weights and the matching terms of the taps
+ * w, w + TP_NP, ... (raster order) for all of the block's candidates and
+ * writes them to shared memory; a consumer warp per candidate folds a chunk of
+ * taps into its sums in raster order while the producers form the next chunk.
+ * So every candidate keeps its order of additions, and its cost the bits of
+ * eval_costs, while the taps of a window are formed TP_NP at a time.  All
+ * candidates that need no other's outcome (1-20) run in one launch, in groups
+ * of 8 that share weights and image-1 reads; the refinements, which need the
+ * best of them, follow in a second launch, one candidate at a time.
+ *
+ * An invalid tap (outside either image) is stored with a NaN in place of its
+ * first term; no valid term is a NaN as long as neither truncation is
+ * (pm_launch_propagate takes the other path then). */
+#define TP_NP 8                                      /* producer warps */
+
+template <bool EXACT> struct TpTerm { typedef float2 type; };
+template <> struct TpTerm<true> { typedef float type; };
+
+/* A candidate's position data per lane: FAST the Q31.32 plane, EXACT the coefficients. */
+template <bool EXACT> struct TpPlane { long long S0, S1, XA; };
+template <> struct TpPlane<true> { float sx, sy, sz; };
+
+template <bool EXACT, int K, int CH>
+struct TpShared {
+    typename TpTerm<EXACT>::type term[2][CH][K][32];
+    float w[2][CH][32];
+    TpPlane<EXACT> plane[K][32];
+    unsigned live;                                   /* candidates with a finite, active plane in some lane */
+};
+
+/* Puts a warp's candidate c into shared memory; every lane calls it. */
+template <bool EXACT, int K, int CH>
+PM_DEV void tp_put_plane(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, int c, float4 s, bool act) {
+    const bool live = act && finite3(s);
+    TpPlane<EXACT> p;
+    if constexpr (EXACT) {
+        p.sx = live ? s.x : 0.0f;
+        p.sy = live ? s.y : 0.0f;
+        p.sz = live ? s.z : -1.0e30f;                /* never inside [0, W) */
+    } else {
+        pm_fix_plane(live, s.x, s.y, s.z, k.W / 2, k.H / 2, &p.S0, &p.S1, &p.XA);
+    }
+    S.plane[c][threadIdx.x] = p;
+    const bool any = __any_sync(0xffffffffu, live);
+    if (threadIdx.x == 0 && any) atomicOr(&S.live, 1u << c);
+}
+
+/* The costs of the planes in S.plane at pixels (x0 + lane, y).  Warps
+ * 0..TP_NP-1 produce, warp CW + c returns candidate c's cost (1e5 for a plane
+ * that is not live); the other warps return garbage.  CH taps per chunk, CH a
+ * multiple of 2 * TP_NP.  All threads call it; it begins and ends with a block
+ * barrier. */
+template <bool EXACT, int K, int CH, int CW>
+PM_DEV float tp_costs(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, const PmView& v1, const PmView& v2, int x0, int y,
+                      bool live_lane) {
+    typedef typename TpTerm<EXACT>::type Term;
+    constexpr int SLOTS = CH / TP_NP;
+    static_assert(SLOTS * TP_NP == CH && SLOTS % 2 == 0, "whole pairs of taps per producer");
+    const int lane = threadIdx.x, w = threadIdx.y, W = k.W, H = k.H, P = k.P;
+    const int x = min(x0 + lane, W - 1);             /* lanes past the row repeat its last pixel */
+    __syncthreads();                                 /* the planes are in place */
+    const unsigned live = S.live;
+    if (!live) return 1e5f;                          /* block-uniform: no plane to evaluate */
+    const int qy0 = max(y - P, 0), ny = min(y + P, H - 1) - qy0 + 1;
+    /* block-uniform columns: every offset that is inside the image for some lane */
+    const int dlo = max(-P, -(x0 + 31)), nx = min(P, W - 1 - x0) - dlo + 1;
+    const int T = nx * ny, nchunk = (T + CH - 1) / CH;
+    const bool producer = w < TP_NP, consumer = w >= CW && w < CW + K;
+    /* producer state: its next tap (row, col) and the candidates' positions there */
+    int col = w, row = 0;
+    long long X[K], SN[K], SW[K];
+    float4 vc = f4s(0.0f);
+    if (producer) {
+        vc = __ldg(&v1.col[(size_t)y * W + x]);
+        while (col >= nx) { col -= nx; ++row; }
+        if constexpr (!EXACT) {
+#pragma unroll
+            for (int c = 0; c < K; ++c) {
+                const TpPlane<EXACT> p = S.plane[c][lane];
+                X[c] = p.XA + (long long)(qy0 + row - H / 2) * p.S1 + (long long)(x + dlo + col - W / 2) * p.S0;
+                SN[c] = (long long)TP_NP * p.S0;     /* to the producer's next tap */
+                SW[c] = p.S1 - (long long)nx * p.S0; /* on each row end it passes */
+            }
+        }
+    }
+    auto produce = [&](int i) {
+        const int buf = i & 1;
+#pragma unroll 1
+        for (int s = 0; s < SLOTS; s += 2) {
+            float4 a1[2], g1[2];
+            int qx[2], qy[2];
+            float prof[2], wt[2];
+            bool in[2];
+            long long Xt[2][K];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                qy[h] = qy0 + min(row, ny - 1);      /* a tap past the last is formed and not read */
+                const int dx = dlo + col, qxr = x + dx;
+                in[h] = qxr >= 0 && qxr < W;
+                qx[h] = clampi(qxr, 0, W - 1);
+                const size_t o = (size_t)qy[h] * W + qx[h];
+                a1[h] = __ldg(&v1.col[o]);
+                g1[h] = __ldg(&v1.grad[o]);
+                prof[h] = c_prof[(qy[h] - y + PM_PMAX) * PM_PROF_N + PM_PMAX + dx];
+                if constexpr (!EXACT) {
+#pragma unroll
+                    for (int c = 0; c < K; ++c) { Xt[h][c] = X[c]; X[c] += SN[c]; }
+                }
+                col += TP_NP;
+                while (col >= nx) {
+                    col -= nx;
+                    ++row;
+                    if constexpr (!EXACT) {
+#pragma unroll
+                        for (int c = 0; c < K; ++c) X[c] += SW[c];
+                    }
+                }
+            }
+            tap_weight2(vc, a1[0], a1[1], prof[0], prof[1], wt[0], wt[1]);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int j = (s + h) * TP_NP + w;
+                S.w[buf][j][lane] = wt[h];
+                const PmRecRow rrow = rec_row(v2, k.rp, qy[h]);
+#pragma unroll
+                for (int c = 0; c < K; ++c) {
+                    if (K > 1 && !((live >> c) & 1u)) continue;
+                    if constexpr (EXACT) {
+                        const TpPlane<EXACT> p = S.plane[c][lane];
+                        float cc, gc;
+                        const bool ok = nb_tap_terms<true>(k, v2, qx[h], qy[h], rrow, p.sx, p.sy, p.sz, 0, a1[h], g1[h], cc, gc);
+                        S.term[buf][j][c][lane] = ok && in[h] ? cc : __int_as_float(0x7fc00000);
+                    } else {
+                        /* the sample column clamped to the row: the load needs no branch */
+                        const int xi = (int)(Xt[h][c] >> 32);
+                        float2 t;
+                        fast_tap_terms(k, rrow, clampi(xi, 0, W - 1), pm_fix_frac(Xt[h][c]), a1[h], g1[h], t.x, t.y);
+                        if (!in[h] || (unsigned)xi >= (unsigned)W) t.x = __int_as_float(0x7fc00000);
+                        S.term[buf][j][c][lane] = t;
+                    }
+                }
+            }
+        }
+    };
+    float r1 = 0.0f, r2 = 0.0f, ws = 0.0f;
+    auto consume = [&](int i) {
+        const int buf = i & 1, n = min(CH, T - i * CH), c = w - CW;
+        auto one = [&](int j) {
+            const Term t = S.term[buf][j][c][lane];
+            const float wt = S.w[buf][j][lane];
+            if constexpr (EXACT) {
+                if (t == t) nb_accumulate<true>(wt, t, 0.0f, r1, r2, ws);
+            } else {
+                if (t.x == t.x) nb_accumulate<false>(wt, t.x, t.y, r1, r2, ws);
+            }
+        };
+        int j = 0;
+        for (; j + 8 <= n; j += 8) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) one(j + u);
+        }
+        for (; j < n; ++j) one(j);
+    };
+    const bool mine = consumer && ((live >> (w - CW)) & 1u);
+    if (producer) produce(0);
+    __syncthreads();
+    for (int i = 0; i < nchunk; ++i) {
+        if (producer && i + 1 < nchunk) produce(i + 1);
+        if (mine) consume(i);
+        __syncthreads();
+    }
+    return nb_final<EXACT>(k, live_lane, r1, r2, ws);
+}
+
+/* The squared distance of a state to the smoothed field (pmhstereo.cl:266-283,
+ * one side of smooth_distance). */
+PM_DEV float state_distance(float4 s, float4 smooth, float cx, float cy, float depthmax, int lr) {
+    const float4 diag = f4(1.0f, 1.0f, 0.0f, 1.0f / (depthmax * depthmax));
+    const float4 d = to_ref_normal_depth(s, cx, cy, lr) - smooth;
+    return dot4(d, diag * d);
+}
+/* The acceptance rule of a propagation pass, from costs and distances formed
+ * beforehand: a state that is not finite makes both distances 0. */
+struct TpBest { float cost, dist; bool fin; };
+PM_DEV bool tp_accepts(const TpBest& cand, const TpBest& self, float theta) {
+    const bool fin = cand.fin && self.fin;
+    return cand.cost + theta * (fin ? cand.dist : 0.0f) <= self.cost + theta * (fin ? self.dist : 0.0f);
+}
+
+/* The smoothed plane's normal and depth at a pixel (:320-323) */
+PM_DEV float4 smooth_at(const PmPassArgs& a, size_t o) {
+    const float4 sm = a.smooth[o];
+    const float nf = fmaxf(pm_sqrt(sm.x * sm.x + sm.y * sm.y) + 0.001f, 1.0f);
+    const float smx = sm.x / nf, smy = sm.y / nf;
+    return f4(smx, smy, pm_sqrt(1.0f - smx * smx - smy * smy), sm.z * a.depthmax);
+}
+
+#define TP_K 8
+#define TP_CH 16       /* taps per chunk of the candidate kernel */
+#define TP_CH1 64      /* taps per chunk of the one-candidate kernels */
+
+/* Candidates 1-8 (blockIdx.z 0), 9-16 (1) and 17-20 (2) of 32 pixels: their
+ * states with their costs go to a.cand[candidate - 1]. */
+template <bool EXACT>
+__global__ void __launch_bounds__(32 * TP_NP, 2) k_taps_candidates(PmPassArgs a) {
+    extern __shared__ __align__(16) unsigned char tp_smem[];
+    TpShared<EXACT, TP_K, TP_CH>& S = *reinterpret_cast<TpShared<EXACT, TP_K, TP_CH>*>(tp_smem);
+    const int W = a.k.W, H = a.k.H, x0 = blockIdx.x * 32, y = blockIdx.y, z = blockIdx.z;
+    const int c = threadIdx.y, x = min(x0 + (int)threadIdx.x, W - 1);
+    const size_t n = (size_t)W * H, o = (size_t)y * W + x;
+    const float cx = (float)x, cy = (float)y;
+    if (c == 0 && threadIdx.x == 0) S.live = 0;
+    __syncthreads();
+    float4 s = f4s(0.0f);
+    bool act = true;
+    if (z == 0) {                                    /* :330-342 */
+        const int nn = c < 4 ? c : c + 1;
+        s = a.old[(size_t)clampi(y + nn / 3 - 1, 0, H - 1) * W + clampi(x + nn % 3 - 1, 0, W - 1)];
+    } else if (z == 1) {
+        if (c == 0) {                                /* :345-352 */
+            const float4 sm = smooth_at(a, o);
+            const float4 sc = f4(1.0f - (-sm.x / sm.z), 0.0f - (-sm.y / sm.z),
+                                 0.0f - ((sm.x * cx + sm.y * cy) / sm.z + sm.w), 0.0f - 0.0f);
+            s = a.lr ? sc : viewprop(sc);
+        } else {
+            PmRng rng;
+            seed_rng(rng, a, x, y, false);
+#pragma unroll 1
+            for (int i = 0; i < 2 * (c - 1); ++i) (void)rng_float(rng);
+            if (c < 7) {                             /* :355-361 */
+                const int ox = (int)(rng_float(rng) * 7.0f + 0.5f);
+                const int oy = (int)(rng_float(rng) * 7.0f + 0.5f);
+                s = a.old[(size_t)clampi(y + oy, 0, H - 1) * W + clampi(x + ox, 0, W - 1)];
+            } else {
+                s = state_init(rng, cx, cy, a.lr, 2.0f, a.depthmax);   /* :364-368 */
+            }
+        }
+    } else {                                         /* :372-379 */
+        const short4 l = a.viewin[o];
+        const short e = c == 0 ? l.x : c == 1 ? l.y : c == 2 ? l.z : l.w;
+        act = c < 4 && e >= 0 && x0 + (int)threadIdx.x < W;
+        if (act) s = viewprop(a.viewsrc[(size_t)y * W + e]);
+    }
+    tp_put_plane(S, a.k, c, s, act);
+    s.w = tp_costs<EXACT, TP_K, TP_CH, 0>(S, a.k, a.v1, a.v2, x0, y, act && finite3(s));
+    if (act && x0 + (int)threadIdx.x < W) a.cand[(size_t)(z * 8 + c) * n + o] = s;
+}
+
+/* One candidate per evaluation: warps 0..TP_NP-1 produce, warp TP_NP owns the
+ * pixels.  MODE 0: the random initial planes (pmhstereo_init).  MODE 1: the
+ * best of a.old and the candidates in a.cand, then the two refinements.
+ * MODE 2: the refinements of the best so far in a.out. */
+template <bool EXACT, int MODE>
+__global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_refine(PmPassArgs a) {
+    extern __shared__ __align__(16) unsigned char tp_smem[];
+    typedef TpShared<EXACT, 1, TP_CH1> Sh;
+    Sh& S = *reinterpret_cast<Sh*>(tp_smem);
+    TpBest (*const best)[32] = reinterpret_cast<TpBest (*)[32]>(tp_smem + sizeof(Sh));   /* [20][32] */
+    const int W = a.k.W, H = a.k.H, x0 = blockIdx.x * 32, y = blockIdx.y;
+    const int lane = threadIdx.x, w = threadIdx.y, x = min(x0 + lane, W - 1);
+    const bool inside = x0 + lane < W, owner = w == TP_NP;
+    const size_t n = (size_t)W * H, o = (size_t)y * W + x;
+    const float cx = (float)x, cy = (float)y, dmax = a.depthmax, theta = a.theta;
+    PmRng rng;
+    if (owner) {
+        seed_rng(rng, a, x, y, MODE == 0);
+        if (lane == 0) S.live = 0;
+    }
+    if constexpr (MODE == 0) {
+        float4 s = f4s(0.0f);
+        __syncwarp();
+        if (owner) {
+            s = state_init(rng, cx, cy, a.lr, 1.0f, dmax);
+            tp_put_plane(S, a.k, 0, s, true);
+        }
+        const float cost = tp_costs<EXACT, 1, TP_CH1, TP_NP>(S, a.k, a.v1, a.v2, x0, y, finite3(s));
+        if (owner && inside) { s.w = cost; a.out[o] = s; }
+        return;
+    }
+    const float4 smooth = smooth_at(a, o);
+    int nview = 0;
+    if (MODE == 1) {
+        if (a.viewin) {
+            const short4 l = a.viewin[o];
+            nview = l.x < 0 ? 0 : l.y < 0 ? 1 : l.z < 0 ? 2 : l.w < 0 ? 3 : 4;
+        }
+        if (!owner) {                                /* the candidates' distances, spread over the producers */
+            for (int i = w; i < 16 + nview; i += TP_NP) {
+                const float4 s = a.cand[(size_t)i * n + o];
+                best[i][lane] = {s.w, state_distance(s, smooth, cx, cy, dmax, a.lr), finite3(s)};
+            }
+        }
+        __syncthreads();
+    }
+    float4 self = f4s(0.0f);
+    TpBest eself = {0.0f, 0.0f, false};
+    int win = MODE == 1 ? 0 : -1;
+    if (owner) {
+        self = MODE == 1 ? a.old[o] : a.out[o];
+        eself = {self.w, state_distance(self, smooth, cx, cy, dmax, a.lr), finite3(self)};
+        if (MODE == 1) {
+            int pick = -1;
+            for (int i = 0; i < 16 + nview; ++i) {
+                const TpBest e = best[i][lane];
+                if (tp_accepts(e, eself, theta)) { eself = e; pick = i; }
+            }
+            if (pick >= 0) { self = a.cand[(size_t)pick * n + o]; win = pick + 1; }
+        }
+#pragma unroll 1
+        for (int i = 0; i < 15; ++i) (void)rng_float(rng);   /* the draws of candidates 10-16 */
+    }
+    /* 21-22: random refinements of the current best (:383-389) */
+    float4 last = f4s(0.0f);
+    bool rejected = false;
+#pragma unroll 1
+    for (int i = 0; i < 2; ++i) {
+        float4 s = f4s(0.0f);
+        bool act = false;
+        if (owner) {
+            s = state_refine(rng, self, cx, cy, dmax, a.lr);
+            /* the right view's refinement (:114-115) does not depend on its
+             * draws: after a rejection the second is the rejected one again */
+            act = !(rejected && s.x == last.x && s.y == last.y && s.z == last.z);
+            if (lane == 0) S.live = 0;
+            tp_put_plane(S, a.k, 0, s, act);
+        }
+        if (__syncthreads_or(act)) {                 /* block-uniform */
+            const float cost = tp_costs<EXACT, 1, TP_CH1, TP_NP>(S, a.k, a.v1, a.v2, x0, y, finite3(s));
+            if (owner && act) {
+                s.w = cost;
+                const TpBest e = {cost, state_distance(s, smooth, cx, cy, dmax, a.lr), finite3(s)};
+                rejected = !tp_accepts(e, eself, theta);
+                last = s;
+                if (!rejected) { self = s; eself = e; win = 21 + i; }
+            }
+        }
+    }
+    if (owner && inside) {
+        a.out[o] = self;
+        if (a.winners && win >= 0) a.winners[o] = (uint8_t)win;
+    }
+    if (MODE == 1 && owner && a.counters) {
+        /* evaluations = 18 + view candidates; taps = in-image window taps */
+        unsigned long long ev = 0, taps = 0;
+        if (inside) {
+            const int P = a.k.P;
+            ev = 18ull + (unsigned long long)nview;
+            taps = ev * (unsigned long long)((min(x + P, W - 1) - max(x - P, 0) + 1) * (min(y + P, H - 1) - max(y - P, 0) + 1));
+        }
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            ev += __shfl_down_sync(0xffffffffu, ev, off);
+            taps += __shfl_down_sync(0xffffffffu, taps, off);
+        }
+        if (lane == 0) {
+            atomicAdd(&a.counters[0], ev);
+            atomicAdd(&a.counters[1], taps);
+        }
+    }
+}
+
+template <bool EXACT> constexpr size_t tp_cand_smem() { return sizeof(TpShared<EXACT, TP_K, TP_CH>); }
+template <bool EXACT, int MODE> constexpr size_t tp_refine_smem() {
+    return sizeof(TpShared<EXACT, 1, TP_CH1>) + (MODE == 1 ? sizeof(TpBest) * 20 * 32 : 0);
 }
 
 /* -------------------------------------------------------- view lists -- */
@@ -1452,7 +1826,15 @@ cudaError_t pm_launch_records(const float4* col, const float4* grad, int W, int 
 
 static inline dim3 pix_grid(int W, int H) { return dim3((W + 31) / 32, (H + 7) / 8); }
 
+static inline dim3 tap_grid(const PmPassArgs& a, int z = 1) { return dim3((a.k.W + 31) / 32, a.k.H, z); }
+
 cudaError_t pm_launch_init(const PmPassArgs& a, bool exact, cudaStream_t st) {
+    if (a.cand) {
+        if (exact) k_taps_refine<true, 0><<<tap_grid(a), dim3(32, TP_NP + 1), tp_refine_smem<true, 0>(), st>>>(a);
+        else k_taps_refine<false, 0><<<tap_grid(a), dim3(32, TP_NP + 1), tp_refine_smem<false, 0>(), st>>>(a);
+        PM_LAUNCH_CHECK();
+        return cudaSuccess;
+    }
     if (exact) k_init<true><<<pix_grid(a.k.W, a.k.H), dim3(32, 8), 0, st>>>(a);
     else k_init<false><<<pix_grid(a.k.W, a.k.H), dim3(32, 8), 0, st>>>(a);
     PM_LAUNCH_CHECK();
@@ -1469,7 +1851,17 @@ cudaError_t pm_launch_cost_field(const PmPassArgs& a, bool exact, const float4* 
 cudaError_t pm_launch_propagate(const PmPassArgs& a, bool exact, cudaStream_t st) {
     const dim3 grid = a.color < 0 ? pix_grid(a.k.W, a.k.H) : pix_grid((a.k.W + 1) / 2, a.k.H);
     PmPassArgs b = a;
-    if (b.color >= 0) b.nbcost = nullptr;   /* red/black: neighbours per pixel */
+    if (b.color >= 0) b.nbcost = nullptr, b.cand = nullptr;   /* red/black: neighbours per pixel */
+    if (b.cand) {
+        const dim3 g = tap_grid(b, b.viewin ? 3 : 2);
+        if (exact) k_taps_candidates<true><<<g, dim3(32, TP_NP), tp_cand_smem<true>(), st>>>(b);
+        else k_taps_candidates<false><<<g, dim3(32, TP_NP), tp_cand_smem<false>(), st>>>(b);
+        PM_LAUNCH_CHECK();
+        if (exact) k_taps_refine<true, 1><<<tap_grid(b), dim3(32, TP_NP + 1), tp_refine_smem<true, 1>(), st>>>(b);
+        else k_taps_refine<false, 1><<<tap_grid(b), dim3(32, TP_NP + 1), tp_refine_smem<false, 1>(), st>>>(b);
+        PM_LAUNCH_CHECK();
+        return cudaSuccess;
+    }
     const dim3 nbgrid((a.k.W + NB_COLS - 1) / NB_COLS, (a.k.H + NB_ROWS - 1) / NB_ROWS);
     if (b.nbcost) {
         const size_t smem = nb_block_smem(a.k.P);
@@ -1537,8 +1929,33 @@ cudaError_t pm_prepare_kernels() {
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(k_pd_block<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pd_block_smem(true));
     if (e != cudaSuccess) return e;
+    auto smem = [&](const void* kern, size_t bytes) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    e = cudaSuccess;
+    smem((const void*)k_taps_candidates<true>, tp_cand_smem<true>());
+    smem((const void*)k_taps_candidates<false>, tp_cand_smem<false>());
+    smem((const void*)k_taps_refine<true, 0>, tp_refine_smem<true, 0>());
+    smem((const void*)k_taps_refine<false, 0>, tp_refine_smem<false, 0>());
+    smem((const void*)k_taps_refine<true, 1>, tp_refine_smem<true, 1>());
+    smem((const void*)k_taps_refine<false, 1>, tp_refine_smem<false, 1>());
+    if (e != cudaSuccess) return e;
     return pm_batch_prepare_kernels();
 }
+
+/* Where the tap-parallel passes stop paying: they form the neighbours'
+ * terms per pixel, which costs more work, and win by filling the GPU.  Per
+ * depthMap of 3 iterations (FAST; EXACT), against one thread per pixel: 64x48
+ * 5.5 against 32.4 ms (6.0; 38.6), 160x120 14.2 against 34.3 (17.4; 40.6),
+ * 240x180 29.9 against 41.5 (35.7; 49.6), 280x210 40.5 against 43.2 (48.8;
+ * 51.5), 321x243 54.3 against 50.1 (63.1; 61.1). */
+#ifndef TP_MAX_PIXELS
+#define TP_MAX_PIXELS 60000
+#endif
+bool pm_tap_parallel(const PmCostConsts& k) {
+    return (size_t)k.W * k.H <= TP_MAX_PIXELS && std::isfinite(k.alpha) && std::isfinite(k.cmax) && std::isfinite(k.gmax);
+}
+size_t pm_tap_parallel_bytes(int W, int H) { return (size_t)20 * W * H * sizeof(float4); }
 
 cudaError_t pm_launch_pd_block(float4* uout, float* pout, const float4* uin, const float* pin, int pzero,
                                const float4* f, const float* wgt, const float* mask, float lambda, int nsteps, int W,

@@ -26,6 +26,7 @@ struct PmPassArgs {
     uint8_t* winners;
     unsigned long long* counters;   /* [0] cost evaluations, [1] in-image taps; may be NULL */
     float* nbcost;             /* FAST: costs of candidates 1-8 by shared windows, [8][W*H], or NULL */
+    float4* cand;              /* tap-parallel passes: states and costs of candidates 1-20, [20][W*H], or NULL */
     int color;                 /* -1: every pixel (Jacobi); 0 / 1: pixels with (x + y) & 1 == color */
 };
 
@@ -116,6 +117,11 @@ cudaError_t pm_launch_normal_depth(const float4* in, int W, int H, float depthma
 /* Kernel attributes (dynamic shared memory limits) for the current device;
  * call once per device before the first launch or stream capture. */
 cudaError_t pm_prepare_kernels();
+
+/* Whether passes of these constants run tap-parallel (small images), given
+ * PmPassArgs::cand of pm_tap_parallel_bytes. */
+bool pm_tap_parallel(const PmCostConsts& k);
+size_t pm_tap_parallel_bytes(int W, int H);
 
 int pm_pd_block_steps();
 /* Bytes of a dual buffer of pm_launch_pd_block: six planes of floats. */
