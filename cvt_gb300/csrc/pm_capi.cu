@@ -57,8 +57,8 @@ struct cvtpm_ctx {
     uint8_t* win[2];
     uint8_t* valid;
     float* occ;                       /* occlusion mask of depthMapInpaint */
-    /* shared-window neighbour costs (FAST and EXACT): the costs of candidates 1-8 per
-     * pixel ([8][W*H] floats), when the budget allows */
+    /* shared plane windows (FAST and EXACT): the costs of the candidates that share none
+     * (PM_COST_PLANES floats per pixel), when the budget allows */
     float* nbcost = nullptr;
     size_t nb_bytes = 0;
     size_t nb_budget = SIZE_MAX;
@@ -328,17 +328,22 @@ cvtpm_status propagate_view(cvtpm_ctx* ctx, PmPassArgs a, bool exact, bool redbl
     return CVTPM_OK;
 }
 
-/* The neighbour-cost buffer of the shared-window path (8 floats per
+/* The cost buffer of the shared-window passes (PM_COST_PLANES floats per
  * pixel).  Used when it fits the context's budget and 60 % of the free device
- * memory; otherwise the propagation evaluates every neighbour per pixel (same
+ * memory; otherwise the propagation evaluates every candidate per pixel (same
  * results). */
-cvtpm_status ensure_nbcost(cvtpm_ctx* ctx, int W, int H) {
-    const size_t need = (size_t)8 * W * H * sizeof(float);
+cvtpm_status ensure_nbcost(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H) {
+    const size_t need = (size_t)PM_COST_PLANES * W * H * sizeof(float);
     ctx->nb_on = false;
-    if (need > ctx->nb_budget) return CVTPM_OK;
+    if (need > ctx->nb_budget || !pm_shared_windows(base_args(ctx, p, W, H, 0).k)) return CVTPM_OK;
     if (ctx->nb_bytes < need) {
-        if (ctx->no_alloc) return CVTPM_OK;          /* capturing: per-pixel neighbours */
-        if (ctx->nbcost) { CK(cudaFree(ctx->nbcost), "free neighbour costs"); ctx->nbcost = nullptr; ctx->nb_bytes = 0; }
+        if (ctx->no_alloc) return CVTPM_OK;          /* capturing: every candidate per pixel */
+        if (ctx->cand && need > ctx->nb_budget - std::min(ctx->nb_budget, ctx->cand_bytes)) {   /* not both */
+            CK(cudaFree(ctx->cand), "free candidates");
+            ctx->cand = nullptr;
+            ctx->cand_bytes = 0;
+        }
+        if (ctx->nbcost) { CK(cudaFree(ctx->nbcost), "free candidate costs"); ctx->nbcost = nullptr; ctx->nb_bytes = 0; }
         size_t fr = 0, tot = 0;
         CK(cudaMemGetInfo(&fr, &tot), "memory info");
         if ((double)need > 0.6 * (double)fr) return CVTPM_OK;
@@ -360,9 +365,8 @@ cvtpm_status ensure_cand(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H, fl
     *cand = nullptr;
     if (p.schedule != CVTPM_SCHEDULE_JACOBI || !pm_tap_parallel(base_args(ctx, p, W, H, 0).k)) return CVTPM_OK;
     const size_t need = pm_tap_parallel_bytes(W, H);
-    if (need > ctx->nb_budget) return CVTPM_OK;
     if (ctx->cand_bytes < need) {
-        if (ctx->no_alloc) return CVTPM_OK;
+        if (ctx->no_alloc || need > ctx->nb_budget - std::min(ctx->nb_budget, ctx->nb_bytes)) return CVTPM_OK;
         if (ctx->cand) { CK(cudaFree(ctx->cand), "free candidates"); ctx->cand = nullptr; ctx->cand_bytes = 0; }
         size_t fr = 0, tot = 0;
         CK(cudaMemGetInfo(&fr, &tot), "memory info");
@@ -491,8 +495,8 @@ cvtpm_status run_depthmap(cvtpm_ctx* ctx, const cvtpm_params& p, float* dmap, si
     if ((s = ensure_cand(ctx, p, W, H, &aL.cand)) != CVTPM_OK) return s;
     aR.cand = aL.cand;
     if (!aL.cand) {
-        if ((s = ensure_nbcost(ctx, W, H)) != CVTPM_OK) return s;
-        if (ctx->nb_on) aL.nbcost = aR.nbcost = ctx->nbcost;
+        if ((s = ensure_nbcost(ctx, p, W, H)) != CVTPM_OK) return s;
+        if (ctx->nb_on) aL.costs = aR.costs = ctx->nbcost;
     }
     if (!ctx->dcount) {
         if (ctx->no_alloc) return fail(ctx, CVTPM_ERR_ALLOC, "counters not allocated before capture");
@@ -632,8 +636,8 @@ cvtpm_status run_depthmap_inpaint(cvtpm_ctx* ctx, const cvtpm_params& p, float* 
     if ((s = ensure_cand(ctx, p, W, H, &aL.cand)) != CVTPM_OK) return s;
     aR.cand = aL.cand;
     if (!aL.cand) {
-        if ((s = ensure_nbcost(ctx, W, H)) != CVTPM_OK) return s;
-        if (ctx->nb_on) aL.nbcost = aR.nbcost = ctx->nbcost;
+        if ((s = ensure_nbcost(ctx, p, W, H)) != CVTPM_OK) return s;
+        if (ctx->nb_on) aL.costs = aR.costs = ctx->nbcost;
     }
     if (!ctx->dcount) {
         if (ctx->no_alloc) return fail(ctx, CVTPM_ERR_ALLOC, "counters not allocated before capture");
@@ -988,7 +992,7 @@ cvtpm_status cvtpm_set_memory_budget(cvtpm_ctx* ctx, size_t bytes) {
     ctx->nb_budget = bytes;
     if (ctx->nbcost && ctx->nb_bytes > bytes) {
         CK(cudaSetDevice(ctx->device), "cudaSetDevice");
-        CK(cudaFree(ctx->nbcost), "free neighbour costs");
+        CK(cudaFree(ctx->nbcost), "free candidate costs");
         ctx->nbcost = nullptr;
         ctx->nb_bytes = 0;
     }
@@ -1177,7 +1181,7 @@ cvtpm_status capture_batch(cvtpm_ctx* ctx, const cvtpm_pair* pairs, int npairs, 
             if ((s = ensure_buffers(c, pairs[i].width, pairs[i].height)) != CVTPM_OK) return fail(ctx, s, c->err);
             float4* cand = nullptr;
             if ((s = ensure_cand(c, p, pairs[i].width, pairs[i].height, &cand)) != CVTPM_OK) return fail(ctx, s, c->err);
-            if (!cand && (s = ensure_nbcost(c, pairs[i].width, pairs[i].height)) != CVTPM_OK) return fail(ctx, s, c->err);
+            if (!cand && (s = ensure_nbcost(c, p, pairs[i].width, pairs[i].height)) != CVTPM_OK) return fail(ctx, s, c->err);
         }
     }
     if (k > 0 && (s = ensure_tables(ctx->lanes[0].c, p, ctx->bstream)) != CVTPM_OK) return fail(ctx, s, ctx->lanes[0].c->err);
@@ -1348,7 +1352,7 @@ cvtpm_status phase_prepare(PhaseState& S) {
         c->nb_budget = S.ctx->nb_budget;
         c->timing = false;
         if ((s = ensure_buffers(c, S.pairs[i].width, S.pairs[i].height)) != CVTPM_OK) return fail(S.ctx, s, c->err);
-        if ((s = ensure_nbcost(c, S.pairs[i].width, S.pairs[i].height)) != CVTPM_OK) return fail(S.ctx, s, c->err);
+        if ((s = ensure_nbcost(c, c->prm, S.pairs[i].width, S.pairs[i].height)) != CVTPM_OK) return fail(S.ctx, s, c->err);
         S.maxW = std::max(S.maxW, S.pairs[i].width);
     }
     return ensure_tables(S.ctx->bpairs[0], S.p, S.st) == CVTPM_OK ? CVTPM_OK
@@ -1383,7 +1387,7 @@ cvtpm_status phase_start(PhaseState& S) {
         const int W = S.pairs[i].width, H = S.pairs[i].height;
         S.aL[i] = base_args(c, c->prm, W, H, 0);
         S.aR[i] = base_args(c, c->prm, W, H, 1);
-        if (c->nb_on) S.aL[i].nbcost = S.aR[i].nbcost = c->nbcost;
+        if (c->nb_on) S.aL[i].costs = S.aR[i].costs = c->nbcost;
         S.aL[i].counters = S.aR[i].counters = c->dcount;
         S.aL[i].out = c->S[0][0];
         S.aR[i].out = c->S[1][0];
@@ -1404,28 +1408,26 @@ cvtpm_status phase_start(PhaseState& S) {
     return CVTPM_OK;
 }
 
-/* One view's propagation pass for every pair: neighbour costs (where the
- * pair's shared windows are on), propagation, view lists. */
+/* One view's propagation pass for every pair (shared windows where the pair
+ * has its cost buffer), then the view lists. */
 cvtpm_status phase_propagate(PhaseState& S, std::vector<PmPassArgs>& args, short4* (*list_of)(cvtpm_ctx*),
                              const float4* (*src_of)(cvtpm_ctx*, int), int sw) {
     cvtpm_ctx* ctx = S.ctx;
     const bool exact = S.p.arith == CVTPM_ARITH_EXACT;
     cvtpm_status s;
-    std::vector<int> nb;
-    for (int i = 0; i < S.n; ++i)
-        if (args[i].nbcost) nb.push_back(i);
-    if (!nb.empty() &&
-        (s = run_phase<PmPassArgs>(ctx, (int)nb.size(), PMB_NBCOST, S.kn, [&](int e, PmPassArgs& a, int& W, int& H) {
-            a = args[nb[e]];
-            W = a.k.W; H = a.k.H;
-        }, [&](const PmBatch<PmPassArgs>& b) { return pm_batch_nbcost(b, exact, S.kn, S.st); }, "batched neighbour costs",
-           &S.launches)) != CVTPM_OK)
-        return s;
-    if ((s = run_phase<PmPassArgs>(ctx, S.n, PMB_PIXEL, S.kn, [&](int e, PmPassArgs& a, int& W, int& H) {
-            a = args[e];
-            W = a.k.W; H = a.k.H;
-        }, [&](const PmBatch<PmPassArgs>& b) { return pm_batch_propagate(b, exact, S.kn, S.st); }, "batched propagate",
-           &S.launches)) != CVTPM_OK)
+    std::vector<int> shared, plain;
+    for (int i = 0; i < S.n; ++i) (args[i].costs ? shared : plain).push_back(i);
+    auto phase = [&](const std::vector<int>& of, PmBatchKernel kind, auto launch, const char* what) -> cvtpm_status {
+        if (of.empty()) return CVTPM_OK;
+        return run_phase<PmPassArgs>(ctx, (int)of.size(), kind, S.kn, [&](int e, PmPassArgs& a, int& W, int& H) {
+                a = args[of[e]];
+                W = a.k.W; H = a.k.H;
+            }, [&](const PmBatch<PmPassArgs>& b) { return launch(b, exact, S.kn, S.st); }, what, &S.launches);
+    };
+    if ((s = phase(shared, PMB_PIXEL, pm_batch_sweep, "batched sweep")) != CVTPM_OK ||
+        (s = phase(shared, PMB_SHARE, pm_batch_share, "batched shared windows")) != CVTPM_OK ||
+        (s = phase(shared, PMB_PIXEL, pm_batch_refine, "batched refinement")) != CVTPM_OK ||
+        (s = phase(plain, PMB_PIXEL, pm_batch_propagate, "batched propagate")) != CVTPM_OK)
         return s;
     return run_phase<PmViewListArgs>(ctx, S.n, PMB_ROW, S.kn, [&](int e, PmViewListArgs& a, int& W, int& H) {
             cvtpm_ctx* c = ctx->bpairs[e];
@@ -1681,7 +1683,7 @@ cvtpm_status tune_mode(PhaseState& full, float ms[2]) {
         ++S.n;
     }
     if (s == CVTPM_OK) s = ensure_buffers(lane, maxW, maxH);
-    if (s == CVTPM_OK) s = ensure_nbcost(lane, maxW, maxH);
+    if (s == CVTPM_OK) s = ensure_nbcost(lane, S.p, maxW, maxH);
     if (s != CVTPM_OK) return fail(ctx, s, lane->err);
     EventPair ev;
     CK(cudaEventCreate(&ev.a), "tune event");

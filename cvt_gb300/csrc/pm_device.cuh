@@ -305,7 +305,7 @@ PM_DEV void fast_tap_terms(const PmCostConsts& k, const PmRecRow& row, int xi, f
 }
 
 /* The bilateral weight of tap (centre colour vc, tap colour a1, profile
- * value prof): the FAST and EXACT paths and k_nbcost share it. */
+ * value prof): the FAST and EXACT paths share it. */
 PM_DEV float tap_weight(float4 vc, float4 a1, float prof) {
     const float d = (fabsf(vc.x - a1.x) + fabsf(vc.y - a1.y)) + fabsf(vc.z - a1.z);
     return pm_wexp(-d * prof);
@@ -348,9 +348,8 @@ PM_DEV void tap_weight2(float4 vc, float4 a, float4 b, float pa, float pb, float
  * Candidates with act[k] == false contribute nothing and return 1e5. */
 /* FAST sweeps of at most PM_PAIR_TAPS_MAXK candidates form their weights two
  * taps at a time (tap_weight2).  Measured per depthMap of the 1242x375 bench
- * pair, same bits: 517.6 -> 509.8 ms with every FAST sweep of 1-4 (the
- * neighbour kernel's weight phase alone: 513.6; sweeps of 3-4 or 2-4 only:
- * within 0.5 ms of 1-4).  The EXACT sweeps keep one tap per step: paired,
+ * pair, same bits: 513.6 -> 509.8 ms with every FAST sweep of 1-4 (sweeps of
+ * 3-4 or 2-4 only: within 0.5 ms of 1-4).  The EXACT sweeps keep one tap per step: paired,
  * its stage-1 sweeps of 4 took 148 registers and one block per SM (596 ->
  * 681 ms). */
 #ifndef PM_PAIR_TAPS_MAXK

@@ -5,9 +5,11 @@
  *  k_prep               pmhstereo_gradxy + pmhstereo_weight (pmhstereo.cl:737-831), input copy
  *  k_records            (fast arithmetic only) value/forward-difference records of a view
  *  k_init<EXACT>        pmhstereo_init (:230-248)
- *  k_propagate<EXACT>   pmhstereo_propagate_view (:286-404) without the scatter
+ *  k_sweep, k_share<EXACT>, k_propagate<EXACT, 2>  pmhstereo_propagate_view (:286-404) without the
+ *                       scatter: candidates 9, 16-20 by pixel; 1-8, 10-15 by plane and the
+ *                       acceptance; the refinements 21, 22
+ *  k_propagate<EXACT, *>  the same with every candidate by pixel
  *  k_taps_*<EXACT>      init and propagate for small images, the taps of a window in parallel
- *  k_nbcost<EXACT>      its candidates 1-8 (:330-342), plane by plane over shared windows
  *  k_view_list          the scatter of :391-400, made deterministic (smallest source x first)
  *  k_consistency        pmhstereo_consistency (:428-464)
  *  k_fill_state         pmhstereo_fill_state (:466-510)
@@ -21,13 +23,9 @@
 #include <cmath>
 #include <type_traits>
 
-/* Blocks of 256 threads per SM the FAST propagation and the neighbour
- * costs are compiled for. */
+/* Blocks of 256 threads per SM the FAST propagation is compiled for. */
 #ifndef PM_PROP_MINB
 #define PM_PROP_MINB 2
-#endif
-#ifndef PM_NB_MINB
-#define PM_NB_MINB 2
 #endif
 /* FAST: candidates 9-16 per window sweep (8: one sweep; 4: two) */
 /* The propagation as two launches: candidates 1-20, then the refinements
@@ -204,10 +202,7 @@ PM_DEV void propagate_tile(const PmPassArgs& a, int tbx, int tby) {
     int nview_total = 0;
     if (STAGE != 2 && STAGE != 3) {
         /* candidates 1-8: the 3x3 neighbourhood of `old`, clamped to the edge
-         * (:330-342).  With the shared-window costs of k_nbcost (FAST), only
-         * neighbours the clamp moves (pixels on the image border) are evaluated
-         * here; the others are read. */
-        const bool shared = a.nbcost != nullptr;
+         * (:330-342) */
 #pragma unroll 1
         for (int b = 0; b < 2; ++b) {
             float4 s[4]; bool act[4]; float c[4];
@@ -215,20 +210,10 @@ PM_DEV void propagate_tile(const PmPassArgs& a, int tbx, int tby) {
             for (int i = 0; i < 4; ++i) {
                 int n = b * 4 + i;                 /* 0..7 over the 8 neighbours in raster order */
                 int nn = n < 4 ? n : n + 1;        /* skip the centre */
-                int px = nn % 3 - 1, py = nn / 3 - 1;
-                s[i] = a.old[(size_t)clampi(yc + py, 0, H - 1) * W + clampi(xc + px, 0, W - 1)];
-                const bool edge = xc + px < 0 || xc + px >= W || yc + py < 0 || yc + py >= H;
-                act[i] = !shared || edge;
-                c[i] = act[i] ? 0.0f : a.nbcost[(size_t)n * W * H + o];
+                s[i] = a.old[(size_t)clampi(yc + nn / 3 - 1, 0, H - 1) * W + clampi(xc + nn % 3 - 1, 0, W - 1)];
+                act[i] = true;
             }
-            bool any = act[0] || act[1] || act[2] || act[3];
-            if (!shared || __any_sync(0xffffffffu, any)) {
-                float ce[4];
-                eval_costs<4, EXACT>(a.k, a.v1, a.v2, xc, yc, s, act, ce);
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-                    if (act[i]) c[i] = ce[i];
-            }
+            eval_costs<4, EXACT>(a.k, a.v1, a.v2, xc, yc, s, act, c);
 #pragma unroll
             for (int i = 0; i < 4; ++i) accept(s[i], c[i], 1 + b * 4 + i);
         }
@@ -334,27 +319,7 @@ k_propagate(PmPassArgs a) {
     propagate_tile<EXACT, STAGE>(a, blockIdx.x, blockIdx.y);
 }
 
-/* ---------------------------------------- shared neighbour windows -- */
-/* Candidates 1-8 (pmhstereo.cl:330-342) evaluated plane by plane.  Thread m
- * owns the plane old[m]; it is candidate k of the pixel u_k = m - o_k for
- * the 8 offsets o_k of the 3x3 neighbourhood (u_k inside the image makes the
- * clamp of :335-336 the identity; border pixels evaluate their clamped
- * neighbours themselves).  A tap's matching terms depend on the tap and the
- * plane only, so they are computed once over the union of the 8 windows
- * (37 x 37) and folded into every user's sums with that user's bilateral
- * weight, formed by tap_weight from the user's centre colour as eval_costs
- * forms it.  Each user receives its taps in raster order with the operations
- * of eval_costs, so its cost has the bits of a separate evaluation.  Costs go
- * to nb[k * W*H + u_k].  Within a warp the window offsets are the same in
- * every lane, so the profile read is a constant-cache broadcast.
- * (Measured alternatives: weights precomputed into a [(2P+1)^2][W*H] volume
- * and loaded, 8 per tap, ran at the same speed for 4.9 KB per pixel; half
- * loaded, half recomputed ran slower than either; staging the volume in a
- * shared-memory ring exposed the latency of the record loads.)  The minimum
- * of 2 blocks per SM makes the allocator use up to 128 registers: without
- * it, it chose 97 and the kernel ran 8 % slower. */
-#define NB_COLS 30   /* planes per warp; lanes 30 and 31 form the weights lanes 28 and 29 read */
-
+/* ---------------------------------------------- shared-window parts -- */
 /* The plane part of a tap for the shared windows: the position and matching
  * terms of plane (sx, sy, sz) [EXACT] or (S0, S1, X) [FAST] at tap (qx, qy).
  * Both depend on the tap's image coordinates and the plane only (EXACT forms
@@ -433,274 +398,342 @@ __device__ __forceinline__ void nb_plane(const PmCostConsts& k, float4 s, bool f
     }
 }
 
-/* Plane (mx, my) with every weight formed by its own lane. */
-template <bool EXACT>
-__device__ __forceinline__ void nbcost_lane(const PmPassArgs& a, int mx, int my) {
-    const int W = a.k.W, H = a.k.H, P = a.k.P;
-    const size_t n = (size_t)W * H, m = (size_t)my * W + mx;
-    const float4 s = a.old[m];
-    long long S0, S1, XA;
-    float sx, sy, sz;
-    const bool fin = finite3(s);
-    nb_plane<EXACT>(a.k, s, fin, sx, sy, sz, S0, S1, XA);
-    unsigned uok = 0;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int nn = k < 4 ? k : k + 1, ox = nn % 3 - 1, oy = nn / 3 - 1;
-        const int ux = mx - ox, uy = my - oy;
-        if (ux >= 0 && ux < W && uy >= 0 && uy < H) uok |= 1u << k;
-    }
-    float4 uc[8];                                   /* the users' centre colours */
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int nn = k < 4 ? k : k + 1, ox = nn % 3 - 1, oy = nn / 3 - 1;
-        const int ux = min(max(mx - ox, 0), W - 1), uy = min(max(my - oy, 0), H - 1);
-        uc[k] = __ldg(&a.v1.col[(size_t)uy * W + ux]);
-    }
-    float r1[8], r2[8], ws[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) { r1[k] = 0.0f; r2[k] = 0.0f; ws[k] = 0.0f; }
-    const int qx0 = max(mx - P - 1, 0), qx1 = min(mx + P + 1, W - 1);
-    const int qy0 = max(my - P - 1, 0), qy1 = min(my + P + 1, H - 1);
-    for (int qy = qy0; qy <= qy1; ++qy) {
-        const int ry = qy - my;
-        unsigned rmask = 0;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int oy = (k < 4 ? k : k + 1) / 3 - 1;
-            if (abs(ry + oy) <= P) rmask |= 1u << k;
-        }
-        rmask &= uok;
-        if (!rmask) continue;
-        const float4* c1row = a.v1.col + (size_t)qy * W;
-        const float4* g1row = a.v1.grad + (size_t)qy * W;
-        const PmRecRow rrow = rec_row(a.v2, a.k.rp, qy);
-        long long X = XA + (long long)(qy - H / 2) * S1 + (long long)(qx0 - W / 2) * S0;
-        for (int qx = qx0; qx <= qx1; ++qx) {
-            const long long Xt = X;
-            X += S0;
-            const int rx = qx - mx;
-            unsigned mask = rmask;
-            if (rx <= -P || rx >= P) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const int ox = (k < 4 ? k : k + 1) % 3 - 1;
-                    if (abs(rx + ox) > P) mask &= ~(1u << k);
-                }
-            }
-            const float4 a1 = __ldg(&c1row[qx]);
-            const float4 g1 = __ldg(&g1row[qx]);
-            float cc, gc;
-            if (!nb_tap_terms<EXACT>(a.k, a.v2, qx, qy, rrow, sx, sy, sz, Xt, a1, g1, cc, gc)) continue;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                if (!((mask >> k) & 1u)) continue;
-                /* user k sees this tap at offset (ry + oy_k, rx + ox_k) */
-                const int nn = k < 4 ? k : k + 1, ox = nn % 3 - 1, oy = nn / 3 - 1;
-                const float w = tap_weight(uc[k], a1, c_prof[(ry + oy + PM_PMAX) * PM_PROF_N + PM_PMAX + rx + ox]);
-                nb_accumulate<EXACT>(w, cc, gc, r1[k], r2[k], ws[k]);
-            }
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        if (!((uok >> k) & 1u)) continue;
-        const int nn = k < 4 ? k : k + 1, ox = nn % 3 - 1, oy = nn / 3 - 1;
-        a.nbcost[(size_t)k * n + m - (size_t)(oy * W + ox)] = nb_final<EXACT>(a.k, fin, r1[k], r2[k], ws[k]);
-    }
-}
-
-/* Interior blocks: the weights shared across the block's rows.
- *
- * A block holds NB_ROWS plane rows (warps 1..NB_ROWS) and NB_WARPS user rows
- * U_w = my0 - 1 + w (w = 0..NB_WARPS-1): the plane rows and the rows just
- * above and below them, whose pixels are users of the edge planes.  The
- * weight of user (mx - 1, U) at tap (mx + rx, Yq) — lane L's "ox = +1"
- * weight — depends on
- * U, Yq, rx and the lane only, so it is needed by the three plane rows
- * U - 1, U and U + 1 at three different window rows.  The block walks the
- * union of its planes' window rows (Yq = my0 - P - 1 .. my0 + NB_ROWS + P)
- * in lockstep; per row:
- *   A. the image-1 row Yq over the block's columns mx0 - P - 1 ..
- *      mx0 + 32 + P (colour and gradient) is staged into shared memory by
- *      cp.async (double-buffered: row Yq + 1 is copied while the taps of
- *      row Yq run, so a row costs two block barriers);
- *   B. warp w forms the weights of its user row at that image row for
- *      every offset rx (one weight per lane and offset) into a table
- *      T[w][rx][lane];
- *   C. each plane warp processes its window row Yq - my: the matching terms
- *      of its plane at each tap (the record loads from global memory
- *      through L1), the 8 users' weights read from the table
- *      (user (mx - ox, U) at tap column mx + rx is lane L + 1 - ox's entry
- *      at offset rx - 1 + ox), folded into the users' sums in raster order
- *      through the operations of eval_costs.
- * A weight is formed once per block, where each plane row forming the
- * weights of its three user rows would form it three times.  Same bits as
- * nbcost_lane. */
-#define NB_ROWS 8
-#define NB_WARPS (NB_ROWS + 2)
-
 PM_DEV void cp_async16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
 
-/* dynamic shared memory of nbcost_block for window radius P */
-__host__ __device__ constexpr size_t nb_block_smem(int P) {
-    return (size_t)4 * (32 + 2 * (P + 1)) * 16 + (size_t)NB_WARPS * (2 * P + 5) * 32 * 4;
+/* The squared distance of a state to the smoothed field (pmhstereo.cl:266-283,
+ * one side of smooth_distance). */
+PM_DEV float state_distance(float4 s, float4 smooth, float cx, float cy, float depthmax, int lr) {
+    const float4 diag = f4(1.0f, 1.0f, 0.0f, 1.0f / (depthmax * depthmax));
+    const float4 d = to_ref_normal_depth(s, cx, cy, lr) - smooth;
+    return dot4(d, diag * d);
+}
+/* The acceptance rule of a propagation pass, from costs and distances formed
+ * beforehand: a state that is not finite makes both distances 0. */
+struct TpBest { float cost, dist; bool fin; };
+PM_DEV bool tp_accepts(const TpBest& cand, const TpBest& self, float theta) {
+    const bool fin = cand.fin && self.fin;
+    return cand.cost + theta * (fin ? cand.dist : 0.0f) <= self.cost + theta * (fin ? self.dist : 0.0f);
+}
+
+/* The smoothed plane's normal and depth at a pixel (:320-323) */
+PM_DEV float4 smooth_at(const PmPassArgs& a, size_t o) {
+    const float4 sm = a.smooth[o];
+    const float nf = fmaxf(pm_sqrt(sm.x * sm.x + sm.y * sm.y) + 0.001f, 1.0f);
+    const float smx = sm.x / nf, smy = sm.y / nf;
+    return f4(smx, smy, pm_sqrt(1.0f - smx * smx - smy * smy), sm.z * a.depthmax);
+}
+
+/* The smoothed plane as a state (candidate 9, :345-352) */
+PM_DEV float4 smooth_state(float4 smooth, float cx, float cy, int lr) {
+    const float4 sc = f4(1.0f - (-smooth.x / smooth.z), 0.0f - (-smooth.y / smooth.z),
+                         0.0f - ((smooth.x * cx + smooth.y * cy) / smooth.z + smooth.w), 0.0f - 0.0f);
+    return lr ? sc : viewprop(sc);
+}
+
+/* Adds a warp's evaluations and in-image window taps (`ev` evaluations at an
+ * inside pixel) to the counters; every lane calls it. */
+PM_DEV void pass_counters(const PmPassArgs& a, bool inside, int x, int y, int nev) {
+    if (!a.counters) return;
+    unsigned long long ev = 0, taps = 0;
+    if (inside) {
+        const int P = a.k.P;
+        const int nx = min(x + P, a.k.W - 1) - max(x - P, 0) + 1;
+        const int ny = min(y + P, a.k.H - 1) - max(y - P, 0) + 1;
+        ev = (unsigned long long)nev;
+        taps = ev * (unsigned long long)(nx * ny);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        ev += __shfl_down_sync(0xffffffffu, ev, off);
+        taps += __shfl_down_sync(0xffffffffu, taps, off);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&a.counters[0], ev);
+        atomicAdd(&a.counters[1], taps);
+    }
+}
+
+/* ------------------------------------------------- shared plane windows -- */
+/* Candidates 1-8 and 10-15 (pmhstereo.cl:330-342,355-361) are planes of the
+ * old field at offsets (-1..7, -1..7): every plane is tested by its 8
+ * neighbours and by about 6 pixels that drew it.  A tap's matching terms
+ * depend on the tap and the plane only, so they are formed once per plane and
+ * tap and read by every pixel that tests the plane; per pixel and plane they
+ * cost a window of record loads, which is what bounds this path (the L1 data
+ * pipe).
+ *
+ * A block owns 32 x SH_TY pixels and the planes they can draw: 40 x (SH_TY + 8)
+ * slots, slot (sx, sy) holding the plane of pixel (x0 - 1 + sx, y0 - 1 + sy)
+ * clamped to the image, so a candidate's slot follows from its offset alone,
+ * also at the border.  The block walks the image rows its windows reach, and
+ * each row by the window offset rx, four at a time: the threads form the terms
+ * of the slots at the next four columns while every pixel folds the current
+ * four into its 14 candidates' sums with the weight of the tap, formed once
+ * for all of them, in raster order.  The terms live in a ring per slot, indexed
+ * by the image column modulo the ring, which has two effects: the lanes of a
+ * warp, whose taps are consecutive columns, read 32 different banks whichever
+ * slots their candidates are in, and the 12 columns in use (offsets -1..7 of
+ * four taps) and the four being formed fill the ring of 16.
+ *
+ * An invalid tap (outside either image) is a NaN in the first term, which no
+ * valid term is for finite truncations (pm_shared_windows).  The sums take
+ * eval_costs' operations in its order, so the costs have its bits.
+ *
+ * Measured at 1242x375 per view pass (ncu): 9.7 ms for the 14 candidates and
+ * the acceptance, where the neighbours by plane (5.9 ms, weights in a table
+ * per block) and the random neighbours by pixel (12.1 of the 16.2 ms of a
+ * sweep of 8) took 18; depthMap 484.7 -> 363.7 ms, 640x480 x 3 iterations
+ * 132 -> 96.3, EXACT 450x375 102 -> 73.4 ms.
+ */
+#define SH_TY 16
+#define SH_NX 40
+#define SH_NY (SH_TY + 8)
+#define SH_NS (SH_NX * SH_NY)
+#define SH_NT (32 * SH_TY)
+#define SH_B 4                                       /* columns per step */
+
+template <bool EXACT> struct ShTerm { typedef float2 type; static constexpr int R = 16; };
+template <> struct ShTerm<true> { typedef float type; static constexpr int R = 32; };   /* 128 bytes per slot */
+
+__host__ __device__ constexpr size_t share_smem(int P) {
+    return (size_t)SH_NS * 128 + 2 * (size_t)(32 + 2 * P) * 32;
+}
+
+/* Candidates 9, 16 and the other view's 17-20, which share no plane with
+ * another pixel: one sweep of as many as the warp's fullest list holds.  Their
+ * costs go to a.costs[0], [1] and [2 + i]. */
+template <bool EXACT>
+PM_DEV void sweep_tile(const PmPassArgs& a, int tbx, int tby) {
+    const int W = a.k.W, H = a.k.H;
+    const int x = tbx * 32 + threadIdx.x, y = tby * 8 + threadIdx.y;
+    const bool inside = x < W && y < H;
+    const int xc = min(x, W - 1), yc = min(y, H - 1);   /* lanes outside still follow the warp */
+    const float cx = (float)xc, cy = (float)yc;
+    const size_t n = (size_t)W * H, o = (size_t)yc * W + xc;
+    const float4 s9 = smooth_state(smooth_at(a, o), cx, cy, a.lr);
+    PmRng rng;
+    seed_rng(rng, a, xc, yc, false);
+#pragma unroll 1
+    for (int i = 0; i < 12; ++i) (void)rng_float(rng);       /* the random neighbours' offsets */
+    const float4 s16 = state_init(rng, cx, cy, a.lr, 2.0f, a.depthmax);
+    short4 l = make_short4(-1, -1, -1, -1);
+    if (a.viewin && inside) l = a.viewin[o];
+    const short li[4] = {l.x, l.y, l.z, l.w};
+    const int nview = (li[0] < 0) ? 0 : (li[1] < 0) ? 1 : (li[2] < 0) ? 2 : (li[3] < 0) ? 3 : 4;
+    auto sweep = [&](auto m) {
+        constexpr int M = decltype(m)::value;
+        float4 s[2 + M]; bool act[2 + M]; float c[2 + M];
+        s[0] = s9; act[0] = true;
+        s[1] = s16; act[1] = true;
+#pragma unroll
+        for (int i = 0; i < M; ++i) {
+            act[2 + i] = i < nview;
+            s[2 + i] = act[2 + i] ? viewprop(a.viewsrc[(size_t)yc * W + li[i]]) : f4s(0.0f);
+        }
+        eval_costs<2 + M, EXACT>(a.k, a.v1, a.v2, xc, yc, s, act, c);
+        if (inside) {
+#pragma unroll
+            for (int i = 0; i < 2 + M; ++i) a.costs[(size_t)i * n + o] = c[i];
+        }
+    };
+    const int nmax = __reduce_max_sync(0xffffffffu, (unsigned)nview);
+    if (nmax == 0) sweep(std::integral_constant<int, 0>());
+    else if (nmax == 1) sweep(std::integral_constant<int, 1>());
+    else if (nmax == 2) sweep(std::integral_constant<int, 2>());
+    else if (nmax == 3) sweep(std::integral_constant<int, 3>());
+    else sweep(std::integral_constant<int, 4>());
 }
 
 template <bool EXACT>
-PM_DEV void nbcost_block(const PmPassArgs& a, int mx0, int my0) {
-    extern __shared__ __align__(16) float4 nb_smem[];
-    const int W = a.k.W, H = a.k.H, P = a.k.P;
-    const int NQ = 32 + 2 * (P + 1);                 /* staged columns mx0 - P - 1 .. mx0 + 32 + P */
-    const int NR = 2 * P + 5;                        /* table columns: offsets rx = -P-3 .. P+1 */
-    /* two staged rows (colour then gradient, NQ float4 each): the copy of
-     * the next row overlaps the taps of the current one */
-    float4* const rows = nb_smem;
-    float* T = reinterpret_cast<float*>(nb_smem + 4 * NQ);
+__global__ void __launch_bounds__(256, 2) k_sweep(PmPassArgs a) { sweep_tile<EXACT>(a, blockIdx.x, blockIdx.y); }
+
+/* The candidates 1-16 and the view candidates of a pixel against its old
+ * state: 9, 16 and 17-20 have their costs in a.costs, the others are formed
+ * here.  The best goes to a.out. */
+template <bool EXACT>
+PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
+    typedef typename ShTerm<EXACT>::type Term;
+    constexpr int R = ShTerm<EXACT>::R;
+    constexpr int SLOTS = (SH_NS + SH_NT - 1) / SH_NT;
+    extern __shared__ __align__(16) unsigned char sh_smem[];
+    Term* const ring = reinterpret_cast<Term*>(sh_smem);             /* [SH_NS][R] */
+    float4* const rows = reinterpret_cast<float4*>(sh_smem + (size_t)SH_NS * 128);
+    const int W = a.k.W, H = a.k.H, P = a.k.P, NQ = 32 + 2 * P;
     const int lane = threadIdx.x, w = threadIdx.y, tid = w * 32 + lane;
-    const int U = my0 + w - 1;                       /* this warp's user row */
-    const float4 uc = __ldg(&a.v1.col[(size_t)clampi(U, 0, H - 1) * W + mx0 + lane - 1]);
-    T[(w * NR + 0) * 32 + lane] = 0.0f;              /* offsets before the window: no weight */
-    T[(w * NR + 1) * 32 + lane] = 0.0f;
-    /* plane role */
-    const int my = U, mx = mx0 + lane;
-    const bool prow = w >= 1 && w <= NB_ROWS && my < H;      /* warp-uniform */
-    const bool own = prow && lane < NB_COLS;
-    const size_t n = (size_t)W * H, m = (size_t)clampi(my, 0, H - 1) * W + mx;
-    const float4 s = a.old[m];
-    long long S0, S1, XA;
-    float sx, sy, sz;
-    const bool fin = finite3(s);
-    nb_plane<EXACT>(a.k, s, fin, sx, sy, sz, S0, S1, XA);
-    unsigned uok = 0;
+    const int x0 = tbx * 32, y0 = tby * SH_TY;
+    const size_t n = (size_t)W * H;
+    /* plane role: slots tid, tid + SH_NT */
+    int smx[SLOTS], slo[SLOTS], shi[SLOTS];          /* nominal column; image rows the slot is needed at */
+    long long S0[SLOTS], S1[SLOTS], X[SLOTS];
+    float sx[SLOTS], sy[SLOTS], sz[SLOTS];
+    const int t0 = max(y0 - P, 0), t1 = min(min(y0 + SH_TY - 1, H - 1) + P, H - 1);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int oy = (k < 4 ? k : k + 1) / 3 - 1;
-        if (my - oy >= 0 && my - oy < H) uok |= 1u << k;
+    for (int i = 0; i < SLOTS; ++i) {
+        const int s = tid + i * SH_NT;
+        const int mx = x0 - 1 + s % SH_NX, my = y0 - 1 + s / SH_NX;
+        const float4 st = a.old[(size_t)clampi(my, 0, H - 1) * W + clampi(mx, 0, W - 1)];
+        long long XA;
+        nb_plane<EXACT>(a.k, st, finite3(st), sx[i], sy[i], sz[i], S0[i], S1[i], XA);
+        smx[i] = mx;
+        slo[i] = max(y0, my - 7) - P;
+        shi[i] = s < SH_NS ? min(min(y0 + SH_TY - 1, H - 1), my + 1) + P : -1;
+        /* the position at column mx - P - 7, row t0 */
+        X[i] = XA + (long long)(t0 - H / 2) * S1[i] + (long long)(mx - P - 7 - W / 2) * S0[i];
     }
-    float r1[8], r2[8], ws[8];
+    /* pixel role */
+    const int x = x0 + lane, y = y0 + w, xc = min(x, W - 1), yc = min(y, H - 1);
+    const size_t o = (size_t)yc * W + xc;
+    const float4 vc = __ldg(&a.v1.col[o]);
+    int roff[6];                                     /* the random neighbours' slots, as ring entries */
+    PmRng rng;
+    seed_rng(rng, a, xc, yc, false);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) { r1[k] = 0.0f; r2[k] = 0.0f; ws[k] = 0.0f; }
-    /* the image rows the block's windows reach: Yq = t0 .. t1 */
-    const int t0 = max(my0 - P - 1, 0), t1 = min(my0 + NB_ROWS + P, H - 1);
-    auto stage = [&](int Yq, int buf) {                 /* A: an image-1 row, by cp.async */
-        const size_t rb = (size_t)Yq * W + (mx0 - P - 1);
+    for (int i = 0; i < 6; ++i) {
+        const int ox = (int)(rng_float(rng) * 7.0f + 0.5f);
+        const int oy = (int)(rng_float(rng) * 7.0f + 0.5f);
+        roff[i] = ((w + 1 + oy) * SH_NX + lane + 1 + ox) * R;
+    }
+    const int own = ((w + 1) * SH_NX + lane + 1) * R;
+    float r1[14], r2[14], ws[14];
+#pragma unroll
+    for (int c = 0; c < 14; ++c) { r1[c] = 0.0f; r2[c] = 0.0f; ws[c] = 0.0f; }
+
+    auto stage = [&](int Yq, int buf) {              /* image-1 row Yq, columns x0 - P .. x0 + 31 + P */
+        const size_t rb = (size_t)Yq * W;
         float4* dst = rows + buf * 2 * NQ;
-        for (int i = tid; i < 2 * NQ; i += NB_WARPS * 32)
-            cp_async16(&dst[i], i < NQ ? (const void*)(a.v1.col + rb + i) : (const void*)(a.v1.grad + rb + i - NQ));
+        for (int i = tid; i < 2 * NQ; i += SH_NT) {
+            const int q = i < NQ ? i : i - NQ, gx = clampi(x0 - P + q, 0, W - 1);
+            cp_async16(&dst[i], i < NQ ? (const void*)(a.v1.col + rb + gx) : (const void*)(a.v1.grad + rb + gx));
+        }
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    auto weights = [&](int Yq, int buf) {               /* B: this user row's weights at image row Yq */
+    auto produce = [&](int Yq, int buf, int t) {     /* columns mx - P - 7 + 4t .. + 3 of every slot */
         const float4* s_col = rows + buf * 2 * NQ;
-        const int dy = Yq - U;
-        if (abs(dy) <= P) {                             /* warp-uniform */
-            const float* prow = c_prof + (dy + PM_PMAX) * PM_PROF_N + PM_PMAX;
-            int rxi = 0;
-            for (; rxi < 2 * P; rxi += 2) {                 /* two offsets at a time, on packed pairs */
-                float wa, wb;
-                tap_weight2(uc, s_col[lane + rxi], s_col[lane + rxi + 1], prow[rxi - P], prow[rxi + 1 - P], wa, wb);
-                T[(w * NR + rxi + 2) * 32 + lane] = wa;
-                T[(w * NR + rxi + 3) * 32 + lane] = wb;
+        const float4* s_grad = s_col + NQ;
+        const PmRecRow rrow = rec_row(a.v2, a.k.rp, Yq);
+#pragma unroll
+        for (int i = 0; i < SLOTS; ++i) {
+            if (Yq < slo[i] || Yq > shi[i]) continue;
+            const int q0 = smx[i] - P - 7 + SH_B * t;
+            Term* const dst = ring + (size_t)(tid + i * SH_NT) * R;
+            long long Xt = X[i] + (long long)(SH_B * t) * S0[i];
+#pragma unroll
+            for (int b = 0; b < SH_B; ++b) {
+                const int q = q0 + b, qs = q - (x0 - P);
+                const long long Xb = Xt;
+                Xt += S0[i];
+                if ((unsigned)qs >= (unsigned)NQ) continue;          /* no pixel of the tile reads it */
+                float cc = 0.0f, gc = 0.0f;
+                bool ok = q >= 0 && q < W;
+                if (ok) ok = nb_tap_terms<EXACT>(a.k, a.v2, q, Yq, rrow, sx[i], sy[i], sz[i], Xb, s_col[qs], s_grad[qs], cc, gc);
+                if (!ok) cc = __int_as_float(0x7fc00000);
+                if constexpr (EXACT) dst[q & (R - 1)] = cc;
+                else dst[q & (R - 1)] = make_float2(cc, gc);
             }
-            for (; rxi < 2 * P + 3; ++rxi) {
-                const int dx = rxi - P;                     /* tap offset from the user: rx + 1 */
-                T[(w * NR + rxi + 2) * 32 + lane] = abs(dx) <= P ? tap_weight(uc, s_col[lane + rxi], prow[dx]) : 0.0f;
-            }
-        } else {
-            for (int rxi = 0; rxi < 2 * P + 3; ++rxi) T[(w * NR + rxi + 2) * 32 + lane] = 0.0f;
         }
     };
+    auto fold = [&](int c, Term t, float wt) {
+        if constexpr (EXACT) {
+            if (t == t) nb_accumulate<true>(wt, t, 0.0f, r1[c], r2[c], ws[c]);
+        } else {
+            if (t.x == t.x) nb_accumulate<false>(wt, t.x, t.y, r1[c], r2[c], ws[c]);
+        }
+    };
+    auto consume = [&](int Yq, int buf, int k) {     /* taps rx = -P + 4k .. + 3 */
+        const float4* s_col = rows + buf * 2 * NQ;
+        const float* prow = c_prof + (Yq - y + PM_PMAX) * PM_PROF_N + PM_PMAX;
+#pragma unroll
+        for (int h = 0; h < SH_B; h += 2) {
+            const int rx = -P + SH_B * k + h;
+            if (rx > P) break;                       /* block-uniform */
+            const int rx1 = min(rx + 1, P);
+            float wt[2];
+            tap_weight2(vc, s_col[lane + P + rx], s_col[lane + P + rx1], prow[rx], prow[rx1], wt[0], wt[1]);
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                if (rx + b > P) break;
+                const Term* const rq = ring + ((x + rx + b) & (R - 1));
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const int nn = c < 4 ? c : c + 1;
+                    fold(c, rq[own + ((nn / 3 - 1) * SH_NX + nn % 3 - 1) * R], wt[b]);
+                }
+#pragma unroll
+                for (int c = 0; c < 6; ++c) fold(8 + c, rq[roff[c]], wt[b]);
+            }
+        }
+    };
+    const int nc = (2 * P + 1 + SH_B - 1) / SH_B;
     stage(t0, 0);
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    weights(t0, 0);
-    __syncthreads();
     for (int Yq = t0; Yq <= t1; ++Yq) {
         const int buf = (Yq - t0) & 1;
-        if (Yq < t1) stage(Yq + 1, buf ^ 1);           /* its buffer was last read before the previous barrier */
-        const float4* s_col = rows + buf * 2 * NQ;
-        const float4* s_grad = s_col + NQ;
-        /* C: the plane rows' window row Yq */
-        const int ry = Yq - my;
-        if (prow && ry >= -P - 1 && ry <= P + 1) {
-            unsigned rmask = 0;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int oy = (k < 4 ? k : k + 1) / 3 - 1;
-                if (abs(ry + oy) <= P) rmask |= 1u << k;
-            }
-            rmask &= uok;
-            if (rmask && own) {
-                const PmRecRow rrow = rec_row(a.v2, a.k.rp, Yq);
-                long long X = XA + (long long)(Yq - H / 2) * S1 + (long long)(mx - P - 1 - W / 2) * S0;
-                /* two taps per iteration: 509.3 -> 507.5 ms per depthMap (4: 508.3) */
-#pragma unroll 2
-                for (int rx = -P - 1; rx <= P + 1; ++rx) {
-                    const int rxi = rx + P + 1;
-                    const long long Xt = X;
-                    X += S0;
-                    unsigned mask = rmask;
-                    if (rx <= -P || rx >= P) {
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) {
-                            const int ox = (k < 4 ? k : k + 1) % 3 - 1;
-                            if (abs(rx + ox) > P) mask &= ~(1u << k);
-                        }
-                    }
-                    const float4 a1 = s_col[lane + rxi];
-                    const float4 g1 = s_grad[lane + rxi];
-                    float cc, gc;
-                    if (!nb_tap_terms<EXACT>(a.k, a.v2, mx + rx, Yq, rrow, sx, sy, sz, Xt, a1, g1, cc, gc)) continue;
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        if (!((mask >> k) & 1u)) continue;
-                        const int nn = k < 4 ? k : k + 1, ox = nn % 3 - 1, r = nn / 3;
-                        const int wu = w + 1 - r;                /* the warp of user row my - (r - 1) */
-                        const float wgt = T[(wu * NR + rxi + 1 + ox) * 32 + lane + 1 - ox];
-                        nb_accumulate<EXACT>(wgt, cc, gc, r1[k], r2[k], ws[k]);
-                    }
-                }
-            }
-        }
-        if (Yq < t1) {
-            asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-            __syncthreads();                            /* the taps of Yq are done with T; row Yq + 1 is staged */
-            weights(Yq + 1, buf ^ 1);
+        if (Yq < t1) stage(Yq + 1, buf ^ 1);         /* last read before the barrier that ended row Yq - 1 */
+        const bool reads = y < H && abs(Yq - y) <= P;                /* warp-uniform */
+        for (int t = 0; t < 3; ++t) produce(Yq, buf, t);
+        __syncthreads();
+        for (int k = 0; k < nc; ++k) {
+            if (k + 1 < nc) produce(Yq, buf, k + 3);
+            if (reads) consume(Yq, buf, k);
+            if (k + 1 == nc) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
             __syncthreads();
         }
-    }
-    if (!own) return;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        if (!((uok >> k) & 1u)) continue;
-        const int nn = k < 4 ? k : k + 1, ox = nn % 3 - 1, oy = nn / 3 - 1;
-        a.nbcost[(size_t)k * n + m - (size_t)(oy * W + ox)] = nb_final<EXACT>(a.k, fin, r1[k], r2[k], ws[k]);
+        for (int i = 0; i < SLOTS; ++i) X[i] += S1[i];
     }
+    if (y >= H) return;
+    /* the acceptance, in candidate order */
+    const float cx = (float)xc, cy = (float)yc, theta = a.theta;
+    const float4 smooth = smooth_at(a, o);
+    const bool inside = x < W;
+    float4 self = a.old[o];
+    TpBest eself = {self.w, state_distance(self, smooth, cx, cy, a.depthmax, a.lr), finite3(self)};
+    int win = 0;
+    auto accept = [&](float4 cand, float cost, int idx) {
+        cand.w = cost;
+        const TpBest e = {cost, state_distance(cand, smooth, cx, cy, a.depthmax, a.lr), finite3(cand)};
+        if (tp_accepts(e, eself, theta)) { self = cand; eself = e; win = idx; }
+    };
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+        const int nn = c < 4 ? c : c + 1;
+        accept(a.old[(size_t)clampi(yc + nn / 3 - 1, 0, H - 1) * W + clampi(xc + nn % 3 - 1, 0, W - 1)],
+               nb_final<EXACT>(a.k, true, r1[c], r2[c], ws[c]), 1 + c);
+    }
+    accept(smooth_state(smooth, cx, cy, a.lr), a.costs[o], 9);
+    seed_rng(rng, a, xc, yc, false);                 /* again: its state is not held over the sweep */
+#pragma unroll
+    for (int c = 0; c < 6; ++c) {
+        const int ox = (int)(rng_float(rng) * 7.0f + 0.5f);
+        const int oy = (int)(rng_float(rng) * 7.0f + 0.5f);
+        accept(a.old[(size_t)min(yc + oy, H - 1) * W + min(xc + ox, W - 1)],
+               nb_final<EXACT>(a.k, true, r1[8 + c], r2[8 + c], ws[8 + c]), 10 + c);
+    }
+    accept(state_init(rng, cx, cy, a.lr, 2.0f, a.depthmax), a.costs[n + o], 16);
+    int nview = 0;
+    if (a.viewin) {
+        const short4 l = a.viewin[o];
+        const short li[4] = {l.x, l.y, l.z, l.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (li[i] >= 0 && nview == i) {
+                accept(viewprop(a.viewsrc[(size_t)yc * W + li[i]]), a.costs[(size_t)(2 + i) * n + o], 17 + i);
+                nview = i + 1;
+            }
+    }
+    if (inside) {
+        a.out[o] = self;
+        if (a.winners) a.winners[o] = (uint8_t)win;
+    }
+    pass_counters(a, inside, x, y, 18 + nview);
 }
 
-/* A block of NB_COLS x NB_ROWS planes: interior blocks (their columns' windows
- * inside the image) share weights across rows (nbcost_block); the others
- * evaluate plane by plane (nbcost_lane). */
 template <bool EXACT>
-PM_DEV void nbcost_tile(const PmPassArgs& a, int tbx, int tby) {
-    const int W = a.k.W, H = a.k.H, P = a.k.P;
-    const int mx0 = tbx * NB_COLS, my0 = tby * NB_ROWS, lane = threadIdx.x, w = threadIdx.y;
-    if (mx0 - P - 1 >= 0 && mx0 + 31 + P + 1 <= W - 1) {   /* block-uniform */
-        nbcost_block<EXACT>(a, mx0, my0);
-        return;
-    }
-    const int mx = mx0 + lane, my = my0 + w - 1;
-    if (w < 1 || w > NB_ROWS || my >= H || lane >= NB_COLS || mx >= W) return;
-    nbcost_lane<EXACT>(a, mx, my);
-}
-
-template <bool EXACT>
-__global__ void __launch_bounds__(32 * NB_WARPS, PM_NB_MINB) k_nbcost(PmPassArgs a) {
-    nbcost_tile<EXACT>(a, blockIdx.x, blockIdx.y);
-}
+__global__ void __launch_bounds__(SH_NT, 1) k_share(PmPassArgs a) { share_tile<EXACT>(a, blockIdx.x, blockIdx.y); }
 
 /* ------------------------------------------------- tap-parallel passes -- */
 /* The propagation of images too small to fill the GPU with one thread per
@@ -882,29 +915,6 @@ PM_DEV float tp_costs(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, const Pm
     return nb_final<EXACT>(k, live_lane, r1, r2, ws);
 }
 
-/* The squared distance of a state to the smoothed field (pmhstereo.cl:266-283,
- * one side of smooth_distance). */
-PM_DEV float state_distance(float4 s, float4 smooth, float cx, float cy, float depthmax, int lr) {
-    const float4 diag = f4(1.0f, 1.0f, 0.0f, 1.0f / (depthmax * depthmax));
-    const float4 d = to_ref_normal_depth(s, cx, cy, lr) - smooth;
-    return dot4(d, diag * d);
-}
-/* The acceptance rule of a propagation pass, from costs and distances formed
- * beforehand: a state that is not finite makes both distances 0. */
-struct TpBest { float cost, dist; bool fin; };
-PM_DEV bool tp_accepts(const TpBest& cand, const TpBest& self, float theta) {
-    const bool fin = cand.fin && self.fin;
-    return cand.cost + theta * (fin ? cand.dist : 0.0f) <= self.cost + theta * (fin ? self.dist : 0.0f);
-}
-
-/* The smoothed plane's normal and depth at a pixel (:320-323) */
-PM_DEV float4 smooth_at(const PmPassArgs& a, size_t o) {
-    const float4 sm = a.smooth[o];
-    const float nf = fmaxf(pm_sqrt(sm.x * sm.x + sm.y * sm.y) + 0.001f, 1.0f);
-    const float smx = sm.x / nf, smy = sm.y / nf;
-    return f4(smx, smy, pm_sqrt(1.0f - smx * smx - smy * smy), sm.z * a.depthmax);
-}
-
 #define TP_K 8
 #define TP_CH 16       /* taps per chunk of the candidate kernel */
 #define TP_CH1 64      /* taps per chunk of the one-candidate kernels */
@@ -928,10 +938,7 @@ __global__ void __launch_bounds__(32 * TP_NP, 2) k_taps_candidates(PmPassArgs a)
         s = a.old[(size_t)clampi(y + nn / 3 - 1, 0, H - 1) * W + clampi(x + nn % 3 - 1, 0, W - 1)];
     } else if (z == 1) {
         if (c == 0) {                                /* :345-352 */
-            const float4 sm = smooth_at(a, o);
-            const float4 sc = f4(1.0f - (-sm.x / sm.z), 0.0f - (-sm.y / sm.z),
-                                 0.0f - ((sm.x * cx + sm.y * cy) / sm.z + sm.w), 0.0f - 0.0f);
-            s = a.lr ? sc : viewprop(sc);
+            s = smooth_state(smooth_at(a, o), cx, cy, a.lr);
         } else {
             PmRng rng;
             seed_rng(rng, a, x, y, false);
@@ -1049,24 +1056,7 @@ __global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_refine(PmPassArgs 
         a.out[o] = self;
         if (a.winners && win >= 0) a.winners[o] = (uint8_t)win;
     }
-    if (MODE == 1 && owner && a.counters) {
-        /* evaluations = 18 + view candidates; taps = in-image window taps */
-        unsigned long long ev = 0, taps = 0;
-        if (inside) {
-            const int P = a.k.P;
-            ev = 18ull + (unsigned long long)nview;
-            taps = ev * (unsigned long long)((min(x + P, W - 1) - max(x - P, 0) + 1) * (min(y + P, H - 1) - max(y - P, 0) + 1));
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            ev += __shfl_down_sync(0xffffffffu, ev, off);
-            taps += __shfl_down_sync(0xffffffffu, taps, off);
-        }
-        if (lane == 0) {
-            atomicAdd(&a.counters[0], ev);
-            atomicAdd(&a.counters[1], taps);
-        }
-    }
+    if (MODE == 1 && owner) pass_counters(a, inside, x, y, 18 + nview);
 }
 
 template <bool EXACT> constexpr size_t tp_cand_smem() { return sizeof(TpShared<EXACT, TP_K, TP_CH>); }
@@ -1730,10 +1720,19 @@ __global__ void __launch_bounds__(256) kb_init(const __grid_constant__ PmBatch<P
 }
 
 template <bool EXACT>
-__global__ void __launch_bounds__(32 * NB_WARPS, PM_NB_MINB) kb_nbcost(const __grid_constant__ PmBatch<PmPassArgs> b) {
+__global__ void __launch_bounds__(256, 2) kb_sweep(const __grid_constant__ PmBatch<PmPassArgs> b) {
     for (int item = blockIdx.x; item < b.first[b.n]; item += gridDim.x) {
         const int p = batch_pair(b, item), t = item - b.first[p];
-        nbcost_tile<EXACT>(b.a[p], t % b.tx[p], t / b.tx[p]);
+        sweep_tile<EXACT>(b.a[p], t % b.tx[p], t / b.tx[p]);
+    }
+}
+
+template <bool EXACT>
+__global__ void __launch_bounds__(SH_NT, 1) kb_share(const __grid_constant__ PmBatch<PmPassArgs> b) {
+    for (int item = blockIdx.x; item < b.first[b.n]; item += gridDim.x) {
+        const int p = batch_pair(b, item), t = item - b.first[p];
+        __syncthreads();                                 /* the rings are reused */
+        share_tile<EXACT>(b.a[p], t % b.tx[p], t / b.tx[p]);
     }
 }
 
@@ -1851,7 +1850,7 @@ cudaError_t pm_launch_cost_field(const PmPassArgs& a, bool exact, const float4* 
 cudaError_t pm_launch_propagate(const PmPassArgs& a, bool exact, cudaStream_t st) {
     const dim3 grid = a.color < 0 ? pix_grid(a.k.W, a.k.H) : pix_grid((a.k.W + 1) / 2, a.k.H);
     PmPassArgs b = a;
-    if (b.color >= 0) b.nbcost = nullptr, b.cand = nullptr;   /* red/black: neighbours per pixel */
+    if (b.color >= 0) b.costs = nullptr, b.cand = nullptr;   /* red/black: every candidate by pixel */
     if (b.cand) {
         const dim3 g = tap_grid(b, b.viewin ? 3 : 2);
         if (exact) k_taps_candidates<true><<<g, dim3(32, TP_NP), tp_cand_smem<true>(), st>>>(b);
@@ -1862,12 +1861,24 @@ cudaError_t pm_launch_propagate(const PmPassArgs& a, bool exact, cudaStream_t st
         PM_LAUNCH_CHECK();
         return cudaSuccess;
     }
-    const dim3 nbgrid((a.k.W + NB_COLS - 1) / NB_COLS, (a.k.H + NB_ROWS - 1) / NB_ROWS);
-    if (b.nbcost) {
-        const size_t smem = nb_block_smem(a.k.P);
-        if (exact) k_nbcost<true><<<nbgrid, dim3(32, NB_WARPS), smem, st>>>(b);
-        else k_nbcost<false><<<nbgrid, dim3(32, NB_WARPS), smem, st>>>(b);
+    if (b.costs) {
+        const dim3 sg((a.k.W + 31) / 32, (a.k.H + SH_TY - 1) / SH_TY);
+        const size_t smem = share_smem(a.k.P);
+        if (exact) {
+            k_sweep<true><<<grid, dim3(32, 8), 0, st>>>(b);
+            PM_LAUNCH_CHECK();
+            k_share<true><<<sg, dim3(32, SH_TY), smem, st>>>(b);
+            PM_LAUNCH_CHECK();
+            k_propagate<true, 2><<<grid, dim3(32, 8), 0, st>>>(b);
+        } else {
+            k_sweep<false><<<grid, dim3(32, 8), 0, st>>>(b);
+            PM_LAUNCH_CHECK();
+            k_share<false><<<sg, dim3(32, SH_TY), smem, st>>>(b);
+            PM_LAUNCH_CHECK();
+            k_propagate<false, 2><<<grid, dim3(32, 8), 0, st>>>(b);
+        }
         PM_LAUNCH_CHECK();
+        return cudaSuccess;
     }
 #if PM_PROP_SPLIT
     if (exact) k_propagate<true, 1><<<grid, dim3(32, 8), 0, st>>>(b);
@@ -1952,9 +1963,10 @@ cudaError_t pm_prepare_kernels() {
 #ifndef TP_MAX_PIXELS
 #define TP_MAX_PIXELS 60000
 #endif
-bool pm_tap_parallel(const PmCostConsts& k) {
-    return (size_t)k.W * k.H <= TP_MAX_PIXELS && std::isfinite(k.alpha) && std::isfinite(k.cmax) && std::isfinite(k.gmax);
+bool pm_shared_windows(const PmCostConsts& k) {
+    return std::isfinite(k.alpha) && std::isfinite(k.cmax) && std::isfinite(k.gmax);
 }
+bool pm_tap_parallel(const PmCostConsts& k) { return (size_t)k.W * k.H <= TP_MAX_PIXELS && pm_shared_windows(k); }
 size_t pm_tap_parallel_bytes(int W, int H) { return (size_t)20 * W * H * sizeof(float4); }
 
 cudaError_t pm_launch_pd_block(float4* uout, float* pout, const float4* uin, const float* pin, int pzero,
@@ -2019,7 +2031,7 @@ void pm_batch_tiles(PmBatchKernel k, int W, int H, const PmBatchKnobs& kn, int* 
     case PMB_PREP: x = (W + PREP_T - 1) / PREP_T; y = (H + PREP_T - 1) / PREP_T; break;
     case PMB_RECORDS: x = (W + 127) / 128; y = H; break;
     case PMB_PIXEL: x = (W + 31) / 32; y = (H + 7) / 8; break;
-    case PMB_NBCOST: x = (W + NB_COLS - 1) / NB_COLS; y = (H + NB_ROWS - 1) / NB_ROWS; break;
+    case PMB_SHARE: x = (W + 31) / 32; y = (H + SH_TY - 1) / SH_TY; break;
     case PMB_ROW: x = 1; y = H; break;
     case PMB_PD: {
         const int rows = kn.pd_rows == 8 ? 8 : 16;
@@ -2072,10 +2084,18 @@ cudaError_t pm_batch_init(const PmBatch<PmPassArgs>& b, bool exact, const PmBatc
     if (exact) PM_BATCH_LAUNCH(kb_init<true>, dim3(32, 8), 0);
     PM_BATCH_LAUNCH(kb_init<false>, dim3(32, 8), 0);
 }
-cudaError_t pm_batch_nbcost(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st) {
-    const size_t smem = nb_block_smem(b.a[0].k.P);           /* one window size per batch */
-    if (exact) PM_BATCH_LAUNCH(kb_nbcost<true>, dim3(32, NB_WARPS), smem);
-    PM_BATCH_LAUNCH(kb_nbcost<false>, dim3(32, NB_WARPS), smem);
+cudaError_t pm_batch_sweep(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st) {
+    if (exact) PM_BATCH_LAUNCH(kb_sweep<true>, dim3(32, 8), 0);
+    PM_BATCH_LAUNCH(kb_sweep<false>, dim3(32, 8), 0);
+}
+cudaError_t pm_batch_share(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st) {
+    const size_t smem = share_smem(b.a[0].k.P);              /* one window size per batch */
+    if (exact) PM_BATCH_LAUNCH(kb_share<true>, dim3(32, SH_TY), smem);
+    PM_BATCH_LAUNCH(kb_share<false>, dim3(32, SH_TY), smem);
+}
+cudaError_t pm_batch_refine(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st) {
+    if (exact) PM_BATCH_LAUNCH((kb_propagate<true, 2>), dim3(32, 8), 0);
+    PM_BATCH_LAUNCH((kb_propagate<false, 2>), dim3(32, 8), 0);
 }
 cudaError_t pm_batch_propagate(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st) {
 #if PM_PROP_SPLIT
@@ -2132,11 +2152,11 @@ cudaError_t pm_batch_pd(const PmBatch<PmPdArgs>& b, const PmBatchKnobs& kn, cuda
 }
 cudaError_t pm_batch_prepare_kernels() {
     cudaError_t e;
-    const int nbmax = (int)nb_block_smem(PM_PMAX);
-    if ((e = cudaFuncSetAttribute(k_nbcost<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, nbmax)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_nbcost<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, nbmax)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(kb_nbcost<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, nbmax)) != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(kb_nbcost<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, nbmax)) != cudaSuccess) return e;
+    const int shmax = (int)share_smem(PM_PMAX);
+    if ((e = cudaFuncSetAttribute(k_share<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, shmax)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_share<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, shmax)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(kb_share<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, shmax)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(kb_share<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, shmax)) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(kb_pd_block<8, 3, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)pds_smem(false, 8, 3))) != cudaSuccess) return e;
     if ((e = cudaFuncSetAttribute(kb_pd_block<8, 2, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -25,7 +25,7 @@ struct PmPassArgs {
     float4* out;
     uint8_t* winners;
     unsigned long long* counters;   /* [0] cost evaluations, [1] in-image taps; may be NULL */
-    float* nbcost;             /* FAST: costs of candidates 1-8 by shared windows, [8][W*H], or NULL */
+    float* costs;              /* shared windows: the costs of candidates 9, 16, 17-20, [PM_COST_PLANES][W*H], or NULL */
     float4* cand;              /* tap-parallel passes: states and costs of candidates 1-20, [20][W*H], or NULL */
     int color;                 /* -1: every pixel (Jacobi); 0 / 1: pixels with (x + y) & 1 == color */
 };
@@ -72,13 +72,17 @@ struct PmBatchKnobs {
 };
 
 /* Tile geometry of each batched kernel (items per pair = tiles). */
-enum PmBatchKernel { PMB_PREP, PMB_RECORDS, PMB_PIXEL, PMB_NBCOST, PMB_ROW, PMB_PD };
+enum PmBatchKernel { PMB_PREP, PMB_RECORDS, PMB_PIXEL, PMB_SHARE, PMB_ROW, PMB_PD };
 void pm_batch_tiles(PmBatchKernel k, int W, int H, const PmBatchKnobs& kn, int* tx, int* tiles);
 
 cudaError_t pm_batch_prep(const PmBatch<PmPrepArgs>& b, const PmBatchKnobs& kn, cudaStream_t st);
 cudaError_t pm_batch_records(const PmBatch<PmRecArgs>& b, const PmBatchKnobs& kn, cudaStream_t st);
 cudaError_t pm_batch_init(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
-cudaError_t pm_batch_nbcost(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
+/* A propagation pass of pairs with PmPassArgs::costs: sweep, share, refine; of
+ * the others: propagate. */
+cudaError_t pm_batch_sweep(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
+cudaError_t pm_batch_share(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
+cudaError_t pm_batch_refine(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
 cudaError_t pm_batch_propagate(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
 cudaError_t pm_batch_view_list(const PmBatch<PmViewListArgs>& b, int maxW, const PmBatchKnobs& kn, cudaStream_t st);
 cudaError_t pm_batch_consistency(const PmBatch<PmConsArgs>& b, const PmBatchKnobs& kn, cudaStream_t st);
@@ -118,6 +122,10 @@ cudaError_t pm_launch_normal_depth(const float4* in, int W, int H, float depthma
  * call once per device before the first launch or stream capture. */
 cudaError_t pm_prepare_kernels();
 
+#define PM_COST_PLANES 6
+/* Whether passes of these constants can share plane windows, given
+ * PmPassArgs::costs. */
+bool pm_shared_windows(const PmCostConsts& k);
 /* Whether passes of these constants run tap-parallel (small images), given
  * PmPassArgs::cand of pm_tap_parallel_bytes. */
 bool pm_tap_parallel(const PmCostConsts& k);

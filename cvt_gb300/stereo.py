@@ -331,9 +331,9 @@ class PMHuberStereo:
         return cost
 
     def set_memory_budget(self, nbytes: int) -> None:
-        """Device bytes the FAST path may use for its shared-window neighbour
-        costs, 32 per pixel (0: evaluate neighbours per pixel; results are the
-        same)."""
+        """Device bytes a propagation pass may use to share work between its
+        candidates: 24 per pixel, 320 for images of at most 60000 pixels (0:
+        every candidate per pixel; results are the same)."""
         self._check(_lib.lib().cvtpm_set_memory_budget(self._h, int(nbytes)))
 
     def cost_adjoint(self, img1: torch.Tensor, img2: torch.Tensor, planes: torch.Tensor, lr: int = 1,

@@ -268,13 +268,14 @@ cvtpm_status cvtpm_polish_planes(cvtpm_ctx* ctx, const float* img1, const float*
                                  float* planes, int lr, int steps, float* cost,
                                  void* stream);
 
-/* Device memory the context may use for the propagation's shared-window
- * neighbour costs (FAST and EXACT): 32 bytes per pixel (the costs of the 8 neighbour
- * candidates).  Within the budget (and 60 % of the free memory) the 8
- * neighbour candidates of a pass are evaluated once per plane over the union
- * of their windows; otherwise per pixel.  Results are identical either way.
- * Default: no limit; 0 turns the shared windows off.  No counterpart in the
- * reference. */
+/* Device memory the context may use to share work between the candidates of
+ * a propagation pass (FAST and EXACT).  With 24 bytes per pixel, planes that
+ * several pixels test (the neighbour and random-neighbour candidates) have
+ * their matching terms formed once per plane; images of at most 60000 pixels
+ * use 320 bytes per pixel instead, to run every candidate's window taps in
+ * parallel.  Otherwise (and beyond 60 % of the free memory) every candidate is
+ * evaluated per pixel.  Results are identical either way.  Default: no limit;
+ * 0 turns both off.  No counterpart in the reference. */
 cvtpm_status cvtpm_set_memory_budget(cvtpm_ctx* ctx, size_t bytes);
 
 /* Enable CUDA-event timing of the propagation and PD phases (on the call's
@@ -312,8 +313,8 @@ cvtpm_status cvtpm_cost_eval_noalloc(const cvtpm_params* params,
  * trace are not produced).
  *
  * Default (lane count 0, Jacobi schedule): phase-batched.  Every phase of
- * the depthMap schedule (prep, init, per iteration the neighbour costs,
- * propagation and view lists of each view, the consistency checks, fills
+ * the depthMap schedule (prep, init, per iteration the propagation stages
+ * and view lists of each view, the consistency checks, fills
  * and PD smoother steps, the final fill) is ONE launch covering all pairs:
  * persistent blocks walk a flat list of (pair, tile) work items, with the
  * pairs' arguments in the kernel parameter (up to 64 pairs per launch).  So
@@ -340,7 +341,7 @@ cvtpm_status cvtpm_depthmap_batched(cvtpm_ctx* ctx, const cvtpm_pair* pairs,
 #define CVTPM_BATCH_MAX_CAND 16
 typedef struct cvtpm_batch_info {
     int lanes;                 /* lanes of the current graph (0: phase-batched) */
-    int shared_windows;        /* shared-window neighbour costs in use for every pair */
+    int shared_windows;        /* shared plane windows in use for every pair */
     int tuned;                 /* 1 if the autotuner ran for the current graph */
     int ncand;
     int cand_lanes[CVTPM_BATCH_MAX_CAND];     /* lane count of a lane candidate, 0 for a phase-batched one */
