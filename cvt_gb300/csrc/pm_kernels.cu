@@ -276,14 +276,26 @@ PM_DEV void propagate_tile(const PmPassArgs& a, int tbx, int tby) {
             else if (nmax == 4) sweep(std::integral_constant<int, 4>());
         }
     }
-    /* 21-22: random refinements of the current best (:383-389) */
+    /* 21-22: random refinements of the current best (:383-389).  The right
+     * view's (:114-115) does not depend on its draws: after a rejection the
+     * second is the rejected one again, and a warp of such pixels skips it. */
+    float4 last = f4s(0.0f);
+    bool rejected = false;
 #pragma unroll 1
     for (int i = 0; i < ((STAGE == 0 || STAGE == 2) ? 2 : 0); ++i) {
         float4 s[1] = {state_refine(rng, self, cx, cy, dmax, lr)};
-        bool act[1] = {true};
+        bool act[1] = {!(rejected && s[0].x == last.x && s[0].y == last.y && s[0].z == last.z)};
+        if (!__any_sync(0xffffffffu, act[0])) continue;
         float c[1];
         eval_costs<1, EXACT>(a.k, a.v1, a.v2, xc, yc, s, act, c);
-        accept(s[0], c[0], 21 + i);
+        if (act[0]) {
+            const int before = win;
+            win = -2;
+            accept(s[0], c[0], 21 + i);
+            rejected = win == -2;
+            if (rejected) win = before;
+            last = s[0];
+        }
     }
     if (inside) {
         a.out[o] = self;
@@ -486,7 +498,8 @@ PM_DEV void pass_counters(const PmPassArgs& a, bool inside, int x, int y, int ne
  * the acceptance, where the neighbours by plane (5.9 ms, weights in a table
  * per block) and the random neighbours by pixel (12.1 of the 16.2 ms of a
  * sweep of 8) took 18; depthMap 484.7 -> 363.7 ms, 640x480 x 3 iterations
- * 132 -> 96.3, EXACT 450x375 102 -> 73.4 ms.
+ * 132 -> 96.3, EXACT 450x375 102 -> 73.4 ms.  With a thread's slots in one
+ * column, sharing their image-1 reads: 9.2 ms.
  */
 #define SH_TY 16
 #define SH_NX 40
@@ -558,6 +571,7 @@ PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
     typedef typename ShTerm<EXACT>::type Term;
     constexpr int R = ShTerm<EXACT>::R;
     constexpr int SLOTS = (SH_NS + SH_NT - 1) / SH_NT;
+    static_assert(SH_NY % SLOTS == 0 && SH_NS / SLOTS <= SH_NT, "a thread's slots share a column");
     extern __shared__ __align__(16) unsigned char sh_smem[];
     Term* const ring = reinterpret_cast<Term*>(sh_smem);             /* [SH_NS][R] */
     float4* const rows = reinterpret_cast<float4*>(sh_smem + (size_t)SH_NS * 128);
@@ -565,21 +579,23 @@ PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
     const int lane = threadIdx.x, w = threadIdx.y, tid = w * 32 + lane;
     const int x0 = tbx * 32, y0 = tby * SH_TY;
     const size_t n = (size_t)W * H;
-    /* plane role: slots tid, tid + SH_NT */
-    int smx[SLOTS], slo[SLOTS], shi[SLOTS];          /* nominal column; image rows the slot is needed at */
+    /* plane role: SLOTS slots of one column, SH_NY / SLOTS rows apart, whose
+     * taps share the image-1 reads */
+    const int pcol = tid % SH_NX, prow0 = tid / SH_NX;
+    const bool plane = prow0 < SH_NY / SLOTS;
+    const int mx = x0 - 1 + pcol;
+    int slo[SLOTS], shi[SLOTS];                      /* image rows the slot is needed at */
     long long S0[SLOTS], S1[SLOTS], X[SLOTS];
     float sx[SLOTS], sy[SLOTS], sz[SLOTS];
     const int t0 = max(y0 - P, 0), t1 = min(min(y0 + SH_TY - 1, H - 1) + P, H - 1);
 #pragma unroll
     for (int i = 0; i < SLOTS; ++i) {
-        const int s = tid + i * SH_NT;
-        const int mx = x0 - 1 + s % SH_NX, my = y0 - 1 + s / SH_NX;
+        const int my = y0 - 1 + prow0 + i * (SH_NY / SLOTS);
         const float4 st = a.old[(size_t)clampi(my, 0, H - 1) * W + clampi(mx, 0, W - 1)];
         long long XA;
         nb_plane<EXACT>(a.k, st, finite3(st), sx[i], sy[i], sz[i], S0[i], S1[i], XA);
-        smx[i] = mx;
         slo[i] = max(y0, my - 7) - P;
-        shi[i] = s < SH_NS ? min(min(y0 + SH_TY - 1, H - 1), my + 1) + P : -1;
+        shi[i] = plane ? min(min(y0 + SH_TY - 1, H - 1), my + 1) + P : -1;
         /* the position at column mx - P - 7, row t0 */
         X[i] = XA + (long long)(t0 - H / 2) * S1[i] + (long long)(mx - P - 7 - W / 2) * S0[i];
     }
@@ -614,25 +630,36 @@ PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
         const float4* s_col = rows + buf * 2 * NQ;
         const float4* s_grad = s_col + NQ;
         const PmRecRow rrow = rec_row(a.v2, a.k.rp, Yq);
+        const int q0 = mx - P - 7 + SH_B * t;
+        long long Xt[SLOTS];
+        bool need[SLOTS];
+        bool any = false;
 #pragma unroll
         for (int i = 0; i < SLOTS; ++i) {
-            if (Yq < slo[i] || Yq > shi[i]) continue;
-            const int q0 = smx[i] - P - 7 + SH_B * t;
-            Term* const dst = ring + (size_t)(tid + i * SH_NT) * R;
-            long long Xt = X[i] + (long long)(SH_B * t) * S0[i];
+            Xt[i] = X[i] + (long long)(SH_B * t) * S0[i];
+            need[i] = Yq >= slo[i] && Yq <= shi[i];
+            any = any || need[i];
+        }
+        if (!any) return;
 #pragma unroll
-            for (int b = 0; b < SH_B; ++b) {
-                const int q = q0 + b, qs = q - (x0 - P);
-                const long long Xb = Xt;
-                Xt += S0[i];
-                if ((unsigned)qs >= (unsigned)NQ) continue;          /* no pixel of the tile reads it */
-                float cc = 0.0f, gc = 0.0f;
-                bool ok = q >= 0 && q < W;
-                if (ok) ok = nb_tap_terms<EXACT>(a.k, a.v2, q, Yq, rrow, sx[i], sy[i], sz[i], Xb, s_col[qs], s_grad[qs], cc, gc);
-                if (!ok) cc = __int_as_float(0x7fc00000);
-                if constexpr (EXACT) dst[q & (R - 1)] = cc;
-                else dst[q & (R - 1)] = make_float2(cc, gc);
+        for (int b = 0; b < SH_B; ++b) {
+            const int q = q0 + b, qs = q - (x0 - P);
+            if ((unsigned)qs < (unsigned)NQ) {       /* else no pixel of the tile reads it */
+                const float4 a1 = s_col[qs], g1 = s_grad[qs];
+                Term* const dst = ring + (size_t)tid * R + (q & (R - 1));
+#pragma unroll
+                for (int i = 0; i < SLOTS; ++i) {
+                    if (!need[i]) continue;
+                    float cc = 0.0f, gc = 0.0f;
+                    bool ok = q >= 0 && q < W;
+                    if (ok) ok = nb_tap_terms<EXACT>(a.k, a.v2, q, Yq, rrow, sx[i], sy[i], sz[i], Xt[i], a1, g1, cc, gc);
+                    if (!ok) cc = __int_as_float(0x7fc00000);
+                    if constexpr (EXACT) dst[i * (SH_NS / SLOTS) * R] = cc;
+                    else dst[i * (SH_NS / SLOTS) * R] = make_float2(cc, gc);
+                }
             }
+#pragma unroll
+            for (int i = 0; i < SLOTS; ++i) Xt[i] += S0[i];
         }
     };
     auto fold = [&](int c, Term t, float wt) {
