@@ -231,7 +231,7 @@ cvtpm_status ensure_buffers(cvtpm_ctx* ctx, int W, int H) {
         add((void**)&ctx->S[v][0], n * 16);
         add((void**)&ctx->S[v][1], n * 16);
         add((void**)&ctx->smooth[v], n * 16);
-        add((void**)&ctx->list[v], n * 8);
+        add((void**)&ctx->list[v], view_list_bytes(W, H));
         add((void**)&ctx->win[v], n);
         add((void**)&ctx->pdP[v], pd);
     }
@@ -286,6 +286,12 @@ cvtpm_status check_image(cvtpm_ctx* ctx, const void* p, int W, int H, size_t pit
     if (pitch % 16 != 0 || pitch < (size_t)W * 16) return fail(ctx, CVTPM_ERR_INVALID_ARGUMENT, std::string(what) + " pitch must be a multiple of 16 and >= 16*width");
     if (((uintptr_t)p & 15) != 0) return fail(ctx, CVTPM_ERR_INVALID_ARGUMENT, std::string(what) + " must be 16-byte aligned");
     return CVTPM_OK;
+}
+
+/* An empty view list: no sources, no entries. */
+cudaError_t clear_view_list(short4* list, int W, int H, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(list, 0xFF, (size_t)W * H * 8, st);
+    return e != cudaSuccess ? e : cudaMemsetAsync(view_counts(list, W, H), 0, (size_t)H * 4, st);
 }
 
 PmPassArgs base_args(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H, int v1) {
@@ -514,7 +520,7 @@ cvtpm_status run_depthmap(cvtpm_ctx* ctx, const cvtpm_params& p, float* dmap, si
         LK(pm_launch_init(aR, exact, st), "init");
         CK(cudaMemsetAsync(ctx->smooth[0], 0, n * 16, st), "clear");   /* :108-113 */
         CK(cudaMemsetAsync(ctx->smooth[1], 0, n * 16, st), "clear");
-        CK(cudaMemsetAsync(ctx->list[1], 0xFF, n * 8, st), "clear");   /* :145-149 */
+        CK(clear_view_list(ctx->list[1], W, H, st), "clear");   /* :145-149 */
     } else {
         /* the state before iteration `first`: both views' planes and smoothed
          * fields; the left pass's view list is the one the right view's
@@ -527,7 +533,7 @@ cvtpm_status run_depthmap(cvtpm_ctx* ctx, const cvtpm_params& p, float* dmap, si
             CK(cudaMemcpyAsync(ctx->smooth[v], resume->smooth + (size_t)v * 4 * n, n * 16, cudaMemcpyDeviceToDevice, st),
                "resume");
         }
-        if (first == 0) CK(cudaMemsetAsync(ctx->list[1], 0xFF, n * 8, st), "clear");
+        if (first == 0) CK(clear_view_list(ctx->list[1], W, H, st), "clear");
         else LK(pm_launch_view_list(ctx->S[1][sw0], W, H, ctx->list[1], st), "view list");
     }
 
@@ -651,7 +657,7 @@ cvtpm_status run_depthmap_inpaint(cvtpm_ctx* ctx, const cvtpm_params& p, float* 
     LK(pm_launch_init(aR, exact, st), "init");
     CK(cudaMemsetAsync(ctx->smooth[0], 0, n * 16, st), "clear");   /* :330-336 */
     CK(cudaMemsetAsync(ctx->smooth[1], 0, n * 16, st), "clear");
-    CK(cudaMemsetAsync(ctx->list[1], 0xFF, n * 8, st), "clear");   /* :365-369 */
+    CK(clear_view_list(ctx->list[1], W, H, st), "clear");   /* :365-369 */
     float theta = 0.0f;
     for (int iter = 0; iter < N; ++iter) {                         /* :371-483 */
         const int sw = iter & 1;
@@ -1403,7 +1409,7 @@ cvtpm_status phase_start(PhaseState& S) {
         const size_t npx = (size_t)S.pairs[i].width * S.pairs[i].height;
         CK(cudaMemsetAsync(c->smooth[0], 0, npx * 16, S.st), "clear");
         CK(cudaMemsetAsync(c->smooth[1], 0, npx * 16, S.st), "clear");
-        CK(cudaMemsetAsync(c->list[1], 0xFF, npx * 8, S.st), "clear");
+        CK(clear_view_list(c->list[1], S.pairs[i].width, S.pairs[i].height, S.st), "clear");
     }
     return CVTPM_OK;
 }
@@ -1425,6 +1431,7 @@ cvtpm_status phase_propagate(PhaseState& S, std::vector<PmPassArgs>& args, short
             }, [&](const PmBatch<PmPassArgs>& b) { return launch(b, exact, S.kn, S.st); }, what, &S.launches);
     };
     if ((s = phase(shared, PMB_PIXEL, pm_batch_sweep, "batched sweep")) != CVTPM_OK ||
+        (s = phase(shared, PMB_PIXEL, pm_batch_views, "batched view candidates")) != CVTPM_OK ||
         (s = phase(shared, PMB_SHARE, pm_batch_share, "batched shared windows")) != CVTPM_OK ||
         (s = phase(shared, PMB_PIXEL, pm_batch_refine, "batched refinement")) != CVTPM_OK ||
         (s = phase(plain, PMB_PIXEL, pm_batch_propagate, "batched propagate")) != CVTPM_OK)

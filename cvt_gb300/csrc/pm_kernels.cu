@@ -6,7 +6,7 @@
  *  k_records            (fast arithmetic only) value/forward-difference records of a view
  *  k_init<EXACT>        pmhstereo_init (:230-248)
  *  k_sweep, k_share<EXACT>, k_propagate<EXACT, 2>  pmhstereo_propagate_view (:286-404) without the
- *                       scatter: candidates 9, 16-20 by pixel; 1-8, 10-15 by plane and the
+ *                       scatter: candidates 9, 16 (k_sweep) and 17-20 (k_views) by pixel; 1-8, 10-15 by plane and the
  *                       acceptance; the refinements 21, 22
  *  k_propagate<EXACT, *>  the same with every candidate by pixel
  *  k_taps_*<EXACT>      init and propagate for small images, the taps of a window in parallel
@@ -515,53 +515,54 @@ __host__ __device__ constexpr size_t share_smem(int P) {
     return (size_t)SH_NS * 128 + 2 * (size_t)(32 + 2 * P) * 32;
 }
 
-/* Candidates 9, 16 and the other view's 17-20, which share no plane with
- * another pixel: one sweep of as many as the warp's fullest list holds.  Their
- * costs go to a.costs[0], [1] and [2 + i]. */
+/* Candidates 9 and 16, which share no plane with another pixel, in one sweep:
+ * their costs go to a.costs[0] and [1]. */
 template <bool EXACT>
 PM_DEV void sweep_tile(const PmPassArgs& a, int tbx, int tby) {
     const int W = a.k.W, H = a.k.H;
     const int x = tbx * 32 + threadIdx.x, y = tby * 8 + threadIdx.y;
-    const bool inside = x < W && y < H;
-    const int xc = min(x, W - 1), yc = min(y, H - 1);   /* lanes outside still follow the warp */
-    const float cx = (float)xc, cy = (float)yc;
-    const size_t n = (size_t)W * H, o = (size_t)yc * W + xc;
-    const float4 s9 = smooth_state(smooth_at(a, o), cx, cy, a.lr);
+    if (x >= W || y >= H) return;
+    const float cx = (float)x, cy = (float)y;
+    const size_t o = (size_t)y * W + x;
     PmRng rng;
-    seed_rng(rng, a, xc, yc, false);
+    seed_rng(rng, a, x, y, false);
 #pragma unroll 1
     for (int i = 0; i < 12; ++i) (void)rng_float(rng);       /* the random neighbours' offsets */
-    const float4 s16 = state_init(rng, cx, cy, a.lr, 2.0f, a.depthmax);
-    short4 l = make_short4(-1, -1, -1, -1);
-    if (a.viewin && inside) l = a.viewin[o];
-    const short li[4] = {l.x, l.y, l.z, l.w};
-    const int nview = (li[0] < 0) ? 0 : (li[1] < 0) ? 1 : (li[2] < 0) ? 2 : (li[3] < 0) ? 3 : 4;
-    auto sweep = [&](auto m) {
-        constexpr int M = decltype(m)::value;
-        float4 s[2 + M]; bool act[2 + M]; float c[2 + M];
-        s[0] = s9; act[0] = true;
-        s[1] = s16; act[1] = true;
-#pragma unroll
-        for (int i = 0; i < M; ++i) {
-            act[2 + i] = i < nview;
-            s[2 + i] = act[2 + i] ? viewprop(a.viewsrc[(size_t)yc * W + li[i]]) : f4s(0.0f);
-        }
-        eval_costs<2 + M, EXACT>(a.k, a.v1, a.v2, xc, yc, s, act, c);
-        if (inside) {
-#pragma unroll
-            for (int i = 0; i < 2 + M; ++i) a.costs[(size_t)i * n + o] = c[i];
-        }
-    };
-    const int nmax = __reduce_max_sync(0xffffffffu, (unsigned)nview);
-    if (nmax == 0) sweep(std::integral_constant<int, 0>());
-    else if (nmax == 1) sweep(std::integral_constant<int, 1>());
-    else if (nmax == 2) sweep(std::integral_constant<int, 2>());
-    else if (nmax == 3) sweep(std::integral_constant<int, 3>());
-    else sweep(std::integral_constant<int, 4>());
+    float4 s[2] = {smooth_state(smooth_at(a, o), cx, cy, a.lr), state_init(rng, cx, cy, a.lr, 2.0f, a.depthmax)};
+    bool act[2] = {true, true};
+    float c[2];
+    eval_costs<2, EXACT>(a.k, a.v1, a.v2, x, y, s, act, c);
+    a.costs[o] = c[0];
+    a.costs[(size_t)W * H + o] = c[1];
 }
 
 template <bool EXACT>
 __global__ void __launch_bounds__(256, 2) k_sweep(PmPassArgs a) { sweep_tile<EXACT>(a, blockIdx.x, blockIdx.y); }
+
+/* The other view's candidates 17-20: entry i of a pixel's list goes to
+ * a.costs[2 + i].  A pixel has 0 to 4 of them, about one on average, so a warp
+ * that followed its pixels would sweep as often as its fullest list; the
+ * threads follow the row's entries (view_entries) instead, each taking one
+ * (1242x375, per pass: 2.2 ms, where a sweep by pixel, joined to that of 9 and
+ * 16, cost 3.4 and the entries of a 32x8 tile taken by its threads 2.7). */
+template <bool EXACT>
+PM_DEV void views_tile(const PmPassArgs& a, int tbx, int tby) {
+    const int W = a.k.W, H = a.k.H, t = tbx * 32 + threadIdx.x, y = tby * 8 + threadIdx.y;
+    if (y >= H || t >= view_counts(a.viewin, W, H)[y]) return;
+    const unsigned e = view_entries(a.viewin, W, H)[(size_t)y * W + t];
+    const int x = e & 16383u, i = e >> 14;
+    const size_t o = (size_t)y * W + x;
+    const short4 l = a.viewin[o];
+    const short src = i == 0 ? l.x : i == 1 ? l.y : i == 2 ? l.z : l.w;
+    float4 s[1] = {viewprop(a.viewsrc[(size_t)y * W + src])};
+    bool act[1] = {true};
+    float c[1];
+    eval_costs<1, EXACT>(a.k, a.v1, a.v2, x, y, s, act, c);
+    a.costs[(size_t)(2 + i) * W * H + o] = c[0];
+}
+
+template <bool EXACT>
+__global__ void __launch_bounds__(256, 3) k_views(PmPassArgs a) { views_tile<EXACT>(a, blockIdx.x, blockIdx.y); }
 
 /* The candidates 1-16 and the view candidates of a pixel against its old
  * state: 9, 16 and 17-20 have their costs in a.costs, the others are formed
@@ -1094,7 +1095,8 @@ template <bool EXACT, int MODE> constexpr size_t tp_refine_smem() {
 /* -------------------------------------------------------- view lists -- */
 /* One warp per row.  Sources are visited in increasing x; the first four
  * that map to a target pixel fill its slots in that order (pmhstereo.cl:394-400
- * executed in raster order). */
+ * executed in raster order).  The row's entries (target | slot << 14, targets
+ * in increasing order) and their number follow the lists in memory. */
 PM_DEV void view_list_row(const float4* __restrict__ src, int W, int H, short4* __restrict__ list, int* cnt, int y) {
     const int lane = threadIdx.x;
     if (y >= H) return;
@@ -1121,6 +1123,20 @@ PM_DEV void view_list_row(const float4* __restrict__ src, int W, int H, short4* 
         }
         __syncwarp();
     }
+    unsigned short* const entries = view_entries(list, W, H) + (size_t)y * W;
+    int total = 0;
+    for (int x0 = 0; x0 < W; x0 += 32) {
+        const int x = x0 + lane, v = x < W ? min(cnt[x], 4) : 0;
+        int sum = v;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, sum, d);
+            if (lane >= d) sum += u;
+        }
+        for (int i = 0; i < v; ++i) entries[total + sum - v + i] = (unsigned short)(x | i << 14);
+        total += __shfl_sync(0xffffffffu, sum, 31);
+    }
+    if (lane == 0) view_counts(list, W, H)[y] = total;
 }
 
 __global__ void __launch_bounds__(32) k_view_list(const float4* __restrict__ src, int W, int H,
@@ -1755,6 +1771,14 @@ __global__ void __launch_bounds__(256, 2) kb_sweep(const __grid_constant__ PmBat
 }
 
 template <bool EXACT>
+__global__ void __launch_bounds__(256, 3) kb_views(const __grid_constant__ PmBatch<PmPassArgs> b) {
+    for (int item = blockIdx.x; item < b.first[b.n]; item += gridDim.x) {
+        const int p = batch_pair(b, item), t = item - b.first[p];
+        views_tile<EXACT>(b.a[p], t % b.tx[p], t / b.tx[p]);
+    }
+}
+
+template <bool EXACT>
 __global__ void __launch_bounds__(SH_NT, 1) kb_share(const __grid_constant__ PmBatch<PmPassArgs> b) {
     for (int item = blockIdx.x; item < b.first[b.n]; item += gridDim.x) {
         const int p = batch_pair(b, item), t = item - b.first[p];
@@ -1894,11 +1918,15 @@ cudaError_t pm_launch_propagate(const PmPassArgs& a, bool exact, cudaStream_t st
         if (exact) {
             k_sweep<true><<<grid, dim3(32, 8), 0, st>>>(b);
             PM_LAUNCH_CHECK();
+            if (b.viewin) k_views<true><<<grid, dim3(32, 8), 0, st>>>(b);
+            PM_LAUNCH_CHECK();
             k_share<true><<<sg, dim3(32, SH_TY), smem, st>>>(b);
             PM_LAUNCH_CHECK();
             k_propagate<true, 2><<<grid, dim3(32, 8), 0, st>>>(b);
         } else {
             k_sweep<false><<<grid, dim3(32, 8), 0, st>>>(b);
+            PM_LAUNCH_CHECK();
+            if (b.viewin) k_views<false><<<grid, dim3(32, 8), 0, st>>>(b);
             PM_LAUNCH_CHECK();
             k_share<false><<<sg, dim3(32, SH_TY), smem, st>>>(b);
             PM_LAUNCH_CHECK();
@@ -2114,6 +2142,11 @@ cudaError_t pm_batch_init(const PmBatch<PmPassArgs>& b, bool exact, const PmBatc
 cudaError_t pm_batch_sweep(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st) {
     if (exact) PM_BATCH_LAUNCH(kb_sweep<true>, dim3(32, 8), 0);
     PM_BATCH_LAUNCH(kb_sweep<false>, dim3(32, 8), 0);
+}
+cudaError_t pm_batch_views(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st) {
+    if (!b.a[0].viewin) return cudaSuccess;
+    if (exact) PM_BATCH_LAUNCH(kb_views<true>, dim3(32, 8), 0);
+    PM_BATCH_LAUNCH(kb_views<false>, dim3(32, 8), 0);
 }
 cudaError_t pm_batch_share(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st) {
     const size_t smem = share_smem(b.a[0].k.P);              /* one window size per batch */

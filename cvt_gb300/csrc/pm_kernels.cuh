@@ -20,7 +20,7 @@ struct PmPassArgs {
     float depthmax, theta;
     const float4* old;         /* previous states of v1            */
     const float4* smooth;      /* PD-smoothed (nx, ny, d/dmax, 1)  */
-    const short4* viewin;      /* up to 4 source x per pixel, or NULL */
+    const short4* viewin;      /* a view list (up to 4 source x per pixel), or NULL */
     const float4* viewsrc;     /* states the view list refers to    */
     float4* out;
     uint8_t* winners;
@@ -29,6 +29,16 @@ struct PmPassArgs {
     float4* cand;              /* tap-parallel passes: states and costs of candidates 1-20, [20][W*H], or NULL */
     int color;                 /* -1: every pixel (Jacobi); 0 / 1: pixels with (x + y) & 1 == color */
 };
+
+/* A view list of a W x H image: a short4 of source positions per pixel, then
+ * the rows' entries (W per row, see k_view_list) and their counts. */
+__host__ __device__ inline unsigned short* view_entries(const short4* list, int W, int H) {
+    return (unsigned short*)(list + (size_t)W * H);
+}
+__host__ __device__ inline int* view_counts(const short4* list, int W, int H) {
+    return (int*)((char*)list + ((size_t)W * H * 10 + 3) / 4 * 4);
+}
+__host__ __device__ inline size_t view_list_bytes(int W, int H) { return ((size_t)W * H * 10 + 3) / 4 * 4 + (size_t)H * 4; }
 
 /* ------------------------------------------------------------------
  * Batched launches (cvtpm_depthmap_batched).  One launch runs one phase of
@@ -78,9 +88,10 @@ void pm_batch_tiles(PmBatchKernel k, int W, int H, const PmBatchKnobs& kn, int* 
 cudaError_t pm_batch_prep(const PmBatch<PmPrepArgs>& b, const PmBatchKnobs& kn, cudaStream_t st);
 cudaError_t pm_batch_records(const PmBatch<PmRecArgs>& b, const PmBatchKnobs& kn, cudaStream_t st);
 cudaError_t pm_batch_init(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
-/* A propagation pass of pairs with PmPassArgs::costs: sweep, share, refine; of
+/* A propagation pass of pairs with PmPassArgs::costs: sweep, views, share, refine; of
  * the others: propagate. */
 cudaError_t pm_batch_sweep(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
+cudaError_t pm_batch_views(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
 cudaError_t pm_batch_share(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
 cudaError_t pm_batch_refine(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
 cudaError_t pm_batch_propagate(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st);
