@@ -57,15 +57,11 @@ struct cvtpm_ctx {
     uint8_t* win[2];
     uint8_t* valid;
     float* occ;                       /* occlusion mask of depthMapInpaint */
-    /* shared plane windows (FAST and EXACT): the costs of the candidates that share none
-     * (PM_COST_PLANES floats per pixel), when the budget allows */
-    float* nbcost = nullptr;
-    size_t nb_bytes = 0;
-    size_t nb_budget = SIZE_MAX;
-    /* tap-parallel passes of small images: the candidates' states and costs */
-    float4* cand = nullptr;
-    size_t cand_bytes = 0;
-    bool nb_on = false;
+    /* what a propagation pass needs to share work between its candidates (plan_pass),
+     * when the budget allows */
+    void* pass = nullptr;
+    size_t pass_bytes = 0;
+    size_t pass_budget = SIZE_MAX;
     /* set while a launch sequence is being captured into a graph: scratch
      * must already be sized, nothing may be allocated */
     bool no_alloc = false;
@@ -320,71 +316,65 @@ PmPassArgs base_args(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H, int v1
  * buffer is overwritten with that intermediate field. */
 cvtpm_status propagate_view(cvtpm_ctx* ctx, PmPassArgs a, bool exact, bool redblack, size_t n, cudaStream_t st) {
     if (!redblack) {
-        a.color = -1;
-        LK(pm_launch_propagate(a, exact, st), "propagate");
+        LK(pm_launch_pass_own(a, exact, st), "propagate");
+        LK(pm_launch_pass_rest(a, exact, st), "propagate");
         return CVTPM_OK;
     }
     float4* A = const_cast<float4*>(a.old);
-    CK(cudaMemcpyAsync(a.out, A, n * 16, cudaMemcpyDeviceToDevice, st), "red/black copy");
-    a.color = 0;
-    LK(pm_launch_propagate(a, exact, st), "propagate red");
-    CK(cudaMemcpyAsync(A, a.out, n * 16, cudaMemcpyDeviceToDevice, st), "red/black copy");
-    a.color = 1;
-    LK(pm_launch_propagate(a, exact, st), "propagate black");
+    for (int c = 0; c < 2; ++c) {
+        if (c == 0) CK(cudaMemcpyAsync(a.out, A, n * 16, cudaMemcpyDeviceToDevice, st), "red/black copy");
+        else CK(cudaMemcpyAsync(A, a.out, n * 16, cudaMemcpyDeviceToDevice, st), "red/black copy");
+        a.color = c;
+        LK(pm_launch_pass_own(a, exact, st), c ? "propagate black" : "propagate red");
+        LK(pm_launch_pass_rest(a, exact, st), c ? "propagate black" : "propagate red");
+    }
     return CVTPM_OK;
 }
 
-/* The cost buffer of the shared-window passes (PM_COST_PLANES floats per
- * pixel).  Used when it fits the context's budget and 60 % of the free device
- * memory; otherwise the propagation evaluates every candidate per pixel (same
- * results). */
-cvtpm_status ensure_nbcost(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H) {
-    const size_t need = (size_t)PM_COST_PLANES * W * H * sizeof(float);
-    ctx->nb_on = false;
-    if (need > ctx->nb_budget || !pm_shared_windows(base_args(ctx, p, W, H, 0).k)) return CVTPM_OK;
-    if (ctx->nb_bytes < need) {
-        if (ctx->no_alloc) return CVTPM_OK;          /* capturing: every candidate per pixel */
-        if (ctx->cand && need > ctx->nb_budget - std::min(ctx->nb_budget, ctx->cand_bytes)) {   /* not both */
-            CK(cudaFree(ctx->cand), "free candidates");
-            ctx->cand = nullptr;
-            ctx->cand_bytes = 0;
+/* Gives the two views' passes the scratch that lets candidates share work:
+ * per pixel of a small image 16 bytes for each of 16 candidates and 4 view
+ * candidates (tap-parallel passes), else 4 bytes for each of 2 and 4 (shared
+ * plane windows).  With the own candidates' part twice, the right view's first
+ * part can run beside the left view's pass (*overlap); the view candidates'
+ * part is used by one view at a time.  The most that fits the context's budget
+ * and 60 % of the free memory is taken; with none of it every candidate is
+ * evaluated per pixel.  Results are the same in every case. */
+cvtpm_status plan_pass(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H, bool taps, PmPassArgs* aL, PmPassArgs* aR,
+                       bool* overlap) {
+    const PmCostConsts k = base_args(ctx, p, W, H, 0).k;
+    *overlap = p.schedule == CVTPM_SCHEDULE_JACOBI;
+    if (!*overlap || !pm_shared_windows(k)) return CVTPM_OK;
+    const size_t n = (size_t)W * H;
+    taps = taps && pm_tap_parallel(k);
+    for (int plan = taps ? 0 : 2; plan < 4; ++plan) {
+        const bool both = (plan & 1) == 0, t = plan < 2;
+        const size_t need = t ? n * sizeof(float4) * (both ? 36 : 20) : n * sizeof(float) * (both ? 8 : 6);
+        if (need > ctx->pass_budget) continue;
+        if (need > ctx->pass_bytes) {
+            if (ctx->no_alloc) continue;             /* capturing: what is there */
+            if (ctx->pass) { CK(cudaFree(ctx->pass), "free pass scratch"); ctx->pass = nullptr; ctx->pass_bytes = 0; }
+            size_t fr = 0, tot = 0;
+            CK(cudaMemGetInfo(&fr, &tot), "memory info");
+            if ((double)need > 0.6 * (double)fr) continue;
+            if (cudaMalloc(&ctx->pass, need) != cudaSuccess) {
+                cudaGetLastError();                  /* clear the failed allocation */
+                ctx->pass = nullptr;
+                continue;
+            }
+            ctx->pass_bytes = need;
         }
-        if (ctx->nbcost) { CK(cudaFree(ctx->nbcost), "free candidate costs"); ctx->nbcost = nullptr; ctx->nb_bytes = 0; }
-        size_t fr = 0, tot = 0;
-        CK(cudaMemGetInfo(&fr, &tot), "memory info");
-        if ((double)need > 0.6 * (double)fr) return CVTPM_OK;
-        if (cudaMalloc(&ctx->nbcost, need) != cudaSuccess) {
-            cudaGetLastError();                      /* clear the failed allocation; use the per-pixel path */
-            ctx->nbcost = nullptr;
-            return CVTPM_OK;
+        if (t) {
+            aL->cand = (float4*)ctx->pass;
+            aR->cand = both ? aL->cand + 16 * n : aL->cand;
+            aL->vcand = aR->vcand = aR->cand + 16 * n;
+        } else {
+            aL->costs = (float*)ctx->pass;
+            aR->costs = both ? aL->costs + 2 * n : aL->costs;
+            aL->vcosts = aR->vcosts = aR->costs + 2 * n;
         }
-        ctx->nb_bytes = need;
+        *overlap = both;
+        return CVTPM_OK;
     }
-    ctx->nb_on = true;
-    return CVTPM_OK;
-}
-
-/* The candidate buffer of the tap-parallel passes (320 bytes per pixel of a
- * small image), under the same budget; without it the passes take the other
- * path (same results). */
-cvtpm_status ensure_cand(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H, float4** cand) {
-    *cand = nullptr;
-    if (p.schedule != CVTPM_SCHEDULE_JACOBI || !pm_tap_parallel(base_args(ctx, p, W, H, 0).k)) return CVTPM_OK;
-    const size_t need = pm_tap_parallel_bytes(W, H);
-    if (ctx->cand_bytes < need) {
-        if (ctx->no_alloc || need > ctx->nb_budget - std::min(ctx->nb_budget, ctx->nb_bytes)) return CVTPM_OK;
-        if (ctx->cand) { CK(cudaFree(ctx->cand), "free candidates"); ctx->cand = nullptr; ctx->cand_bytes = 0; }
-        size_t fr = 0, tot = 0;
-        CK(cudaMemGetInfo(&fr, &tot), "memory info");
-        if ((double)need > 0.6 * (double)fr) return CVTPM_OK;
-        if (cudaMalloc(&ctx->cand, need) != cudaSuccess) {
-            cudaGetLastError();
-            ctx->cand = nullptr;
-            return CVTPM_OK;
-        }
-        ctx->cand_bytes = need;
-    }
-    *cand = ctx->cand;
     return CVTPM_OK;
 }
 
@@ -498,12 +488,8 @@ cvtpm_status run_depthmap(cvtpm_ctx* ctx, const cvtpm_params& p, float* dmap, si
     const float dscale = p.dscale <= 0.0f ? 1.0f / dmax : p.dscale;
     const int N = p.iterations;
     PmPassArgs aL = base_args(ctx, p, W, H, 0), aR = base_args(ctx, p, W, H, 1);
-    if ((s = ensure_cand(ctx, p, W, H, &aL.cand)) != CVTPM_OK) return s;
-    aR.cand = aL.cand;
-    if (!aL.cand) {
-        if ((s = ensure_nbcost(ctx, p, W, H)) != CVTPM_OK) return s;
-        if (ctx->nb_on) aL.costs = aR.costs = ctx->nbcost;
-    }
+    bool overlap = false;
+    if ((s = plan_pass(ctx, p, W, H, true, &aL, &aR, &overlap)) != CVTPM_OK) return s;
     if (!ctx->dcount) {
         if (ctx->no_alloc) return fail(ctx, CVTPM_ERR_ALLOC, "counters not allocated before capture");
         CK(cudaMalloc(&ctx->dcount, 2 * sizeof(unsigned long long)), "counters");
@@ -538,27 +524,52 @@ cvtpm_status run_depthmap(cvtpm_ctx* ctx, const cvtpm_params& p, float* dmap, si
     }
 
     float theta = theta_at(first, N);
+    aL.counters = aR.counters = ctx->dcount;
+    aL.winners = ctx->win[0];
+    aR.winners = ctx->win[1];
+    /* The right view's candidates 1-16 need its own planes and smoothed field
+     * only, so they run on the side stream behind its smoother, beside the left
+     * view's smoother and pass: the launches of the two chains fill the SMs
+     * that the other's last waves leave idle (321x243 51.0 -> 44.5 ms, 1242x375
+     * 339.3 -> 335.5).  The right view's pass then takes the left view's planes
+     * and refines on `st`. */
+    auto right_own = [&](int iter, float th) -> cvtpm_status {
+        const int sw = iter & 1;
+        aR.iter = iter;
+        aR.theta = th;
+        aR.old = ctx->S[1][sw]; aR.out = ctx->S[1][1 - sw]; aR.smooth = ctx->smooth[1];
+        LK(pm_launch_pass_own(aR, exact, ctx->side), "propagate");
+        return CVTPM_OK;
+    };
+    if (overlap && first < last) {
+        CK(cudaEventRecord(ctx->side_fork, st), "fork");
+        CK(cudaStreamWaitEvent(ctx->side, ctx->side_fork, 0), "fork");
+        if ((s = right_own(first, theta)) != CVTPM_OK) return s;
+        CK(cudaEventRecord(ctx->side_join, ctx->side), "join");
+    }
     for (int iter = first; iter < last; ++iter) {                  /* :151-266 */
         const int sw = iter & 1;
-        aL.iter = aR.iter = iter;
-        aL.theta = aR.theta = theta;
-        aL.old = ctx->S[0][sw]; aL.out = ctx->S[0][1 - sw]; aL.smooth = ctx->smooth[0];
-        aL.viewin = ctx->list[1]; aL.viewsrc = ctx->S[1][sw]; aL.winners = ctx->win[0];
-        aL.counters = aR.counters = ctx->dcount;
+        const bool redblack = p.schedule == CVTPM_SCHEDULE_REDBLACK;
+        const float next = iter >= 5 ? smoothstep01(((float)iter - 5.0f) / ((float)N - 5.0f)) * 1.0f : theta;
         {
-            NvtxRange r("propagate left");
+            NvtxRange r("propagate left and right");
             PhaseTimer tm(ctx, st, ctx->ev_prop);
-            if ((s = propagate_view(ctx, aL, exact, p.schedule == CVTPM_SCHEDULE_REDBLACK, n, st)) != CVTPM_OK) return s;
-            tm.stop();
-        }
-        LK(pm_launch_view_list(ctx->S[0][1 - sw], W, H, ctx->list[0], st), "view list");
-        aR.old = ctx->S[1][sw]; aR.out = ctx->S[1][1 - sw]; aR.smooth = ctx->smooth[1];
-        aR.viewin = ctx->list[0]; aR.viewsrc = ctx->S[0][1 - sw]; aR.winners = ctx->win[1];
-        if (iter > first) CK(cudaStreamWaitEvent(st, ctx->side_join, 0), "join");   /* smooth[1] */
-        {
-            NvtxRange r("propagate right");
-            PhaseTimer tm(ctx, st, ctx->ev_prop);
-            if ((s = propagate_view(ctx, aR, exact, p.schedule == CVTPM_SCHEDULE_REDBLACK, n, st)) != CVTPM_OK) return s;
+            aL.iter = iter;
+            aL.theta = theta;
+            aL.old = ctx->S[0][sw]; aL.out = ctx->S[0][1 - sw]; aL.smooth = ctx->smooth[0];
+            aL.viewin = ctx->list[1]; aL.viewsrc = ctx->S[1][sw];
+            if ((s = propagate_view(ctx, aL, exact, redblack, n, st)) != CVTPM_OK) return s;
+            LK(pm_launch_view_list(ctx->S[0][1 - sw], W, H, ctx->list[0], st), "view list");
+            if (overlap || iter > first) CK(cudaStreamWaitEvent(st, ctx->side_join, 0), "join");   /* smooth[1] */
+            aR.viewin = ctx->list[0]; aR.viewsrc = ctx->S[0][1 - sw];
+            if (overlap) {
+                LK(pm_launch_pass_rest(aR, exact, st), "propagate");
+            } else {
+                aR.iter = iter;
+                aR.theta = theta;
+                aR.old = ctx->S[1][sw]; aR.out = ctx->S[1][1 - sw]; aR.smooth = ctx->smooth[1];
+                if ((s = propagate_view(ctx, aR, exact, redblack, n, st)) != CVTPM_OK) return s;
+            }
             tm.stop();
         }
         ctx->stats.propagate_launches += 2;
@@ -566,10 +577,8 @@ cvtpm_status run_depthmap(cvtpm_ctx* ctx, const cvtpm_params& p, float* dmap, si
         const float lambda = theta * p.thetascale + 5.0f;
         /* :228-261.  The right view's consistency, fill and smoother need only
          * this iteration's planes and write only smooth[1] and scratch of
-         * their own, so they run on the side stream while the left view's
-         * smoother and the next left pass run here: the side work fills the
-         * SMs the tails of those launches leave idle.  The next right pass
-         * waits for it (side_join). */
+         * their own, so they run on the side stream beside the left view's and
+         * the next left pass.  The next right pass waits for them (side_join). */
         CK(cudaEventRecord(ctx->side_fork, st), "fork");
         CK(cudaStreamWaitEvent(ctx->side, ctx->side_fork, 0), "fork");
         for (int v = 1; v >= 0; --v) {
@@ -582,9 +591,12 @@ cvtpm_status run_depthmap(cvtpm_ctx* ctx, const cvtpm_params& p, float* dmap, si
             LK(pm_launch_fill_state(t1, W, H, dmax, v == 0 ? 1 : 0, t2, sv), "fill");
             if ((s = pd_apply(ctx, ctx->smooth[v], t2, ctx->wgt[v], lambda, p.pd_iterations, W, H, sv, nullptr, v)) != CVTPM_OK)
                 return s;
+            if (v == 1) {
+                if (overlap && iter + 1 < last && (s = right_own(iter + 1, next)) != CVTPM_OK) return s;
+                CK(cudaEventRecord(ctx->side_join, ctx->side), "join");
+            }
         }
-        CK(cudaEventRecord(ctx->side_join, ctx->side), "join");
-        if (iter >= 5) theta = smoothstep01(((float)iter - 5.0f) / ((float)N - 5.0f)) * 1.0f;
+        theta = next;
     }
     if (last > first) CK(cudaStreamWaitEvent(st, ctx->side_join, 0), "join");
     if (save) {
@@ -639,12 +651,8 @@ cvtpm_status run_depthmap_inpaint(cvtpm_ctx* ctx, const cvtpm_params& p, float* 
     const float dmax = p.depthmax;
     const int N = p.iterations;
     PmPassArgs aL = base_args(ctx, p, W, H, 0), aR = base_args(ctx, p, W, H, 1);
-    if ((s = ensure_cand(ctx, p, W, H, &aL.cand)) != CVTPM_OK) return s;
-    aR.cand = aL.cand;
-    if (!aL.cand) {
-        if ((s = ensure_nbcost(ctx, p, W, H)) != CVTPM_OK) return s;
-        if (ctx->nb_on) aL.costs = aR.costs = ctx->nbcost;
-    }
+    bool overlap = false;                                          /* not used: one stream here */
+    if ((s = plan_pass(ctx, p, W, H, true, &aL, &aR, &overlap)) != CVTPM_OK) return s;
     if (!ctx->dcount) {
         if (ctx->no_alloc) return fail(ctx, CVTPM_ERR_ALLOC, "counters not allocated before capture");
         CK(cudaMalloc(&ctx->dcount, 2 * sizeof(unsigned long long)), "counters");
@@ -817,8 +825,7 @@ cvtpm_status cvtpm_destroy(cvtpm_ctx* ctx) {
     if (ctx->bfork) cudaEventDestroy(ctx->bfork);
     if (ctx->bjoin) cudaEventDestroy(ctx->bjoin);
     if (ctx->stage) cudaFree(ctx->stage);
-    if (ctx->nbcost) cudaFree(ctx->nbcost);
-    if (ctx->cand) cudaFree(ctx->cand);
+    if (ctx->pass) cudaFree(ctx->pass);
     if (ctx->istage) cudaFree(ctx->istage);
     if (ctx->dcount) cudaFree(ctx->dcount);
     for (auto& pr : ctx->ev_prop) { cudaEventDestroy(pr.first); cudaEventDestroy(pr.second); }
@@ -995,18 +1002,12 @@ cvtpm_status cvtpm_cost_eval(cvtpm_ctx* ctx, const float* img1, const float* img
 
 cvtpm_status cvtpm_set_memory_budget(cvtpm_ctx* ctx, size_t bytes) {
     if (!ctx) return CVTPM_ERR_INVALID_ARGUMENT;
-    ctx->nb_budget = bytes;
-    if (ctx->nbcost && ctx->nb_bytes > bytes) {
+    ctx->pass_budget = bytes;
+    if (ctx->pass && ctx->pass_bytes > bytes) {
         CK(cudaSetDevice(ctx->device), "cudaSetDevice");
-        CK(cudaFree(ctx->nbcost), "free candidate costs");
-        ctx->nbcost = nullptr;
-        ctx->nb_bytes = 0;
-    }
-    if (ctx->cand && ctx->cand_bytes > bytes) {
-        CK(cudaSetDevice(ctx->device), "cudaSetDevice");
-        CK(cudaFree(ctx->cand), "free candidates");
-        ctx->cand = nullptr;
-        ctx->cand_bytes = 0;
+        CK(cudaFree(ctx->pass), "free pass scratch");
+        ctx->pass = nullptr;
+        ctx->pass_bytes = 0;
     }
     return CVTPM_OK;
 }
@@ -1181,13 +1182,14 @@ cvtpm_status capture_batch(cvtpm_ctx* ctx, const cvtpm_pair* pairs, int npairs, 
     for (int j = 0; j < k; ++j) {
         cvtpm_ctx* c = ctx->lanes[j].c;
         c->prm = p;
-        if ((s = cvtpm_set_memory_budget(c, ctx->nb_budget)) != CVTPM_OK) return fail(ctx, s, c->err);
+        if ((s = cvtpm_set_memory_budget(c, ctx->pass_budget)) != CVTPM_OK) return fail(ctx, s, c->err);
         c->timing = false;
         for (int i : plan[j]) {
             if ((s = ensure_buffers(c, pairs[i].width, pairs[i].height)) != CVTPM_OK) return fail(ctx, s, c->err);
-            float4* cand = nullptr;
-            if ((s = ensure_cand(c, p, pairs[i].width, pairs[i].height, &cand)) != CVTPM_OK) return fail(ctx, s, c->err);
-            if (!cand && (s = ensure_nbcost(c, p, pairs[i].width, pairs[i].height)) != CVTPM_OK) return fail(ctx, s, c->err);
+            PmPassArgs aL, aR;
+            bool overlap;
+            if ((s = plan_pass(c, p, pairs[i].width, pairs[i].height, true, &aL, &aR, &overlap)) != CVTPM_OK)
+                return fail(ctx, s, c->err);
         }
     }
     if (k > 0 && (s = ensure_tables(ctx->lanes[0].c, p, ctx->bstream)) != CVTPM_OK) return fail(ctx, s, ctx->lanes[0].c->err);
@@ -1355,10 +1357,13 @@ cvtpm_status phase_prepare(PhaseState& S) {
         cvtpm_ctx* c = S.ctx->bpairs[i];
         c->prm = S.p;
         c->prm.depthmax = S.pairs[i].depthmax;
-        c->nb_budget = S.ctx->nb_budget;
+        c->pass_budget = S.ctx->pass_budget;
         c->timing = false;
         if ((s = ensure_buffers(c, S.pairs[i].width, S.pairs[i].height)) != CVTPM_OK) return fail(S.ctx, s, c->err);
-        if ((s = ensure_nbcost(c, c->prm, S.pairs[i].width, S.pairs[i].height)) != CVTPM_OK) return fail(S.ctx, s, c->err);
+        PmPassArgs aL, aR;
+        bool overlap;
+        if ((s = plan_pass(c, c->prm, S.pairs[i].width, S.pairs[i].height, false, &aL, &aR, &overlap)) != CVTPM_OK)
+            return fail(S.ctx, s, c->err);
         S.maxW = std::max(S.maxW, S.pairs[i].width);
     }
     return ensure_tables(S.ctx->bpairs[0], S.p, S.st) == CVTPM_OK ? CVTPM_OK
@@ -1393,7 +1398,8 @@ cvtpm_status phase_start(PhaseState& S) {
         const int W = S.pairs[i].width, H = S.pairs[i].height;
         S.aL[i] = base_args(c, c->prm, W, H, 0);
         S.aR[i] = base_args(c, c->prm, W, H, 1);
-        if (c->nb_on) S.aL[i].costs = S.aR[i].costs = c->nbcost;
+        bool overlap;
+        if ((s = plan_pass(c, c->prm, W, H, false, &S.aL[i], &S.aR[i], &overlap)) != CVTPM_OK) return fail(ctx, s, c->err);
         S.aL[i].counters = S.aR[i].counters = c->dcount;
         S.aL[i].out = c->S[0][0];
         S.aR[i].out = c->S[1][0];
@@ -1679,18 +1685,18 @@ cvtpm_status tune_mode(PhaseState& full, float ms[2]) {
     int maxW = 1, maxH = 1;
     cvtpm_ctx* ctx = S.ctx;
     cvtpm_ctx* lane = ctx->lanes[0].c;
-    cvtpm_status s = cvtpm_set_memory_budget(lane, ctx->nb_budget);
+    cvtpm_status s = cvtpm_set_memory_budget(lane, ctx->pass_budget);
     S.n = 0;
     while (S.n < full.n && (S.n == 0 || px < 4000000)) {
-        float4* cand = nullptr;
-        if (s == CVTPM_OK) s = ensure_cand(lane, S.p, full.pairs[S.n].width, full.pairs[S.n].height, &cand);
+        PmPassArgs aL, aR;
+        bool overlap;
+        if (s == CVTPM_OK) s = plan_pass(lane, S.p, full.pairs[S.n].width, full.pairs[S.n].height, true, &aL, &aR, &overlap);
         px += (long long)full.pairs[S.n].width * full.pairs[S.n].height;
         maxW = std::max(maxW, full.pairs[S.n].width);
         maxH = std::max(maxH, full.pairs[S.n].height);
         ++S.n;
     }
     if (s == CVTPM_OK) s = ensure_buffers(lane, maxW, maxH);
-    if (s == CVTPM_OK) s = ensure_nbcost(lane, S.p, maxW, maxH);
     if (s != CVTPM_OK) return fail(ctx, s, lane->err);
     EventPair ev;
     CK(cudaEventCreate(&ev.a), "tune event");
@@ -1734,7 +1740,7 @@ static cvtpm_status batch_lanes(cvtpm_ctx* ctx, const cvtpm_pair* pairs, int npa
     if ((s = capture_batch(ctx, pairs, npairs, k, ctx->prm.iterations, &ctx->bexec, &nodes)) != CVTPM_OK) return s;
     ctx->bkey = key;
     ctx->binfo.lanes = k;
-    ctx->binfo.shared_windows = ctx->prm.arith == CVTPM_ARITH_FAST && ctx->nb_budget > 0 ? 1 : 0;
+    ctx->binfo.shared_windows = ctx->prm.arith == CVTPM_ARITH_FAST && ctx->pass_budget > 0 ? 1 : 0;
     ctx->binfo.graph_nodes = (long long)nodes;
     ctx->binfo.replays = 0;
     ctx->binfo.launches = 0;
@@ -1763,7 +1769,7 @@ static cvtpm_status depthmap_batched(cvtpm_ctx* ctx, const cvtpm_pair* pairs, in
     put(&ctx->batch_lanes, sizeof(int));
     put(&ctx->pinned_knobs, sizeof(bool));
     put(&ctx->knobs.grid_mult, sizeof(int)); put(&ctx->knobs.pd_rows, sizeof(int)); put(&ctx->knobs.pd_halo, sizeof(int));
-    put(&ctx->nb_budget, sizeof(size_t));
+    put(&ctx->pass_budget, sizeof(size_t));
     for (int i = 0; i < npairs; ++i) {
         const cvtpm_pair& q = pairs[i];
         put(&q.width, sizeof(int)); put(&q.height, sizeof(int)); put(&q.depthmax, sizeof(float));
@@ -1826,7 +1832,7 @@ static cvtpm_status depthmap_batched(cvtpm_ctx* ctx, const cvtpm_pair* pairs, in
         ctx->binfo.pd_halo = S.kn.pd_halo;
         ctx->binfo.launches = S.launches;
         int nb = 0;
-        for (int i = 0; i < npairs; ++i) nb += ctx->bpairs[i]->nb_on ? 1 : 0;
+        for (int i = 0; i < npairs; ++i) nb += S.aL[i].costs ? 1 : 0;
         ctx->binfo.shared_windows = nb == npairs ? 1 : 0;
         ctx->binfo.graph_nodes = (long long)nodes;
         ctx->binfo.replays = 0;

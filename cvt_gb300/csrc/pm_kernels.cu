@@ -27,26 +27,12 @@
 #ifndef PM_PROP_MINB
 #define PM_PROP_MINB 2
 #endif
-/* FAST: candidates 9-16 per window sweep (8: one sweep; 4: two) */
-/* The propagation as two launches: candidates 1-20, then the refinements
- * at PM_REFINE_MINB blocks of 256 per SM (0: one launch). */
-#ifndef PM_PROP_SPLIT
-#define PM_PROP_SPLIT 1
-#endif
-#ifndef PM_REFINE_MINB
+/* The refinements and the other view's candidates are launches of their own,
+ * at the blocks per SM their registers allow. */
 #define PM_REFINE_MINB 4
-#endif
-/* The other view's candidates as a launch of their own (at PM_VIEW_MINB
- * blocks per SM) between the two. */
-#ifndef PM_VIEW_SPLIT
-#define PM_VIEW_SPLIT 1
-#endif
-#ifndef PM_VIEW_MINB
 #define PM_VIEW_MINB 3
-#endif
-#ifndef PM_FAST_SWEEP
+/* FAST: candidates 9-16 per window sweep */
 #define PM_FAST_SWEEP 8
-#endif
 
 
 /* ------------------------------------------------------------- prep -- */
@@ -151,20 +137,42 @@ __global__ void __launch_bounds__(256) k_cost_field(PmPassArgs a, const float4* 
     cost[(size_t)y * a.k.W + x] = c[0];
 }
 
+/* Adds a warp's evaluations and in-image window taps (`ev` evaluations at an
+ * inside pixel) to the counters; every lane calls it. */
+PM_DEV void pass_counters(const PmPassArgs& a, bool inside, int x, int y, int nev) {
+    if (!a.counters) return;
+    unsigned long long ev = 0, taps = 0;
+    if (inside) {
+        const int P = a.k.P;
+        const int nx = min(x + P, a.k.W - 1) - max(x - P, 0) + 1;
+        const int ny = min(y + P, a.k.H - 1) - max(y - P, 0) + 1;
+        ev = (unsigned long long)nev;
+        taps = ev * (unsigned long long)(nx * ny);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        ev += __shfl_down_sync(0xffffffffu, ev, off);
+        taps += __shfl_down_sync(0xffffffffu, taps, off);
+    }
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&a.counters[0], ev);
+        atomicAdd(&a.counters[1], taps);
+    }
+}
+
 /* --------------------------------------------------------- propagate -- */
 /* Register budgets, measured per 1242x375 depthMap: EXACT allowed one block
  * per SM takes 128 registers and still fits two (630 against 644 ms with
  * the 111 it took under the plain 256-thread bound); FAST needs the
  * two-block cap (it takes 153 registers and one block per SM otherwise: pass
  * 39.2 against 31.6 ms), where it also stops spilling. */
-/* STAGE 0: the whole candidate schedule.  STAGE 1: candidates 1-16 (and
- * 17-20 unless PM_VIEW_SPLIT), the best so far written to out (its index to
+/* STAGE 1: candidates 1-16, the best so far written to out (its index to
  * winners).  STAGE 3: the other view's candidates 17-20 against that best.
  * STAGE 2: the two refinements of the best (read back from out), from the
  * random stream after the 15 draws stage 1 made (12 for the random
- * neighbours' offsets, 3 for the random plane).  Stages 1, (3,) 2 in order
- * give the bits of stage 0; the split lets each sweep run at the occupancy
- * its registers allow. */
+ * neighbours' offsets, 3 for the random plane); with a.vcosts it first
+ * accepts 17-20 by the costs that holds.  The split lets each sweep run at the
+ * occupancy its registers allow. */
 template <bool EXACT, int STAGE>
 PM_DEV void propagate_tile(const PmPassArgs& a, int tbx, int tby) {
     const int W = a.k.W, H = a.k.H;
@@ -200,7 +208,7 @@ PM_DEV void propagate_tile(const PmPassArgs& a, int tbx, int tby) {
     };
 
     int nview_total = 0;
-    if (STAGE != 2 && STAGE != 3) {
+    if (STAGE == 1) {
         /* candidates 1-8: the 3x3 neighbourhood of `old`, clamped to the edge
          * (:330-342) */
 #pragma unroll 1
@@ -246,7 +254,16 @@ PM_DEV void propagate_tile(const PmPassArgs& a, int tbx, int tby) {
             for (int j = 0; j < NB; ++j) accept(s[j], c[j], 9 + b0 + j);
         }
     }
-    if (STAGE == 0 || STAGE == 3 || (STAGE == 1 && !PM_VIEW_SPLIT)) {
+    if (STAGE == 2 && a.vcosts && a.viewin) {
+        /* 17-20 with their costs from k_views */
+        const short4 l = a.viewin[o];
+        const short li[4] = {l.x, l.y, l.z, l.w};
+        nview_total = (li[0] < 0) ? 0 : (li[1] < 0) ? 1 : (li[2] < 0) ? 2 : (li[3] < 0) ? 3 : 4;
+#pragma unroll 1
+        for (int i = 0; i < nview_total; ++i)
+            accept(viewprop(a.viewsrc[(size_t)yc * W + li[i]]), a.vcosts[(size_t)i * W * H + o], 17 + i);
+    }
+    if (STAGE == 3) {
         /* 17-20: candidates from the other view (:372-379) */
         if (a.viewin) {
             short4 l = a.viewin[o];
@@ -282,7 +299,7 @@ PM_DEV void propagate_tile(const PmPassArgs& a, int tbx, int tby) {
     float4 last = f4s(0.0f);
     bool rejected = false;
 #pragma unroll 1
-    for (int i = 0; i < ((STAGE == 0 || STAGE == 2) ? 2 : 0); ++i) {
+    for (int i = 0; i < (STAGE == 2 ? 2 : 0); ++i) {
         float4 s[1] = {state_refine(rng, self, cx, cy, dmax, lr)};
         bool act[1] = {!(rejected && s[0].x == last.x && s[0].y == last.y && s[0].z == last.z)};
         if (!__any_sync(0xffffffffu, act[0])) continue;
@@ -301,26 +318,8 @@ PM_DEV void propagate_tile(const PmPassArgs& a, int tbx, int tby) {
         a.out[o] = self;
         if (a.winners && win >= 0) a.winners[o] = (uint8_t)win;
     }
-    if (STAGE != 2 && a.counters) {
-        /* evaluations = 18 + view candidates; taps = in-image window taps */
-        unsigned long long ev = 0, taps = 0;
-        if (inside) {
-            const int P = a.k.P;
-            const int nx = min(xc + P, W - 1) - max(xc - P, 0) + 1;
-            const int ny = min(yc + P, H - 1) - max(yc - P, 0) + 1;
-            ev = (STAGE == 3 ? 0ull : 18ull) + (unsigned long long)nview_total;
-            taps = ev * (unsigned long long)(nx * ny);
-        }
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            ev += __shfl_down_sync(0xffffffffu, ev, off);
-            taps += __shfl_down_sync(0xffffffffu, taps, off);
-        }
-        if ((threadIdx.x & 31) == 0) {
-            atomicAdd(&a.counters[0], ev);
-            atomicAdd(&a.counters[1], taps);
-        }
-    }
+    /* 18 evaluations and those of the view candidates */
+    if (STAGE != 2 || a.vcosts) pass_counters(a, inside, x, y, (STAGE >= 2 ? 0 : 18) + nview_total);
 }
 
 /* Registers: the candidate stages at two blocks per SM (FAST) or one
@@ -445,29 +444,6 @@ PM_DEV float4 smooth_state(float4 smooth, float cx, float cy, int lr) {
     return lr ? sc : viewprop(sc);
 }
 
-/* Adds a warp's evaluations and in-image window taps (`ev` evaluations at an
- * inside pixel) to the counters; every lane calls it. */
-PM_DEV void pass_counters(const PmPassArgs& a, bool inside, int x, int y, int nev) {
-    if (!a.counters) return;
-    unsigned long long ev = 0, taps = 0;
-    if (inside) {
-        const int P = a.k.P;
-        const int nx = min(x + P, a.k.W - 1) - max(x - P, 0) + 1;
-        const int ny = min(y + P, a.k.H - 1) - max(y - P, 0) + 1;
-        ev = (unsigned long long)nev;
-        taps = ev * (unsigned long long)(nx * ny);
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        ev += __shfl_down_sync(0xffffffffu, ev, off);
-        taps += __shfl_down_sync(0xffffffffu, taps, off);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&a.counters[0], ev);
-        atomicAdd(&a.counters[1], taps);
-    }
-}
-
 /* ------------------------------------------------- shared plane windows -- */
 /* Candidates 1-8 and 10-15 (pmhstereo.cl:330-342,355-361) are planes of the
  * old field at offsets (-1..7, -1..7): every plane is tested by its 8
@@ -540,7 +516,7 @@ template <bool EXACT>
 __global__ void __launch_bounds__(256, 2) k_sweep(PmPassArgs a) { sweep_tile<EXACT>(a, blockIdx.x, blockIdx.y); }
 
 /* The other view's candidates 17-20: entry i of a pixel's list goes to
- * a.costs[2 + i].  A pixel has 0 to 4 of them, about one on average, so a warp
+ * a.vcosts[i].  A pixel has 0 to 4 of them, about one on average, so a warp
  * that followed its pixels would sweep as often as its fullest list; the
  * threads follow the row's entries (view_entries) instead, each taking one
  * (1242x375, per pass: 2.2 ms, where a sweep by pixel, joined to that of 9 and
@@ -558,15 +534,14 @@ PM_DEV void views_tile(const PmPassArgs& a, int tbx, int tby) {
     bool act[1] = {true};
     float c[1];
     eval_costs<1, EXACT>(a.k, a.v1, a.v2, x, y, s, act, c);
-    a.costs[(size_t)(2 + i) * W * H + o] = c[0];
+    a.vcosts[(size_t)i * W * H + o] = c[0];
 }
 
 template <bool EXACT>
 __global__ void __launch_bounds__(256, 3) k_views(PmPassArgs a) { views_tile<EXACT>(a, blockIdx.x, blockIdx.y); }
 
-/* The candidates 1-16 and the view candidates of a pixel against its old
- * state: 9, 16 and 17-20 have their costs in a.costs, the others are formed
- * here.  The best goes to a.out. */
+/* The candidates 1-16 of a pixel against its old state: 9 and 16 have their
+ * costs in a.costs, the others are formed here.  The best goes to a.out. */
 template <bool EXACT>
 PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
     typedef typename ShTerm<EXACT>::type Term;
@@ -742,22 +717,11 @@ PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
                nb_final<EXACT>(a.k, true, r1[8 + c], r2[8 + c], ws[8 + c]), 10 + c);
     }
     accept(state_init(rng, cx, cy, a.lr, 2.0f, a.depthmax), a.costs[n + o], 16);
-    int nview = 0;
-    if (a.viewin) {
-        const short4 l = a.viewin[o];
-        const short li[4] = {l.x, l.y, l.z, l.w};
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (li[i] >= 0 && nview == i) {
-                accept(viewprop(a.viewsrc[(size_t)yc * W + li[i]]), a.costs[(size_t)(2 + i) * n + o], 17 + i);
-                nview = i + 1;
-            }
-    }
     if (inside) {
         a.out[o] = self;
         if (a.winners) a.winners[o] = (uint8_t)win;
     }
-    pass_counters(a, inside, x, y, 18 + nview);
+    pass_counters(a, inside, x, y, 18);
 }
 
 template <bool EXACT>
@@ -947,13 +911,14 @@ PM_DEV float tp_costs(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, const Pm
 #define TP_CH 16       /* taps per chunk of the candidate kernel */
 #define TP_CH1 64      /* taps per chunk of the one-candidate kernels */
 
-/* Candidates 1-8 (blockIdx.z 0), 9-16 (1) and 17-20 (2) of 32 pixels: their
- * states with their costs go to a.cand[candidate - 1]. */
+/* Candidates 1-8 (group 0), 9-16 (1) and 17-20 (2) of 32 pixels: their
+ * states with their costs go to a.cand[candidate - 1] and a.vcand[candidate - 17];
+ * z0 is the first group. */
 template <bool EXACT>
-__global__ void __launch_bounds__(32 * TP_NP, 2) k_taps_candidates(PmPassArgs a) {
+__global__ void __launch_bounds__(32 * TP_NP, 2) k_taps_candidates(PmPassArgs a, int z0) {
     extern __shared__ __align__(16) unsigned char tp_smem[];
     TpShared<EXACT, TP_K, TP_CH>& S = *reinterpret_cast<TpShared<EXACT, TP_K, TP_CH>*>(tp_smem);
-    const int W = a.k.W, H = a.k.H, x0 = blockIdx.x * 32, y = blockIdx.y, z = blockIdx.z;
+    const int W = a.k.W, H = a.k.H, x0 = blockIdx.x * 32, y = blockIdx.y, z = z0 + blockIdx.z;
     const int c = threadIdx.y, x = min(x0 + (int)threadIdx.x, W - 1);
     const size_t n = (size_t)W * H, o = (size_t)y * W + x;
     const float cx = (float)x, cy = (float)y;
@@ -988,12 +953,12 @@ __global__ void __launch_bounds__(32 * TP_NP, 2) k_taps_candidates(PmPassArgs a)
     }
     tp_put_plane(S, a.k, c, s, act);
     s.w = tp_costs<EXACT, TP_K, TP_CH, 0>(S, a.k, a.v1, a.v2, x0, y, act && finite3(s));
-    if (act && x0 + (int)threadIdx.x < W) a.cand[(size_t)(z * 8 + c) * n + o] = s;
+    if (act && x0 + (int)threadIdx.x < W) (z < 2 ? a.cand + (size_t)(z * 8 + c) * n : a.vcand + (size_t)c * n)[o] = s;
 }
 
 /* One candidate per evaluation: warps 0..TP_NP-1 produce, warp TP_NP owns the
  * pixels.  MODE 0: the random initial planes (pmhstereo_init).  MODE 1: the
- * best of a.old and the candidates in a.cand, then the two refinements.
+ * best of a.old and the candidates in a.cand and a.vcand, then the two refinements.
  * MODE 2: the refinements of the best so far in a.out. */
 template <bool EXACT, int MODE>
 __global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_refine(PmPassArgs a) {
@@ -1031,7 +996,7 @@ __global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_refine(PmPassArgs 
         }
         if (!owner) {                                /* the candidates' distances, spread over the producers */
             for (int i = w; i < 16 + nview; i += TP_NP) {
-                const float4 s = a.cand[(size_t)i * n + o];
+                const float4 s = (i < 16 ? a.cand + (size_t)i * n : a.vcand + (size_t)(i - 16) * n)[o];
                 best[i][lane] = {s.w, state_distance(s, smooth, cx, cy, dmax, a.lr), finite3(s)};
             }
         }
@@ -1049,7 +1014,10 @@ __global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_refine(PmPassArgs 
                 const TpBest e = best[i][lane];
                 if (tp_accepts(e, eself, theta)) { eself = e; pick = i; }
             }
-            if (pick >= 0) { self = a.cand[(size_t)pick * n + o]; win = pick + 1; }
+            if (pick >= 0) {
+                self = (pick < 16 ? a.cand + (size_t)pick * n : a.vcand + (size_t)(pick - 16) * n)[o];
+                win = pick + 1;
+            }
         }
 #pragma unroll 1
         for (int i = 0; i < 15; ++i) (void)rng_float(rng);   /* the draws of candidates 10-16 */
@@ -1898,60 +1866,44 @@ cudaError_t pm_launch_cost_field(const PmPassArgs& a, bool exact, const float4* 
     return cudaSuccess;
 }
 
-cudaError_t pm_launch_propagate(const PmPassArgs& a, bool exact, cudaStream_t st) {
-    const dim3 grid = a.color < 0 ? pix_grid(a.k.W, a.k.H) : pix_grid((a.k.W + 1) / 2, a.k.H);
-    PmPassArgs b = a;
-    if (b.color >= 0) b.costs = nullptr, b.cand = nullptr;   /* red/black: every candidate by pixel */
-    if (b.cand) {
-        const dim3 g = tap_grid(b, b.viewin ? 3 : 2);
-        if (exact) k_taps_candidates<true><<<g, dim3(32, TP_NP), tp_cand_smem<true>(), st>>>(b);
-        else k_taps_candidates<false><<<g, dim3(32, TP_NP), tp_cand_smem<false>(), st>>>(b);
+static inline dim3 pass_grid(const PmPassArgs& a) {
+    return a.color < 0 ? pix_grid(a.k.W, a.k.H) : pix_grid((a.k.W + 1) / 2, a.k.H);
+}
+
+cudaError_t pm_launch_pass_own(const PmPassArgs& a, bool exact, cudaStream_t st) {
+    if (a.cand) {
+        const size_t smem = exact ? tp_cand_smem<true>() : tp_cand_smem<false>();
+        (exact ? k_taps_candidates<true> : k_taps_candidates<false>)<<<tap_grid(a, 2), dim3(32, TP_NP), smem, st>>>(a, 0);
+    } else if (a.costs) {
+        (exact ? k_sweep<true> : k_sweep<false>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
         PM_LAUNCH_CHECK();
-        if (exact) k_taps_refine<true, 1><<<tap_grid(b), dim3(32, TP_NP + 1), tp_refine_smem<true, 1>(), st>>>(b);
-        else k_taps_refine<false, 1><<<tap_grid(b), dim3(32, TP_NP + 1), tp_refine_smem<false, 1>(), st>>>(b);
-        PM_LAUNCH_CHECK();
-        return cudaSuccess;
+        const dim3 g((a.k.W + 31) / 32, (a.k.H + SH_TY - 1) / SH_TY);
+        (exact ? k_share<true> : k_share<false>)<<<g, dim3(32, SH_TY), share_smem(a.k.P), st>>>(a);
+    } else {
+        (exact ? k_propagate<true, 1> : k_propagate<false, 1>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
     }
-    if (b.costs) {
-        const dim3 sg((a.k.W + 31) / 32, (a.k.H + SH_TY - 1) / SH_TY);
-        const size_t smem = share_smem(a.k.P);
-        if (exact) {
-            k_sweep<true><<<grid, dim3(32, 8), 0, st>>>(b);
-            PM_LAUNCH_CHECK();
-            if (b.viewin) k_views<true><<<grid, dim3(32, 8), 0, st>>>(b);
-            PM_LAUNCH_CHECK();
-            k_share<true><<<sg, dim3(32, SH_TY), smem, st>>>(b);
-            PM_LAUNCH_CHECK();
-            k_propagate<true, 2><<<grid, dim3(32, 8), 0, st>>>(b);
-        } else {
-            k_sweep<false><<<grid, dim3(32, 8), 0, st>>>(b);
-            PM_LAUNCH_CHECK();
-            if (b.viewin) k_views<false><<<grid, dim3(32, 8), 0, st>>>(b);
-            PM_LAUNCH_CHECK();
-            k_share<false><<<sg, dim3(32, SH_TY), smem, st>>>(b);
-            PM_LAUNCH_CHECK();
-            k_propagate<false, 2><<<grid, dim3(32, 8), 0, st>>>(b);
-        }
-        PM_LAUNCH_CHECK();
-        return cudaSuccess;
-    }
-#if PM_PROP_SPLIT
-    if (exact) k_propagate<true, 1><<<grid, dim3(32, 8), 0, st>>>(b);
-    else k_propagate<false, 1><<<grid, dim3(32, 8), 0, st>>>(b);
     PM_LAUNCH_CHECK();
-#if PM_VIEW_SPLIT
-    if (b.viewin) {
-        if (exact) k_propagate<true, 3><<<grid, dim3(32, 8), 0, st>>>(b);
-        else k_propagate<false, 3><<<grid, dim3(32, 8), 0, st>>>(b);
+    return cudaSuccess;
+}
+
+cudaError_t pm_launch_pass_rest(const PmPassArgs& a, bool exact, cudaStream_t st) {
+    if (a.cand) {
+        if (a.viewin) {
+            const size_t smem = exact ? tp_cand_smem<true>() : tp_cand_smem<false>();
+            (exact ? k_taps_candidates<true> : k_taps_candidates<false>)<<<tap_grid(a), dim3(32, TP_NP), smem, st>>>(a, 2);
+            PM_LAUNCH_CHECK();
+        }
+        const size_t smem = exact ? tp_refine_smem<true, 1>() : tp_refine_smem<false, 1>();
+        (exact ? k_taps_refine<true, 1> : k_taps_refine<false, 1>)<<<tap_grid(a), dim3(32, TP_NP + 1), smem, st>>>(a);
+        PM_LAUNCH_CHECK();
+        return cudaSuccess;
+    }
+    if (a.viewin) {
+        if (a.costs) (exact ? k_views<true> : k_views<false>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
+        else (exact ? k_propagate<true, 3> : k_propagate<false, 3>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
         PM_LAUNCH_CHECK();
     }
-#endif
-    if (exact) k_propagate<true, 2><<<grid, dim3(32, 8), 0, st>>>(b);
-    else k_propagate<false, 2><<<grid, dim3(32, 8), 0, st>>>(b);
-#else
-    if (exact) k_propagate<true, 0><<<grid, dim3(32, 8), 0, st>>>(b);
-    else k_propagate<false, 0><<<grid, dim3(32, 8), 0, st>>>(b);
-#endif
+    (exact ? k_propagate<true, 2> : k_propagate<false, 2>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
     PM_LAUNCH_CHECK();
     return cudaSuccess;
 }
@@ -2022,7 +1974,6 @@ bool pm_shared_windows(const PmCostConsts& k) {
     return std::isfinite(k.alpha) && std::isfinite(k.cmax) && std::isfinite(k.gmax);
 }
 bool pm_tap_parallel(const PmCostConsts& k) { return (size_t)k.W * k.H <= TP_MAX_PIXELS && pm_shared_windows(k); }
-size_t pm_tap_parallel_bytes(int W, int H) { return (size_t)20 * W * H * sizeof(float4); }
 
 cudaError_t pm_launch_pd_block(float4* uout, float* pout, const float4* uin, const float* pin, int pzero,
                                const float4* f, const float* wgt, const float* mask, float lambda, int nsteps, int W,
@@ -2158,38 +2109,18 @@ cudaError_t pm_batch_refine(const PmBatch<PmPassArgs>& b, bool exact, const PmBa
     PM_BATCH_LAUNCH((kb_propagate<false, 2>), dim3(32, 8), 0);
 }
 cudaError_t pm_batch_propagate(const PmBatch<PmPassArgs>& b, bool exact, const PmBatchKnobs& kn, cudaStream_t st) {
-#if PM_PROP_SPLIT
-    {
-        const int items_ = b.first[b.n];
-        if (items_ <= 0) return cudaSuccess;
-        if (exact) {
-            kb_propagate<true, 1><<<batch_grid(kb_propagate<true, 1>, 256, 0, items_, kn.grid_mult), dim3(32, 8), 0, st>>>(b);
-            PM_LAUNCH_CHECK();
-#if PM_VIEW_SPLIT
-            if (b.a[0].viewin) {
-                kb_propagate<true, 3><<<batch_grid(kb_propagate<true, 3>, 256, 0, items_, kn.grid_mult), dim3(32, 8), 0, st>>>(b);
-                PM_LAUNCH_CHECK();
-            }
-#endif
-            kb_propagate<true, 2><<<batch_grid(kb_propagate<true, 2>, 256, 0, items_, kn.grid_mult), dim3(32, 8), 0, st>>>(b);
-        } else {
-            kb_propagate<false, 1><<<batch_grid(kb_propagate<false, 1>, 256, 0, items_, kn.grid_mult), dim3(32, 8), 0, st>>>(b);
-            PM_LAUNCH_CHECK();
-#if PM_VIEW_SPLIT
-            if (b.a[0].viewin) {
-                kb_propagate<false, 3><<<batch_grid(kb_propagate<false, 3>, 256, 0, items_, kn.grid_mult), dim3(32, 8), 0, st>>>(b);
-                PM_LAUNCH_CHECK();
-            }
-#endif
-            kb_propagate<false, 2><<<batch_grid(kb_propagate<false, 2>, 256, 0, items_, kn.grid_mult), dim3(32, 8), 0, st>>>(b);
-        }
+    const int items = b.first[b.n];
+    if (items <= 0) return cudaSuccess;
+    auto grid = [&](auto kern) { return batch_grid(kern, 256, 0, items, kn.grid_mult); };
+    if (exact) kb_propagate<true, 1><<<grid(kb_propagate<true, 1>), dim3(32, 8), 0, st>>>(b);
+    else kb_propagate<false, 1><<<grid(kb_propagate<false, 1>), dim3(32, 8), 0, st>>>(b);
+    PM_LAUNCH_CHECK();
+    if (b.a[0].viewin) {
+        if (exact) kb_propagate<true, 3><<<grid(kb_propagate<true, 3>), dim3(32, 8), 0, st>>>(b);
+        else kb_propagate<false, 3><<<grid(kb_propagate<false, 3>), dim3(32, 8), 0, st>>>(b);
         PM_LAUNCH_CHECK();
-        return cudaSuccess;
     }
-#else
-    if (exact) PM_BATCH_LAUNCH((kb_propagate<true, 0>), dim3(32, 8), 0);
-    PM_BATCH_LAUNCH((kb_propagate<false, 0>), dim3(32, 8), 0);
-#endif
+    return pm_batch_refine(b, exact, kn, st);
 }
 cudaError_t pm_batch_view_list(const PmBatch<PmViewListArgs>& b, int maxW, const PmBatchKnobs& kn, cudaStream_t st) {
     PM_BATCH_LAUNCH(kb_view_list, dim3(32), sizeof(int) * (size_t)maxW);

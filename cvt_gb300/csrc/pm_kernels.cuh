@@ -25,8 +25,10 @@ struct PmPassArgs {
     float4* out;
     uint8_t* winners;
     unsigned long long* counters;   /* [0] cost evaluations, [1] in-image taps; may be NULL */
-    float* costs;              /* shared windows: the costs of candidates 9, 16, 17-20, [PM_COST_PLANES][W*H], or NULL */
-    float4* cand;              /* tap-parallel passes: states and costs of candidates 1-20, [20][W*H], or NULL */
+    float* costs;              /* shared windows: the costs of candidates 9 and 16, [2][W*H], or NULL */
+    float* vcosts;             /*   and those of 17-20, [4][W*H] */
+    float4* cand;              /* tap-parallel passes: states and costs of candidates 1-16, [16][W*H], or NULL */
+    float4* vcand;             /*   and those of 17-20, [4][W*H] */
     int color;                 /* -1: every pixel (Jacobi); 0 / 1: pixels with (x + y) & 1 == color */
 };
 
@@ -112,7 +114,11 @@ cudaError_t pm_launch_records(const float4* col, const float4* grad, int W, int 
 cudaError_t pm_launch_init(const PmPassArgs& a, bool exact, cudaStream_t st);
 cudaError_t pm_launch_cost_field(const PmPassArgs& a, bool exact, const float4* states, float* cost,
                                  cudaStream_t st);
-cudaError_t pm_launch_propagate(const PmPassArgs& a, bool exact, cudaStream_t st);
+/* A propagation pass in two parts: candidates 1-16 against a.old into a.out,
+ * which need nothing of the other view; then 17-20 from the other view's
+ * planes and the refinements, in a.out. */
+cudaError_t pm_launch_pass_own(const PmPassArgs& a, bool exact, cudaStream_t st);
+cudaError_t pm_launch_pass_rest(const PmPassArgs& a, bool exact, cudaStream_t st);
 cudaError_t pm_launch_view_list(const float4* src, int W, int H, short4* list, cudaStream_t st);
 cudaError_t pm_launch_consistency(const float4* L, const float4* R, int W, int H, float maxdisp,
                                   float maxangle, int lr, float4* out, uint8_t* valid, cudaStream_t st);
@@ -133,14 +139,12 @@ cudaError_t pm_launch_normal_depth(const float4* in, int W, int H, float depthma
  * call once per device before the first launch or stream capture. */
 cudaError_t pm_prepare_kernels();
 
-#define PM_COST_PLANES 6
 /* Whether passes of these constants can share plane windows, given
- * PmPassArgs::costs. */
+ * PmPassArgs::costs and vcosts. */
 bool pm_shared_windows(const PmCostConsts& k);
 /* Whether passes of these constants run tap-parallel (small images), given
- * PmPassArgs::cand of pm_tap_parallel_bytes. */
+ * PmPassArgs::cand and vcand. */
 bool pm_tap_parallel(const PmCostConsts& k);
-size_t pm_tap_parallel_bytes(int W, int H);
 
 int pm_pd_block_steps();
 /* Bytes of a dual buffer of pm_launch_pd_block: six planes of floats. */

@@ -269,10 +269,10 @@ cvtpm_status cvtpm_polish_planes(cvtpm_ctx* ctx, const float* img1, const float*
                                  void* stream);
 
 /* Device memory the context may use to share work between the candidates of
- * a propagation pass (FAST and EXACT).  With 24 bytes per pixel, planes that
+ * a propagation pass (FAST and EXACT).  With 32 bytes per pixel (24: one view at a time), planes that
  * several pixels test (the neighbour and random-neighbour candidates) have
  * their matching terms formed once per plane; images of at most 60000 pixels
- * use 320 bytes per pixel instead, to run every candidate's window taps in
+ * use 576 (320) instead, to run every candidate's window taps in
  * parallel.  Otherwise (and beyond 60 % of the free memory) every candidate is
  * evaluated per pixel.  Results are identical either way.  Default: no limit;
  * 0 turns both off.  No counterpart in the reference. */

@@ -12,7 +12,8 @@ from cvt_gb300 import scenes
 
 pytestmark = pytest.mark.gpu
 
-PER_PIXEL = {"taps": 320, "windows": 32, "pixel": 0}      # budget, bytes per pixel
+# budget, bytes per pixel: with both views' scratch apart, or one view at a time
+PER_PIXEL = {"taps": 576, "taps_one": 320, "windows": 32, "windows_one": 24, "pixel": 0}
 
 
 def _run(route, p, left, right):
@@ -30,7 +31,7 @@ def _run(route, p, left, right):
 @pytest.mark.parametrize("W,H,patch", [(1, 1, 1), (1, 40, 3), (31, 5, 2), (32, 16, 1), (33, 17, 4), (39, 15, 6),
                                        (64, 33, 5), (65, 9, 31), (70, 50, 17), (97, 4, 9)])
 @pytest.mark.parametrize("exact", [False, True])
-@pytest.mark.parametrize("route", ["taps", "windows", "pixel"])
+@pytest.mark.parametrize("route", list(PER_PIXEL))
 def test_route_bits(cuda, oracle, W, H, patch, exact, route):
     sc = scenes.make_scene(max(W, 6), max(H, 6), 2, 9.0, seed=W * 7 + H)
     left, right = np.ascontiguousarray(sc.left[:H, :W]), np.ascontiguousarray(sc.right[:H, :W])
