@@ -22,9 +22,9 @@
  * S and R (the cost), once for the gradients — so the window weights are
  * recomputed, never stored.  The plane gradient is a register sum; the image
  * terms at the centre pixel are summed in registers, the terms at the window
- * pixel q and at the two interpolation columns of the other image are added
- * with 128-bit float atomics into four accumulators (colour and gradient-
- * image adjoints of each image).  A second kernel pulls the gradient-image
+ * pixel q and at the two interpolation columns of the other image over the
+ * taps that share them (k_cost_adjoint), then added with 128-bit float atomics
+ * into four accumulators (colour and gradient-image adjoints of each image).  A second kernel pulls the gradient-image
  * adjoints back through the transposed 3x3 stencil and the grey weights and
  * writes dL/d(image).  Summation order of the atomics is not fixed, so image
  * gradients vary in the last bits from run to run.
@@ -82,120 +82,215 @@ struct PmAdjArgs {
     float4 *dI1, *dG1, *dI2, *dG2;   /* accumulators (IMG kernels only) */
 };
 
+/* The window sums of a plane at its Q31.32 position (S0, S1, XC at the pixel):
+ * the operations of the FAST evaluator in raster order, two taps' weights at a
+ * time. */
+__device__ __forceinline__ void cost_sums(const PmCostConsts& k, const PmView& v1, const PmView& v2, int x, int y, float4 vc,
+                                          long long S0, long long S1, long long XC, float& ws, float& r1, float& r2) {
+    const int dxlo = max(-k.P, -x), dxhi = min(k.P, k.W - 1 - x);
+    const int qy0 = max(y - k.P, 0), qy1 = min(y + k.P, k.H - 1);
+    ws = r1 = r2 = 0.0f;
+    for (int qy = qy0; qy <= qy1; ++qy) {
+        const float4* c1row = v1.col + (size_t)qy * k.W + x;
+        const float4* g1row = v1.grad + (size_t)qy * k.W + x;
+        const float* prow = c_prof + (qy - y + PM_PMAX) * PM_PROF_N + PM_PMAX;
+        const PmRecRow rrow = rec_row(v2, k.rp, qy);
+        long long X = XC + (long long)(qy - y) * S1 + (long long)dxlo * S0;
+        auto one = [&](float4 a1, float4 g1, float w1) {
+            const long long Xt = X;
+            X += S0;
+            const int xi = (int)(Xt >> 32);
+            if ((unsigned)xi >= (unsigned)k.W) return;
+            float cc, gc;
+            fast_tap_terms(k, rrow, xi, pm_fix_frac(Xt), a1, g1, cc, gc);
+            r1 = fmaf(w1, cc, r1);
+            r2 = fmaf(w1, gc, r2);
+            ws = ws + w1;
+        };
+        int dx = dxlo;
+        for (; dx < dxhi; dx += 2) {
+            const float4 a1 = __ldg(&c1row[dx]), a1b = __ldg(&c1row[dx + 1]);
+            const float4 g1 = __ldg(&g1row[dx]), g1b = __ldg(&g1row[dx + 1]);
+            float w1, w1b;
+            tap_weight2(vc, a1, a1b, prow[dx], prow[dx + 1], w1, w1b);
+            one(a1, g1, w1);
+            one(a1b, g1b, w1b);
+        }
+        if (dx == dxhi) {
+            const float4 a1 = __ldg(&c1row[dx]);
+            one(a1, __ldg(&g1row[dx]), tap_weight(vc, a1, prow[dx]));
+        }
+    }
+}
+
+/* Seven image-adjoint terms: colour 0, 1 | colour 2, gradient image 0 |
+ * gradient image 1, 2 | 3. */
+struct SevenTerms {
+    float2 v0, v1, v2;
+    float v3;
+    __device__ __forceinline__ void add(float w, float2 s0, float2 s1, float2 s2, float s3) {
+        v0 = ffma2(f2s(w), s0, v0);
+        v1 = ffma2(f2s(w), s1, v1);
+        v2 = ffma2(f2s(w), s2, v2);
+        v3 = fmaf(w, s3, v3);
+    }
+    /* takes the terms of the lane above; the last lane starts anew */
+    __device__ __forceinline__ void shift_down(int lane) {
+        float* const v = &v0.x;
+#pragma unroll
+        for (int k = 0; k < 7; ++k) {
+            const float t = __shfl_down_sync(0xffffffffu, v[k], 1);
+            v[k] = lane == 31 ? 0.0f : t;
+        }
+    }
+};
+__device__ __forceinline__ void add_image(float4* dI, float4* dG, size_t o, const SevenTerms& t) {
+    atomicAdd(&dI[o], make_float4(t.v0.x, t.v0.y, t.v1.x, 0.0f));
+    atomicAdd(&dG[o], make_float4(t.v1.y, t.v2.x, t.v2.y, t.v3));
+}
+/* w with the sign of e, 0 for e == 0 (w sgn(e)); with a cap, also 0 where |e| is not below it */
+__device__ __forceinline__ float wsgn(float w, float e) {
+    const float s = __int_as_float(__float_as_int(w) ^ (__float_as_int(e) & 0x80000000));
+    return e > 0.0f || e < 0.0f ? s : 0.0f;
+}
+__device__ __forceinline__ float wsgn(float w, float e, float cap) {
+    const float s = __int_as_float(__float_as_int(w) ^ (__float_as_int(e) & 0x80000000));
+    return fabsf(e) < cap && e != 0.0f ? s : 0.0f;
+}
+
+/* What bounds the gradient sweep is the atomics on the image accumulators: a
+ * tap has terms at one pixel of image 1 and two of image 2, seven floats each,
+ * six 128-bit additions.  Two things take most of them away.  The lanes of a
+ * warp are neighbours in a row and walk the window together, so the image-1
+ * pixel of lane l at offset dx is that of lane l - 1 at dx + 1: its sum moves
+ * down one lane per offset and is added to memory when lane 0 has had its turn
+ * (two additions by one lane, instead of 32).  And a lane's sample moves about
+ * one column per offset, so it holds the sums of the two columns it is between
+ * and adds one to memory when it leaves it (two additions instead of four).
+ * 640x480, 35x35 window (ncu): 8.36 -> 5.27 ms; what bounds it now is
+ * instruction issue (334 per tap over both sweeps, issue 63 %). */
 template <bool IMG>
 __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
-    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
-    const int W = a.k.W, H = a.k.H, P = a.k.P;
-    if (x >= W || y >= H) return;
+    const int W = a.k.W, H = a.k.H, P = a.k.P, lane = threadIdx.x;
+    const int x0 = blockIdx.x * 32, xr = x0 + lane, y = blockIdx.y * 8 + threadIdx.y;
+    if (y >= H) return;                                  /* warp-uniform */
+    const bool inside = xr < W;
+    const int x = min(xr, W - 1);                        /* lanes past the row follow the warp */
     const size_t o = (size_t)y * W + x;
     const float4 pl = a.planes[o];
     const float ds = a.lr ? -1.0f : 1.0f;               /* d(state)/d(plane) */
     long long S0, S1, XC;
     const bool live = fix_plane_d(1.0 + (double)ds * pl.x, (double)ds * pl.y, (double)ds * pl.z, x, y, S0, S1, XC);
     const float4 vc = __ldg(&a.v1.col[o]);
-    const int dxlo = max(-P, -x), dxhi = min(P, W - 1 - x);
 
-    /* sweep 1: the cost (same operations as the FAST evaluator) */
-    float ws = 0.0f, r1 = 0.0f, r2 = 0.0f;
-    for (int dy = -P; dy <= P; ++dy) {
-        const int qy = y + dy;
-        if (qy < 0 || qy >= H) continue;
-        const float* prow = c_prof + (dy + PM_PMAX) * PM_PROF_N + PM_PMAX;
-        long long X = XC + (long long)dy * S1 + (long long)dxlo * S0;
-        for (int dx = dxlo; dx <= dxhi; ++dx) {
-            const long long Xt = X;
-            X += S0;
-            const int xi = (int)(Xt >> 32);
-            if ((unsigned)xi >= (unsigned)W) continue;
-            const size_t q = (size_t)qy * W + x + dx;
-            const float4 a1 = __ldg(&a.v1.col[q]);
-            const float4 g1 = __ldg(&a.v1.grad[q]);
-            const float d = (fabsf(vc.x - a1.x) + fabsf(vc.y - a1.y)) + fabsf(vc.z - a1.z);
-            const float w1 = pm_wexp(-d * prow[dx]);
-            TapVals t;
-            load_tap(a.v2, (size_t)qy * a.k.rp + xi, pm_fix_frac(Xt), t);
-            const float cc = (fminf(fabsf(a1.x - t.v[0]), a.k.cmax) + fminf(fabsf(a1.y - t.v[1]), a.k.cmax)) +
-                             fminf(fabsf(a1.z - t.v[2]), a.k.cmax);
-            const float gc = ((fminf(fabsf(g1.x - t.v[3]), a.k.gmax) + fminf(fabsf(g1.y - t.v[4]), a.k.gmax)) +
-                              fminf(fabsf(g1.z - t.v[5]), a.k.gmax)) + fminf(fabsf(g1.w - t.v[6]), a.k.gmax);
-            r1 = fmaf(w1, cc, r1);
-            r2 = fmaf(w1, gc, r2);
-            ws = ws + w1;
-        }
-    }
+    /* sweep 1: the cost */
+    float ws, r1, r2;
+    cost_sums(a.k, a.v1, a.v2, x, y, vc, S0, S1, XC, ws, r1, r2);
     const bool valid = live && ws > 1.1f;
     const float C = valid ? fmaf(a.k.alpha, r1, a.k.oma * r2) / ws : 1e5f;
-    if (a.cost) a.cost[o] = C;
+    if (a.cost && inside) a.cost[o] = C;
     if (!a.dcost) return;
 
     /* sweep 2: gradients */
     const float g = a.dcost[o];
+    const bool act = inside && valid && g != 0.0f;
     float gs0 = 0.0f, gs1 = 0.0f, gs2 = 0.0f;
-    float cr = 0.0f, cgc = 0.0f, cb = 0.0f;                   /* centre colour */
-    if (valid && g != 0.0f) {
-        const float u = g / ws;
+    float centre[3] = {0.0f, 0.0f, 0.0f};               /* terms of the centre colour */
+    if (__any_sync(0xffffffffu, act)) {
+        const float u = act ? g / ws : 0.0f;
         const float al = a.k.alpha, oma = a.k.oma;
-        for (int dy = -P; dy <= P; ++dy) {
-            const int qy = y + dy;
-            if (qy < 0 || qy >= H) continue;
-            const float* prow = c_prof + (dy + PM_PMAX) * PM_PROF_N + PM_PMAX;
-            long long X = XC + (long long)dy * S1 + (long long)dxlo * S0;
+        const int qy0 = max(y - P, 0), qy1 = min(y + P, H - 1);
+        const int dlo = max(-P, -(x0 + 31)), dhi = min(P, W - 1 - x0);   /* inside the image for some lane */
+        for (int qy = qy0; qy <= qy1; ++qy) {
+            const float* prow = c_prof + (qy - y + PM_PMAX) * PM_PROF_N + PM_PMAX;
+            const size_t rb = (size_t)qy * W;
             const float qyf = (float)qy;
-            for (int dx = dxlo; dx <= dxhi; ++dx) {
+            long long X = XC + (long long)(qy - y) * S1 + (long long)dlo * S0;
+            SevenTerms m = {}, lo = {}, hi = {};         /* image 1 at the lane's tap; image 2 at columns col, col + 1 */
+            int col = -2;
+            const PmRecRow rrow = rec_row(a.v2, a.k.rp, qy);
+            for (int dx = dlo; dx <= dhi; ++dx) {
                 const long long Xt = X;
                 X += S0;
-                const int xi = (int)(Xt >> 32);
-                if ((unsigned)xi >= (unsigned)W) continue;
-                const int qx = x + dx;
-                const size_t q = (size_t)qy * W + qx;
+                if (IMG && dx > dlo) {                   /* column x0 + dx - 1 is complete: lane 0 had it last */
+                    const int qc = x0 + dx - 1;
+                    if (lane == 0 && qc >= 0) add_image(a.dI1, a.dG1, rb + qc, m);
+                    m.shift_down(lane);
+                }
+                const int qx = xr + dx, xi = (int)(Xt >> 32);
+                if (!act || qx < 0 || qx >= W || (unsigned)xi >= (unsigned)W) continue;
+                const size_t q = rb + qx;
                 const float4 a1 = __ldg(&a.v1.col[q]);
                 const float4 g1 = __ldg(&a.v1.grad[q]);
                 const float dcx = vc.x - a1.x, dcy = vc.y - a1.y, dcz = vc.z - a1.z;
                 const float prof = prow[dx];
                 const float w1 = pm_wexp(-((fabsf(dcx) + fabsf(dcy)) + fabsf(dcz)) * prof);
                 const float af = pm_fix_frac(Xt);
-                TapVals t;
-                load_tap(a.v2, (size_t)qy * a.k.rp + xi, af, t);
-                const float e[7] = {a1.x - t.v[0], a1.y - t.v[1], a1.z - t.v[2],
-                                    g1.x - t.v[3], g1.y - t.v[4], g1.z - t.v[5], g1.w - t.v[6]};
-                const float cc = (fminf(fabsf(e[0]), a.k.cmax) + fminf(fabsf(e[1]), a.k.cmax)) + fminf(fabsf(e[2]), a.k.cmax);
-                const float gc = ((fminf(fabsf(e[3]), a.k.gmax) + fminf(fabsf(e[4]), a.k.gmax)) +
-                                  fminf(fabsf(e[5]), a.k.gmax)) + fminf(fabsf(e[6]), a.k.gmax);
+                const float4 A = __ldg(rrow.A + xi), B = __ldg(rrow.B + xi), Cc = __ldg(rrow.C + xi);
+                const float2 D = __ldg(rrow.D + xi);
+                /* residuals of channels (c0, c1), (c2, g0), (g1, g2), g3 */
+                const float2 e0 = fsub2(make_float2(a1.x, a1.y), ffma2(f2s(af), make_float2(B.x, B.y), make_float2(A.x, A.y)));
+                const float2 e1 = fsub2(make_float2(a1.z, g1.x), ffma2(f2s(af), make_float2(B.z, B.w), make_float2(A.z, A.w)));
+                const float2 e2 = fsub2(make_float2(g1.y, g1.z), ffma2(f2s(af), make_float2(Cc.z, Cc.w), make_float2(Cc.x, Cc.y)));
+                const float e3 = g1.w - fmaf(af, D.y, D.x);
+                const float cm = a.k.cmax, gm = a.k.gmax;
+                const float cc = (fminf(fabsf(e0.x), cm) + fminf(fabsf(e0.y), cm)) + fminf(fabsf(e1.x), cm);
+                const float gc = ((fminf(fabsf(e1.y), gm) + fminf(fabsf(e2.x), gm)) + fminf(fabsf(e2.y), gm)) + fminf(fabsf(e3), gm);
                 const float ct = fmaf(al, cc, oma * gc);
                 const float gct = u * w1;                            /* dL/dc_t */
                 const float gdt = -(u * (ct - C)) * (prof * w1);     /* dL/dd_t */
-                float sc[7];
-#pragma unroll
-                for (int k = 0; k < 3; ++k) sc[k] = al * tsgn(e[k], a.k.cmax);
-#pragma unroll
-                for (int k = 3; k < 7; ++k) sc[k] = oma * tsgn(e[k], a.k.gmax);
-                float slope = 0.0f;
-#pragma unroll
-                for (int k = 0; k < 7; ++k) slope = fmaf(sc[k], t.D[k], slope);
+                /* the channels' slopes of c_t: the share with the residual's sign below its truncation */
+                const float2 s0 = make_float2(wsgn(al, e0.x, cm), wsgn(al, e0.y, cm));
+                const float2 s1 = make_float2(wsgn(al, e1.x, cm), wsgn(oma, e1.y, gm));
+                const float2 s2 = make_float2(wsgn(oma, e2.x, gm), wsgn(oma, e2.y, gm));
+                const float s3 = wsgn(oma, e3, gm);
+                float slope = fmaf(s0.y, B.y, s0.x * B.x);
+                slope = fmaf(s1.x, B.z, slope);
+                slope = fmaf(s1.y, B.w, slope);
+                slope = fmaf(s2.x, Cc.z, slope);
+                slope = fmaf(s2.y, Cc.w, slope);
+                slope = fmaf(s3, D.y, slope);
                 const float gx = -gct * slope;                       /* dL/dx' */
                 gs0 = fmaf(gx, (float)qx, gs0);
                 gs1 = fmaf(gx, qyf, gs1);
                 gs2 += gx;
                 if (IMG) {
-                    const float sx = sgnf(dcx), sy = sgnf(dcy), sz = sgnf(dcz);
-                    cr = fmaf(gdt, sx, cr);
-                    cgc = fmaf(gdt, sy, cgc);
-                    cb = fmaf(gdt, sz, cb);
-                    atomicAdd(&a.dI1[q], make_float4(fmaf(gct, sc[0], -gdt * sx), fmaf(gct, sc[1], -gdt * sy),
-                                                     fmaf(gct, sc[2], -gdt * sz), 0.0f));
-                    atomicAdd(&a.dG1[q], make_float4(gct * sc[3], gct * sc[4], gct * sc[5], gct * sc[6]));
-                    const float w0 = -gct * (1.0f - af), w1i = -gct * af;
-                    const size_t j0 = (size_t)qy * W + xi, j1 = (size_t)qy * W + min(xi + 1, W - 1);
-                    atomicAdd(&a.dI2[j0], make_float4(w0 * sc[0], w0 * sc[1], w0 * sc[2], 0.0f));
-                    atomicAdd(&a.dI2[j1], make_float4(w1i * sc[0], w1i * sc[1], w1i * sc[2], 0.0f));
-                    atomicAdd(&a.dG2[j0], make_float4(w0 * sc[3], w0 * sc[4], w0 * sc[5], w0 * sc[6]));
-                    atomicAdd(&a.dG2[j1], make_float4(w1i * sc[3], w1i * sc[4], w1i * sc[5], w1i * sc[6]));
+                    const float dr = wsgn(gdt, dcx), dg = wsgn(gdt, dcy), db = wsgn(gdt, dcz);
+                    centre[0] += dr;
+                    centre[1] += dg;
+                    centre[2] += db;
+                    m.add(gct, s0, s1, s2, s3);
+                    m.v0 = fsub2(m.v0, make_float2(dr, dg));
+                    m.v1.x -= db;
+                    if (xi != col) {
+                        const bool next = xi == col + 1;
+                        if (col >= 0) {
+                            add_image(a.dI2, a.dG2, rb + col, lo);
+                            if (!next) add_image(a.dI2, a.dG2, rb + min(col + 1, W - 1), hi);
+                        }
+                        const SevenTerms zero = {};
+                        lo = next ? hi : zero;
+                        hi = zero;
+                        col = xi;
+                    }
+                    lo.add(-gct * (1.0f - af), s0, s1, s2, s3);
+                    hi.add(-gct * af, s0, s1, s2, s3);
+                }
+            }
+            if (IMG) {                                   /* the row's last columns */
+                const int qc = xr + dhi;
+                if (qc >= 0 && qc < W) add_image(a.dI1, a.dG1, rb + qc, m);
+                if (col >= 0) {
+                    add_image(a.dI2, a.dG2, rb + col, lo);
+                    add_image(a.dI2, a.dG2, rb + min(col + 1, W - 1), hi);
                 }
             }
         }
     }
+    if (!inside) return;
     if (a.dplanes) a.dplanes[o] = make_float4(ds * gs0, ds * gs1, ds * gs2, 0.0f);
-    if (IMG && (cr != 0.0f || cgc != 0.0f || cb != 0.0f)) atomicAdd(&a.dI1[o], make_float4(cr, cgc, cb, 0.0f));
+    if (IMG && (centre[0] != 0.0f || centre[1] != 0.0f || centre[2] != 0.0f))
+        atomicAdd(&a.dI1[o], make_float4(centre[0], centre[1], centre[2], 0.0f));
 }
 
 /* dL/d(image) = colour accumulator + grey weights x (transposed gradient
