@@ -37,18 +37,6 @@
 
 namespace {
 
-/* Fixed-point plane from double state coefficients (see pm_fix_plane). */
-__device__ __forceinline__ bool fix_plane_d(double s0, double s1, double s2, int x, int y, long long& S0,
-                                            long long& S1, long long& XC) {
-    const bool ok0 = isfinite(s0) && isfinite(s1) && isfinite(s2) && fabs(s0) < 16777216.0 && fabs(s1) < 16777216.0;
-    const double xc = ok0 ? __fma_rn(s0, (double)x, __fma_rn(s1, (double)y, s2)) : 0.0;
-    const bool ok = ok0 && fabs(xc) < 1073741824.0;
-    S0 = ok ? __double2ll_rn(s0 * 4294967296.0) : 0;
-    S1 = ok ? __double2ll_rn(s1 * 4294967296.0) : 0;
-    XC = ok ? __double2ll_rn(xc * 4294967296.0) : PM_FIX_NONE;
-    return ok;
-}
-
 __device__ __forceinline__ float sgnf(float v) { return v > 0.0f ? 1.0f : (v < 0.0f ? -1.0f : 0.0f); }
 /* sign(e) inside the truncation, 0 outside (the slope of min(|e|, cap)). */
 __device__ __forceinline__ float tsgn(float e, float cap) { return fabsf(e) < cap ? sgnf(e) : 0.0f; }
@@ -80,6 +68,7 @@ struct PmAdjArgs {
     float* cost;               /* may be NULL */
     float4* dplanes;           /* may be NULL */
     float4 *dI1, *dG1, *dI2, *dG2;   /* accumulators (IMG kernels only) */
+    const float* sums;         /* ROWS kernels: the weight sums, with the costs in `cost` */
 };
 
 /* The window sums of a plane at its Q31.32 position (S0, S1, XC at the pixel):
@@ -168,12 +157,16 @@ __device__ __forceinline__ float wsgn(float w, float e, float cap) {
  * one column per offset, so it holds the sums of the two columns it is between
  * and adds one to memory when it leaves it (two additions instead of four).
  * 640x480, 35x35 window (ncu): 8.36 -> 5.27 ms; what bounds it now is
- * instruction issue (334 per tap over both sweeps, issue 63 %). */
-template <bool IMG>
+ * instruction issue (334 per tap over both sweeps, issue 63 %).
+ *
+ * ROWS: images too small to fill the GPU (pm_tap_parallel) get their costs and
+ * weight sums tap-parallel beforehand, and the 8 warps of a block share the
+ * window rows of one row of 32 pixels. */
+template <bool IMG, bool ROWS>
 __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
     const int W = a.k.W, H = a.k.H, P = a.k.P, lane = threadIdx.x;
-    const int x0 = blockIdx.x * 32, xr = x0 + lane, y = blockIdx.y * 8 + threadIdx.y;
-    if (y >= H) return;                                  /* warp-uniform */
+    const int x0 = blockIdx.x * 32, xr = x0 + lane, y = ROWS ? blockIdx.y : blockIdx.y * 8 + threadIdx.y;
+    if (y >= H) return;                                  /* warp-uniform; no row past the last with ROWS */
     const bool inside = xr < W;
     const int x = min(xr, W - 1);                        /* lanes past the row follow the warp */
     const size_t o = (size_t)y * W + x;
@@ -184,12 +177,20 @@ __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
     const float4 vc = __ldg(&a.v1.col[o]);
 
     /* sweep 1: the cost */
-    float ws, r1, r2;
-    cost_sums(a.k, a.v1, a.v2, x, y, vc, S0, S1, XC, ws, r1, r2);
-    const bool valid = live && ws > 1.1f;
-    const float C = valid ? fmaf(a.k.alpha, r1, a.k.oma * r2) / ws : 1e5f;
-    if (a.cost && inside) a.cost[o] = C;
-    if (!a.dcost) return;
+    float ws, C;
+    bool valid;
+    if (ROWS) {
+        ws = a.sums[o];
+        C = a.cost[o];
+        valid = live && ws > 1.1f;
+    } else {
+        float r1, r2;
+        cost_sums(a.k, a.v1, a.v2, x, y, vc, S0, S1, XC, ws, r1, r2);
+        valid = live && ws > 1.1f;
+        C = valid ? fmaf(a.k.alpha, r1, a.k.oma * r2) / ws : 1e5f;
+        if (a.cost && inside) a.cost[o] = C;
+        if (!a.dcost) return;
+    }
 
     /* sweep 2: gradients */
     const float g = a.dcost[o];
@@ -201,7 +202,7 @@ __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
         const float al = a.k.alpha, oma = a.k.oma;
         const int qy0 = max(y - P, 0), qy1 = min(y + P, H - 1);
         const int dlo = max(-P, -(x0 + 31)), dhi = min(P, W - 1 - x0);   /* inside the image for some lane */
-        for (int qy = qy0; qy <= qy1; ++qy) {
+        for (int qy = qy0 + (ROWS ? (int)threadIdx.y : 0); qy <= qy1; qy += ROWS ? 8 : 1) {
             const float* prow = c_prof + (qy - y + PM_PMAX) * PM_PROF_N + PM_PMAX;
             const size_t rb = (size_t)qy * W;
             const float qyf = (float)qy;
@@ -287,6 +288,20 @@ __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
             }
         }
     }
+    if (ROWS) {                                          /* the warps' sums, in warp order */
+        __shared__ float part[8][6][32];
+        const float v[6] = {gs0, gs1, gs2, centre[0], centre[1], centre[2]};
+#pragma unroll
+        for (int k = 0; k < 6; ++k) part[threadIdx.y][k][lane] = v[k];
+        __syncthreads();
+        if (threadIdx.y) return;
+        float t[6] = {};
+        for (int w = 0; w < 8; ++w)
+#pragma unroll
+            for (int k = 0; k < 6; ++k) t[k] += part[w][k][lane];
+        gs0 = t[0]; gs1 = t[1]; gs2 = t[2];
+        centre[0] = t[3]; centre[1] = t[4]; centre[2] = t[5];
+    }
     if (!inside) return;
     if (a.dplanes) a.dplanes[o] = make_float4(ds * gs0, ds * gs1, ds * gs2, 0.0f);
     if (IMG && (centre[0] != 0.0f || centre[1] != 0.0f || centre[2] != 0.0f))
@@ -329,13 +344,14 @@ cudaError_t pm_adjoint_upload_profile(const float* prof, cudaStream_t st) {
 
 cudaError_t pm_launch_cost_adjoint(const PmCostConsts& k, const PmView& v1, const PmView& v2, const float4* planes,
                                    int lr, const float* dcost, float* cost, float4* dplanes, float4* dI1, float4* dG1,
-                                   float4* dI2, float4* dG2, cudaStream_t st) {
+                                   float4* dI2, float4* dG2, const float* sums, cudaStream_t st) {
     PmAdjArgs a;
+    a.sums = sums;
     a.k = k; a.v1 = v1; a.v2 = v2; a.planes = planes; a.lr = lr; a.dcost = dcost; a.cost = cost;
     a.dplanes = dplanes; a.dI1 = dI1; a.dG1 = dG1; a.dI2 = dI2; a.dG2 = dG2;
-    dim3 grid((k.W + 31) / 32, (k.H + 7) / 8), block(32, 8);
-    if (dI1) k_cost_adjoint<true><<<grid, block, 0, st>>>(a);
-    else k_cost_adjoint<false><<<grid, block, 0, st>>>(a);
+    const dim3 grid((k.W + 31) / 32, sums ? k.H : (k.H + 7) / 8), block(32, 8);
+    if (sums) (dI1 ? k_cost_adjoint<true, true> : k_cost_adjoint<false, true>)<<<grid, block, 0, st>>>(a);
+    else (dI1 ? k_cost_adjoint<true, false> : k_cost_adjoint<false, false>)<<<grid, block, 0, st>>>(a);
     return cudaGetLastError();
 }
 

@@ -1108,8 +1108,15 @@ cvtpm_status cvtpm_cost_adjoint(cvtpm_ctx* ctx, const float* img1, const float* 
     if (img) {
         for (float4* b : {dI1, dG1, dI2, dG2}) CK(cudaMemsetAsync(b, 0, n * 16, st), "adjoint clear");
     }
-    LK(pm_launch_cost_adjoint(a.k, a.v1, a.v2, (const float4*)planes, lr, dcost, cost, (float4*)dplanes,
-                              img ? dI1 : nullptr, dG1, dI2, dG2, st), "cost adjoint");
+    float* sums = nullptr;
+    if (pm_tap_parallel(a.k)) {                      /* small images: costs and weight sums first, into free scratch */
+        sums = (float*)ctx->smooth[0];
+        if (!cost) cost = (float*)ctx->smooth[1];
+        LK(pm_launch_plane_sums(a, (const float4*)planes, lr, cost, sums, st), "plane sums");
+    }
+    if (!sums || dcost)
+        LK(pm_launch_cost_adjoint(a.k, a.v1, a.v2, (const float4*)planes, lr, dcost, cost, (float4*)dplanes,
+                                  img ? dI1 : nullptr, dG1, dI2, dG2, sums, st), "cost adjoint");
     if (dimg1) LK(pm_launch_adjoint_finish(dI1, dG1, width, height, dimg1, st), "adjoint image 1");
     if (dimg2) LK(pm_launch_adjoint_finish(dI2, dG2, width, height, dimg2, st), "adjoint image 2");
     return CVTPM_OK;

@@ -311,17 +311,12 @@ PM_DEV float tap_weight(float4 vc, float4 a1, float prof) {
     return pm_wexp(-d * prof);
 }
 
-/* tap_weight of two taps (colours a, b; profile values pa, pb) on packed
- * pairs: each half of every packed operation is the scalar operation
- * tap_weight and pm_wexp perform on that tap, so wa and wb are their floats.
- * -d * prof is formed as -(d * prof) (the same float: RN is symmetric), and
- * fmaf(-kf, c, r) as a fused kf * (-c) + r (the same exact product). */
-PM_DEV void tap_weight2(float4 vc, float4 a, float4 b, float pa, float pb, float& wa, float& wb) {
-    const float2 ex = fsub2(f2s(vc.x), make_float2(a.x, b.x));
-    const float2 ey = fsub2(f2s(vc.y), make_float2(a.y, b.y));
-    const float2 ez = fsub2(f2s(vc.z), make_float2(a.z, b.z));
-    const float da = (fabsf(ex.x) + fabsf(ey.x)) + fabsf(ez.x);
-    const float db = (fabsf(ex.y) + fabsf(ey.y)) + fabsf(ez.y);
+/* exp(-d * prof) of two colour distances on packed pairs: each half of every
+ * packed operation is the scalar operation tap_weight and pm_wexp perform on
+ * it, so wa and wb are their floats.  -d * prof is formed as -(d * prof) (the
+ * same float: RN is symmetric), and fmaf(-kf, c, r) as a fused kf * (-c) + r
+ * (the same exact product). */
+PM_DEV void weight_pair(float da, float db, float pa, float pb, float& wa, float& wb) {
     const float2 y = fmul2(make_float2(da, db), make_float2(pa, pb));
     const float2 xc = make_float2(fminf(fmaxf(-y.x, -87.3f), 88.7f), fminf(fmaxf(-y.y, -87.3f), 88.7f));
     const float2 big = ffma2(xc, f2s(1.44269504088896341f), f2s(12582912.0f));
@@ -338,6 +333,34 @@ PM_DEV void tap_weight2(float4 vc, float4 a, float4 b, float pa, float pb, float
     p = ffma2(p, r, f2s(1.0f));
     wa = __int_as_float(__float_as_int(p.x) + ((__float_as_int(big.x) - 0x4B400000) << 23));
     wb = __int_as_float(__float_as_int(p.y) + ((__float_as_int(big.y) - 0x4B400000) << 23));
+}
+
+/* tap_weight of two taps (colours a, b; profile values pa, pb) of one centre. */
+PM_DEV void tap_weight2(float4 vc, float4 a, float4 b, float pa, float pb, float& wa, float& wb) {
+    const float2 ex = fsub2(f2s(vc.x), make_float2(a.x, b.x));
+    const float2 ey = fsub2(f2s(vc.y), make_float2(a.y, b.y));
+    const float2 ez = fsub2(f2s(vc.z), make_float2(a.z, b.z));
+    weight_pair((fabsf(ex.x) + fabsf(ey.x)) + fabsf(ez.x), (fabsf(ex.y) + fabsf(ey.y)) + fabsf(ez.y), pa, pb, wa, wb);
+}
+
+/* Fixed-point plane from double state coefficients, anchored at pixel (x, y)
+ * (see pm_fix_plane). */
+PM_DEV bool fix_plane_d(double s0, double s1, double s2, int x, int y, long long& S0, long long& S1, long long& XC) {
+    const bool ok0 = isfinite(s0) && isfinite(s1) && isfinite(s2) && fabs(s0) < 16777216.0 && fabs(s1) < 16777216.0;
+    const double xc = ok0 ? __fma_rn(s0, (double)x, __fma_rn(s1, (double)y, s2)) : 0.0;
+    const bool ok = ok0 && fabs(xc) < 1073741824.0;
+    S0 = ok ? __double2ll_rn(s0 * 4294967296.0) : 0;
+    S1 = ok ? __double2ll_rn(s1 * 4294967296.0) : 0;
+    XC = ok ? __double2ll_rn(xc * 4294967296.0) : PM_FIX_NONE;
+    return ok;
+}
+
+/* tap_weight of one tap (colour a1) for two centres, as tap_weight2. */
+PM_DEV void tap_weight_centres(float4 va, float4 vb, float4 a1, float pa, float pb, float& wa, float& wb) {
+    const float2 ex = fsub2(make_float2(va.x, vb.x), f2s(a1.x));
+    const float2 ey = fsub2(make_float2(va.y, vb.y), f2s(a1.y));
+    const float2 ez = fsub2(make_float2(va.z, vb.z), f2s(a1.z));
+    weight_pair((fabsf(ex.x) + fabsf(ey.x)) + fabsf(ez.x), (fabsf(ex.y) + fabsf(ey.y)) + fabsf(ez.y), pa, pb, wa, wb);
 }
 
 #ifdef PM_KERNELS_TU
@@ -473,6 +496,66 @@ PM_DEV void eval_costs(const PmCostConsts& k, const PmView& v1, const PmView& v2
         float v;
         if (EXACT) v = r1[c] / ws[c];
         else v = fmaf(k.alpha, r1[c], k.oma * r2[c]) / ws[c];
+        cost[c] = (!live[c] || ws[c] <= 1.1f) ? 1e5f : v;
+    }
+}
+
+/* The FAST costs of plane s[0] at pixel (x, y) and s[1] at (x, y + 1), the
+ * pixels below each other sharing the image-1 reads of the window rows they
+ * have in common: eval_costs' operations in its order, so its bits.  The second pixel
+ * is left out (cost 1e5) where `two` is false. */
+PM_DEV void eval_column(const PmCostConsts& k, const PmView& v1, const PmView& v2, int x, int y, bool two,
+                        const float4 (&s)[2], float (&cost)[2]) {
+    const int P = k.P;
+    const int dxlo = max(-P, -x), dxhi = min(P, k.W - 1 - x);
+    const int qy0 = max(y - P, 0), qy1 = min(y + P + 1, k.H - 1);
+    long long S0[2], D[2], X[2];
+    bool live[2];
+    float ws[2], r1[2], r2[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        live[c] = (c == 0 || two) && finite3(s[c]);
+        long long S1, XC;
+        pm_fix_plane(live[c], s[c].x, s[c].y, s[c].z, k.W / 2, k.H / 2, &S0[c], &S1, &XC);
+        X[c] = XC + (long long)(qy0 - k.H / 2) * S1 + (long long)(x + dxlo - k.W / 2) * S0[c];
+        D[c] = S1 - (long long)(dxhi - dxlo + 1) * S0[c];
+        ws[c] = r1[c] = r2[c] = 0.0f;
+    }
+    const size_t o = (size_t)y * k.W + x;
+    const float4 va = __ldg(&v1.col[o]), vb = __ldg(&v1.col[two ? o + k.W : o]);
+    for (int qy = qy0; qy <= qy1; ++qy) {
+        const bool run[2] = {qy <= y + P, qy >= y + 1 - P};
+        const float4* c1row = v1.col + (size_t)qy * k.W + x;
+        const float4* g1row = v1.grad + (size_t)qy * k.W + x;
+        const float* pa = c_prof + (min(qy - y, P) + PM_PMAX) * PM_PROF_N + PM_PMAX;
+        const float* pb = c_prof + (max(qy - y - 1, -P) + PM_PMAX) * PM_PROF_N + PM_PMAX;
+        const PmRecRow rrow = rec_row(v2, k.rp, qy);
+#pragma unroll 2
+        for (int dx = dxlo; dx <= dxhi; ++dx) {
+            const float4 a1 = __ldg(&c1row[dx]);
+            const float4 g1 = __ldg(&g1row[dx]);
+            float w[2];
+            tap_weight_centres(va, vb, a1, pa[dx], pb[dx], w[0], w[1]);
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const long long Xt = X[c];
+                X[c] += S0[c];
+                const int xi = (int)(Xt >> 32);
+                if (!run[c] || (unsigned)xi >= (unsigned)k.W) continue;
+                float cc, gc;
+                fast_tap_terms(k, rrow, xi, pm_fix_frac(Xt), a1, g1, cc, gc);
+                const float2 r = ffma2(make_float2(w[c], w[c]), make_float2(cc, gc), make_float2(r1[c], r2[c]));
+                r1[c] = r.x;                       /* fmaf(w, cc, r1), fmaf(w, gc, r2) */
+                r2[c] = r.y;
+                ws[c] = ws[c] + w[c];
+            }
+        }
+        X[0] += D[0];
+        X[1] += D[1];
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        const float v = fmaf(k.alpha, r1[c], k.oma * r2[c]) / ws[c];
         cost[c] = (!live[c] || ws[c] <= 1.1f) ? 1e5f : v;
     }
 }

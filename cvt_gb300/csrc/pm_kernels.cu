@@ -15,7 +15,7 @@
  *  k_fill_state         pmhstereo_fill_state (:466-510)
  *  k_pd_step            PDHuberWeighted (PDHuberWeighted.cl:34-104)
  *  k_fill_output        pmhstereo_fill_depthmap / fill_normalmap (:512-603)
- *  k_cost_field<EXACT>  the cost of a fixed state field (test/adjoint entry)
+ *  k_cost_field_*       the cost of a fixed state field
  */
 #define PM_KERNELS_TU 1
 #include "pm_kernels.cuh"
@@ -125,15 +125,33 @@ PM_DEV void init_tile(const PmPassArgs& a, int tbx, int tby) {
 template <bool EXACT>
 __global__ void __launch_bounds__(256) k_init(PmPassArgs a) { init_tile<EXACT>(a, blockIdx.x, blockIdx.y); }
 
-template <bool EXACT>
-__global__ void __launch_bounds__(256) k_cost_field(PmPassArgs a, const float4* __restrict__ states,
-                                                   float* __restrict__ cost) {
+/* The cost of a state field.  FAST: two pixels of a column per thread, whose
+ * windows share 36 of 37 image-1 rows (the L1 data pipe bounds this sweep:
+ * 85 % busy with one pixel per thread; 640x480 1.50 -> 1.35 ms, 1242x375 2.28
+ * -> 2.08).  EXACT, whose arithmetic outweighs those reads, gains nothing by it
+ * (1.62 against 1.67 ms) and takes one. */
+#define CF_ROWS 2                                    /* warps per block */
+__global__ void __launch_bounds__(32 * CF_ROWS, 8) k_cost_field_fast(PmPassArgs a, const float4* __restrict__ states,
+                                                                    float* __restrict__ cost) {
+    const int x = blockIdx.x * 32 + threadIdx.x, y = 2 * (blockIdx.y * CF_ROWS + threadIdx.y);
+    if (x >= a.k.W || y >= a.k.H) return;
+    const bool two = y + 1 < a.k.H;
+    const size_t o = (size_t)y * a.k.W + x;
+    const float4 s[2] = {states[o], states[two ? o + a.k.W : o]};
+    float c[2];
+    eval_column(a.k, a.v1, a.v2, x, y, two, s, c);
+    cost[o] = c[0];
+    if (two) cost[o + a.k.W] = c[1];
+}
+
+__global__ void __launch_bounds__(256) k_cost_field_exact(PmPassArgs a, const float4* __restrict__ states,
+                                                          float* __restrict__ cost) {
     const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
     if (x >= a.k.W || y >= a.k.H) return;
     float4 s[1] = {states[(size_t)y * a.k.W + x]};
     bool act[1] = {true};
     float c[1];
-    eval_costs<1, EXACT>(a.k, a.v1, a.v2, x, y, s, act, c);
+    eval_costs<1, true>(a.k, a.v1, a.v2, x, y, s, act, c);
     cost[(size_t)y * a.k.W + x] = c[0];
 }
 
@@ -787,7 +805,7 @@ PM_DEV void tp_put_plane(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, int c
  * barrier. */
 template <bool EXACT, int K, int CH, int CW>
 PM_DEV float tp_costs(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, const PmView& v1, const PmView& v2, int x0, int y,
-                      bool live_lane) {
+                      bool live_lane, float* wsum = nullptr) {
     typedef typename TpTerm<EXACT>::type Term;
     constexpr int SLOTS = CH / TP_NP;
     static_assert(SLOTS * TP_NP == CH && SLOTS % 2 == 0, "whole pairs of taps per producer");
@@ -812,7 +830,9 @@ PM_DEV float tp_costs(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, const Pm
 #pragma unroll
             for (int c = 0; c < K; ++c) {
                 const TpPlane<EXACT> p = S.plane[c][lane];
-                X[c] = p.XA + (long long)(qy0 + row - H / 2) * p.S1 + (long long)(x + dlo + col - W / 2) * p.S0;
+                X[c] = (long long)((unsigned long long)p.XA +
+                                   (unsigned long long)(qy0 + row - H / 2) * (unsigned long long)p.S1 +
+                                   (unsigned long long)(x + dlo + col - W / 2) * (unsigned long long)p.S0);
                 SN[c] = (long long)TP_NP * p.S0;     /* to the producer's next tap */
                 SW[c] = p.S1 - (long long)nx * p.S0; /* on each row end it passes */
             }
@@ -904,6 +924,7 @@ PM_DEV float tp_costs(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, const Pm
         if (mine) consume(i);
         __syncthreads();
     }
+    if (wsum) *wsum = ws;
     return nb_final<EXACT>(k, live_lane, r1, r2, ws);
 }
 
@@ -1055,6 +1076,43 @@ __global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_refine(PmPassArgs 
     if (MODE == 1 && owner) pass_counters(a, inside, x, y, 18 + nview);
 }
 
+/* The cost of a state field, one plane per pixel.  PLANES: of planes (a, b, c)
+ * at the positions of the adjoint (formed in double), with the weight sums. */
+template <bool EXACT, bool PLANES>
+__global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_field(PmPassArgs a, const float4* __restrict__ field, int lr,
+                                                                   float* __restrict__ cost, float* __restrict__ sums) {
+    extern __shared__ __align__(16) unsigned char tp_smem[];
+    TpShared<EXACT, 1, TP_CH1>& S = *reinterpret_cast<TpShared<EXACT, 1, TP_CH1>*>(tp_smem);
+    const int W = a.k.W, x0 = blockIdx.x * 32, y = blockIdx.y, lane = threadIdx.x, x = min(x0 + lane, W - 1);
+    const bool owner = threadIdx.y == TP_NP;
+    const size_t o = (size_t)y * W + x;
+    bool live = false;
+    if (owner) {
+        const float4 s = field[o];
+        if (lane == 0) S.live = 0;
+        if constexpr (PLANES) {
+            const float ds = lr ? -1.0f : 1.0f;
+            TpPlane<EXACT> p;
+            live = fix_plane_d(1.0 + (double)ds * s.x, (double)ds * s.y, (double)ds * s.z, x, y, p.S0, p.S1, p.XA);
+            /* from the pixel to the image centre; modulo 2^64, as steep planes pass it */
+            p.XA = (long long)((unsigned long long)p.XA - (unsigned long long)(y - a.k.H / 2) * (unsigned long long)p.S1 -
+                               (unsigned long long)(x - W / 2) * (unsigned long long)p.S0);
+            S.plane[0][lane] = p;
+            if (__any_sync(0xffffffffu, live) && lane == 0) S.live = 1;
+        } else {
+            live = finite3(s);
+            tp_put_plane(S, a.k, 0, s, true);
+        }
+    }
+    float ws = 0.0f;
+    const float c = tp_costs<EXACT, 1, TP_CH1, TP_NP>(S, a.k, a.v1, a.v2, x0, y, live, &ws);
+    if (owner && x0 + lane < W) {
+        cost[o] = c;
+        if (PLANES) sums[o] = ws;
+    }
+}
+
+template <bool EXACT> constexpr size_t tp_field_smem() { return sizeof(TpShared<EXACT, 1, TP_CH1>); }
 template <bool EXACT> constexpr size_t tp_cand_smem() { return sizeof(TpShared<EXACT, TP_K, TP_CH>); }
 template <bool EXACT, int MODE> constexpr size_t tp_refine_smem() {
     return sizeof(TpShared<EXACT, 1, TP_CH1>) + (MODE == 1 ? sizeof(TpBest) * 20 * 32 : 0);
@@ -1860,8 +1918,22 @@ cudaError_t pm_launch_init(const PmPassArgs& a, bool exact, cudaStream_t st) {
 }
 
 cudaError_t pm_launch_cost_field(const PmPassArgs& a, bool exact, const float4* states, float* cost, cudaStream_t st) {
-    if (exact) k_cost_field<true><<<pix_grid(a.k.W, a.k.H), dim3(32, 8), 0, st>>>(a, states, cost);
-    else k_cost_field<false><<<pix_grid(a.k.W, a.k.H), dim3(32, 8), 0, st>>>(a, states, cost);
+    const int W = a.k.W, H = a.k.H;
+    if (pm_tap_parallel(a.k)) {
+        const size_t smem = exact ? tp_field_smem<true>() : tp_field_smem<false>();
+        (exact ? k_taps_field<true, false> : k_taps_field<false, false>)<<<tap_grid(a), dim3(32, TP_NP + 1), smem, st>>>(
+            a, states, 0, cost, nullptr);
+    } else if (exact) {
+        k_cost_field_exact<<<pix_grid(W, H), dim3(32, 8), 0, st>>>(a, states, cost);
+    } else {
+        k_cost_field_fast<<<dim3((W + 31) / 32, (H + 2 * CF_ROWS - 1) / (2 * CF_ROWS)), dim3(32, CF_ROWS), 0, st>>>(a, states, cost);
+    }
+    PM_LAUNCH_CHECK();
+    return cudaSuccess;
+}
+
+cudaError_t pm_launch_plane_sums(const PmPassArgs& a, const float4* planes, int lr, float* cost, float* ws, cudaStream_t st) {
+    k_taps_field<false, true><<<tap_grid(a), dim3(32, TP_NP + 1), tp_field_smem<false>(), st>>>(a, planes, lr, cost, ws);
     PM_LAUNCH_CHECK();
     return cudaSuccess;
 }
@@ -1955,6 +2027,9 @@ cudaError_t pm_prepare_kernels() {
     smem((const void*)k_taps_candidates<false>, tp_cand_smem<false>());
     smem((const void*)k_taps_refine<true, 0>, tp_refine_smem<true, 0>());
     smem((const void*)k_taps_refine<false, 0>, tp_refine_smem<false, 0>());
+    smem((const void*)k_taps_field<true, false>, tp_field_smem<true>());
+    smem((const void*)k_taps_field<false, false>, tp_field_smem<false>());
+    smem((const void*)k_taps_field<false, true>, tp_field_smem<false>());
     smem((const void*)k_taps_refine<true, 1>, tp_refine_smem<true, 1>());
     smem((const void*)k_taps_refine<false, 1>, tp_refine_smem<false, 1>());
     if (e != cudaSuccess) return e;

@@ -112,6 +112,9 @@ cudaError_t pm_launch_prep(const float4* img, size_t pitch4, int W, int H, float
 cudaError_t pm_launch_records(const float4* col, const float4* grad, int W, int H, int rp, float4* A, float4* B,
                               float4* C, float2* D, cudaStream_t st);
 cudaError_t pm_launch_init(const PmPassArgs& a, bool exact, cudaStream_t st);
+/* The FAST cost and weight sum of a plane field (a, b, c) of an image that
+ * pm_tap_parallel takes, at the adjoint's positions and with its bits. */
+cudaError_t pm_launch_plane_sums(const PmPassArgs& a, const float4* planes, int lr, float* cost, float* ws, cudaStream_t st);
 cudaError_t pm_launch_cost_field(const PmPassArgs& a, bool exact, const float4* states, float* cost,
                                  cudaStream_t st);
 /* A propagation pass in two parts: candidates 1-16 against a.old into a.out,
@@ -156,9 +159,11 @@ cudaError_t pm_launch_ffma_peak(float* out, int blocks, int iters, cudaStream_t 
 
 /* pm_adjoint.cu */
 cudaError_t pm_adjoint_upload_profile(const float* prof, cudaStream_t st);
+/* sums: the weight sums of pm_launch_plane_sums, whose costs are in `cost`
+ * (small images); NULL: the kernel forms both. */
 cudaError_t pm_launch_cost_adjoint(const PmCostConsts& k, const PmView& v1, const PmView& v2, const float4* planes,
                                    int lr, const float* dcost, float* cost, float4* dplanes, float4* dI1, float4* dG1,
-                                   float4* dI2, float4* dG2, cudaStream_t st);
+                                   float4* dI2, float4* dG2, const float* sums, cudaStream_t st);
 cudaError_t pm_launch_adjoint_finish(const float4* dI, const float4* dG, int W, int H, float* out, cudaStream_t st);
 cudaError_t pm_launch_gn_polish(const PmCostConsts& k, const PmView& v1, const PmView& v2, float4* planes, int lr,
                                 int steps, float* cost, cudaStream_t st);

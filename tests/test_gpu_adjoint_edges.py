@@ -13,7 +13,8 @@ from cvt_gb300.params import PRESET_BASELINE, default_params
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("W,H,patch", [(1, 1, 2), (5, 30, 3), (31, 7, 2), (32, 6, 4), (33, 9, 3), (66, 5, 6), (70, 12, 1)])
+@pytest.mark.parametrize("W,H,patch", [(1, 1, 2), (5, 30, 3), (31, 7, 2), (32, 6, 4), (33, 9, 3), (66, 5, 6), (70, 12, 1),
+                                       (301, 203, 2)])      # above 60000 pixels: a thread per pixel
 @pytest.mark.parametrize("lr", [1, 0])
 def test_adjoint_edges(cuda, oracle, W, H, patch, lr):
     from cvt_gb300.stereo import PMHuberStereo

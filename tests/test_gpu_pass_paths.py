@@ -65,3 +65,18 @@ def test_route_special_values(cuda, oracle, route, what):
     assert np.array_equal(ex["winners"], wex["winners"])
     assert not bit_diff(ex["states"], wex["states"]).any()
     assert not bit_diff(got, want).any()
+
+
+@pytest.mark.parametrize("W,H,patch", [(33, 7, 3), (301, 203, 2), (64, 941, 1)])      # below and above 60000 pixels
+@pytest.mark.parametrize("exact", [False, True])
+def test_cost_field_bits(cuda, oracle, W, H, patch, exact):
+    from cvt_gb300.stereo import PMHuberStereo
+    rng = np.random.default_rng(W + H)
+    left, right = rng.random((H, W, 4), np.float32), rng.random((H, W, 4), np.float32)
+    s = np.zeros((H, W, 4), np.float32)
+    s[..., 0] = rng.choice([1.0, 0.9, 1.4, -0.7, np.nan], (H, W))
+    s[..., 1] = rng.uniform(-0.3, 0.3, (H, W))
+    s[..., 2] = rng.uniform(-4, W / 3, (H, W))
+    p = P.default_params(P.PRESET_REFERENCE if exact else P.PRESET_BASELINE, patchsize=patch)
+    got = PMHuberStereo(0, p).cost(*(torch.from_numpy(t).cuda() for t in (left, right, s)))
+    assert not bit_diff(got.cpu().numpy(), oracle.cost_field(p, left, right, s)).any()
