@@ -159,7 +159,7 @@ __device__ __forceinline__ float wsgn(float w, float e, float cap) {
  * 640x480, 35x35 window (ncu): 8.36 -> 5.27 ms; what bounds it now is
  * instruction issue (334 per tap over both sweeps, issue 63 %).
  *
- * ROWS: images too small to fill the GPU (pm_tap_parallel) get their costs and
+ * ROWS: images too small to fill the GPU (pm_tap_field) get their costs and
  * weight sums tap-parallel beforehand, and the 8 warps of a block share the
  * window rows of one row of 32 pixels. */
 template <bool IMG, bool ROWS>

@@ -1109,7 +1109,7 @@ cvtpm_status cvtpm_cost_adjoint(cvtpm_ctx* ctx, const float* img1, const float* 
         for (float4* b : {dI1, dG1, dI2, dG2}) CK(cudaMemsetAsync(b, 0, n * 16, st), "adjoint clear");
     }
     float* sums = nullptr;
-    if (pm_tap_parallel(a.k)) {                      /* small images: costs and weight sums first, into free scratch */
+    if (pm_tap_field(a.k)) {                         /* small images: costs and weight sums first, into free scratch */
         sums = (float*)ctx->smooth[0];
         if (!cost) cost = (float*)ctx->smooth[1];
         LK(pm_launch_plane_sums(a, (const float4*)planes, lr, cost, sums, st), "plane sums");

@@ -471,8 +471,8 @@ PM_DEV float4 smooth_state(float4 smooth, float cx, float cy, int lr) {
  * cost a window of record loads, which is what bounds this path (the L1 data
  * pipe).
  *
- * A block owns 32 x SH_TY pixels and the planes they can draw: 40 x (SH_TY + 8)
- * slots, slot (sx, sy) holding the plane of pixel (x0 - 1 + sx, y0 - 1 + sy)
+ * A block owns 32 x ty pixels (ty <= SH_TY) and the planes they can draw: 40 x
+ * (ty + 8) slots, slot (sx, sy) holding the plane of pixel (x0 - 1 + sx, y0 - 1 + sy)
  * clamped to the image, so a candidate's slot follows from its offset alone,
  * also at the border.  The block walks the image rows its windows reach, and
  * each row by the window offset rx, four at a time: the threads form the terms
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(256, 3) k_views(PmPassArgs a) { views_tile<EXA
 /* The candidates 1-16 of a pixel against its old state: 9 and 16 have their
  * costs in a.costs, the others are formed here.  The best goes to a.out. */
 template <bool EXACT>
-PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
+PM_DEV void share_tile(const PmPassArgs& a, int ty, int tbx, int tby) {
     typedef typename ShTerm<EXACT>::type Term;
     constexpr int R = ShTerm<EXACT>::R;
     constexpr int SLOTS = (SH_NS + SH_NT - 1) / SH_NT;
@@ -571,7 +571,7 @@ PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
     float4* const rows = reinterpret_cast<float4*>(sh_smem + (size_t)SH_NS * 128);
     const int W = a.k.W, H = a.k.H, P = a.k.P, NQ = 32 + 2 * P;
     const int lane = threadIdx.x, w = threadIdx.y, tid = w * 32 + lane;
-    const int x0 = tbx * 32, y0 = tby * SH_TY;
+    const int x0 = tbx * 32, y0 = tby * ty, ylast = min(y0 + ty, H) - 1;
     const size_t n = (size_t)W * H;
     /* plane role: SLOTS slots of one column, SH_NY / SLOTS rows apart, whose
      * taps share the image-1 reads */
@@ -581,7 +581,7 @@ PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
     int slo[SLOTS], shi[SLOTS];                      /* image rows the slot is needed at */
     long long S0[SLOTS], S1[SLOTS], X[SLOTS];
     float sx[SLOTS], sy[SLOTS], sz[SLOTS];
-    const int t0 = max(y0 - P, 0), t1 = min(min(y0 + SH_TY - 1, H - 1) + P, H - 1);
+    const int t0 = max(y0 - P, 0), t1 = min(ylast + P, H - 1);
 #pragma unroll
     for (int i = 0; i < SLOTS; ++i) {
         const int my = y0 - 1 + prow0 + i * (SH_NY / SLOTS);
@@ -589,7 +589,7 @@ PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
         long long XA;
         nb_plane<EXACT>(a.k, st, finite3(st), sx[i], sy[i], sz[i], S0[i], S1[i], XA);
         slo[i] = max(y0, my - 7) - P;
-        shi[i] = plane ? min(min(y0 + SH_TY - 1, H - 1), my + 1) + P : -1;
+        shi[i] = plane && my - 7 <= ylast ? min(ylast, my + 1) + P : -1;
         /* the position at column mx - P - 7, row t0 */
         X[i] = XA + (long long)(t0 - H / 2) * S1[i] + (long long)(mx - P - 7 - W / 2) * S0[i];
     }
@@ -694,7 +694,7 @@ PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
     for (int Yq = t0; Yq <= t1; ++Yq) {
         const int buf = (Yq - t0) & 1;
         if (Yq < t1) stage(Yq + 1, buf ^ 1);         /* last read before the barrier that ended row Yq - 1 */
-        const bool reads = y < H && abs(Yq - y) <= P;                /* warp-uniform */
+        const bool reads = y <= ylast && abs(Yq - y) <= P;                /* warp-uniform */
         for (int t = 0; t < 3; ++t) produce(Yq, buf, t);
         __syncthreads();
         for (int k = 0; k < nc; ++k) {
@@ -706,7 +706,7 @@ PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
 #pragma unroll
         for (int i = 0; i < SLOTS; ++i) X[i] += S1[i];
     }
-    if (y >= H) return;
+    if (y > ylast) return;
     /* the acceptance, in candidate order */
     const float cx = (float)xc, cy = (float)yc, theta = a.theta;
     const float4 smooth = smooth_at(a, o);
@@ -743,7 +743,7 @@ PM_DEV void share_tile(const PmPassArgs& a, int tbx, int tby) {
 }
 
 template <bool EXACT>
-__global__ void __launch_bounds__(SH_NT, 1) k_share(PmPassArgs a) { share_tile<EXACT>(a, blockIdx.x, blockIdx.y); }
+__global__ void __launch_bounds__(SH_NT, 1) k_share(PmPassArgs a, int ty) { share_tile<EXACT>(a, ty, blockIdx.x, blockIdx.y); }
 
 /* ------------------------------------------------- tap-parallel passes -- */
 /* The propagation of images too small to fill the GPU with one thread per
@@ -928,59 +928,68 @@ PM_DEV float tp_costs(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, const Pm
     return nb_final<EXACT>(k, live_lane, r1, r2, ws);
 }
 
-#define TP_K 8
-#define TP_CH 16       /* taps per chunk of the candidate kernel */
+#define TP_CH 16       /* taps per chunk of the candidate kernels */
 #define TP_CH1 64      /* taps per chunk of the one-candidate kernels */
 
-/* Candidates 1-8 (group 0), 9-16 (1) and 17-20 (2) of 32 pixels: their
- * states with their costs go to a.cand[candidate - 1] and a.vcand[candidate - 17];
- * z0 is the first group. */
-template <bool EXACT>
-__global__ void __launch_bounds__(32 * TP_NP, 2) k_taps_candidates(PmPassArgs a, int z0) {
+/* Candidates of 32 pixels, a group per block: KIND 0 takes 8 of 1-16
+ * (blockIdx.z 0 and 1) and leaves states with their costs in
+ * a.cand[candidate - 1]; KIND 1 takes 9 and 16 and leaves their costs in
+ * a.costs; KIND 2 takes the other view's 17-20 and leaves costs in a.vcosts or,
+ * without it, states with costs in a.vcand. */
+__host__ __device__ constexpr int tp_group(int kind) { return kind == 0 ? 8 : kind == 1 ? 2 : 4; }
+template <bool EXACT, int KIND>
+__global__ void __launch_bounds__(32 * TP_NP, 2) k_taps_candidates(PmPassArgs a) {
+    constexpr int K = tp_group(KIND);
     extern __shared__ __align__(16) unsigned char tp_smem[];
-    TpShared<EXACT, TP_K, TP_CH>& S = *reinterpret_cast<TpShared<EXACT, TP_K, TP_CH>*>(tp_smem);
-    const int W = a.k.W, H = a.k.H, x0 = blockIdx.x * 32, y = blockIdx.y, z = z0 + blockIdx.z;
+    TpShared<EXACT, K, TP_CH>& S = *reinterpret_cast<TpShared<EXACT, K, TP_CH>*>(tp_smem);
+    const int W = a.k.W, H = a.k.H, x0 = blockIdx.x * 32, y = blockIdx.y;
     const int c = threadIdx.y, x = min(x0 + (int)threadIdx.x, W - 1);
+    const int i = KIND == 0 ? blockIdx.z * 8 + c : KIND == 1 ? (c == 0 ? 8 : 15) : 16 + c;   /* the candidate less 1 */
     const size_t n = (size_t)W * H, o = (size_t)y * W + x;
     const float cx = (float)x, cy = (float)y;
     if (c == 0 && threadIdx.x == 0) S.live = 0;
     __syncthreads();
     float4 s = f4s(0.0f);
-    bool act = true;
-    if (z == 0) {                                    /* :330-342 */
-        const int nn = c < 4 ? c : c + 1;
-        s = a.old[(size_t)clampi(y + nn / 3 - 1, 0, H - 1) * W + clampi(x + nn % 3 - 1, 0, W - 1)];
-    } else if (z == 1) {
-        if (c == 0) {                                /* :345-352 */
+    bool act = c < K;
+    if (act) {                                       /* warp-uniform */
+        if (i < 8) {                                 /* :330-342 */
+            const int nn = i < 4 ? i : i + 1;
+            s = a.old[(size_t)clampi(y + nn / 3 - 1, 0, H - 1) * W + clampi(x + nn % 3 - 1, 0, W - 1)];
+        } else if (i == 8) {                         /* :345-352 */
             s = smooth_state(smooth_at(a, o), cx, cy, a.lr);
-        } else {
+        } else if (i < 16) {
             PmRng rng;
             seed_rng(rng, a, x, y, false);
 #pragma unroll 1
-            for (int i = 0; i < 2 * (c - 1); ++i) (void)rng_float(rng);
-            if (c < 7) {                             /* :355-361 */
+            for (int d = 0; d < 2 * (i - 9); ++d) (void)rng_float(rng);
+            if (i < 15) {                            /* :355-361 */
                 const int ox = (int)(rng_float(rng) * 7.0f + 0.5f);
                 const int oy = (int)(rng_float(rng) * 7.0f + 0.5f);
                 s = a.old[(size_t)clampi(y + oy, 0, H - 1) * W + clampi(x + ox, 0, W - 1)];
             } else {
                 s = state_init(rng, cx, cy, a.lr, 2.0f, a.depthmax);   /* :364-368 */
             }
+        } else {                                     /* :372-379 */
+            const short4 l = a.viewin[o];
+            const short e = i == 16 ? l.x : i == 17 ? l.y : i == 18 ? l.z : l.w;
+            act = e >= 0 && x0 + (int)threadIdx.x < W;
+            if (act) s = viewprop(a.viewsrc[(size_t)y * W + e]);
         }
-    } else {                                         /* :372-379 */
-        const short4 l = a.viewin[o];
-        const short e = c == 0 ? l.x : c == 1 ? l.y : c == 2 ? l.z : l.w;
-        act = c < 4 && e >= 0 && x0 + (int)threadIdx.x < W;
-        if (act) s = viewprop(a.viewsrc[(size_t)y * W + e]);
+        tp_put_plane(S, a.k, c, s, act);
     }
-    tp_put_plane(S, a.k, c, s, act);
-    s.w = tp_costs<EXACT, TP_K, TP_CH, 0>(S, a.k, a.v1, a.v2, x0, y, act && finite3(s));
-    if (act && x0 + (int)threadIdx.x < W) (z < 2 ? a.cand + (size_t)(z * 8 + c) * n : a.vcand + (size_t)c * n)[o] = s;
+    s.w = tp_costs<EXACT, K, TP_CH, 0>(S, a.k, a.v1, a.v2, x0, y, act && finite3(s));
+    if (!act || x0 + (int)threadIdx.x >= W) return;
+    if (KIND == 0) a.cand[(size_t)i * n + o] = s;
+    else if (KIND == 1) a.costs[(size_t)c * n + o] = s.w;
+    else if (a.vcosts) a.vcosts[(size_t)c * n + o] = s.w;
+    else a.vcand[(size_t)c * n + o] = s;
 }
 
 /* One candidate per evaluation: warps 0..TP_NP-1 produce, warp TP_NP owns the
  * pixels.  MODE 0: the random initial planes (pmhstereo_init).  MODE 1: the
  * best of a.old and the candidates in a.cand and a.vcand, then the two refinements.
- * MODE 2: the refinements of the best so far in a.out. */
+ * MODE 2: the best of a.out and the view candidates with a.vcosts, then the
+ * refinements. */
 template <bool EXACT, int MODE>
 __global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_refine(PmPassArgs a) {
     extern __shared__ __align__(16) unsigned char tp_smem[];
@@ -1010,11 +1019,12 @@ __global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_refine(PmPassArgs 
     }
     const float4 smooth = smooth_at(a, o);
     int nview = 0;
+    short4 list = make_short4(-1, -1, -1, -1);
+    if (a.viewin) {
+        list = a.viewin[o];
+        nview = list.x < 0 ? 0 : list.y < 0 ? 1 : list.z < 0 ? 2 : list.w < 0 ? 3 : 4;
+    }
     if (MODE == 1) {
-        if (a.viewin) {
-            const short4 l = a.viewin[o];
-            nview = l.x < 0 ? 0 : l.y < 0 ? 1 : l.z < 0 ? 2 : l.w < 0 ? 3 : 4;
-        }
         if (!owner) {                                /* the candidates' distances, spread over the producers */
             for (int i = w; i < 16 + nview; i += TP_NP) {
                 const float4 s = (i < 16 ? a.cand + (size_t)i * n : a.vcand + (size_t)(i - 16) * n)[o];
@@ -1038,6 +1048,16 @@ __global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_refine(PmPassArgs 
             if (pick >= 0) {
                 self = (pick < 16 ? a.cand + (size_t)pick * n : a.vcand + (size_t)(pick - 16) * n)[o];
                 win = pick + 1;
+            }
+        }
+        if (MODE == 2) {
+#pragma unroll 1
+            for (int i = 0; i < nview; ++i) {
+                const short e = i == 0 ? list.x : i == 1 ? list.y : i == 2 ? list.z : list.w;
+                float4 s = viewprop(a.viewsrc[(size_t)y * W + e]);
+                s.w = a.vcosts[(size_t)i * n + o];
+                const TpBest b = {s.w, state_distance(s, smooth, cx, cy, dmax, a.lr), finite3(s)};
+                if (tp_accepts(b, eself, theta)) { self = s; eself = b; win = 17 + i; }
             }
         }
 #pragma unroll 1
@@ -1073,7 +1093,7 @@ __global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_refine(PmPassArgs 
         a.out[o] = self;
         if (a.winners && win >= 0) a.winners[o] = (uint8_t)win;
     }
-    if (MODE == 1 && owner) pass_counters(a, inside, x, y, 18 + nview);
+    if (owner) pass_counters(a, inside, x, y, (MODE == 1 ? 18 : 0) + nview);
 }
 
 /* The cost of a state field, one plane per pixel.  PLANES: of planes (a, b, c)
@@ -1113,7 +1133,7 @@ __global__ void __launch_bounds__(32 * (TP_NP + 1), 2) k_taps_field(PmPassArgs a
 }
 
 template <bool EXACT> constexpr size_t tp_field_smem() { return sizeof(TpShared<EXACT, 1, TP_CH1>); }
-template <bool EXACT> constexpr size_t tp_cand_smem() { return sizeof(TpShared<EXACT, TP_K, TP_CH>); }
+template <bool EXACT, int KIND> constexpr size_t tp_cand_smem() { return sizeof(TpShared<EXACT, tp_group(KIND), TP_CH>); }
 template <bool EXACT, int MODE> constexpr size_t tp_refine_smem() {
     return sizeof(TpShared<EXACT, 1, TP_CH1>) + (MODE == 1 ? sizeof(TpBest) * 20 * 32 : 0);
 }
@@ -1809,7 +1829,7 @@ __global__ void __launch_bounds__(SH_NT, 1) kb_share(const __grid_constant__ PmB
     for (int item = blockIdx.x; item < b.first[b.n]; item += gridDim.x) {
         const int p = batch_pair(b, item), t = item - b.first[p];
         __syncthreads();                                 /* the rings are reused */
-        share_tile<EXACT>(b.a[p], t % b.tx[p], t / b.tx[p]);
+        share_tile<EXACT>(b.a[p], SH_TY, t % b.tx[p], t / b.tx[p]);
     }
 }
 
@@ -1905,7 +1925,7 @@ static inline dim3 pix_grid(int W, int H) { return dim3((W + 31) / 32, (H + 7) /
 static inline dim3 tap_grid(const PmPassArgs& a, int z = 1) { return dim3((a.k.W + 31) / 32, a.k.H, z); }
 
 cudaError_t pm_launch_init(const PmPassArgs& a, bool exact, cudaStream_t st) {
-    if (a.cand) {
+    if (pm_tap_sweeps(a.k)) {
         if (exact) k_taps_refine<true, 0><<<tap_grid(a), dim3(32, TP_NP + 1), tp_refine_smem<true, 0>(), st>>>(a);
         else k_taps_refine<false, 0><<<tap_grid(a), dim3(32, TP_NP + 1), tp_refine_smem<false, 0>(), st>>>(a);
         PM_LAUNCH_CHECK();
@@ -1919,7 +1939,7 @@ cudaError_t pm_launch_init(const PmPassArgs& a, bool exact, cudaStream_t st) {
 
 cudaError_t pm_launch_cost_field(const PmPassArgs& a, bool exact, const float4* states, float* cost, cudaStream_t st) {
     const int W = a.k.W, H = a.k.H;
-    if (pm_tap_parallel(a.k)) {
+    if (pm_tap_field(a.k)) {
         const size_t smem = exact ? tp_field_smem<true>() : tp_field_smem<false>();
         (exact ? k_taps_field<true, false> : k_taps_field<false, false>)<<<tap_grid(a), dim3(32, TP_NP + 1), smem, st>>>(
             a, states, 0, cost, nullptr);
@@ -1942,15 +1962,41 @@ static inline dim3 pass_grid(const PmPassArgs& a) {
     return a.color < 0 ? pix_grid(a.k.W, a.k.H) : pix_grid((a.k.W + 1) / 2, a.k.H);
 }
 
+template <int KIND>
+static void launch_taps(const PmPassArgs& a, bool exact, int groups, cudaStream_t st) {
+    const size_t smem = exact ? tp_cand_smem<true, KIND>() : tp_cand_smem<false, KIND>();
+    (exact ? k_taps_candidates<true, KIND> : k_taps_candidates<false, KIND>)<<<tap_grid(a, groups), dim3(32, TP_NP), smem, st>>>(a);
+}
+template <int MODE>
+static void launch_refine(const PmPassArgs& a, bool exact, cudaStream_t st) {
+    const size_t smem = exact ? tp_refine_smem<true, MODE>() : tp_refine_smem<false, MODE>();
+    (exact ? k_taps_refine<true, MODE> : k_taps_refine<false, MODE>)<<<tap_grid(a), dim3(32, TP_NP + 1), smem, st>>>(a);
+}
+
+/* Rows of a k_share tile: SH_TY, which repeats the fewest planes, unless fewer
+ * let the tiles of both views (they run side by side) fill the SMs once:
+ * 160x120 11.8 ms per depthMap with 16 rows, 10.7 with 8; 240x180, where 16
+ * already fill them, 18.2 and 20.2. */
+static int share_rows(const PmCostConsts& k) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return SH_TY;
+    const int cols = (k.W + 31) / 32;
+    for (int ty = SH_TY / 2; ty < SH_TY; ++ty)
+        if (2 * cols * ((k.H + ty - 1) / ty) <= sms) return ty;
+    return SH_TY;
+}
+
 cudaError_t pm_launch_pass_own(const PmPassArgs& a, bool exact, cudaStream_t st) {
     if (a.cand) {
-        const size_t smem = exact ? tp_cand_smem<true>() : tp_cand_smem<false>();
-        (exact ? k_taps_candidates<true> : k_taps_candidates<false>)<<<tap_grid(a, 2), dim3(32, TP_NP), smem, st>>>(a, 0);
+        launch_taps<0>(a, exact, 2, st);
     } else if (a.costs) {
-        (exact ? k_sweep<true> : k_sweep<false>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
+        if (pm_tap_sweeps(a.k)) launch_taps<1>(a, exact, 1, st);
+        else (exact ? k_sweep<true> : k_sweep<false>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
         PM_LAUNCH_CHECK();
-        const dim3 g((a.k.W + 31) / 32, (a.k.H + SH_TY - 1) / SH_TY);
-        (exact ? k_share<true> : k_share<false>)<<<g, dim3(32, SH_TY), share_smem(a.k.P), st>>>(a);
+        const int ty = share_rows(a.k);
+        const dim3 g((a.k.W + 31) / 32, (a.k.H + ty - 1) / ty);
+        (exact ? k_share<true> : k_share<false>)<<<g, dim3(32, SH_TY), share_smem(a.k.P), st>>>(a, ty);
     } else {
         (exact ? k_propagate<true, 1> : k_propagate<false, 1>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
     }
@@ -1959,23 +2005,16 @@ cudaError_t pm_launch_pass_own(const PmPassArgs& a, bool exact, cudaStream_t st)
 }
 
 cudaError_t pm_launch_pass_rest(const PmPassArgs& a, bool exact, cudaStream_t st) {
-    if (a.cand) {
-        if (a.viewin) {
-            const size_t smem = exact ? tp_cand_smem<true>() : tp_cand_smem<false>();
-            (exact ? k_taps_candidates<true> : k_taps_candidates<false>)<<<tap_grid(a), dim3(32, TP_NP), smem, st>>>(a, 2);
-            PM_LAUNCH_CHECK();
-        }
-        const size_t smem = exact ? tp_refine_smem<true, 1>() : tp_refine_smem<false, 1>();
-        (exact ? k_taps_refine<true, 1> : k_taps_refine<false, 1>)<<<tap_grid(a), dim3(32, TP_NP + 1), smem, st>>>(a);
-        PM_LAUNCH_CHECK();
-        return cudaSuccess;
-    }
+    const bool taps = a.cand || (a.costs && pm_tap_sweeps(a.k));
     if (a.viewin) {
-        if (a.costs) (exact ? k_views<true> : k_views<false>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
+        if (taps) launch_taps<2>(a, exact, 1, st);
+        else if (a.costs) (exact ? k_views<true> : k_views<false>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
         else (exact ? k_propagate<true, 3> : k_propagate<false, 3>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
         PM_LAUNCH_CHECK();
     }
-    (exact ? k_propagate<true, 2> : k_propagate<false, 2>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
+    if (a.cand) launch_refine<1>(a, exact, st);
+    else if (taps) launch_refine<2>(a, exact, st);
+    else (exact ? k_propagate<true, 2> : k_propagate<false, 2>)<<<pass_grid(a), dim3(32, 8), 0, st>>>(a);
     PM_LAUNCH_CHECK();
     return cudaSuccess;
 }
@@ -2023,8 +2062,14 @@ cudaError_t pm_prepare_kernels() {
         if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     };
     e = cudaSuccess;
-    smem((const void*)k_taps_candidates<true>, tp_cand_smem<true>());
-    smem((const void*)k_taps_candidates<false>, tp_cand_smem<false>());
+    smem((const void*)k_taps_candidates<true, 0>, tp_cand_smem<true, 0>());
+    smem((const void*)k_taps_candidates<false, 0>, tp_cand_smem<false, 0>());
+    smem((const void*)k_taps_candidates<true, 1>, tp_cand_smem<true, 1>());
+    smem((const void*)k_taps_candidates<false, 1>, tp_cand_smem<false, 1>());
+    smem((const void*)k_taps_candidates<true, 2>, tp_cand_smem<true, 2>());
+    smem((const void*)k_taps_candidates<false, 2>, tp_cand_smem<false, 2>());
+    smem((const void*)k_taps_refine<true, 2>, tp_refine_smem<true, 2>());
+    smem((const void*)k_taps_refine<false, 2>, tp_refine_smem<false, 2>());
     smem((const void*)k_taps_refine<true, 0>, tp_refine_smem<true, 0>());
     smem((const void*)k_taps_refine<false, 0>, tp_refine_smem<false, 0>());
     smem((const void*)k_taps_field<true, false>, tp_field_smem<true>());
@@ -2036,19 +2081,26 @@ cudaError_t pm_prepare_kernels() {
     return pm_batch_prepare_kernels();
 }
 
-/* Where the tap-parallel passes stop paying: they form the neighbours'
- * terms per pixel, which costs more work, and win by filling the GPU.  Per
- * depthMap of 3 iterations (FAST; EXACT), against one thread per pixel: 64x48
- * 5.5 against 32.4 ms (6.0; 38.6), 160x120 14.2 against 34.3 (17.4; 40.6),
- * 240x180 29.9 against 41.5 (35.7; 49.6), 280x210 40.5 against 43.2 (48.8;
- * 51.5), 321x243 54.3 against 50.1 (63.1; 61.1). */
-#ifndef TP_MAX_PIXELS
-#define TP_MAX_PIXELS 60000
-#endif
+/* Where the tap-parallel kernels stop paying: they fill the GPU on small
+ * images, at more work and more L1 traffic per tap than a thread per pixel, and
+ * (for candidates 1-8 and 10-15) than shared plane windows.  Per depthMap of 3
+ * iterations (FAST; EXACT), ms:
+ *   all candidates tap-parallel against shared windows: 96x72 7.1, 9.3 (8.0,
+ *   10.1); 128x96 10.3, 10.6 (11.5, 11.3); 160x120 14.0, 11.8 (17.1, 13.6);
+ *   the others tap-parallel against a thread per pixel, with shared windows:
+ *   160x120 11.8, 15.2 (13.6, 17.9); 200x150 15.1, 16.1 (16.1, 18.7); 240x180
+ *   18.8, 18.2 (20.6, 21.3); 280x210 24.7, 22.3 (28.5, 26.8).
+ * A cost field: 160x120 0.162 against 0.454 (0.198, 0.427); 321x243 0.544
+ * against 0.525 (0.704, 0.596). */
+#define TP_MAX_PIXELS 12500
+#define TS_MAX_PIXELS 40000
+#define TF_MAX_PIXELS 60000
 bool pm_shared_windows(const PmCostConsts& k) {
     return std::isfinite(k.alpha) && std::isfinite(k.cmax) && std::isfinite(k.gmax);
 }
 bool pm_tap_parallel(const PmCostConsts& k) { return (size_t)k.W * k.H <= TP_MAX_PIXELS && pm_shared_windows(k); }
+bool pm_tap_sweeps(const PmCostConsts& k) { return (size_t)k.W * k.H <= TS_MAX_PIXELS && pm_shared_windows(k); }
+bool pm_tap_field(const PmCostConsts& k) { return (size_t)k.W * k.H <= TF_MAX_PIXELS && pm_shared_windows(k); }
 
 cudaError_t pm_launch_pd_block(float4* uout, float* pout, const float4* uin, const float* pin, int pzero,
                                const float4* f, const float* wgt, const float* mask, float lambda, int nsteps, int W,
