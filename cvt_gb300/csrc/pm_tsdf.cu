@@ -183,13 +183,24 @@ __device__ __forceinline__ float trilinear(const float2* __restrict__ cv, int W,
     const float bx = floorf(px), by = floorf(py), bz = floorf(pz);
     const float ax = px - bx, ay = py - by, az = pz - bz;
     const int ix = (int)bx, iy = (int)by, iz = (int)bz;
+    /* s0..s7: x fastest, then y, then z.  The first alone settles most empty
+     * samples; the others are in flight together (a test between them would
+     * make each wait for the one before). */
+    const float2* const p = cv + ((size_t)iz * H + iy) * W + ix;
+    const float2 t0 = __ldg(p);
+    if (t0.y < 1.0f) return 1e10f;
+    float2 t[8];
     float v[8];
+    t[0] = t0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {   /* s0..s7: x fastest, then y, then z */
-        const float2 t = cv[((size_t)(iz + (k >> 2)) * H + (iy + ((k >> 1) & 1))) * W + (ix + (k & 1))];
-        if (t.y < 1.0f) return 1e10f;
-        v[k] = t.x;
+    for (int k = 1; k < 8; ++k) t[k] = __ldg(p + ((size_t)(k >> 2) * H + ((k >> 1) & 1)) * W + (k & 1));
+    bool seen = true;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        seen = seen && !(t[k].y < 1.0f);
+        v[k] = t[k].x;
     }
+    if (!seen) return 1e10f;
     const float z0 = mixf(v[0], v[4], az), z1 = mixf(v[1], v[5], az), z2 = mixf(v[2], v[6], az), z3 = mixf(v[3], v[7], az);
     const float y0 = mixf(z0, z2, ay), y1 = mixf(z1, z3, ay);
     return mixf(y0, y1, ax);
@@ -199,8 +210,55 @@ __device__ __forceinline__ float ray_bound(float o, float d, int extent, bool st
     return (((d > 0.0f) == start ? 0.0f : (float)extent) - o) / d;
 }
 
+/* Which bricks of 8^3 voxels hold a voxel of weight >= 1 (or NaN: the test of
+ * trilinear, inverted), one byte each, and in `coarse` which bricks of 32^3
+ * do (cleared before).  A thread reads a column of 64 voxels of one x; the
+ * volume is read once, 8 bytes per voxel (HBM-bound). */
+#define TSDF_FINE 3                                  /* log2 of the extents */
+#define TSDF_COARSE 5
+struct BrickGrid {
+    const unsigned char *fine, *coarse;              /* NULL: no bricks */
+    int fw, fh, cw, ch;                              /* bricks per row and per column */
+};
+__global__ void __launch_bounds__(256) k_tsdf_bricks(const float2* __restrict__ cv, int W, int H, int D,
+                                                     unsigned char* __restrict__ fine, unsigned char* __restrict__ coarse,
+                                                     BrickGrid g) {
+    const int x = blockIdx.x * 256 + threadIdx.x, y0 = blockIdx.y * 8, z0 = blockIdx.z * 8;
+    bool any = false;
+    if (x < W) {
+        const int y1 = min(y0 + 8, H), z1 = min(z0 + 8, D);
+#pragma unroll 2
+        for (int z = z0; z < z1; ++z) {
+            const float2* p = cv + ((size_t)z * H + y0) * W + x;
+            if (y1 == y0 + 8) {
+                float w[8];
+#pragma unroll
+                for (int y = 0; y < 8; ++y) w[y] = __ldg(p + (size_t)y * W).y;
+#pragma unroll
+                for (int y = 0; y < 8; ++y) any = any || !(w[y] < 1.0f);
+            } else {
+                for (int y = y0; y < y1; ++y, p += W) any = any || !(__ldg(p).y < 1.0f);
+            }
+        }
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, any);
+    if ((threadIdx.x & 7) == 0 && x < W)
+        fine[((size_t)blockIdx.z * g.fh + blockIdx.y) * g.fw + (x >> 3)] = (m >> (threadIdx.x & 31)) & 0xffu ? 1 : 0;
+    if (m && (threadIdx.x & 31) == 0 && x < W)
+        coarse[((size_t)(blockIdx.z >> 2) * g.ch + (blockIdx.y >> 2)) * g.cw + (x >> 5)] = 1;
+}
+
+/* The march evaluates samples half a voxel apart, and most of them lie where
+ * nothing was integrated: a corner of weight < 1 makes the value 1e10.  With
+ * bricks, a sample whose first corner lies in a brick without weights has that
+ * value at once.  It then steps to the last sample it expects inside the brick,
+ * with the additions to lambda alone: if that one is in the brick, so are those
+ * between (a position is monotone in lambda, rounded or not) and all have the
+ * value 1e10; if not, it takes one step.  The values met, and so the results,
+ * are those of the plain march. */
 __global__ void __launch_bounds__(256) k_tsdf_raycast(float* __restrict__ out, size_t opitch4, int iw, int ih,
                                                       const float2* __restrict__ cv, int W, int H, int D,
+                                                      BrickGrid bg,
                                                       DMat4 tcam2g, DMat4 tg2cam, float scale, int max_steps) {
     const int gx = blockIdx.x * 32 + threadIdx.x, gy = blockIdx.y * 8 + threadIdx.y;
     if (gx >= iw || gy >= ih) return;
@@ -215,12 +273,52 @@ __global__ void __launch_bounds__(256) k_tsdf_raycast(float* __restrict__ out, s
     if (rs < re && isfinite(rs) && isfinite(re) && isfinite(dx) && isfinite(dy) && isfinite(dz)) {
         const float vx = fabsf(dx * (re - rs)), vy = fabsf(dy * (re - rs)), vz = fabsf(dz * (re - rs));
         const float step = 0.5f * sqrtf((vx * vx + vy * vy) + vz * vz) / fmaxf(vx, fmaxf(vy, vz));
-        float ppx = o4.x + dx * rs, ppy = o4.y + dy * rs, ppz = o4.z + dz * rs;
-        float vp = trilinear(cv, W, H, D, ppx, ppy, ppz);
+        const float mx = (float)(W - 2), my = (float)(H - 2), mz = (float)(D - 2);
+        /* the first corner of the sample at lambda (trilinear's clamps) */
+        auto corner = [&](float lambda) {
+            return make_int3((int)fminf(fmaxf(0.0f, o4.x + dx * lambda), mx), (int)fminf(fmaxf(0.0f, o4.y + dy * lambda), my),
+                             (int)fminf(fmaxf(0.0f, o4.z + dz * lambda), mz));
+        };
+        const float ix = 1.0f / (dx * step), iy = 1.0f / (dy * step), iz = 1.0f / (dz * step);   /* steps per voxel */
+        float ppz = o4.z + dz * rs;
+        float vp = trilinear(cv, W, H, D, o4.x + dx * rs, o4.y + dy * rs, ppz);
         int n = 0;
-        for (float lambda = rs + step; lambda <= re && n < max_steps; lambda += step, ++n) {
-            const float px = o4.x + dx * lambda, py = o4.y + dy * lambda, pz = o4.z + dz * lambda;
-            const float v = trilinear(cv, W, H, D, px, py, pz);
+        float lambda = rs + step;
+        while (lambda <= re && n < max_steps) {
+            bool empty = false;
+            if (bg.fine) {
+                const int3 c = corner(lambda);
+                int sh = TSDF_COARSE;
+                empty = !__ldg(&bg.coarse[((c.z >> sh) * bg.ch + (c.y >> sh)) * bg.cw + (c.x >> sh)]);
+                if (!empty) {
+                    sh = TSDF_FINE;
+                    empty = !__ldg(&bg.fine[((c.z >> sh) * bg.fh + (c.y >> sh)) * bg.fw + (c.x >> sh)]);
+                }
+                if (empty && !(vp < 0.0f)) {             /* 1e10 from here on makes no crossing */
+                    const int3 b = make_int3(c.x >> sh, c.y >> sh, c.z >> sh);
+                    /* the steps to the brick's far sides, less a little */
+                    const float ex = (float)((b.x + (dx > 0.0f)) << sh) - (o4.x + dx * lambda);
+                    const float ey = (float)((b.y + (dy > 0.0f)) << sh) - (o4.y + dy * lambda);
+                    const float ez = (float)((b.z + (dz > 0.0f)) << sh) - (o4.z + dz * lambda);
+                    const float far = fminf(fminf(dx != 0.0f ? ex * ix : 1e9f, dy != 0.0f ? ey * iy : 1e9f),
+                                            dz != 0.0f ? ez * iz : 1e9f) - 0.01f;
+                    const int hop = min((int)fminf(fmaxf(far, 0.0f), 256.0f), max_steps - n - 1);
+                    if (hop > 0) {
+                        float last = lambda;
+                        for (int i = 0; i < hop; ++i) last += step;
+                        const int3 l = corner(last);
+                        if (last <= re && l.x >> sh == b.x && l.y >> sh == b.y && l.z >> sh == b.z) {
+                            vp = 1e10f;
+                            ppz = o4.z + dz * last;
+                            lambda = last + step;
+                            n += hop + 1;
+                            continue;
+                        }
+                    }
+                }
+            }
+            const float pz = o4.z + dz * lambda;
+            const float v = empty ? 1e10f : trilinear(cv, W, H, D, o4.x + dx * lambda, o4.y + dy * lambda, pz);
             if (vp < 0.0f && v > 0.0f) break;
             if (vp > 0.0f && v < 0.0f) {
                 const float alpha = -v / (vp - v);
@@ -229,7 +327,9 @@ __global__ void __launch_bounds__(256) k_tsdf_raycast(float* __restrict__ out, s
                 break;
             }
             vp = v;
-            ppx = px; ppy = py; ppz = pz;
+            ppz = pz;
+            lambda += step;
+            ++n;
         }
     }
     out[(size_t)gy * opitch4 + gx] = ret;
@@ -264,7 +364,11 @@ struct cvtpm_tsdf {
     float trunc;
     Mat4 g2w;
     float2* vol;
+    unsigned char* bricks;     /* scratch of a ray cast, behind the volume; NULL: no room for it */
 };
+
+/* bricks of 1 << sh voxels along an extent */
+static int tsdf_bricks(int extent, int sh) { return (extent + (1 << sh) - 1) >> sh; }
 
 /* Vision::disparityToDepthmap (cvt/vision/Vision.cpp:147-168): the depth
  * (focallength * baseline) / (disparity * dispscale) where the scaled
@@ -304,7 +408,13 @@ cvtpm_status cvtpm_tsdf_create(cvtpm_tsdf** out, int device, const float* grid_t
     v->W = width; v->H = height; v->D = depth;
     v->trunc = truncation;
     memcpy(v->g2w.m, grid_to_world, sizeof v->g2w.m);
-    if (cudaMalloc(&v->vol, sizeof(float2) * (size_t)width * height * depth) != cudaSuccess) {
+    const size_t bytes = sizeof(float2) * (size_t)width * height * depth;
+    size_t bricks = 0;
+    for (int sh : {TSDF_FINE, TSDF_COARSE})
+        bricks += (size_t)tsdf_bricks(width, sh) * tsdf_bricks(height, sh) * tsdf_bricks(depth, sh);
+    if (cudaMalloc(&v->vol, bytes + bricks) == cudaSuccess) {
+        v->bricks = (unsigned char*)v->vol + bytes;
+    } else if (cudaGetLastError(), cudaMalloc(&v->vol, bytes) != cudaSuccess) {
         cudaGetLastError();
         delete v;
         return fail(CVTPM_ERR_ALLOC, "tsdf create: volume allocation failed");
@@ -373,8 +483,24 @@ cvtpm_status cvtpm_tsdf_raycast(cvtpm_tsdf* v, const float* proj, float* depthma
     const DMat4 T = to_dev(all), Ti = to_dev(mat4_inverse(all));
     const int max_steps = 2 * (v->W > v->H ? (v->W > v->D ? v->W : v->D) : (v->H > v->D ? v->H : v->D)) + 16;
     cudaSetDevice(v->device);
+    BrickGrid g = {nullptr, nullptr, tsdf_bricks(v->W, TSDF_FINE), tsdf_bricks(v->H, TSDF_FINE),
+                   tsdf_bricks(v->W, TSDF_COARSE), tsdf_bricks(v->H, TSDF_COARSE)};
+    /* The bricks cost a pass over the volume and two launches, and save the
+     * evaluations of empty samples, which count where there are many rays: 256^3
+     * with 640x480 rays 0.30 -> 0.24 ms, 128^3 0.17 -> 0.15, 512^3 0.66 -> 0.53;
+     * but 256^3 with 320x240 0.19 -> 0.22 and 48^3 with 640x480 0.09 -> 0.12. */
+    const size_t samples = (size_t)dwidth * dheight * (size_t)(max_steps / 2);
+    if (v->bricks && samples >= 30000000) {
+        /* formed anew for each cast: the caller may write the volume (cvtpm_tsdf_info) */
+        const int fd = tsdf_bricks(v->D, TSDF_FINE), cd = tsdf_bricks(v->D, TSDF_COARSE);
+        unsigned char *fine = v->bricks, *coarse = fine + (size_t)g.fw * g.fh * fd;
+        cudaMemsetAsync(coarse, 0, (size_t)g.cw * g.ch * cd, (cudaStream_t)stream);
+        k_tsdf_bricks<<<dim3((v->W + 255) / 256, g.fh, fd), 256, 0, (cudaStream_t)stream>>>(v->vol, v->W, v->H, v->D, fine, coarse, g);
+        g.fine = fine;
+        g.coarse = coarse;
+    }
     k_tsdf_raycast<<<dim3((dwidth + 31) / 32, (dheight + 7) / 8), dim3(32, 8), 0, (cudaStream_t)stream>>>(
-        depthmap, dpitch / 4, dwidth, dheight, v->vol, v->W, v->H, v->D, Ti, T, scale, max_steps);
+        depthmap, dpitch / 4, dwidth, dheight, v->vol, v->W, v->H, v->D, g, Ti, T, scale, max_steps);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CVTPM_OK : fail(CVTPM_ERR_CUDA, std::string("tsdf raycast: ") + cudaGetErrorString(e));
 }
