@@ -199,7 +199,10 @@ __global__ void k_scan_vert(Stk2 p) {
  * row], top(X) = pre(X, top) [+ pre(left, top)], the reference's two steps
  * on its local buffer.  Here 16 lanes walk the 16 columns of a window down
  * its rows: the left column's value comes by shuffle from the window's lane
- * 0, the top row's stays in a register — no shared memory, no barriers.
+ * 0, the top row's stays in a register — no shared memory, no barriers; the
+ * window's rows are read before the first is written, so that their reads are
+ * in flight together: 0.27 ms over the 954 MB of 128 slices at 1242x375, the
+ * time of a copy, against 0.65 row by row.
  * Windows are disjoint, and the fix-ups of the image's last row and column
  * read only pixels no window covers. */
 __global__ void __launch_bounds__(128) k_scan_block2(Stk2 p, int nbx, int nby) {
@@ -211,15 +214,19 @@ __global__ void __launch_bounds__(128) k_scan_block2(Stk2 p, int nbx, int nby) {
     const int bx = wx * 16, by = wy * 16;
     const int X = bx + lx - 1;
     const unsigned src = lane & 16;                         /* the window's lane 0 */
-    float4 top = tex(m, X, by - 1);
+    float4 row[16];                                         /* the window's rows, before any is written */
+#pragma unroll
+    for (int ly = 0; ly < 16; ++ly) row[ly] = tex(m, X, by + ly - 1);
+    float4 top = row[0];
     {
         const float4 l0 = shfl4(top, src);
         if (lx) top = add4(top, l0);
     }
+#pragma unroll
     for (int ly = 0; ly < 16; ++ly) {
         float4 v = top;
         if (ly) {
-            v = tex(m, X, by + ly - 1);
+            v = row[ly];
             const float4 l = shfl4(v, src);
             if (lx) v = add4(v, l);
             v = add4(v, top);
@@ -264,54 +271,95 @@ __global__ void __launch_bounds__(256) k_gradx(Img out, Img src) {
     put(out, x, y, sub4(tex(src, x + 1, y), tex(src, x - 1, y)));
 }
 
-/* stereogcv_costdepthgrad (point cost) at (x, y) for disparity depth:
- * img0 at the pixel, img1 at x - depth */
-__device__ __forceinline__ float point_cost(const Img& img0, const Img& img1, const Img& grad0, const Img& grad1,
-                                            int x, int y, float depth) {
-    const int W = img0.w, H = img1.h;
-    const float u = (float)x + 0.5f - depth, v = (float)y + 0.5f;
-    if (u < 0.0f || u >= (float)W || v < 0.0f || v >= (float)H) return 0.008f + 0.028f;
-    const float4 dm = make_float4(0.3333f, 0.3333f, 0.3333f, 0.0f);
-    const float4 I0 = tex(img0, x, y), G0 = tex(grad0, x, y);
-    const float4 I1 = bilinear(img1, u, v), G1 = bilinear(grad1, u, v);
-    const float ci = fminf(dotf4(abs4(sub4(I1, I0)), dm), 0.028f);
-    const float cg = fminf(dotf4(abs4(sub4(G1, G0)), dm), 0.008f);
-    return ci + (cg - ci) * 0.10f;   /* mix(ci, cg, ALPHA) */
-}
-
 /* Disparities of one batch: slice z of every stack belongs to d[z]. */
 struct Depths {
     float d[GCV_BATCH_MAX];
 };
 
-/* The cost image of disparity dl.d[z] and the 16 x 16 block scans of its two
- * integral images, the cost (GRAY) and img0 * cost (prefixsum_pblock_mul2),
- * in one pass: the same sums in the same order as the two block scans of the
- * stored cost image.  Pixels outside the image scan as 0, as the reference's
- * out-of-image reads return 0. */
-__global__ void __launch_bounds__(256) k_cost_scan(Stk ig, Stk iint, Img img0, Img img1, Img grad0, Img grad1,
-                                                   Depths dl) {
-    __shared__ float4 b4[256];
-    __shared__ float b1[256];
-    const int lx = threadIdx.x, ly = threadIdx.y, lid = ly * 16 + lx;
-    const int x = blockIdx.x * 16 + lx, y = blockIdx.y * 16 + ly, z = blockIdx.z;
-    float c = 0.0f;
-    if (x < img0.w && y < img0.h) c = point_cost(img0, img1, grad0, grad1, x, y, dl.d[z]);
-    float4 t = mul4(tex(img0, x, y), make_float4(c, c, c, c));
-    b4[lid] = t;
-    b1[lid] = c;
+/* Two 16 x 16 blocks side by side, channel by channel: [channel][row][column]. */
+typedef float ScanTile[4][16][32];
+
+/* The 16 x 16 block scans (prefixsum_pblock*) of a tile that its four warps
+ * filled, four rows each; out's pixels from (x0, y0).  Warp c scans channel c,
+ * one lane per column with the 16 rows in registers: the Hillis-Steele x steps
+ * by shuffle among a block's 16 lanes, the y steps within the lane, in place of
+ * a barrier on either side of every step.  A tile's values come from all four
+ * warps rather than from a lane per column of 16 rows, whose registers left too
+ * few warps to hide the reads (cost 1.11 ms, (a, b) 1.89 ms). */
+__device__ __forceinline__ void scan_tile(ScanTile& s, Img out, int x0, int y0) {
+    const int lane = threadIdx.x, c = threadIdx.y, lx = lane & 15;
+    __syncthreads();
+    float t[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) t[r] = s[c][r][lane];
+#pragma unroll
     for (int off = 1; off < 16; off <<= 1) {
-        __syncthreads();
-        if (lx >= off) { t = add4(t, b4[lid - off]); c = c + b1[lid - off]; }
-        __syncthreads();
-        b4[lid] = t; b1[lid] = c;
-        __syncthreads();
-        if (ly >= off) { t = add4(t, b4[lid - 16 * off]); c = c + b1[lid - 16 * off]; }
-        __syncthreads();
-        b4[lid] = t; b1[lid] = c;
+#pragma unroll
+        for (int r = 0; r < 16; ++r) {
+            const float l = __shfl_up_sync(0xffffffffu, t[r], off, 16);
+            if (lx >= off) t[r] += l;
+        }
+#pragma unroll
+        for (int r = 15; r >= off; --r) t[r] += t[r - off];
     }
-    put(iint.at(z), x, y, t);
-    put(ig.at(z), x, y, make_float4(c, c, c, c));
+#pragma unroll
+    for (int r = 0; r < 16; ++r) s[c][r][lane] = t[r];
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int r = 4 * threadIdx.y + k;
+        put(out, x0 + lane, y0 + r, make_float4(s[0][r][lane], s[1][r][lane], s[2][r][lane], s[3][r][lane]));
+    }
+}
+__device__ __forceinline__ void tile_set(ScanTile& s, int r, float4 v) {
+    s[0][r][threadIdx.x] = v.x; s[1][r][threadIdx.x] = v.y; s[2][r][threadIdx.x] = v.z; s[3][r][threadIdx.x] = v.w;
+}
+
+/* The cost image (stereogcv_costdepthgrad, point cost: img0 at the pixel, img1
+ * at x - depth) of disparity dl.d[z] and the block scans of img0.rgb * cost
+ * (prefixsum_pblock_mul2) and the cost, as one image (r, g, b, cost): the sums
+ * of the two block scans of the stored cost image, in their order.  (The guided
+ * filter reads no alpha of the first, so the cost takes its place.)  A lane owns
+ * four rows of a column; a sample's v lies on its row, so the bilinear read's
+ * lower texels are the next row's upper ones and each is read once.  0.67 ms for 128
+ * disparities at 1242x375, against 1.18 with a thread per pixel, the scans in
+ * shared memory and the cost in a stack of its own.  Pixels
+ * outside the image scan as 0, as the reference's out-of-image reads return 0. */
+__global__ void __launch_bounds__(128) k_cost_scan(Stk iint, Img img0, Img img1, Img grad0, Img grad1, Depths dl) {
+    __shared__ ScanTile s;
+    const int x = blockIdx.x * 32 + threadIdx.x, y0 = blockIdx.y * 16 + 4 * threadIdx.y;
+    const float depth = dl.d[blockIdx.z];
+    const int W = img0.w, H = img0.h;
+    const float u = (float)x + 0.5f - depth;
+    const bool in = x < W && !(u < 0.0f || u >= (float)W);
+    const float tu = u - 0.5f, fu = floorf(tu), fa = tu - fu;
+    const int i0 = in ? (int)fu : -2;
+    float4 i00 = tex(img1, i0, y0), i10 = tex(img1, i0 + 1, y0), g00 = tex(grad1, i0, y0), g10 = tex(grad1, i0 + 1, y0);
+    const float4 dm = make_float4(0.3333f, 0.3333f, 0.3333f, 0.0f);
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int y = y0 + r;
+        const float4 I0 = tex(img0, x, y);
+        float c = 0.0f;
+        if (in) {
+            const float4 i01 = tex(img1, i0, y + 1), i11 = tex(img1, i0 + 1, y + 1);
+            const float4 g01 = tex(grad1, i0, y + 1), g11 = tex(grad1, i0 + 1, y + 1);
+            if (y < H) {
+                const float tv = ((float)y + 0.5f) - 0.5f, b = tv - floorf(tv);
+                const float w00 = (1.0f - fa) * (1.0f - b), w10 = fa * (1.0f - b), w01 = (1.0f - fa) * b, w11 = fa * b;
+                const float4 I1 = add4(add4(add4(scl4(w00, i00), scl4(w10, i10)), scl4(w01, i01)), scl4(w11, i11));
+                const float4 G1 = add4(add4(add4(scl4(w00, g00), scl4(w10, g10)), scl4(w01, g01)), scl4(w11, g11));
+                const float ci = fminf(dotf4(abs4(sub4(I1, I0)), dm), 0.028f);
+                const float cg = fminf(dotf4(abs4(sub4(G1, tex(grad0, x, y))), dm), 0.008f);
+                c = ci + (cg - ci) * 0.10f;                 /* mix(ci, cg, ALPHA) */
+            }
+            i00 = i01; i10 = i11; g00 = g01; g10 = g11;
+        } else if (x < W && y < H) {
+            c = 0.008f + 0.028f;
+        }
+        tile_set(s, 4 * threadIdx.y + r, make_float4(I0.x * c, I0.y * c, I0.z * c, c));
+    }
+    scan_tile(s, iint.at(blockIdx.z), blockIdx.x * 32, blockIdx.y * 16);
 }
 
 /* guidedfilter_calcab_outerrgb at one pixel: the 3x3 system (covariance of
@@ -350,35 +398,26 @@ __device__ __forceinline__ float4 calcab_px(float4 g, float4 s, float4 sg, float
 
 /* Per pixel of disparity slice z: the box means of the cost and of
  * guide * cost, the guided filter's (a, b), and the 16 x 16 block scans of a
- * and b — the first steps of their integral images.  b's four channels are
- * equal (s - dot(g, a) with s a GRAY mean), so one is stored. */
-__global__ void __launch_bounds__(256) k_calcab_scan(Stk iaI, Stk ibI, Stk ig, Stk iint, Img mG, Img mRR, Img mGG,
-                                                     float eps, int r) {
-    __shared__ float4 b4[256];
-    __shared__ float b1[256];
-    const int lx = threadIdx.x, ly = threadIdx.y, lid = ly * 16 + lx;
-    const int x = blockIdx.x * 16 + lx, y = blockIdx.y * 16 + ly, z = blockIdx.z;
-    float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    float b = 0.0f;
-    if (x < mG.w && y < mG.h) {
-        const float s = box_px(ig.at(z), x, y, r).x;
-        a = calcab_px(tex(mG, x, y), make_float4(s, s, s, s), box_px(iint.at(z), x, y, r), tex(mRR, x, y),
-                      tex(mGG, x, y), eps, &b);
+ * and b — the first steps of their integral images, as one image (a, b): a has
+ * no fourth channel, and b's four are equal (s - dot(g, a) with s a GRAY mean).
+ * 0.88 ms for 128 disparities at 1242x375, against 1.30 with two stacks. */
+__global__ void __launch_bounds__(128) k_calcab_scan(Stk iab, Stk iint, Img mG, Img mRR, Img mGG, float eps, int r) {
+    __shared__ ScanTile s;
+    const int x = blockIdx.x * 32 + threadIdx.x, y0 = blockIdx.y * 16 + 4 * threadIdx.y;
+    const Img in = iint.at(blockIdx.z);
+#pragma unroll 2
+    for (int k = 0; k < 4; ++k) {
+        const int y = y0 + k;
+        float4 t = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (x < mG.w && y < mG.h) {
+            const float4 m = box_px(in, x, y, r);
+            float b;
+            t = calcab_px(tex(mG, x, y), make_float4(m.w, m.w, m.w, m.w), m, tex(mRR, x, y), tex(mGG, x, y), eps, &b);
+            t.w = b;
+        }
+        tile_set(s, 4 * threadIdx.y + k, t);
     }
-    b4[lid] = a;
-    b1[lid] = b;
-    for (int off = 1; off < 16; off <<= 1) {
-        __syncthreads();
-        if (lx >= off) { a = add4(a, b4[lid - off]); b = b + b1[lid - off]; }
-        __syncthreads();
-        b4[lid] = a; b1[lid] = b;
-        __syncthreads();
-        if (ly >= off) { a = add4(a, b4[lid - 16 * off]); b = b + b1[lid - 16 * off]; }
-        __syncthreads();
-        b4[lid] = a; b1[lid] = b;
-    }
-    put(iaI.at(z), x, y, a);
-    put(ibI.at(z), x, y, make_float4(b, b, b, b));
+    scan_tile(s, iab.at(blockIdx.z), blockIdx.x * 32, blockIdx.y * 16);
 }
 
 /* Per pixel, the batch's disparities in order: the box means of a and b,
@@ -390,10 +429,10 @@ __global__ void __launch_bounds__(256) k_calcab_scan(Stk iaI, Stk ibI, Stk ig, S
  * sequential rule picks the first disparity of the smallest cost below the
  * start (NaN never compares less), and so does this. */
 #define FM_CHUNKS 8
-/* 4 blocks per SM (64 registers): 11.44 ms per apply at 1242x375 x 128
- * disparities, against 11.95 with 77 registers and 3 blocks, 12.4 with 5 */
-__global__ void __launch_bounds__(32 * FM_CHUNKS, 4) k_filter_min(Img c, Stk iaI, Stk ibI, Img guide, Depths nd, int nz,
-                                                              int r) {
+/* 5 blocks per SM: 6.31 ms per apply at 1242x375 x 128 disparities, against
+ * 6.44 with 3 or 4 blocks.  One stack to read where a and b had one each: 0.56
+ * ms for 1.08 at 4 blocks. */
+__global__ void __launch_bounds__(32 * FM_CHUNKS, 5) k_filter_min(Img c, Stk iab, Img guide, Depths nd, int nz, int r) {
     __shared__ float bv[FM_CHUNKS][32];
     __shared__ int bz[FM_CHUNKS][32];
     const int lx = threadIdx.x, k = threadIdx.y;
@@ -405,8 +444,10 @@ __global__ void __launch_bounds__(32 * FM_CHUNKS, 4) k_filter_min(Img c, Stk iaI
         const int z1 = (k + 1) * nz / FM_CHUNKS;
 #pragma unroll 2
         for (int z = k * nz / FM_CHUNKS; z < z1; ++z) {
-            const float d = dotf4(box_px(iaI.at(z), x, y, r), g);
-            const float n = d + box_px(ibI.at(z), x, y, r).x;
+            float4 m = box_px(iab.at(z), x, y, r);
+            const float b = m.w;
+            m.w = 0.0f;                    /* a's fourth channel */
+            const float n = dotf4(m, g) + b;
             if (n < best) { best = n; bi = z; }
         }
     }
@@ -452,7 +493,6 @@ cvtpm_status fail(cvtpm_status s, const std::string& m) {
 dim3 g16(int W, int H) { return dim3((W + 15) / 16, (H + 15) / 16); }
 dim3 g32(int W, int H) { return dim3((W + 31) / 32, (H + 7) / 8); }
 
-
 Stk2 one(Stk a) { return Stk2{{a, a}, 1}; }
 Stk2 two(Stk a, Stk b) { return Stk2{{a, b}, 2}; }
 
@@ -469,8 +509,9 @@ void scan_rest(Stk2 p, int nz, cudaStream_t st) {
 Stk stack(float* d, int W, int H, int c) { return Stk{d, W, H, c, (size_t)W * H * c}; }
 
 /* Scratch: GCV_VIEW_FLOATS per pixel for a view, GCV_SLICE_FLOATS per pixel
- * and disparity of a batch (cost integral 1, guide * cost integral 4, the
- * integrals of a 4 and b 1). */
+ * and disparity of a batch: the integrals of (guide * cost, cost) 4 and of
+ * (a, b) 4, and 2 that nothing uses — the figure is what plans have reported
+ * and what sets where a large image's batches are cut. */
 const int GCV_VIEW_FLOATS = 22, GCV_SLICE_FLOATS = 10;
 
 std::atomic<int> g_batch{0};
@@ -511,10 +552,9 @@ void depthmap(float* dst, size_t dpitch, Img cam0, Img cam1, float dmin, float d
     /* RGBA images and stacks first: every float4 buffer starts on a
      * multiple of 4 floats whatever W * H is */
     const Img g0 = take(4), g1 = take(4), mG = take(4), mRR = take(4), mGG = take(4);
-    const Stk iint = stack(s, W, H, 4), iaI = stack(s + 4 * n * batch, W, H, 4);
+    const Stk iint = stack(s, W, H, 4), iab = stack(s + 4 * n * batch, W, H, 4);
     s += 8 * n * batch;
     const Img c = take(2);
-    const Stk ig = stack(s, W, H, 1), ibI = stack(s + n * batch, W, H, 1);
     /* the view's set-up integrals, before the first batch: 8 floats per pixel
      * of the RGBA stacks */
     const Stk t0 = stack(iint.d, W, H, 4), t1 = stack(iint.d + 4 * n, W, H, 4);
@@ -540,12 +580,12 @@ void depthmap(float* dst, size_t dpitch, Img cam0, Img cam1, float dmin, float d
             nd.d[z] = fabsf(d - dmin) / fabsf(dmax - dmin);
         }
         steps -= nz;
-        const dim3 gz((W + 15) / 16, (H + 15) / 16, nz);
-        k_cost_scan<<<gz, dim3(16, 16), 0, st>>>(ig, iint, cam1, cam0, g1, g0, dd);
-        scan_rest(two(ig, iint), nz, st);
-        k_calcab_scan<<<gz, dim3(16, 16), 0, st>>>(iaI, ibI, ig, iint, mG, mRR, mGG, 1e-3f, R);
-        scan_rest(two(iaI, ibI), nz, st);
-        k_filter_min<<<dim3((W + 31) / 32, H), dim3(32, FM_CHUNKS), 0, st>>>(c, iaI, ibI, cam1, nd, nz, R);
+        const dim3 gz((W + 31) / 32, (H + 15) / 16, nz);
+        k_cost_scan<<<gz, dim3(32, 4), 0, st>>>(iint, cam1, cam0, g1, g0, dd);
+        scan_rest(one(iint), nz, st);
+        k_calcab_scan<<<gz, dim3(32, 4), 0, st>>>(iab, iint, mG, mRR, mGG, 1e-3f, R);
+        scan_rest(one(iab), nz, st);
+        k_filter_min<<<dim3((W + 31) / 32, H), dim3(32, FM_CHUNKS), 0, st>>>(c, iab, cam1, nd, nz, R);
     }
     k_depthconv<<<g32(W, H), dim3(32, 8), 0, st>>>(dst, dpitch / 4, c, 1.0f, 0.0f);
 }
