@@ -1470,8 +1470,9 @@ k_pd_step(float4* __restrict__ uout, float4* __restrict__ pout, const float4* __
  * Q2 = -RN(x / b) (Markstein's theorem on division by a correctly rounded
  * reciprocal, "Computation of elementary functions on the IBM RISC System/6000
  * processor", 1990), including the sign of a zero x.  The theorem wants no
- * underflow or overflow: a cell with 0 < |x| < 2^-100 takes IEEE divisions,
- * and so does a block whose values are not all of moderate size (`tame`).
+ * underflow or overflow: in a row with some 0 < |x| < 2^-100 the tiny values
+ * are scaled up, divided and scaled back (`neg_div2_any`), and a block whose
+ * values are not all of moderate size (`tame`) takes IEEE divisions.
  *
  * Measured at 1242x375, 4 steps per launch (ncu): 29-38 us per launch, where
  * the form that kept everything in shared memory as float4 and divided with
@@ -1496,6 +1497,31 @@ PM_DEV float2 neg_div2(float2 x, float2 b, float2 ny) {
     r = ffma2(q1, b, x);
     return ffma2(r, ny, q1);
 }
+/* The same for any |x| < 2^60, with 1 <= b <= 2^20: a tiny x is multiplied by
+ * 2^100, which is exact, and its quotient by 2^-100.  That rounds a second time
+ * where the result is subnormal, and wrongly only where the first rounding made
+ * it half a subnormal's unit off (d): the remainder's sign then says on which
+ * side of the tie the quotient lies.
+ * The smoothed field's support grows by a cell a step, its values falling off
+ * so fast that a band of subnormals lies around every empty region: with IEEE
+ * divisions, which leave for a subroutine there, the first two iterations'
+ * launches took 70-140 us at 1242x375, against 40-49 (ncu); depthMap of 640x480
+ * 88.3 -> 85.8 ms, of 1242x375 335 -> 327.  (A vote that gives a whole warp one
+ * form costs 0.4 ms at 640x480 and 0.4 of 64x48's 5.5.) */
+PM_DEV float2 neg_div2_any(float2 x, float2 b, float2 ny) {
+    const bool tx = fabsf(x.x) < 7.8886091e-31f, ty = fabsf(x.y) < 7.8886091e-31f;     /* 2^-100 */
+    const float2 up = make_float2(tx ? 1.2676506e30f : 1.0f, ty ? 1.2676506e30f : 1.0f);
+    const float2 down = make_float2(tx ? 7.8886091e-31f : 1.0f, ty ? 7.8886091e-31f : 1.0f);
+    const float2 xs = fmul2(x, up);
+    const float2 q = neg_div2(xs, b, ny);
+    const float2 r = ffma2(q, b, xs);
+    float2 t = fmul2(q, down);
+    const float2 d = ffma2(t, up, fmul2(q, f2s(-1.0f)));
+    const float half = 8.8817842e-16f;                                                  /* 2^-50 */
+    if (fabsf(d.x) == half && r.x != 0.0f) t.x = copysignf((q.x - copysignf(half, r.x)) * down.x, q.x);
+    if (fabsf(d.y) == half && r.y != 0.0f) t.y = copysignf((q.y - copysignf(half, r.y)) * down.y, q.y);
+    return t;
+}
 /* s = RN(sqrt(v)) and ny = -RN(1 / s) for both halves, 1 <= v <= PDS_VMAX:
  * Newton's iteration for 1 / sqrt(v) from rsqrt.approx and one fused residual
  * step each for the root and its reciprocal (Markstein, as above).  Compared
@@ -1503,7 +1529,7 @@ PM_DEV float2 neg_div2(float2 x, float2 b, float2 ny) {
  * all equal, and so are the reciprocals but those of significands of ones.
  * Those, and they alone, leave a residual of 2^-24 before the last step: the
  * return value is the larger residual. */
-#define PDS_VMAX 1.2676506e30f                       /* 2^100 */
+#define PDS_VMAX 1.0995116e12f                       /* 2^40: s <= 2^20 */
 #define PDS_RESID 5.9604645e-8f                      /* 2^-24 */
 PM_DEV float norm2(float2 v, float2& s, float2& ny) {
     float2 y;
@@ -1523,9 +1549,11 @@ PM_DEV float norm2(float2 v, float2& s, float2& ny) {
 }
 /* x / s for both halves (multiplying by -1 is exact) */
 PM_DEV float2 div_norm2(float2 x, float2 s, float2 ny) { return fmul2(neg_div2(x, s, ny), f2s(-1.0f)); }
+PM_DEV float2 div_norm2_any(float2 x, float2 s, float2 ny) { return fmul2(neg_div2_any(x, s, ny), f2s(-1.0f)); }
 /* 2 bits(x) - 1 as unsigned: 0xffffffff for zeros, small for tiny values */
 PM_DEV unsigned pds_mag(float x) { return 2u * (unsigned)__float_as_int(x) - 1u; }
 #define PDS_TINY (2u * (27u << 23) - 1u)             /* pds_mag(2^-100) */
+#define PDS_SMALL (2u * (47u << 23) - 1u)            /* pds_mag(2^-80): not tiny after a division by <= 2^20 either */
 PM_DEV unsigned pds_mag2(unsigned m, float2 x) { return min(m, min(pds_mag(x.x), pds_mag(x.y))); }
 PM_DEV float neg_div_ieee(float x, float b) { return x == 0.0f ? -x : -(x / b); }
 
@@ -1641,6 +1669,12 @@ PM_DEV void pds_tile(float4* __restrict__ uout, float* __restrict__ pout, const 
                     nl[c] = neg_div2(nl[c], cd, cn);
                     nh[c] = neg_div2(nh[c], cd, cn);
                 }
+            } else if (tame) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    nl[c] = neg_div2_any(nl[c], cd, cn);
+                    nh[c] = neg_div2_any(nh[c], cd, cn);
+                }
             } else {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) {
@@ -1674,10 +1708,18 @@ PM_DEV void pds_tile(float4* __restrict__ uout, float* __restrict__ pout, const 
                     else e = fmaxf(e, norm2(make_float2(fmaxf(v[c].x, 1.0f), fmaxf(v[c].y, 1.0f)), s[c], ny[c]));
                 }
                 if (tame && vmax <= PDS_VMAX && e < PDS_RESID) {
+                    if (m >= PDS_SMALL) {
 #pragma unroll
-                    for (int c = 0; c < 3; ++c) {
-                        nl[c] = div_norm2(nl[c], s[c], ny[c]);
-                        nh[c] = div_norm2(nh[c], s[c], ny[c]);
+                        for (int c = 0; c < 3; ++c) {
+                            nl[c] = div_norm2(nl[c], s[c], ny[c]);
+                            nh[c] = div_norm2(nh[c], s[c], ny[c]);
+                        }
+                    } else if (!(vmax <= 1.0f)) {                     /* else every s is 1 */
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) {
+                            nl[c] = div_norm2_any(nl[c], s[c], ny[c]);
+                            nh[c] = div_norm2_any(nh[c], s[c], ny[c]);
+                        }
                     }
                 } else {
 #pragma unroll
@@ -1716,6 +1758,9 @@ PM_DEV void pds_tile(float4* __restrict__ uout, float* __restrict__ pout, const 
             if (tame && m >= PDS_TINY) {
 #pragma unroll
                 for (int c = 0; c < 3; ++c) num[c] = neg_div2(num[c], bu, nu);
+            } else if (tame) {
+#pragma unroll
+                for (int c = 0; c < 3; ++c) num[c] = neg_div2_any(num[c], bu, nu);
             } else {
 #pragma unroll
                 for (int c = 0; c < 3; ++c)

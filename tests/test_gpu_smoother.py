@@ -1,8 +1,8 @@
 """The blocked PD smoother against the oracle's steps, bit for bit, where its
 tiling and its branches can go wrong: image sizes around the tile (56 x 16) and
 column-pair edges, step counts that are no multiple of the steps per launch,
-warm starts that reach the IEEE divisions (values below 2^-100, of 1e30, not
-finite) and a non-finite image weight."""
+warm starts that reach the scaled divisions (values below 2^-100, alone and
+beside norms above 1) and the IEEE ones (1e30, not finite) and a non-finite image weight."""
 import numpy as np
 import pytest
 import torch
@@ -24,6 +24,9 @@ def _warm(kind, rng, shape):
         u[rng.random(shape[:-1]) < 0.3, :3] = 0.0
     elif kind == "steep":                    # norms well above 1
         u[..., :3] *= 300.0
+    elif kind == "steeptiny":                # norms above 1 beside components of 1e-20 .. 1e-44
+        u[..., 0] *= 300.0
+        u[..., 1:3] *= (10.0 ** rng.uniform(-44, -20, shape[:-1] + (2,))).astype(np.float32)
     elif kind == "huge":
         u[rng.random(shape[:-1]) < 0.02, :3] = 1e30
     elif kind == "nonfinite":
@@ -34,8 +37,8 @@ def _warm(kind, rng, shape):
 
 
 @pytest.mark.parametrize("W,H", [(1, 1), (2, 3), (3, 40), (55, 15), (56, 16), (57, 17), (61, 33), (113, 49)])
-@pytest.mark.parametrize("kind,steps", [("mixed", 3), ("zeros", 30), ("tiny", 9), ("steep", 8), ("huge", 6),
-                                        ("nonfinite", 5)])
+@pytest.mark.parametrize("kind,steps", [("mixed", 3), ("zeros", 30), ("tiny", 9), ("steep", 8), ("steeptiny", 2),
+                                        ("huge", 6),                                         ("nonfinite", 5)])
 def test_smoother_bits(cuda, oracle, W, H, kind, steps):
     from cvt_gb300.stereo import PMHuberStereo
     rng = np.random.default_rng(W * 1000 + H * 10 + steps)
