@@ -281,17 +281,15 @@ PM_DEV PmRecRow rec_row(const PmView& v, int rp, int y) {
     return {v.recA + o, v.recB + o, v.recC + o, v.recD + o};
 }
 
-PM_DEV void fast_tap_terms(const PmCostConsts& k, const PmRecRow& row, int xi, float a, float4 a1, float4 g1,
-                           float& cc, float& gc) {
-    const float4 A = __ldg(row.A + xi);
-    const float4 B = __ldg(row.B + xi);
-    const float4 Cc = __ldg(row.C + xi);
-    const float2 D = __ldg(row.D + xi);
+/* The truncated differences of a tap at fraction a between the values
+ * (A; Cv; dx) and with the forward differences (B; Cd; dy). */
+PM_DEV void fast_terms(const PmCostConsts& k, float2 A0, float2 A1, float2 C0, float D0, float2 B0, float2 B1, float2 C1,
+                       float D1, float a, float4 a1, float4 g1, float& cc, float& gc) {
     const float2 aa = make_float2(a, a);
-    const float2 v01 = ffma2(aa, make_float2(B.x, B.y), make_float2(A.x, A.y));     /* c0, c1 */
-    const float2 v23 = ffma2(aa, make_float2(B.z, B.w), make_float2(A.z, A.w));     /* c2, g0 */
-    const float2 v45 = ffma2(aa, make_float2(Cc.z, Cc.w), make_float2(Cc.x, Cc.y)); /* g1, g2 */
-    const float v6 = fmaf(a, D.y, D.x);                                              /* g3 */
+    const float2 v01 = ffma2(aa, B0, A0);                                            /* c0, c1 */
+    const float2 v23 = ffma2(aa, B1, A1);                                            /* c2, g0 */
+    const float2 v45 = ffma2(aa, C1, C0);                                            /* g1, g2 */
+    const float v6 = fmaf(a, D1, D0);                                                /* g3 */
     const float2 d01 = fsub2(make_float2(a1.x, a1.y), v01);
     const float2 d23 = fsub2(make_float2(a1.z, g1.x), v23);
     const float2 d45 = fsub2(make_float2(g1.y, g1.z), v45);
@@ -302,6 +300,16 @@ PM_DEV void fast_tap_terms(const PmCostConsts& k, const PmRecRow& row, int xi, f
     const float2 s = fadd2(fadd2(make_float2(m0, m3), make_float2(m1, m4)), make_float2(m2, m5));
     cc = s.x;                                      /* (m0 + m1) + m2 */
     gc = s.y + m6;                                 /* ((m3 + m4) + m5) + m6 */
+}
+
+PM_DEV void fast_tap_terms(const PmCostConsts& k, const PmRecRow& row, int xi, float a, float4 a1, float4 g1,
+                           float& cc, float& gc) {
+    const float4 A = __ldg(row.A + xi);
+    const float4 B = __ldg(row.B + xi);
+    const float4 Cc = __ldg(row.C + xi);
+    const float2 D = __ldg(row.D + xi);
+    fast_terms(k, make_float2(A.x, A.y), make_float2(A.z, A.w), make_float2(Cc.x, Cc.y), D.x, make_float2(B.x, B.y),
+               make_float2(B.z, B.w), make_float2(Cc.z, Cc.w), D.y, a, a1, g1, cc, gc);
 }
 
 /* The bilateral weight of tap (centre colour vc, tap colour a1, profile
@@ -387,6 +395,15 @@ PM_DEV void tap_weight_centres(float4 va, float4 vb, float4 a1, float pa, float 
 template <int K, bool EXACT>
 PM_DEV void eval_costs(const PmCostConsts& k, const PmView& v1, const PmView& v2, int x, int y,
                        const float4 (&s)[K], const bool (&act)[K], float (&cost)[K]) {
+    /* FAST, up to two candidates: a plane's slope is near 1, so the next tap
+     * mostly lies between the columns xi + 1 and xi + 2.  The values at xi + 1
+     * are kept and each tap loads those of one more column, in place of a
+     * record's values and differences (8 L1 wavefronts a warp for 14), and forms
+     * the record's differences itself; a lane that did not advance by one loads
+     * its own column again.  1242x375, per launch (ncu): k_sweep 4.73 -> 4.31 ms,
+     * k_init 3.2 -> 2.5, the first refinements 5.4 -> 4.8; depthMap 327 -> 319
+     * ms.  More candidates would spill the 8 registers each. */
+    constexpr bool NEXT = !EXACT && K <= 2;
     float sx[K], sy[K], sz[K];
     /* FAST: X is the candidate's Q31.32 position at the current tap, S0 its
      * step along a row and D the step from a row's end to the next row's
@@ -414,8 +431,14 @@ PM_DEV void eval_costs(const PmCostConsts& k, const PmView& v1, const PmView& v2
         }
     }
     float ws[K], r1[K], r2[K];
+    /* the second image's values at column at + 1 (clamped) of the row */
+    float4 nc[K], ng[K];
+    int at[K];
 #pragma unroll
-    for (int c = 0; c < K; ++c) { ws[c] = 0.0f; r1[c] = 0.0f; r2[c] = 0.0f; }
+    for (int c = 0; c < K; ++c) {
+        ws[c] = 0.0f; r1[c] = 0.0f; r2[c] = 0.0f;
+        if constexpr (NEXT) nc[c] = ng[c] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
     const float4 vc = __ldg(&v1.col[(size_t)y * k.W + x]);
     for (int qy = qy0; qy <= qy1; ++qy) {
         const int dy = qy - y;
@@ -424,6 +447,9 @@ PM_DEV void eval_costs(const PmCostConsts& k, const PmView& v1, const PmView& v2
         const float4* g1row = v1.grad + (size_t)qy * k.W;
         const float* prow = c_prof + (dy + PM_PMAX) * PM_PROF_N + PM_PMAX;
         const PmRecRow rrow = rec_row(v2, k.rp, qy);
+        const float4 *c2row = v2.col + (size_t)qy * k.W, *g2row = v2.grad + (size_t)qy * k.W;
+#pragma unroll
+        for (int c = 0; c < K; ++c) at[c] = -2;
         /* candidate c's terms at tap column qx, folded into its sums */
         auto one = [&](int c, int qx, float4 a1, float4 g1, float w1) {
                 if (EXACT) {
@@ -454,7 +480,20 @@ PM_DEV void eval_costs(const PmCostConsts& k, const PmView& v1, const PmView& v2
                     const int xi = (int)(Xt >> 32);
                     if ((unsigned)xi >= (unsigned)k.W) return;
                     float cc, gc;
-                    fast_tap_terms(k, rrow, xi, pm_fix_frac(Xt), a1, g1, cc, gc);
+                    if constexpr (NEXT) {
+                        float4 c0 = nc[c], h0 = ng[c];
+                        if (xi != at[c] + 1) { c0 = __ldg(&c2row[xi]); h0 = __ldg(&g2row[xi]); }
+                        const int xn = min(xi + 1, k.W - 1);
+                        nc[c] = __ldg(&c2row[xn]);
+                        ng[c] = __ldg(&g2row[xn]);
+                        at[c] = xi;
+                        const float4 c1 = nc[c], h1 = ng[c];
+                        fast_terms(k, make_float2(c0.x, c0.y), make_float2(c0.z, h0.x), make_float2(h0.y, h0.z), h0.w,
+                                   make_float2(c1.x - c0.x, c1.y - c0.y), make_float2(c1.z - c0.z, h1.x - h0.x),
+                                   make_float2(h1.y - h0.y, h1.z - h0.z), h1.w - h0.w, pm_fix_frac(Xt), a1, g1, cc, gc);
+                    } else {
+                        fast_tap_terms(k, rrow, xi, pm_fix_frac(Xt), a1, g1, cc, gc);
+                    }
                     const float2 r = ffma2(make_float2(w1, w1), make_float2(cc, gc), make_float2(r1[c], r2[c]));
                     r1[c] = r.x;                   /* fmaf(w1, cc, r1), fmaf(w1, gc, r2) */
                     r2[c] = r.y;
