@@ -2130,14 +2130,15 @@ cudaError_t pm_prepare_kernels() {
  * images, at more work and more L1 traffic per tap than a thread per pixel, and
  * (for candidates 1-8 and 10-15) than shared plane windows.  Per depthMap of 3
  * iterations (FAST; EXACT), ms:
- *   all candidates tap-parallel against shared windows: 96x72 7.1, 9.3 (8.0,
- *   10.1); 128x96 10.3, 10.6 (11.5, 11.3); 160x120 14.0, 11.8 (17.1, 13.6);
+ *   all candidates tap-parallel against shared windows: 96x72 7.1, 8.2 (8.0,
+ *   8.9); 100x80 8.1, 8.5; 100x90 8.8, 8.7 (10.1, 9.6); 112x98 10.0, 9.3 (11.5,
+ *   10.2); 124x100 10.6, 9.7 (12.2, 10.6);
  *   the others tap-parallel against a thread per pixel, with shared windows:
  *   160x120 11.8, 15.2 (13.6, 17.9); 200x150 15.1, 16.1 (16.1, 18.7); 240x180
  *   18.8, 18.2 (20.6, 21.3); 280x210 24.7, 22.3 (28.5, 26.8).
  * A cost field: 160x120 0.162 against 0.454 (0.198, 0.427); 321x243 0.544
  * against 0.525 (0.704, 0.596). */
-#define TP_MAX_PIXELS 12500
+#define TP_MAX_PIXELS 8500
 #define TS_MAX_PIXELS 40000
 #define TF_MAX_PIXELS 60000
 bool pm_shared_windows(const PmCostConsts& k) {

@@ -332,7 +332,7 @@ class PMHuberStereo:
 
     def set_memory_budget(self, nbytes: int) -> None:
         """Device bytes a propagation pass may use to share work between its
-        candidates: 32 per pixel, 576 for images of at most 12500 pixels (0:
+        candidates: 32 per pixel, 576 for images of at most 8500 pixels (0:
         every candidate per pixel; results are the same)."""
         self._check(_lib.lib().cvtpm_set_memory_budget(self._h, int(nbytes)))
 
