@@ -293,7 +293,7 @@ def run_ours(args, rank, world, local_rank):
     flops_launch = (stats["cost_taps"] * FLOPS_PER_TAP) / nprop + in_image_taps(W, H, PATCH) * FLOPS_PER_WEIGHT_TAP
     achieved = flops_launch / (prop_ms * 1e-3) / 1e12
     traffic = read_traffic()
-    roofline = {"kernel": "k_propagate<fast>", "bound": "fp32", "achieved": achieved,
+    roofline = {"kernel": "k_sweep + k_share + k_views + k_propagate (the propagation pass, fast)", "bound": "fp32", "achieved": achieved,
                 "peak": fp32_tflops, "unit": "TFLOP/s",
                 "frac": (achieved / fp32_tflops) if fp32_tflops else None,
                 "traffic": traffic.get("k_propagate_bytes_per_launch"),
@@ -316,8 +316,8 @@ def run_ours(args, rank, world, local_rank):
                    "steps_per_launch": stats["pd_steps"] / max(1, stats["pd_launches"]),
                    "timed": "the blocked PD kernel alone, 248 steps on the bench pair's left smoother input "
                             "(cvtpm_tool_pd_time); inside depthMap the two views' smoothers run concurrently",
-                   "note": "the blocked kernel keeps 4 steps in shared memory, so it moves fewer bytes than one step's algorithmic count"}
-    # the propagation's limiter is the L1 data path: its record bytes against
+                   "note": "the blocked kernel keeps 4 steps in registers, so it moves fewer bytes than one step's algorithmic count"}
+    # the propagation's L1 rate: the algorithm's record bytes against
     # 128 B per clock and SM at the sampled clock
     clocks = clk.summary()
     n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
@@ -328,12 +328,12 @@ def run_ours(args, rank, world, local_rank):
     roofline["peak_derived_source"] = (f"{n_sm} SMs x {FP32_LANES_PER_SM} FP32 lanes x 2 flops x the median SM clock "
                                        "sampled during the timed region")
     l1_achieved = stats["cost_taps"] / nprop * RECORD_BYTES_PER_TAP / (prop_ms * 1e-3) / 1e9
-    roofline_l1 = {"kernel": "k_propagate<fast> + k_nbcost (the propagation pass)", "bound": "l1",
+    roofline_l1 = {"kernel": "k_sweep + k_share + k_views + k_propagate (the propagation pass, fast)", "bound": "l1",
                    "achieved": l1_achieved, "peak": l1_peak, "unit": "GB/s",
                    "frac": (l1_achieved / l1_peak) if l1_peak else None,
-                   "per": "pass: device-counted evaluated taps x 56 record bytes (a lower bound: image-1 reads, "
-                          "weights and misaligned 128-byte lines come on top; ncu measures the L1 data pipe at "
-                          "81-88 % busy) / pass time",
+                   "per": "pass: device-counted evaluated taps x 56 record bytes, as if every candidate read its own "
+                          "window (k_share reads a plane's window once for all candidates that test it, and the "
+                          "sweeps 28 bytes a tap, so the rate can pass the peak) / pass time",
                    "peak_source": f"{n_sm} SMs (from the device) x 128 B/clk x the median SM clock sampled during "
                                   "the timed region"}
     cpu = None
