@@ -211,9 +211,12 @@ __device__ __forceinline__ float ray_bound(float o, float d, int extent, bool st
 }
 
 /* Which bricks of 8^3 voxels hold a voxel of weight >= 1 (or NaN: the test of
- * trilinear, inverted), one byte each, and in `coarse` which bricks of 32^3
- * do (cleared before).  A thread reads a column of 64 voxels of one x; the
- * volume is read once, 8 bytes per voxel (HBM-bound). */
+ * trilinear, inverted), one byte each; and from those, which bricks of 32^3
+ * do.  A thread reads a column of 64 voxels of one x; the volume is read once,
+ * 8 bytes per voxel (HBM-bound).  The bytes are a volume's own and every cast
+ * forms them anew, each byte stored once and never cleared first: casts of one
+ * volume on several streams store the values that are there, so one may march
+ * while another marks. */
 #define TSDF_FINE 3                                  /* log2 of the extents */
 #define TSDF_COARSE 5
 struct BrickGrid {
@@ -221,8 +224,7 @@ struct BrickGrid {
     int fw, fh, cw, ch;                              /* bricks per row and per column */
 };
 __global__ void __launch_bounds__(256) k_tsdf_bricks(const float2* __restrict__ cv, int W, int H, int D,
-                                                     unsigned char* __restrict__ fine, unsigned char* __restrict__ coarse,
-                                                     BrickGrid g) {
+                                                     unsigned char* __restrict__ fine, BrickGrid g) {
     const int x = blockIdx.x * 256 + threadIdx.x, y0 = blockIdx.y * 8, z0 = blockIdx.z * 8;
     bool any = false;
     if (x < W) {
@@ -244,8 +246,19 @@ __global__ void __launch_bounds__(256) k_tsdf_bricks(const float2* __restrict__ 
     const unsigned m = __ballot_sync(0xffffffffu, any);
     if ((threadIdx.x & 7) == 0 && x < W)
         fine[((size_t)blockIdx.z * g.fh + blockIdx.y) * g.fw + (x >> 3)] = (m >> (threadIdx.x & 31)) & 0xffu ? 1 : 0;
-    if (m && (threadIdx.x & 31) == 0 && x < W)
-        coarse[((size_t)(blockIdx.z >> 2) * g.ch + (blockIdx.y >> 2)) * g.cw + (x >> 5)] = 1;
+}
+
+/* A coarse brick per thread: any of its 4^3 fine ones (fd of them in z). */
+__global__ void __launch_bounds__(128) k_tsdf_coarse(const unsigned char* __restrict__ fine, unsigned char* __restrict__ coarse,
+                                                     BrickGrid g, int fd, int cd) {
+    const size_t i = (size_t)blockIdx.x * 128 + threadIdx.x;
+    if (i >= (size_t)g.cw * g.ch * cd) return;
+    const int cx = (int)(i % g.cw), cy = (int)(i / g.cw % g.ch), cz = (int)(i / g.cw / g.ch);
+    unsigned char any = 0;
+    for (int z = 4 * cz; z < min(4 * cz + 4, fd); ++z)
+        for (int y = 4 * cy; y < min(4 * cy + 4, g.fh); ++y)
+            for (int x = 4 * cx; x < min(4 * cx + 4, g.fw); ++x) any |= fine[((size_t)z * g.fh + y) * g.fw + x];
+    coarse[i] = any;
 }
 
 /* The march evaluates samples half a voxel apart, and most of them lie where
@@ -364,7 +377,7 @@ struct cvtpm_tsdf {
     float trunc;
     Mat4 g2w;
     float2* vol;
-    unsigned char* bricks;     /* scratch of a ray cast, behind the volume; NULL: no room for it */
+    unsigned char* bricks;     /* marks of the ray casts, behind the volume; NULL: no room for them */
 };
 
 /* bricks of 1 << sh voxels along an extent */
@@ -494,8 +507,9 @@ cvtpm_status cvtpm_tsdf_raycast(cvtpm_tsdf* v, const float* proj, float* depthma
         /* formed anew for each cast: the caller may write the volume (cvtpm_tsdf_info) */
         const int fd = tsdf_bricks(v->D, TSDF_FINE), cd = tsdf_bricks(v->D, TSDF_COARSE);
         unsigned char *fine = v->bricks, *coarse = fine + (size_t)g.fw * g.fh * fd;
-        cudaMemsetAsync(coarse, 0, (size_t)g.cw * g.ch * cd, (cudaStream_t)stream);
-        k_tsdf_bricks<<<dim3((v->W + 255) / 256, g.fh, fd), 256, 0, (cudaStream_t)stream>>>(v->vol, v->W, v->H, v->D, fine, coarse, g);
+        k_tsdf_bricks<<<dim3((v->W + 255) / 256, g.fh, fd), 256, 0, (cudaStream_t)stream>>>(v->vol, v->W, v->H, v->D, fine, g);
+        const size_t nc = (size_t)g.cw * g.ch * cd;
+        k_tsdf_coarse<<<(unsigned)((nc + 127) / 128), 128, 0, (cudaStream_t)stream>>>(fine, coarse, g, fd, cd);
         g.fine = fine;
         g.coarse = coarse;
     }

@@ -570,7 +570,8 @@ cvtpm_status cvtpm_tsdf_add_depthmap(cvtpm_tsdf* vol, const float* proj, const f
  * surface along each pixel's ray, 0 where there is none.  A ray whose march
  * cannot advance in float (a camera about 2^24 voxels from the volume) stops
  * after 2 * max(width, height, depth) + 16 steps with 0, where the
- * reference's loop does not end. */
+ * reference's loop does not end.  A cast only reads the volume: casts of one
+ * volume may run at once on several streams, ordered against what writes it. */
 cvtpm_status cvtpm_tsdf_raycast(cvtpm_tsdf* vol, const float* proj, float* depthmap,
                                 int dwidth, int dheight, size_t dpitch, float scale, void* stream);
 /* The slice kernels TSDFVolume_sliceX/Y/Z (axis 0/1/2, plane `index`) into
