@@ -764,7 +764,7 @@ __global__ void __launch_bounds__(SH_NT, 1) k_share(PmPassArgs a, int ty) { shar
  *
  * An invalid tap (outside either image) is stored with a NaN in place of its
  * first term; no valid term is a NaN as long as neither truncation is
- * (pm_launch_propagate takes the other path then). */
+ * (pm_shared_windows sends the others to the per-pixel stages). */
 #define TP_NP 8                                      /* producer warps */
 
 template <bool EXACT> struct TpTerm { typedef float2 type; };
@@ -814,7 +814,10 @@ PM_DEV float tp_costs(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, const Pm
     const int x = min(x0 + lane, W - 1);             /* lanes past the row repeat its last pixel */
     __syncthreads();                                 /* the planes are in place */
     const unsigned live = S.live;
-    if (!live) return 1e5f;                          /* block-uniform: no plane to evaluate */
+    if (!live) {                                     /* block-uniform: no plane to evaluate */
+        __syncthreads();                             /* every warp has read it: the caller may write S again */
+        return 1e5f;
+    }
     const int qy0 = max(y - P, 0), ny = min(y + P, H - 1) - qy0 + 1;
     /* block-uniform columns: every offset that is inside the image for some lane */
     const int dlo = max(-P, -(x0 + 31)), nx = min(P, W - 1 - x0) - dlo + 1;
