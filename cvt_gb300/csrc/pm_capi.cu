@@ -61,6 +61,7 @@ struct cvtpm_ctx {
      * when the budget allows */
     void* pass = nullptr;
     size_t pass_bytes = 0;
+    size_t pass_pixels = 0;           /* the largest image it was allocated for */
     size_t pass_budget = SIZE_MAX;
     /* set while a launch sequence is being captured into a graph: scratch
      * must already be sized, nothing may be allocated */
@@ -338,30 +339,43 @@ cvtpm_status propagate_view(cvtpm_ctx* ctx, PmPassArgs a, bool exact, bool redbl
  * part can run beside the left view's pass (*overlap); the view candidates'
  * part is used by one view at a time.  The most that fits the context's budget
  * and 60 % of the free memory is taken; with none of it every candidate is
- * evaluated per pixel.  Results are the same in every case. */
-cvtpm_status plan_pass(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H, bool taps, PmPassArgs* aL, PmPassArgs* aR,
-                       bool* overlap) {
+ * evaluated per pixel.  Results are the same in every case.
+ *
+ * A caller's captured graphs hold the scratch's address, so it is replaced, as
+ * the pool of ensure_buffers is, only for an image of more pixels than any
+ * before: an allocation is large enough for every smaller image too (their
+ * tap-parallel passes take more than the shared windows of larger ones), and
+ * where memory was short then, what there is stays.  While `st` is captured
+ * nothing is allocated. */
+cvtpm_status plan_pass(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H, bool taps, cudaStream_t st, PmPassArgs* aL,
+                       PmPassArgs* aR, bool* overlap) {
     const PmCostConsts k = base_args(ctx, p, W, H, 0).k;
     *overlap = p.schedule == CVTPM_SCHEDULE_JACOBI;
     if (!*overlap || !pm_shared_windows(k)) return CVTPM_OK;
     const size_t n = (size_t)W * H;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cap), "capture status");
+    const bool grow = !ctx->no_alloc && cap == cudaStreamCaptureStatusNone && (!ctx->pass || n > ctx->pass_pixels);
+    const size_t small = taps ? std::min(n, (size_t)pm_tap_parallel_pixels()) * sizeof(float4) * 36 : 0;
     taps = taps && pm_tap_parallel(k);
     for (int plan = taps ? 0 : 2; plan < 4; ++plan) {
         const bool both = (plan & 1) == 0, t = plan < 2;
         const size_t need = t ? n * sizeof(float4) * (both ? 36 : 20) : n * sizeof(float) * (both ? 8 : 6);
         if (need > ctx->pass_budget) continue;
         if (need > ctx->pass_bytes) {
-            if (ctx->no_alloc) continue;             /* capturing: what is there */
+            if (!grow) continue;                     /* what is there */
             if (ctx->pass) { CK(cudaFree(ctx->pass), "free pass scratch"); ctx->pass = nullptr; ctx->pass_bytes = 0; }
             size_t fr = 0, tot = 0;
             CK(cudaMemGetInfo(&fr, &tot), "memory info");
             if ((double)need > 0.6 * (double)fr) continue;
-            if (cudaMalloc(&ctx->pass, need) != cudaSuccess) {
+            const size_t most = std::min(std::max(need, small), std::min(ctx->pass_budget, (size_t)(0.6 * (double)fr)));
+            if (cudaMalloc(&ctx->pass, most) != cudaSuccess) {
                 cudaGetLastError();                  /* clear the failed allocation */
                 ctx->pass = nullptr;
                 continue;
             }
-            ctx->pass_bytes = need;
+            ctx->pass_bytes = most;
+            ctx->pass_pixels = n;
         }
         if (t) {
             aL->cand = (float4*)ctx->pass;
@@ -489,7 +503,7 @@ cvtpm_status run_depthmap(cvtpm_ctx* ctx, const cvtpm_params& p, float* dmap, si
     const int N = p.iterations;
     PmPassArgs aL = base_args(ctx, p, W, H, 0), aR = base_args(ctx, p, W, H, 1);
     bool overlap = false;
-    if ((s = plan_pass(ctx, p, W, H, true, &aL, &aR, &overlap)) != CVTPM_OK) return s;
+    if ((s = plan_pass(ctx, p, W, H, true, st, &aL, &aR, &overlap)) != CVTPM_OK) return s;
     if (!ctx->dcount) {
         if (ctx->no_alloc) return fail(ctx, CVTPM_ERR_ALLOC, "counters not allocated before capture");
         CK(cudaMalloc(&ctx->dcount, 2 * sizeof(unsigned long long)), "counters");
@@ -652,7 +666,7 @@ cvtpm_status run_depthmap_inpaint(cvtpm_ctx* ctx, const cvtpm_params& p, float* 
     const int N = p.iterations;
     PmPassArgs aL = base_args(ctx, p, W, H, 0), aR = base_args(ctx, p, W, H, 1);
     bool overlap = false;                                          /* not used: one stream here */
-    if ((s = plan_pass(ctx, p, W, H, true, &aL, &aR, &overlap)) != CVTPM_OK) return s;
+    if ((s = plan_pass(ctx, p, W, H, true, st, &aL, &aR, &overlap)) != CVTPM_OK) return s;
     if (!ctx->dcount) {
         if (ctx->no_alloc) return fail(ctx, CVTPM_ERR_ALLOC, "counters not allocated before capture");
         CK(cudaMalloc(&ctx->dcount, 2 * sizeof(unsigned long long)), "counters");
@@ -1002,6 +1016,7 @@ cvtpm_status cvtpm_cost_eval(cvtpm_ctx* ctx, const float* img1, const float* img
 
 cvtpm_status cvtpm_set_memory_budget(cvtpm_ctx* ctx, size_t bytes) {
     if (!ctx) return CVTPM_ERR_INVALID_ARGUMENT;
+    if (bytes != ctx->pass_budget) ctx->pass_pixels = 0;   /* the next call may size the scratch anew */
     ctx->pass_budget = bytes;
     if (ctx->pass && ctx->pass_bytes > bytes) {
         CK(cudaSetDevice(ctx->device), "cudaSetDevice");
@@ -1195,7 +1210,7 @@ cvtpm_status capture_batch(cvtpm_ctx* ctx, const cvtpm_pair* pairs, int npairs, 
             if ((s = ensure_buffers(c, pairs[i].width, pairs[i].height)) != CVTPM_OK) return fail(ctx, s, c->err);
             PmPassArgs aL, aR;
             bool overlap;
-            if ((s = plan_pass(c, p, pairs[i].width, pairs[i].height, true, &aL, &aR, &overlap)) != CVTPM_OK)
+            if ((s = plan_pass(c, p, pairs[i].width, pairs[i].height, true, ctx->bstream, &aL, &aR, &overlap)) != CVTPM_OK)
                 return fail(ctx, s, c->err);
         }
     }
@@ -1369,7 +1384,7 @@ cvtpm_status phase_prepare(PhaseState& S) {
         if ((s = ensure_buffers(c, S.pairs[i].width, S.pairs[i].height)) != CVTPM_OK) return fail(S.ctx, s, c->err);
         PmPassArgs aL, aR;
         bool overlap;
-        if ((s = plan_pass(c, c->prm, S.pairs[i].width, S.pairs[i].height, false, &aL, &aR, &overlap)) != CVTPM_OK)
+        if ((s = plan_pass(c, c->prm, S.pairs[i].width, S.pairs[i].height, false, S.st, &aL, &aR, &overlap)) != CVTPM_OK)
             return fail(S.ctx, s, c->err);
         S.maxW = std::max(S.maxW, S.pairs[i].width);
     }
@@ -1406,7 +1421,7 @@ cvtpm_status phase_start(PhaseState& S) {
         S.aL[i] = base_args(c, c->prm, W, H, 0);
         S.aR[i] = base_args(c, c->prm, W, H, 1);
         bool overlap;
-        if ((s = plan_pass(c, c->prm, W, H, false, &S.aL[i], &S.aR[i], &overlap)) != CVTPM_OK) return fail(ctx, s, c->err);
+        if ((s = plan_pass(c, c->prm, W, H, false, S.st, &S.aL[i], &S.aR[i], &overlap)) != CVTPM_OK) return fail(ctx, s, c->err);
         S.aL[i].counters = S.aR[i].counters = c->dcount;
         S.aL[i].out = c->S[0][0];
         S.aR[i].out = c->S[1][0];
@@ -1697,7 +1712,8 @@ cvtpm_status tune_mode(PhaseState& full, float ms[2]) {
     while (S.n < full.n && (S.n == 0 || px < 4000000)) {
         PmPassArgs aL, aR;
         bool overlap;
-        if (s == CVTPM_OK) s = plan_pass(lane, S.p, full.pairs[S.n].width, full.pairs[S.n].height, true, &aL, &aR, &overlap);
+        if (s == CVTPM_OK)
+            s = plan_pass(lane, S.p, full.pairs[S.n].width, full.pairs[S.n].height, true, S.st, &aL, &aR, &overlap);
         px += (long long)full.pairs[S.n].width * full.pairs[S.n].height;
         maxW = std::max(maxW, full.pairs[S.n].width);
         maxH = std::max(maxH, full.pairs[S.n].height);

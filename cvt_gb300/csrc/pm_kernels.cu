@@ -2148,6 +2148,7 @@ cudaError_t pm_prepare_kernels() {
 bool pm_shared_windows(const PmCostConsts& k) {
     return std::isfinite(k.alpha) && std::isfinite(k.cmax) && std::isfinite(k.gmax);
 }
+int pm_tap_parallel_pixels() { return TP_MAX_PIXELS; }
 bool pm_tap_parallel(const PmCostConsts& k) { return (size_t)k.W * k.H <= TP_MAX_PIXELS && pm_shared_windows(k); }
 bool pm_tap_sweeps(const PmCostConsts& k) { return (size_t)k.W * k.H <= TS_MAX_PIXELS && pm_shared_windows(k); }
 bool pm_tap_field(const PmCostConsts& k) { return (size_t)k.W * k.H <= TF_MAX_PIXELS && pm_shared_windows(k); }

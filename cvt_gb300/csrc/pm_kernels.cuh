@@ -148,6 +148,7 @@ bool pm_shared_windows(const PmCostConsts& k);
 /* Whether all candidates of a pass run tap-parallel (the smallest images),
  * given PmPassArgs::cand and vcand; whether single candidates do (small ones). */
 bool pm_tap_parallel(const PmCostConsts& k);
+int pm_tap_parallel_pixels();                        /* the most pixels of such an image */
 bool pm_tap_sweeps(const PmCostConsts& k);
 /* Whether a cost field does. */
 bool pm_tap_field(const PmCostConsts& k);

@@ -274,7 +274,10 @@ cvtpm_status cvtpm_polish_planes(cvtpm_ctx* ctx, const float* img1, const float*
  * their matching terms formed once per plane; images of at most 8500 pixels
  * use 576 (320) instead, to run every candidate's window taps in
  * parallel.  Otherwise (and beyond 60 % of the free memory) every candidate is
- * evaluated per pixel.  Results are identical either way.  Default: no limit;
+ * evaluated per pixel.  Results are identical either way.  The context keeps
+ * the memory, replaces it for an image of more pixels than any before, as its
+ * other scratch, and allocates none under stream capture (a graph holds its
+ * address); after a change of the limit, capture anew.  Default: no limit;
  * 0 turns both off.  No counterpart in the reference. */
 cvtpm_status cvtpm_set_memory_budget(cvtpm_ctx* ctx, size_t bytes);
 
