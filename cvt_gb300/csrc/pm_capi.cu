@@ -351,7 +351,7 @@ cvtpm_status plan_pass(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H, bool
                        PmPassArgs* aR, bool* overlap) {
     const PmCostConsts k = base_args(ctx, p, W, H, 0).k;
     *overlap = p.schedule == CVTPM_SCHEDULE_JACOBI;
-    if (!*overlap || !pm_shared_windows(k)) return CVTPM_OK;
+    if (!*overlap) return CVTPM_OK;
     const size_t n = (size_t)W * H;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(st, &cap), "capture status");

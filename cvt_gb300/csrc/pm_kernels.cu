@@ -20,7 +20,6 @@
 #define PM_KERNELS_TU 1
 #include "pm_kernels.cuh"
 
-#include <cmath>
 #include <type_traits>
 
 /* Blocks of 256 threads per SM the FAST propagation is compiled for. */
@@ -389,6 +388,15 @@ __device__ __forceinline__ bool nb_tap_terms(const PmCostConsts& k, const PmView
     }
 }
 
+/* The mark of an invalid tap (outside either image) in the term a block shares
+ * for it: a NaN of this payload.  A valid term can be a NaN too (a truncation
+ * that is not finite; EXACT: 0 or an overflow times an infinite sum), but it is
+ * the result of an addition, whose NaN is always 0x7fffffff, and counts. */
+#define PM_NO_TERM 0x7fe5a5a5
+PM_DEV float no_term() { return __int_as_float(PM_NO_TERM); }
+PM_DEV bool is_term(float t) { return __float_as_int(t) != PM_NO_TERM; }
+PM_DEV bool is_term(float2 t) { return is_term(t.x); }
+
 /* One user's sums, in eval_costs' operations: EXACT ws += w, r1 += w * C;
  * FAST r1 = fma(w, cc, r1), r2 = fma(w, gc, r2), ws += w. */
 template <bool EXACT>
@@ -484,9 +492,8 @@ PM_DEV float4 smooth_state(float4 smooth, float cx, float cy, int lr) {
  * slots their candidates are in, and the 12 columns in use (offsets -1..7 of
  * four taps) and the four being formed fill the ring of 16.
  *
- * An invalid tap (outside either image) is a NaN in the first term, which no
- * valid term is for finite truncations (pm_shared_windows).  The sums take
- * eval_costs' operations in its order, so the costs have its bits.
+ * An invalid tap (outside either image) is marked in its first term (no_term).
+ * The sums take eval_costs' operations in its order, so the costs have its bits.
  *
  * Measured at 1242x375 per view pass (ncu): 9.7 ms for the 14 candidates and
  * the acceptance, where the neighbours by plane (5.9 ms, weights in a table
@@ -648,7 +655,7 @@ PM_DEV void share_tile(const PmPassArgs& a, int ty, int tbx, int tby) {
                     float cc = 0.0f, gc = 0.0f;
                     bool ok = q >= 0 && q < W;
                     if (ok) ok = nb_tap_terms<EXACT>(a.k, a.v2, q, Yq, rrow, sx[i], sy[i], sz[i], Xt[i], a1, g1, cc, gc);
-                    if (!ok) cc = __int_as_float(0x7fc00000);
+                    if (!ok) cc = no_term();
                     if constexpr (EXACT) dst[i * (SH_NS / SLOTS) * R] = cc;
                     else dst[i * (SH_NS / SLOTS) * R] = make_float2(cc, gc);
                 }
@@ -659,9 +666,9 @@ PM_DEV void share_tile(const PmPassArgs& a, int ty, int tbx, int tby) {
     };
     auto fold = [&](int c, Term t, float wt) {
         if constexpr (EXACT) {
-            if (t == t) nb_accumulate<true>(wt, t, 0.0f, r1[c], r2[c], ws[c]);
+            if (is_term(t)) nb_accumulate<true>(wt, t, 0.0f, r1[c], r2[c], ws[c]);
         } else {
-            if (t.x == t.x) nb_accumulate<false>(wt, t.x, t.y, r1[c], r2[c], ws[c]);
+            if (is_term(t)) nb_accumulate<false>(wt, t.x, t.y, r1[c], r2[c], ws[c]);
         }
     };
     auto consume = [&](int Yq, int buf, int k) {     /* taps rx = -P + 4k .. + 3 */
@@ -762,9 +769,7 @@ __global__ void __launch_bounds__(SH_NT, 1) k_share(PmPassArgs a, int ty) { shar
  * of 8 that share weights and image-1 reads; the refinements, which need the
  * best of them, follow in a second launch, one candidate at a time.
  *
- * An invalid tap (outside either image) is stored with a NaN in place of its
- * first term; no valid term is a NaN as long as neither truncation is
- * (pm_shared_windows sends the others to the per-pixel stages). */
+ * An invalid tap (outside either image) is stored as no_term. */
 #define TP_NP 8                                      /* producer warps */
 
 template <bool EXACT> struct TpTerm { typedef float2 type; };
@@ -888,13 +893,13 @@ PM_DEV float tp_costs(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, const Pm
                         const TpPlane<EXACT> p = S.plane[c][lane];
                         float cc, gc;
                         const bool ok = nb_tap_terms<true>(k, v2, qx[h], qy[h], rrow, p.sx, p.sy, p.sz, 0, a1[h], g1[h], cc, gc);
-                        S.term[buf][j][c][lane] = ok && in[h] ? cc : __int_as_float(0x7fc00000);
+                        S.term[buf][j][c][lane] = ok && in[h] ? cc : no_term();
                     } else {
                         /* the sample column clamped to the row: the load needs no branch */
                         const int xi = (int)(Xt[h][c] >> 32);
                         float2 t;
                         fast_tap_terms(k, rrow, clampi(xi, 0, W - 1), pm_fix_frac(Xt[h][c]), a1[h], g1[h], t.x, t.y);
-                        if (!in[h] || (unsigned)xi >= (unsigned)W) t.x = __int_as_float(0x7fc00000);
+                        if (!in[h] || (unsigned)xi >= (unsigned)W) t.x = no_term();
                         S.term[buf][j][c][lane] = t;
                     }
                 }
@@ -908,9 +913,9 @@ PM_DEV float tp_costs(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, const Pm
             const Term t = S.term[buf][j][c][lane];
             const float wt = S.w[buf][j][lane];
             if constexpr (EXACT) {
-                if (t == t) nb_accumulate<true>(wt, t, 0.0f, r1, r2, ws);
+                if (is_term(t)) nb_accumulate<true>(wt, t, 0.0f, r1, r2, ws);
             } else {
-                if (t.x == t.x) nb_accumulate<false>(wt, t.x, t.y, r1, r2, ws);
+                if (is_term(t)) nb_accumulate<false>(wt, t.x, t.y, r1, r2, ws);
             }
         };
         int j = 0;
@@ -2145,13 +2150,10 @@ cudaError_t pm_prepare_kernels() {
 #define TP_MAX_PIXELS 8500
 #define TS_MAX_PIXELS 40000
 #define TF_MAX_PIXELS 60000
-bool pm_shared_windows(const PmCostConsts& k) {
-    return std::isfinite(k.alpha) && std::isfinite(k.cmax) && std::isfinite(k.gmax);
-}
 int pm_tap_parallel_pixels() { return TP_MAX_PIXELS; }
-bool pm_tap_parallel(const PmCostConsts& k) { return (size_t)k.W * k.H <= TP_MAX_PIXELS && pm_shared_windows(k); }
-bool pm_tap_sweeps(const PmCostConsts& k) { return (size_t)k.W * k.H <= TS_MAX_PIXELS && pm_shared_windows(k); }
-bool pm_tap_field(const PmCostConsts& k) { return (size_t)k.W * k.H <= TF_MAX_PIXELS && pm_shared_windows(k); }
+bool pm_tap_parallel(const PmCostConsts& k) { return (size_t)k.W * k.H <= TP_MAX_PIXELS; }
+bool pm_tap_sweeps(const PmCostConsts& k) { return (size_t)k.W * k.H <= TS_MAX_PIXELS; }
+bool pm_tap_field(const PmCostConsts& k) { return (size_t)k.W * k.H <= TF_MAX_PIXELS; }
 
 cudaError_t pm_launch_pd_block(float4* uout, float* pout, const float4* uin, const float* pin, int pzero,
                                const float4* f, const float* wgt, const float* mask, float lambda, int nsteps, int W,

@@ -142,9 +142,6 @@ cudaError_t pm_launch_normal_depth(const float4* in, int W, int H, float depthma
  * call once per device before the first launch or stream capture. */
 cudaError_t pm_prepare_kernels();
 
-/* Whether passes of these constants can share plane windows, given
- * PmPassArgs::costs and vcosts. */
-bool pm_shared_windows(const PmCostConsts& k);
 /* Whether all candidates of a pass run tap-parallel (the smallest images),
  * given PmPassArgs::cand and vcand; whether single candidates do (small ones). */
 bool pm_tap_parallel(const PmCostConsts& k);
