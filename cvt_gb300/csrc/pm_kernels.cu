@@ -20,6 +20,7 @@
 #define PM_KERNELS_TU 1
 #include "pm_kernels.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 /* Blocks of 256 threads per SM the FAST propagation is compiled for. */
@@ -825,7 +826,7 @@ PM_DEV float tp_costs(TpShared<EXACT, K, CH>& S, const PmCostConsts& k, const Pm
     }
     const int qy0 = max(y - P, 0), ny = min(y + P, H - 1) - qy0 + 1;
     /* block-uniform columns: every offset that is inside the image for some lane */
-    const int dlo = max(-P, -(x0 + 31)), nx = min(P, W - 1 - x0) - dlo + 1;
+    const int dlo = max(-P, -min(x0 + 31, W - 1)), nx = min(P, W - 1 - x0) - dlo + 1;
     const int T = nx * ny, nchunk = (T + CH - 1) / CH;
     const bool producer = w < TP_NP, consumer = w >= CW && w < CW + K;
     /* producer state: its next tap (row, col) and the candidates' positions there */
@@ -1993,7 +1994,7 @@ cudaError_t pm_launch_init(const PmPassArgs& a, bool exact, cudaStream_t st) {
 
 cudaError_t pm_launch_cost_field(const PmPassArgs& a, bool exact, const float4* states, float* cost, cudaStream_t st) {
     const int W = a.k.W, H = a.k.H;
-    if (pm_tap_field(a.k)) {
+    if (pm_tap_field(a.k, exact)) {
         const size_t smem = exact ? tp_field_smem<true>() : tp_field_smem<false>();
         (exact ? k_taps_field<true, false> : k_taps_field<false, false>)<<<tap_grid(a), dim3(32, TP_NP + 1), smem, st>>>(
             a, states, 0, cost, nullptr);
@@ -2137,23 +2138,42 @@ cudaError_t pm_prepare_kernels() {
 
 /* Where the tap-parallel kernels stop paying: they fill the GPU on small
  * images, at more work and more L1 traffic per tap than a thread per pixel, and
- * (for candidates 1-8 and 10-15) than shared plane windows.  Per depthMap of 3
- * iterations (FAST; EXACT), ms:
- *   all candidates tap-parallel against shared windows: 96x72 7.1, 8.2 (8.0,
- *   8.9); 100x80 8.1, 8.5; 100x90 8.8, 8.7 (10.1, 9.6); 112x98 10.0, 9.3 (11.5,
- *   10.2); 124x100 10.6, 9.7 (12.2, 10.6);
- *   the others tap-parallel against a thread per pixel, with shared windows:
- *   160x120 11.8, 15.2 (13.6, 17.9); 200x150 15.1, 16.1 (16.1, 18.7); 240x180
- *   18.8, 18.2 (20.6, 21.3); 280x210 24.7, 22.3 (28.5, 26.8).
- * A cost field: 160x120 0.162 against 0.454 (0.198, 0.427); 321x243 0.544
- * against 0.525 (0.704, 0.596). */
-#define TP_MAX_PIXELS 8500
-#define TS_MAX_PIXELS 40000
-#define TF_MAX_PIXELS 60000
-int pm_tap_parallel_pixels() { return TP_MAX_PIXELS; }
-bool pm_tap_parallel(const PmCostConsts& k) { return (size_t)k.W * k.H <= TP_MAX_PIXELS; }
-bool pm_tap_sweeps(const PmCostConsts& k) { return (size_t)k.W * k.H <= TS_MAX_PIXELS; }
-bool pm_tap_field(const PmCostConsts& k) { return (size_t)k.W * k.H <= TF_MAX_PIXELS; }
+ * (for candidates 1-8 and 10-15) than shared plane windows.
+ *
+ * What they take grows with their blocks (32 pixels of a row, however few a
+ * narrow image has there) times the taps of a block's window and a fixed cost
+ * of some `fixed` taps; what a thread per pixel takes is the chain of its own
+ * window's taps, of which a narrow image has fewer than a block of it.  So they
+ * are taken while blocks * (block's taps + fixed) <= most * (pixel's taps).
+ * Tap-parallel and a thread per pixel at 35x35 windows (11x11; 3x3), ms:
+ *   cost field, FAST: 160x120 0.166, 0.501 (0.057, 0.087; equal); 240x160 0.289,
+ *   0.479 (0.077, 0.093; 0.053, 0.047); 310x200 0.445, 0.523 (0.103, 0.096);
+ *   321x243 equal (0.112, 0.102; 0.067, 0.047); 8x4500 0.431, 0.158; 1x8000
+ *   0.177, 0.079.  EXACT: 240x160 0.341, 0.466 (0.078, 0.073; 0.043, 0.034);
+ *   310x200 0.537, 0.547; 280x280 0.661, 0.619.
+ *   adjoint with images: 240x160 0.978, 1.126 (0.212, 0.191; 0.123, 0.085);
+ *   240x250 1.53, 1.47 (0.283, 0.219).
+ *   candidates 9, 16-20, the refinements and the initial planes beside shared
+ *   windows, depthMap of 2 iterations, FAST (EXACT): 160x120 5.67, 8.29 (6.31,
+ *   9.54), 11x11 1.20, 1.40 (1.34, 1.60), 7x7 0.86, 0.90; 240x160 9.77, 10.16
+ *   (10.7, 12.4), 11x11 2.05, 1.86 (2.28, 2.11); 321x243 19.3, 16.9; 24x1500
+ *   11.1, 10.1.
+ * All candidates tap-parallel against shared windows with the others so (3x3: a
+ * thread per pixel): 96x72 (216 blocks) 3.29, 3.81 (EXACT 3.73, 4.35), 11x11
+ * 0.72, 0.89, 3x3 0.43, 0.52; 100x90 (360) 4.25, 4.13 (5.11, 4.73), 11x11 0.92,
+ * 1.01, 3x3 equal; 160x120 8.26, 5.67. */
+static long long row_blocks(const PmCostConsts& k) { return (long long)((k.W + 31) / 32) * k.H; }
+static bool taps_pay(const PmCostConsts& k, int most, int fixed) {
+    const long long rows = std::min(2 * k.P + 1, k.H);
+    const long long own = std::min(2 * k.P + 1, k.W) * rows, block = std::min(2 * k.P + 1, 2 * k.W - 1) * rows;
+    return row_blocks(k) * (block + fixed) <= most * own;
+}
+#define TP_MAX_BLOCKS 320
+int pm_tap_parallel_pixels() { return 32 * TP_MAX_BLOCKS; }
+bool pm_tap_parallel(const PmCostConsts& k) { return row_blocks(k) <= TP_MAX_BLOCKS; }
+bool pm_tap_sweeps(const PmCostConsts& k) { return taps_pay(k, 1500, 70); }
+bool pm_tap_field(const PmCostConsts& k, bool exact) { return taps_pay(k, exact ? 2200 : 2700, 100); }
+bool pm_tap_adjoint(const PmCostConsts& k, bool images) { return images ? taps_pay(k, 2000, 200) : pm_tap_field(k, false); }
 
 cudaError_t pm_launch_pd_block(float4* uout, float* pout, const float4* uin, const float* pin, int pzero,
                                const float4* f, const float* wgt, const float* mask, float lambda, int nsteps, int W,

@@ -113,7 +113,7 @@ cudaError_t pm_launch_records(const float4* col, const float4* grad, int W, int 
                               float4* C, float2* D, cudaStream_t st);
 cudaError_t pm_launch_init(const PmPassArgs& a, bool exact, cudaStream_t st);
 /* The FAST cost and weight sum of a plane field (a, b, c) of an image that
- * pm_tap_field takes, at the adjoint's positions and with its bits. */
+ * pm_tap_adjoint takes, at the adjoint's positions and with its bits. */
 cudaError_t pm_launch_plane_sums(const PmPassArgs& a, const float4* planes, int lr, float* cost, float* ws, cudaStream_t st);
 cudaError_t pm_launch_cost_field(const PmPassArgs& a, bool exact, const float4* states, float* cost,
                                  cudaStream_t st);
@@ -147,8 +147,9 @@ cudaError_t pm_prepare_kernels();
 bool pm_tap_parallel(const PmCostConsts& k);
 int pm_tap_parallel_pixels();                        /* the most pixels of such an image */
 bool pm_tap_sweeps(const PmCostConsts& k);
-/* Whether a cost field does. */
-bool pm_tap_field(const PmCostConsts& k);
+/* Whether a cost field does; the adjoint, with or without image gradients. */
+bool pm_tap_field(const PmCostConsts& k, bool exact);
+bool pm_tap_adjoint(const PmCostConsts& k, bool images);
 
 int pm_pd_block_steps();
 /* Bytes of a dual buffer of pm_launch_pd_block: six planes of floats. */

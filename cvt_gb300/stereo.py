@@ -332,8 +332,8 @@ class PMHuberStereo:
 
     def set_memory_budget(self, nbytes: int) -> None:
         """Device bytes a propagation pass may use to share work between its
-        candidates: 32 per pixel, 576 for images of at most 8500 pixels (0:
-        every candidate per pixel; results are the same)."""
+        candidates: 32 per pixel, 576 for images of at most 320 blocks of 32
+        pixels of a row (0: every candidate per pixel; results are the same)."""
         self._check(_lib.lib().cvtpm_set_memory_budget(self._h, int(nbytes)))
 
     def cost_adjoint(self, img1: torch.Tensor, img2: torch.Tensor, planes: torch.Tensor, lr: int = 1,

@@ -271,8 +271,8 @@ cvtpm_status cvtpm_polish_planes(cvtpm_ctx* ctx, const float* img1, const float*
 /* Device memory the context may use to share work between the candidates of
  * a propagation pass (FAST and EXACT).  With 32 bytes per pixel (24: one view at a time), planes that
  * several pixels test (the neighbour and random-neighbour candidates) have
- * their matching terms formed once per plane; images of at most 8500 pixels
- * use 576 (320) instead, to run every candidate's window taps in
+ * their matching terms formed once per plane; images of at most 320
+ * blocks of 32 pixels of a row use 576 (320) instead, to run every candidate's window taps in
  * parallel.  Otherwise (and beyond 60 % of the free memory) every candidate is
  * evaluated per pixel.  Results are identical either way.  The context keeps
  * the memory, replaces it for an image of more pixels than any before, as its

@@ -1,7 +1,8 @@
 /*
  * cvtpm_tools.h — measurement helpers exported by libcvtpm.so beside the
  * drop-in ABI of cvtpm.h.  They have no counterpart in the reference: they
- * supply denominators for roofline reporting.
+ * supply denominators for roofline reporting and show what tests cannot see
+ * from results.
  */
 #ifndef CVTPM_TOOLS_H
 #define CVTPM_TOOLS_H
@@ -22,6 +23,15 @@ cvtpm_status cvtpm_tool_fp32_peak(int device, void* stream, float* tflops);
  * best of two timed runs after a warm-up).  depthMap runs the two views'
  * smoothers concurrently, so its per-phase timings cannot give this. */
 cvtpm_status cvtpm_tool_pd_time(cvtpm_ctx* ctx, int steps, void* stream, float* us_per_step);
+
+/* The routes that calls of these parameters (patchsize, arith) take for an image
+ * size; -1 for a bad argument.  No device is needed.  Routes never change
+ * results. */
+#define CVTPM_ROUTE_TAPS 1          /* every candidate of a pass tap-parallel */
+#define CVTPM_ROUTE_TAP_SWEEPS 2    /* the candidates outside shared windows */
+#define CVTPM_ROUTE_TAP_COST 4      /* cvtpm_cost_eval */
+#define CVTPM_ROUTE_TAP_ADJOINT 8   /* cvtpm_cost_adjoint with image gradients */
+int cvtpm_tool_routes(const cvtpm_params* params, int width, int height);
 
 #ifdef __cplusplus
 }
