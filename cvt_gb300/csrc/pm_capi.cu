@@ -358,7 +358,7 @@ cvtpm_status plan_pass(cvtpm_ctx* ctx, const cvtpm_params& p, int W, int H, bool
     const bool grow = !ctx->no_alloc && cap == cudaStreamCaptureStatusNone && (!ctx->pass || n > ctx->pass_pixels);
     const size_t small = taps ? std::min(n, (size_t)pm_tap_parallel_pixels()) * sizeof(float4) * 36 : 0;
     taps = taps && pm_tap_parallel(k);
-    for (int plan = taps ? 0 : 2; plan < 4; ++plan) {
+    for (int plan = taps ? 0 : 2; plan < (pm_shared_windows(k) ? 4 : 2); ++plan) {
         const bool both = (plan & 1) == 0, t = plan < 2;
         const size_t need = t ? n * sizeof(float4) * (both ? 36 : 20) : n * sizeof(float) * (both ? 8 : 6);
         if (need > ctx->pass_budget) continue;
@@ -1947,6 +1947,7 @@ int cvtpm_tool_routes(const cvtpm_params* params, int width, int height) {
     memset(&k, 0, sizeof(k));
     k.W = width; k.H = height; k.P = params->patchsize;
     return (pm_tap_parallel(k) ? CVTPM_ROUTE_TAPS : 0) | (pm_tap_sweeps(k) ? CVTPM_ROUTE_TAP_SWEEPS : 0) |
+           (pm_shared_windows(k) ? CVTPM_ROUTE_WINDOWS : 0) |
            (pm_tap_field(k, params->arith == CVTPM_ARITH_EXACT) ? CVTPM_ROUTE_TAP_COST : 0) |
            (pm_tap_adjoint(k, true) ? CVTPM_ROUTE_TAP_ADJOINT : 0);
 }

@@ -2172,6 +2172,13 @@ static bool taps_pay(const PmCostConsts& k, int most, int fixed) {
 int pm_tap_parallel_pixels() { return 32 * TP_MAX_BLOCKS; }
 bool pm_tap_parallel(const PmCostConsts& k) { return row_blocks(k) <= TP_MAX_BLOCKS; }
 bool pm_tap_sweeps(const PmCostConsts& k) { return taps_pay(k, 1500, 70); }
+/* Shared plane windows form and fold all 2P + 1 columns of a window whatever
+ * the image holds of them, and a step of four columns ends with a barrier.
+ * depthMap of 2 iterations, windows against every candidate per pixel, ms:
+ * 35x35 16x3000 12.0, 12.7, 8x4500 12.3, 9.3, 1x8000 14.4, 3.0; 19x19 8x4500
+ * 6.0, 5.5; 11x11 8x4500 3.6, 3.8; 640x480 7x7 5.4, 6.3 (EXACT 6.0, 6.3), 5x5
+ * 4.3, 4.1 (4.9, 4.1), 3x3 2.9, 2.5 (3.3, 2.5). */
+bool pm_shared_windows(const PmCostConsts& k) { return k.P >= 3 && 9 * std::min(2 * k.P + 1, k.W) >= 4 * (2 * k.P + 1); }
 bool pm_tap_field(const PmCostConsts& k, bool exact) { return taps_pay(k, exact ? 2200 : 2700, 100); }
 bool pm_tap_adjoint(const PmCostConsts& k, bool images) { return images ? taps_pay(k, 2000, 200) : pm_tap_field(k, false); }
 

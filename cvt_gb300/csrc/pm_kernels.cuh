@@ -147,6 +147,8 @@ cudaError_t pm_prepare_kernels();
 bool pm_tap_parallel(const PmCostConsts& k);
 int pm_tap_parallel_pixels();                        /* the most pixels of such an image */
 bool pm_tap_sweeps(const PmCostConsts& k);
+/* Whether passes share plane windows, given PmPassArgs::costs and vcosts. */
+bool pm_shared_windows(const PmCostConsts& k);
 /* Whether a cost field does; the adjoint, with or without image gradients. */
 bool pm_tap_field(const PmCostConsts& k, bool exact);
 bool pm_tap_adjoint(const PmCostConsts& k, bool images);

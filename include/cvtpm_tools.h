@@ -29,6 +29,7 @@ cvtpm_status cvtpm_tool_pd_time(cvtpm_ctx* ctx, int steps, void* stream, float* 
  * results. */
 #define CVTPM_ROUTE_TAPS 1          /* every candidate of a pass tap-parallel */
 #define CVTPM_ROUTE_TAP_SWEEPS 2    /* the candidates outside shared windows */
+#define CVTPM_ROUTE_WINDOWS 16      /* larger images' passes share plane windows */
 #define CVTPM_ROUTE_TAP_COST 4      /* cvtpm_cost_eval */
 #define CVTPM_ROUTE_TAP_ADJOINT 8   /* cvtpm_cost_adjoint with image gradients */
 int cvtpm_tool_routes(const cvtpm_params* params, int width, int height);
