@@ -72,42 +72,64 @@ struct PmAdjArgs {
 };
 
 /* The window sums of a plane at its Q31.32 position (S0, S1, XC at the pixel):
- * the operations of the FAST evaluator in raster order, two taps' weights at a
- * time. */
+ * the operations of the FAST evaluator in raster order, on packed pairs or
+ * (SCALAR) one by one, which are the same operations.  Packed, the kernel
+ * without image terms takes 3.06 ms at 640x480 and scalar 3.19, but the one with
+ * them 5.59 and 5.46; and rows of few taps pay for the addresses of the four
+ * record rows (the cost alone of 16x5000 0.54 and 0.38 ms). */
+template <bool SCALAR>
 __device__ __forceinline__ void cost_sums(const PmCostConsts& k, const PmView& v1, const PmView& v2, int x, int y, float4 vc,
                                           long long S0, long long S1, long long XC, float& ws, float& r1, float& r2) {
-    const int dxlo = max(-k.P, -x), dxhi = min(k.P, k.W - 1 - x);
-    const int qy0 = max(y - k.P, 0), qy1 = min(y + k.P, k.H - 1);
+    const int W = k.W, dxlo = max(-k.P, -x), dxhi = min(k.P, W - 1 - x);
     ws = r1 = r2 = 0.0f;
+    if (SCALAR) {
+        for (int dy = -k.P; dy <= k.P; ++dy) {
+            const int qy = y + dy;
+            if (qy < 0 || qy >= k.H) continue;
+            const float* prow = c_prof + (dy + PM_PMAX) * PM_PROF_N + PM_PMAX;
+            long long X = XC + (long long)dy * S1 + (long long)dxlo * S0;
+            for (int dx = dxlo; dx <= dxhi; ++dx) {
+                const long long Xt = X;
+                X += S0;
+                const int xi = (int)(Xt >> 32);
+                if ((unsigned)xi >= (unsigned)W) continue;
+                const size_t q = (size_t)qy * W + x + dx;
+                const float4 a1 = __ldg(&v1.col[q]);
+                const float4 g1 = __ldg(&v1.grad[q]);
+                const float w1 = tap_weight(vc, a1, prow[dx]);
+                TapVals t;
+                load_tap(v2, (size_t)qy * k.rp + xi, pm_fix_frac(Xt), t);
+                const float cc = (fminf(fabsf(a1.x - t.v[0]), k.cmax) + fminf(fabsf(a1.y - t.v[1]), k.cmax)) +
+                                 fminf(fabsf(a1.z - t.v[2]), k.cmax);
+                const float gc = ((fminf(fabsf(g1.x - t.v[3]), k.gmax) + fminf(fabsf(g1.y - t.v[4]), k.gmax)) +
+                                  fminf(fabsf(g1.z - t.v[5]), k.gmax)) + fminf(fabsf(g1.w - t.v[6]), k.gmax);
+                r1 = fmaf(w1, cc, r1);
+                r2 = fmaf(w1, gc, r2);
+                ws = ws + w1;
+            }
+        }
+        return;
+    }
+    const int qy0 = max(y - k.P, 0), qy1 = min(y + k.P, k.H - 1);
     for (int qy = qy0; qy <= qy1; ++qy) {
-        const float4* c1row = v1.col + (size_t)qy * k.W + x;
-        const float4* g1row = v1.grad + (size_t)qy * k.W + x;
+        const float4* c1row = v1.col + (size_t)qy * W + x;
+        const float4* g1row = v1.grad + (size_t)qy * W + x;
         const float* prow = c_prof + (qy - y + PM_PMAX) * PM_PROF_N + PM_PMAX;
         const PmRecRow rrow = rec_row(v2, k.rp, qy);
         long long X = XC + (long long)(qy - y) * S1 + (long long)dxlo * S0;
-        auto one = [&](float4 a1, float4 g1, float w1) {
+        for (int dx = dxlo; dx <= dxhi; ++dx) {
+            const float4 a1 = __ldg(&c1row[dx]);
+            const float4 g1 = __ldg(&g1row[dx]);
+            const float w1 = tap_weight(vc, a1, prow[dx]);
             const long long Xt = X;
             X += S0;
             const int xi = (int)(Xt >> 32);
-            if ((unsigned)xi >= (unsigned)k.W) return;
+            if ((unsigned)xi >= (unsigned)W) continue;
             float cc, gc;
             fast_tap_terms(k, rrow, xi, pm_fix_frac(Xt), a1, g1, cc, gc);
             r1 = fmaf(w1, cc, r1);
             r2 = fmaf(w1, gc, r2);
             ws = ws + w1;
-        };
-        int dx = dxlo;
-        for (; dx < dxhi; dx += 2) {
-            const float4 a1 = __ldg(&c1row[dx]), a1b = __ldg(&c1row[dx + 1]);
-            const float4 g1 = __ldg(&g1row[dx]), g1b = __ldg(&g1row[dx + 1]);
-            float w1, w1b;
-            tap_weight2(vc, a1, a1b, prow[dx], prow[dx + 1], w1, w1b);
-            one(a1, g1, w1);
-            one(a1b, g1b, w1b);
-        }
-        if (dx == dxhi) {
-            const float4 a1 = __ldg(&c1row[dx]);
-            one(a1, __ldg(&g1row[dx]), tap_weight(vc, a1, prow[dx]));
         }
     }
 }
@@ -147,6 +169,24 @@ __device__ __forceinline__ float wsgn(float w, float e, float cap) {
     return fabsf(e) < cap && e != 0.0f ? s : 0.0f;
 }
 
+/* The cost alone: without the registers of the gradients, and in blocks of 4
+ * rows, which spread small images over the SMs better than 8 (321x243 0.55 ->
+ * 0.49 ms, 63x63 window 1.72 -> 1.42, 500x400 1.20 -> 1.15). */
+#define PC_ROWS 4                                    /* warps per block */
+template <bool NARROW>
+__global__ void __launch_bounds__(32 * PC_ROWS) k_plane_cost(PmAdjArgs a) {
+    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * PC_ROWS + threadIdx.y;
+    if (x >= a.k.W || y >= a.k.H) return;
+    const size_t o = (size_t)y * a.k.W + x;
+    const float4 pl = a.planes[o];
+    const float ds = a.lr ? -1.0f : 1.0f;
+    long long S0, S1, XC;
+    const bool live = fix_plane_d(1.0 + (double)ds * pl.x, (double)ds * pl.y, (double)ds * pl.z, x, y, S0, S1, XC);
+    float ws, r1, r2;
+    cost_sums<NARROW>(a.k, a.v1, a.v2, x, y, __ldg(&a.v1.col[o]), S0, S1, XC, ws, r1, r2);
+    a.cost[o] = live && ws > 1.1f ? fmaf(a.k.alpha, r1, a.k.oma * r2) / ws : 1e5f;
+}
+
 /* What bounds the gradient sweep is the atomics on the image accumulators: a
  * tap has terms at one pixel of image 1 and two of image 2, seven floats each,
  * six 128-bit additions.  Two things take most of them away.  The lanes of a
@@ -159,11 +199,16 @@ __device__ __forceinline__ float wsgn(float w, float e, float cap) {
  * 640x480, 35x35 window (ncu): 8.36 -> 5.27 ms; what bounds it now is
  * instruction issue (334 per tap over both sweeps, issue 63 %).
  *
- * ROWS: images too small to fill the GPU (pm_tap_field) get their costs and
+ * NARROW: where a row is shorter than a warp few lanes share an image-1 pixel,
+ * and each adds its terms per tap (35x35 window: 31x4000 2.38 -> 2.15 ms, 16x5000
+ * 2.06 -> 1.33, 4x20000 0.80 -> 0.41; 40x1500 2.21 that way, 1.75 along the lanes).
+ *
+ * ROWS: images too small to fill the GPU (pm_tap_adjoint) get their costs and
  * weight sums tap-parallel beforehand, and the 8 warps of a block share the
  * window rows of one row of 32 pixels. */
-template <bool IMG, bool ROWS>
+template <bool IMG, bool NARROW, bool ROWS>
 __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
+    constexpr bool LANES = IMG && !NARROW;
     const int W = a.k.W, H = a.k.H, P = a.k.P, lane = threadIdx.x;
     const int x0 = blockIdx.x * 32, xr = x0 + lane, y = ROWS ? blockIdx.y : blockIdx.y * 8 + threadIdx.y;
     if (y >= H) return;                                  /* warp-uniform; no row past the last with ROWS */
@@ -185,11 +230,10 @@ __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
         valid = live && ws > 1.1f;
     } else {
         float r1, r2;
-        cost_sums(a.k, a.v1, a.v2, x, y, vc, S0, S1, XC, ws, r1, r2);
+        cost_sums<IMG || NARROW>(a.k, a.v1, a.v2, x, y, vc, S0, S1, XC, ws, r1, r2);
         valid = live && ws > 1.1f;
         C = valid ? fmaf(a.k.alpha, r1, a.k.oma * r2) / ws : 1e5f;
         if (a.cost && inside) a.cost[o] = C;
-        if (!a.dcost) return;
     }
 
     /* sweep 2: gradients */
@@ -201,7 +245,8 @@ __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
         const float u = act ? g / ws : 0.0f;
         const float al = a.k.alpha, oma = a.k.oma;
         const int qy0 = max(y - P, 0), qy1 = min(y + P, H - 1);
-        const int dlo = max(-P, -(x0 + 31)), dhi = min(P, W - 1 - x0);   /* inside the image for some lane */
+        /* inside the image for some lane, which the shuffles and uniform reads of the profile want, or for this one */
+        const int dlo = max(-P, NARROW ? -x : -min(x0 + 31, W - 1)), dhi = min(P, W - 1 - (NARROW ? x : x0));
         for (int qy = qy0 + (ROWS ? (int)threadIdx.y : 0); qy <= qy1; qy += ROWS ? 8 : 1) {
             const float* prow = c_prof + (qy - y + PM_PMAX) * PM_PROF_N + PM_PMAX;
             const size_t rb = (size_t)qy * W;
@@ -213,7 +258,7 @@ __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
             for (int dx = dlo; dx <= dhi; ++dx) {
                 const long long Xt = X;
                 X += S0;
-                if (IMG && dx > dlo) {                   /* column x0 + dx - 1 is complete: lane 0 had it last */
+                if (LANES && dx > dlo) {                 /* column x0 + dx - 1 is complete: lane 0 had it last */
                     const int qc = x0 + dx - 1;
                     if (lane == 0 && qc >= 0) add_image(a.dI1, a.dG1, rb + qc, m);
                     m.shift_down(lane);
@@ -260,9 +305,11 @@ __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
                     centre[0] += dr;
                     centre[1] += dg;
                     centre[2] += db;
+                    if (NARROW) m = {};
                     m.add(gct, s0, s1, s2, s3);
                     m.v0 = fsub2(m.v0, make_float2(dr, dg));
                     m.v1.x -= db;
+                    if (NARROW) add_image(a.dI1, a.dG1, q, m);
                     if (xi != col) {
                         const bool next = xi == col + 1;
                         if (col >= 0) {
@@ -280,7 +327,7 @@ __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
             }
             if (IMG) {                                   /* the row's last columns */
                 const int qc = xr + dhi;
-                if (qc >= 0 && qc < W) add_image(a.dI1, a.dG1, rb + qc, m);
+                if (LANES && qc >= 0 && qc < W) add_image(a.dI1, a.dG1, rb + qc, m);
                 if (col >= 0) {
                     add_image(a.dI2, a.dG2, rb + col, lo);
                     add_image(a.dI2, a.dG2, rb + min(col + 1, W - 1), hi);
@@ -350,8 +397,18 @@ cudaError_t pm_launch_cost_adjoint(const PmCostConsts& k, const PmView& v1, cons
     a.k = k; a.v1 = v1; a.v2 = v2; a.planes = planes; a.lr = lr; a.dcost = dcost; a.cost = cost;
     a.dplanes = dplanes; a.dI1 = dI1; a.dG1 = dG1; a.dI2 = dI2; a.dG2 = dG2;
     const dim3 grid((k.W + 31) / 32, sums ? k.H : (k.H + 7) / 8), block(32, 8);
-    if (sums) (dI1 ? k_cost_adjoint<true, true> : k_cost_adjoint<false, true>)<<<grid, block, 0, st>>>(a);
-    else (dI1 ? k_cost_adjoint<true, false> : k_cost_adjoint<false, false>)<<<grid, block, 0, st>>>(a);
+    const bool narrow = k.W < 32;
+    auto launch = [&](auto kern) { kern<<<grid, block, 0, st>>>(a); };
+    if (!dcost) {
+        const dim3 g((k.W + 31) / 32, (k.H + PC_ROWS - 1) / PC_ROWS);
+        if (cost) (narrow ? k_plane_cost<true> : k_plane_cost<false>)<<<g, dim3(32, PC_ROWS), 0, st>>>(a);
+    } else if (sums) {
+        if (dI1) launch(narrow ? k_cost_adjoint<true, true, true> : k_cost_adjoint<true, false, true>);
+        else launch(narrow ? k_cost_adjoint<false, true, true> : k_cost_adjoint<false, false, true>);
+    } else {
+        if (dI1) launch(narrow ? k_cost_adjoint<true, true, false> : k_cost_adjoint<true, false, false>);
+        else launch(narrow ? k_cost_adjoint<false, true, false> : k_cost_adjoint<false, false, false>);
+    }
     return cudaGetLastError();
 }
 

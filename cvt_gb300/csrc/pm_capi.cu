@@ -1124,7 +1124,7 @@ cvtpm_status cvtpm_cost_adjoint(cvtpm_ctx* ctx, const float* img1, const float* 
         for (float4* b : {dI1, dG1, dI2, dG2}) CK(cudaMemsetAsync(b, 0, n * 16, st), "adjoint clear");
     }
     float* sums = nullptr;
-    if (pm_tap_adjoint(a.k, img)) {                       /* small images: costs and weight sums first, into free scratch */
+    if (pm_tap_adjoint(a.k, dcost != nullptr, img)) {    /* small images: costs and weight sums first, into free scratch */
         sums = (float*)ctx->smooth[0];
         if (!cost) cost = (float*)ctx->smooth[1];
         LK(pm_launch_plane_sums(a, (const float4*)planes, lr, cost, sums, st), "plane sums");
@@ -1949,7 +1949,7 @@ int cvtpm_tool_routes(const cvtpm_params* params, int width, int height) {
     return (pm_tap_parallel(k) ? CVTPM_ROUTE_TAPS : 0) | (pm_tap_sweeps(k) ? CVTPM_ROUTE_TAP_SWEEPS : 0) |
            (pm_shared_windows(k) ? CVTPM_ROUTE_WINDOWS : 0) |
            (pm_tap_field(k, params->arith == CVTPM_ARITH_EXACT) ? CVTPM_ROUTE_TAP_COST : 0) |
-           (pm_tap_adjoint(k, true) ? CVTPM_ROUTE_TAP_ADJOINT : 0);
+           (pm_tap_adjoint(k, true, true) ? CVTPM_ROUTE_TAP_ADJOINT : 0);
 }
 
 cvtpm_status cvtpm_tool_pd_time(cvtpm_ctx* ctx, int steps, void* stream, float* us_per_step) {

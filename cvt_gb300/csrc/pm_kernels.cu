@@ -2152,7 +2152,9 @@ cudaError_t pm_prepare_kernels() {
  *   0.177, 0.079.  EXACT: 240x160 0.341, 0.466 (0.078, 0.073; 0.043, 0.034);
  *   310x200 0.537, 0.547; 280x280 0.661, 0.619.
  *   adjoint with images: 240x160 0.978, 1.126 (0.212, 0.191; 0.123, 0.085);
- *   240x250 1.53, 1.47 (0.283, 0.219).
+ *   240x250 1.53, 1.47 (0.283, 0.219); with planes alone 240x250 0.78, 0.92
+ *   (0.155, 0.137), 450x200 1.11, 1.23, 31x4000 equal; the cost alone 240x250
+ *   equal, 321x243 0.55, 0.49.
  *   candidates 9, 16-20, the refinements and the initial planes beside shared
  *   windows, depthMap of 2 iterations, FAST (EXACT): 160x120 5.67, 8.29 (6.31,
  *   9.54), 11x11 1.20, 1.40 (1.34, 1.60), 7x7 0.86, 0.90; 240x160 9.77, 10.16
@@ -2180,7 +2182,9 @@ bool pm_tap_sweeps(const PmCostConsts& k) { return taps_pay(k, 1500, 70); }
  * 4.3, 4.1 (4.9, 4.1), 3x3 2.9, 2.5 (3.3, 2.5). */
 bool pm_shared_windows(const PmCostConsts& k) { return k.P >= 3 && 9 * std::min(2 * k.P + 1, k.W) >= 4 * (2 * k.P + 1); }
 bool pm_tap_field(const PmCostConsts& k, bool exact) { return taps_pay(k, exact ? 2200 : 2700, 100); }
-bool pm_tap_adjoint(const PmCostConsts& k, bool images) { return images ? taps_pay(k, 2000, 200) : pm_tap_field(k, false); }
+bool pm_tap_adjoint(const PmCostConsts& k, bool planes, bool images) {
+    return images ? taps_pay(k, 2000, 200) : planes ? taps_pay(k, 3800, 240) : taps_pay(k, 2200, 100);
+}
 
 cudaError_t pm_launch_pd_block(float4* uout, float* pout, const float4* uin, const float* pin, int pzero,
                                const float4* f, const float* wgt, const float* mask, float lambda, int nsteps, int W,

@@ -149,9 +149,10 @@ int pm_tap_parallel_pixels();                        /* the most pixels of such 
 bool pm_tap_sweeps(const PmCostConsts& k);
 /* Whether passes share plane windows, given PmPassArgs::costs and vcosts. */
 bool pm_shared_windows(const PmCostConsts& k);
-/* Whether a cost field does; the adjoint, with or without image gradients. */
+/* Whether a cost field does; the adjoint, with plane or image gradients
+ * or neither. */
 bool pm_tap_field(const PmCostConsts& k, bool exact);
-bool pm_tap_adjoint(const PmCostConsts& k, bool images);
+bool pm_tap_adjoint(const PmCostConsts& k, bool planes, bool images);
 
 int pm_pd_block_steps();
 /* Bytes of a dual buffer of pm_launch_pd_block: six planes of floats. */
