@@ -392,18 +392,20 @@ PM_DEV void tap_weight_centres(float4 va, float4 vb, float4 a1, float pa, float 
 #ifndef PM_PAIR_TAPS_EXACT
 #define PM_PAIR_TAPS_EXACT 0
 #endif
-template <int K, bool EXACT>
+template <int K, bool EXACT, bool NEXT = !EXACT && K <= 2>
 PM_DEV void eval_costs(const PmCostConsts& k, const PmView& v1, const PmView& v2, int x, int y,
                        const float4 (&s)[K], const bool (&act)[K], float (&cost)[K]) {
-    /* FAST, up to two candidates: a plane's slope is near 1, so the next tap
+    /* NEXT (FAST, up to two candidates): a plane's slope is near 1, so the next tap
      * mostly lies between the columns xi + 1 and xi + 2.  The values at xi + 1
      * are kept and each tap loads those of one more column, in place of a
      * record's values and differences (8 L1 wavefronts a warp for 14), and forms
      * the record's differences itself; a lane that did not advance by one loads
      * its own column again.  1242x375, per launch (ncu): k_sweep 4.73 -> 4.31 ms,
      * k_init 3.2 -> 2.5, the first refinements 5.4 -> 4.8; depthMap 327 -> 319
-     * ms.  More candidates would spill the 8 registers each. */
-    constexpr bool NEXT = !EXACT && K <= 2;
+     * ms.  More candidates would spill the 8 registers each; a field of fixed
+     * planes, one launch for one plane a pixel, is faster from the records
+     * (640x480 1.36 ms, 1.65 so). */
+    static_assert(!NEXT || !EXACT, "EXACT reads no records");
     float sx[K], sy[K], sz[K];
     /* FAST: X is the candidate's Q31.32 position at the current tap, S0 its
      * step along a row and D the step from a row's end to the next row's

@@ -125,14 +125,27 @@ PM_DEV void init_tile(const PmPassArgs& a, int tbx, int tby) {
 template <bool EXACT>
 __global__ void __launch_bounds__(256) k_init(PmPassArgs a) { init_tile<EXACT>(a, blockIdx.x, blockIdx.y); }
 
-/* The cost of a state field.  FAST: two pixels of a column per thread, whose
- * windows share 36 of 37 image-1 rows (the L1 data pipe bounds this sweep:
- * 85 % busy with one pixel per thread; 640x480 1.50 -> 1.35 ms, 1242x375 2.28
- * -> 2.08).  EXACT, whose arithmetic outweighs those reads, gains nothing by it
- * (1.62 against 1.67 ms) and takes one. */
+/* The cost of a state field, a pixel per thread. */
+template <bool EXACT>
+__global__ void __launch_bounds__(256) k_cost_field(PmPassArgs a, const float4* __restrict__ states,
+                                                    float* __restrict__ cost) {
+    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
+    if (x >= a.k.W || y >= a.k.H) return;
+    float4 s[1] = {states[(size_t)y * a.k.W + x]};
+    bool act[1] = {true};
+    float c[1];
+    eval_costs<1, EXACT, false>(a.k, a.v1, a.v2, x, y, s, act, c);
+    cost[(size_t)y * a.k.W + x] = c[0];
+}
+
+/* FAST, large fields (cost_field_pairs): two pixels of a column per thread,
+ * whose windows share all but one image-1 row (the L1 data pipe bounds this
+ * sweep: 85 % busy with one pixel per thread; 640x480 1.36 -> 1.23 ms, 1242x375
+ * 1.92 -> 1.76, 1920x1080 8.2 -> 7.4).  EXACT, whose arithmetic outweighs those
+ * reads, gains nothing by it (1.62 against 1.67 ms). */
 #define CF_ROWS 2                                    /* warps per block */
-__global__ void __launch_bounds__(32 * CF_ROWS, 8) k_cost_field_fast(PmPassArgs a, const float4* __restrict__ states,
-                                                                    float* __restrict__ cost) {
+__global__ void __launch_bounds__(32 * CF_ROWS, 8) k_cost_field_pairs(PmPassArgs a, const float4* __restrict__ states,
+                                                                     float* __restrict__ cost) {
     const int x = blockIdx.x * 32 + threadIdx.x, y = 2 * (blockIdx.y * CF_ROWS + threadIdx.y);
     if (x >= a.k.W || y >= a.k.H) return;
     const bool two = y + 1 < a.k.H;
@@ -142,17 +155,6 @@ __global__ void __launch_bounds__(32 * CF_ROWS, 8) k_cost_field_fast(PmPassArgs 
     eval_column(a.k, a.v1, a.v2, x, y, two, s, c);
     cost[o] = c[0];
     if (two) cost[o + a.k.W] = c[1];
-}
-
-__global__ void __launch_bounds__(256) k_cost_field_exact(PmPassArgs a, const float4* __restrict__ states,
-                                                          float* __restrict__ cost) {
-    const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y;
-    if (x >= a.k.W || y >= a.k.H) return;
-    float4 s[1] = {states[(size_t)y * a.k.W + x]};
-    bool act[1] = {true};
-    float c[1];
-    eval_costs<1, true>(a.k, a.v1, a.v2, x, y, s, act, c);
-    cost[(size_t)y * a.k.W + x] = c[0];
 }
 
 /* Adds a warp's evaluations and in-image window taps (`ev` evaluations at an
@@ -1975,6 +1977,9 @@ cudaError_t pm_launch_records(const float4* col, const float4* grad, int W, int 
     return cudaSuccess;
 }
 
+/* blocks of 32 pixels of a row */
+static long long row_blocks(const PmCostConsts& k) { return (long long)((k.W + 31) / 32) * k.H; }
+
 static inline dim3 pix_grid(int W, int H) { return dim3((W + 31) / 32, (H + 7) / 8); }
 
 static inline dim3 tap_grid(const PmPassArgs& a, int z = 1) { return dim3((a.k.W + 31) / 32, a.k.H, z); }
@@ -1992,16 +1997,24 @@ cudaError_t pm_launch_init(const PmPassArgs& a, bool exact, cudaStream_t st) {
     return cudaSuccess;
 }
 
+/* Two pixels a thread pay from about the size on that fills the SMs with half
+ * the threads, and where a window's rows are long enough to share: FAST, two
+ * and one, ms: 35x35 240x250 0.525, 0.475, 321x243 0.536, 0.553, 16x5000 0.530,
+ * 0.507; 19x19 240x250 0.186, 0.167, 321x243 equal, 500x300 0.231, 0.250; 11x11
+ * 321x243 0.101, 0.094, 640x480 0.181, 0.183, 1920x1080 0.97, 0.93; 5x5 640x480
+ * 0.083, 0.080. */
+static bool cost_field_pairs(const PmCostConsts& k) { return k.P >= 6 && k.W >= 32 && row_blocks(k) >= 2600; }
+
 cudaError_t pm_launch_cost_field(const PmPassArgs& a, bool exact, const float4* states, float* cost, cudaStream_t st) {
     const int W = a.k.W, H = a.k.H;
     if (pm_tap_field(a.k, exact)) {
         const size_t smem = exact ? tp_field_smem<true>() : tp_field_smem<false>();
         (exact ? k_taps_field<true, false> : k_taps_field<false, false>)<<<tap_grid(a), dim3(32, TP_NP + 1), smem, st>>>(
             a, states, 0, cost, nullptr);
-    } else if (exact) {
-        k_cost_field_exact<<<pix_grid(W, H), dim3(32, 8), 0, st>>>(a, states, cost);
+    } else if (!exact && cost_field_pairs(a.k)) {
+        k_cost_field_pairs<<<dim3((W + 31) / 32, (H + 2 * CF_ROWS - 1) / (2 * CF_ROWS)), dim3(32, CF_ROWS), 0, st>>>(a, states, cost);
     } else {
-        k_cost_field_fast<<<dim3((W + 31) / 32, (H + 2 * CF_ROWS - 1) / (2 * CF_ROWS)), dim3(32, CF_ROWS), 0, st>>>(a, states, cost);
+        (exact ? k_cost_field<true> : k_cost_field<false>)<<<pix_grid(W, H), dim3(32, 8), 0, st>>>(a, states, cost);
     }
     PM_LAUNCH_CHECK();
     return cudaSuccess;
@@ -2143,13 +2156,15 @@ cudaError_t pm_prepare_kernels() {
  * What they take grows with their blocks (32 pixels of a row, however few a
  * narrow image has there) times the taps of a block's window and a fixed cost
  * of some `fixed` taps; what a thread per pixel takes is the chain of its own
- * window's taps, of which a narrow image has fewer than a block of it.  So they
- * are taken while blocks * (block's taps + fixed) <= most * (pixel's taps).
+ * window's taps, of which a narrow image has fewer than a block of it, and
+ * reads faster where less than a warp wide.  So they are taken while blocks *
+ * (block's taps + fixed) <= most * (pixel's taps), these counted down to half
+ * at a width of 1.
  * Tap-parallel and a thread per pixel at 35x35 windows (11x11; 3x3), ms:
  *   cost field, FAST: 160x120 0.166, 0.501 (0.057, 0.087; equal); 240x160 0.289,
  *   0.479 (0.077, 0.093; 0.053, 0.047); 310x200 0.445, 0.523 (0.103, 0.096);
- *   321x243 equal (0.112, 0.102; 0.067, 0.047); 8x4500 0.431, 0.158; 1x8000
- *   0.177, 0.079.  EXACT: 240x160 0.341, 0.466 (0.078, 0.073; 0.043, 0.034);
+ *   321x243 equal (0.112, 0.102; 0.067, 0.047); 8x1000 0.132, 0.111; 8x4500
+ *   0.431, 0.158; 1x8000 0.177, 0.079.  EXACT: 240x160 0.341, 0.466 (0.078, 0.073; 0.043, 0.034);
  *   310x200 0.537, 0.547; 280x280 0.661, 0.619.
  *   adjoint with images: 240x160 0.978, 1.126 (0.212, 0.191; 0.123, 0.085);
  *   240x250 1.53, 1.47 (0.283, 0.219); with planes alone 240x250 0.78, 0.92
@@ -2164,11 +2179,10 @@ cudaError_t pm_prepare_kernels() {
  * thread per pixel): 96x72 (216 blocks) 3.29, 3.81 (EXACT 3.73, 4.35), 11x11
  * 0.72, 0.89, 3x3 0.43, 0.52; 100x90 (360) 4.25, 4.13 (5.11, 4.73), 11x11 0.92,
  * 1.01, 3x3 equal; 160x120 8.26, 5.67. */
-static long long row_blocks(const PmCostConsts& k) { return (long long)((k.W + 31) / 32) * k.H; }
 static bool taps_pay(const PmCostConsts& k, int most, int fixed) {
     const long long rows = std::min(2 * k.P + 1, k.H);
     const long long own = std::min(2 * k.P + 1, k.W) * rows, block = std::min(2 * k.P + 1, 2 * k.W - 1) * rows;
-    return row_blocks(k) * (block + fixed) <= most * own;
+    return row_blocks(k) * (block + fixed) * 64 <= most * own * (std::min(k.W, 32) + 32);
 }
 #define TP_MAX_BLOCKS 320
 int pm_tap_parallel_pixels() { return 32 * TP_MAX_BLOCKS; }
@@ -2181,7 +2195,7 @@ bool pm_tap_sweeps(const PmCostConsts& k) { return taps_pay(k, 1500, 70); }
  * 6.0, 5.5; 11x11 8x4500 3.6, 3.8; 640x480 7x7 5.4, 6.3 (EXACT 6.0, 6.3), 5x5
  * 4.3, 4.1 (4.9, 4.1), 3x3 2.9, 2.5 (3.3, 2.5). */
 bool pm_shared_windows(const PmCostConsts& k) { return k.P >= 3 && 9 * std::min(2 * k.P + 1, k.W) >= 4 * (2 * k.P + 1); }
-bool pm_tap_field(const PmCostConsts& k, bool exact) { return taps_pay(k, exact ? 2200 : 2700, 100); }
+bool pm_tap_field(const PmCostConsts& k, bool exact) { return taps_pay(k, exact ? 2200 : 2750, 100); }
 bool pm_tap_adjoint(const PmCostConsts& k, bool planes, bool images) {
     return images ? taps_pay(k, 2000, 200) : planes ? taps_pay(k, 3800, 240) : taps_pay(k, 2200, 100);
 }

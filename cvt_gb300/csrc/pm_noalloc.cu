@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(256) k_cost_field_noalloc(PmPassArgs a, const 
     float4 s[1] = {states[(size_t)y * a.k.W + x]};
     bool act[1] = {true};
     float c[1];
-    eval_costs<1, EXACT>(a.k, a.v1, a.v2, x, y, s, act, c);
+    eval_costs<1, EXACT, false>(a.k, a.v1, a.v2, x, y, s, act, c);
     cost[(size_t)y * a.k.W + x] = c[0];
 }
 
