@@ -40,6 +40,7 @@
 #include <vector>
 
 #include "cvtpm.h"
+#include "cvtpm_tools.h"
 #include "pm_kernels.cuh"
 
 namespace {
@@ -225,11 +226,11 @@ struct BrickGrid {
 };
 __global__ void __launch_bounds__(256) k_tsdf_bricks(const float2* __restrict__ cv, int W, int H, int D,
                                                      unsigned char* __restrict__ fine, BrickGrid g) {
-    const int x = blockIdx.x * 256 + threadIdx.x, y0 = blockIdx.y * 8, z0 = blockIdx.z * 8;
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y0 = blockIdx.y * 8, z0 = blockIdx.z * 8;
     bool any = false;
     if (x < W) {
         const int y1 = min(y0 + 8, H), z1 = min(z0 + 8, D);
-#pragma unroll 2
+#pragma unroll 4
         for (int z = z0; z < z1; ++z) {
             const float2* p = cv + ((size_t)z * H + y0) * W + x;
             if (y1 == y0 + 8) {
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(256) k_tsdf_bricks(const float2* __restrict__ 
 #pragma unroll
                 for (int y = 0; y < 8; ++y) w[y] = __ldg(p + (size_t)y * W).y;
 #pragma unroll
-                for (int y = 0; y < 8; ++y) any = any || !(w[y] < 1.0f);
+                for (int y = 0; y < 8; ++y) any |= !(w[y] < 1.0f);
             } else {
                 for (int y = y0; y < y1; ++y, p += W) any = any || !(__ldg(p).y < 1.0f);
             }
@@ -248,27 +249,33 @@ __global__ void __launch_bounds__(256) k_tsdf_bricks(const float2* __restrict__ 
         fine[((size_t)blockIdx.z * g.fh + blockIdx.y) * g.fw + (x >> 3)] = (m >> (threadIdx.x & 31)) & 0xffu ? 1 : 0;
 }
 
-/* A coarse brick per thread: any of its 4^3 fine ones (fd of them in z). */
-__global__ void __launch_bounds__(128) k_tsdf_coarse(const unsigned char* __restrict__ fine, unsigned char* __restrict__ coarse,
+/* A coarse brick per warp: any of its 4^3 fine ones (fd of them in z). */
+__global__ void __launch_bounds__(256) k_tsdf_coarse(const unsigned char* __restrict__ fine, unsigned char* __restrict__ coarse,
                                                      BrickGrid g, int fd, int cd) {
-    const size_t i = (size_t)blockIdx.x * 128 + threadIdx.x;
-    if (i >= (size_t)g.cw * g.ch * cd) return;
+    const unsigned i = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (i >= (unsigned)(g.cw * g.ch * cd)) return;
     const int cx = (int)(i % g.cw), cy = (int)(i / g.cw % g.ch), cz = (int)(i / g.cw / g.ch);
-    unsigned char any = 0;
-    for (int z = 4 * cz; z < min(4 * cz + 4, fd); ++z)
-        for (int y = 4 * cy; y < min(4 * cy + 4, g.fh); ++y)
-            for (int x = 4 * cx; x < min(4 * cx + 4, g.fw); ++x) any |= fine[((size_t)z * g.fh + y) * g.fw + x];
-    coarse[i] = any;
+    const int x = 4 * cx + (lane & 3), y = 4 * cy + (lane >> 2 & 3), z = 4 * cz + (lane >> 4);
+    bool any = false;
+    if (x < g.fw && y < g.fh) {
+        if (z < fd) any = fine[((size_t)z * g.fh + y) * g.fw + x];
+        if (z + 2 < fd) any = any || fine[((size_t)(z + 2) * g.fh + y) * g.fw + x];
+    }
+    any = __any_sync(0xffffffffu, any);
+    if (lane == 0) coarse[i] = any;
 }
 
 /* The march evaluates samples half a voxel apart, and most of them lie where
  * nothing was integrated: a corner of weight < 1 makes the value 1e10.  With
- * bricks, a sample whose first corner lies in a brick without weights has that
+ * BRICKS, a sample whose first corner lies in a brick without weights has that
  * value at once.  It then steps to the last sample it expects inside the brick,
  * with the additions to lambda alone: if that one is in the brick, so are those
  * between (a position is monotone in lambda, rounded or not) and all have the
  * value 1e10; if not, it takes one step.  The values met, and so the results,
- * are those of the plain march. */
+ * are those of the plain march.  That is a kernel of its own: with the bricks'
+ * registers in its loop it took 10-16 % longer (256^3, 64x48 rays, empty, 0.146
+ * -> 0.168 ms). */
+template <bool BRICKS>
 __global__ void __launch_bounds__(256) k_tsdf_raycast(float* __restrict__ out, size_t opitch4, int iw, int ih,
                                                       const float2* __restrict__ cv, int W, int H, int D,
                                                       BrickGrid bg,
@@ -286,63 +293,74 @@ __global__ void __launch_bounds__(256) k_tsdf_raycast(float* __restrict__ out, s
     if (rs < re && isfinite(rs) && isfinite(re) && isfinite(dx) && isfinite(dy) && isfinite(dz)) {
         const float vx = fabsf(dx * (re - rs)), vy = fabsf(dy * (re - rs)), vz = fabsf(dz * (re - rs));
         const float step = 0.5f * sqrtf((vx * vx + vy * vy) + vz * vz) / fmaxf(vx, fmaxf(vy, vz));
-        const float mx = (float)(W - 2), my = (float)(H - 2), mz = (float)(D - 2);
-        /* the first corner of the sample at lambda (trilinear's clamps) */
-        auto corner = [&](float lambda) {
-            return make_int3((int)fminf(fmaxf(0.0f, o4.x + dx * lambda), mx), (int)fminf(fmaxf(0.0f, o4.y + dy * lambda), my),
-                             (int)fminf(fmaxf(0.0f, o4.z + dz * lambda), mz));
-        };
-        const float ix = 1.0f / (dx * step), iy = 1.0f / (dy * step), iz = 1.0f / (dz * step);   /* steps per voxel */
         float ppz = o4.z + dz * rs;
         float vp = trilinear(cv, W, H, D, o4.x + dx * rs, o4.y + dy * rs, ppz);
         int n = 0;
         float lambda = rs + step;
-        while (lambda <= re && n < max_steps) {
-            bool empty = false;
-            if (bg.fine) {
-                const int3 c = corner(lambda);
-                int sh = TSDF_COARSE;
-                empty = !__ldg(&bg.coarse[((c.z >> sh) * bg.ch + (c.y >> sh)) * bg.cw + (c.x >> sh)]);
-                if (!empty) {
-                    sh = TSDF_FINE;
-                    empty = !__ldg(&bg.fine[((c.z >> sh) * bg.fh + (c.y >> sh)) * bg.fw + (c.x >> sh)]);
-                }
-                if (empty && !(vp < 0.0f)) {             /* 1e10 from here on makes no crossing */
-                    const int3 b = make_int3(c.x >> sh, c.y >> sh, c.z >> sh);
-                    /* the steps to the brick's far sides, less a little */
-                    const float ex = (float)((b.x + (dx > 0.0f)) << sh) - (o4.x + dx * lambda);
-                    const float ey = (float)((b.y + (dy > 0.0f)) << sh) - (o4.y + dy * lambda);
-                    const float ez = (float)((b.z + (dz > 0.0f)) << sh) - (o4.z + dz * lambda);
-                    const float far = fminf(fminf(dx != 0.0f ? ex * ix : 1e9f, dy != 0.0f ? ey * iy : 1e9f),
-                                            dz != 0.0f ? ez * iz : 1e9f) - 0.01f;
-                    const int hop = min((int)fminf(fmaxf(far, 0.0f), 256.0f), max_steps - n - 1);
-                    if (hop > 0) {
-                        float last = lambda;
-                        for (int i = 0; i < hop; ++i) last += step;
-                        const int3 l = corner(last);
-                        if (last <= re && l.x >> sh == b.x && l.y >> sh == b.y && l.z >> sh == b.z) {
-                            vp = 1e10f;
-                            ppz = o4.z + dz * last;
-                            lambda = last + step;
-                            n += hop + 1;
-                            continue;
-                        }
-                    }
-                }
-            }
-            const float pz = o4.z + dz * lambda;
-            const float v = empty ? 1e10f : trilinear(cv, W, H, D, o4.x + dx * lambda, o4.y + dy * lambda, pz);
-            if (vp < 0.0f && v > 0.0f) break;
+        /* a sample's value against the one before: true where the march ends */
+        auto met = [&](float v, float pz) {
+            if (vp < 0.0f && v > 0.0f) return true;
             if (vp > 0.0f && v < 0.0f) {
                 const float alpha = -v / (vp - v);
                 const float g = mixf(pz, ppz, alpha);   /* the reference mixes z only and uses it for x, y, z */
                 ret = fmaxf(-(dot4(tg2cam.r[2], make_float4(g, g, g, 1.0f))) * scale, 0.0f);
-                break;
+                return true;
             }
             vp = v;
             ppz = pz;
-            lambda += step;
-            ++n;
+            return false;
+        };
+        if (!BRICKS) {
+            for (; lambda <= re && n < max_steps; lambda += step, ++n) {
+                const float px = o4.x + dx * lambda, py = o4.y + dy * lambda, pz = o4.z + dz * lambda;
+                if (met(trilinear(cv, W, H, D, px, py, pz), pz)) break;
+            }
+        } else {
+            const float mx = (float)(W - 2), my = (float)(H - 2), mz = (float)(D - 2);
+            /* the first corner of the sample at lambda (trilinear's clamps) */
+            auto corner = [&](float lambda) {
+                return make_int3((int)fminf(fmaxf(0.0f, o4.x + dx * lambda), mx), (int)fminf(fmaxf(0.0f, o4.y + dy * lambda), my),
+                                 (int)fminf(fmaxf(0.0f, o4.z + dz * lambda), mz));
+            };
+            const float ix = 1.0f / (dx * step), iy = 1.0f / (dy * step), iz = 1.0f / (dz * step);   /* steps per voxel */
+            while (lambda <= re && n < max_steps) {
+                bool empty = false;
+                {
+                    const int3 c = corner(lambda);
+                    int sh = TSDF_COARSE;
+                    empty = !__ldg(&bg.coarse[((c.z >> sh) * bg.ch + (c.y >> sh)) * bg.cw + (c.x >> sh)]);
+                    if (!empty) {
+                        sh = TSDF_FINE;
+                        empty = !__ldg(&bg.fine[((c.z >> sh) * bg.fh + (c.y >> sh)) * bg.fw + (c.x >> sh)]);
+                    }
+                    if (empty && !(vp < 0.0f)) {             /* 1e10 from here on makes no crossing */
+                        const int3 b = make_int3(c.x >> sh, c.y >> sh, c.z >> sh);
+                        /* the steps to the brick's far sides, less a little */
+                        const float ex = (float)((b.x + (dx > 0.0f)) << sh) - (o4.x + dx * lambda);
+                        const float ey = (float)((b.y + (dy > 0.0f)) << sh) - (o4.y + dy * lambda);
+                        const float ez = (float)((b.z + (dz > 0.0f)) << sh) - (o4.z + dz * lambda);
+                        const float far = fminf(fminf(dx != 0.0f ? ex * ix : 1e9f, dy != 0.0f ? ey * iy : 1e9f),
+                                                dz != 0.0f ? ez * iz : 1e9f) - 0.01f;
+                        const int hop = min((int)fminf(fmaxf(far, 0.0f), 256.0f), max_steps - n - 1);
+                        if (hop > 0) {
+                            float last = lambda;
+                            for (int i = 0; i < hop; ++i) last += step;
+                            const int3 l = corner(last);
+                            if (last <= re && l.x >> sh == b.x && l.y >> sh == b.y && l.z >> sh == b.z) {
+                                vp = 1e10f;
+                                ppz = o4.z + dz * last;
+                                lambda = last + step;
+                                n += hop + 1;
+                                continue;
+                            }
+                        }
+                    }
+                }
+                const float pz = o4.z + dz * lambda;
+                if (met(empty ? 1e10f : trilinear(cv, W, H, D, o4.x + dx * lambda, o4.y + dy * lambda, pz), pz)) break;
+                lambda += step;
+                ++n;
+            }
         }
     }
     out[(size_t)gy * opitch4 + gx] = ret;
@@ -379,6 +397,20 @@ struct cvtpm_tsdf {
     float2* vol;
     unsigned char* bricks;     /* marks of the ray casts, behind the volume; NULL: no room for them */
 };
+
+/* The bricks cost a pass over the volume and two launches, and save the
+ * evaluations of empty samples: time that grows with the rays times an extent,
+ * and with the extent alone where the rays are too few to fill the GPU.  Without
+ * and with, ms, a scene with a surface: 640x480 rays 96^3 0.112, 0.111, 256^3
+ * 0.264, 0.210, 512^3 0.622, 0.496, 768^3 1.06, 1.03, 1024^3 1.58, 1.95; 320x240
+ * rays 256^3 0.152, 0.195, 384^3 0.404, 0.339, 512^3 0.534, 0.508, 768^3 0.88,
+ * 1.03, 64x512x512 0.136, 0.101, 512x512x64 0.048, 0.053; 1280x960 rays 48^3
+ * 0.187, 0.200; 1920x1080 rays 1024^3 5.3, 2.7.  (Empty volumes gain more; where
+ * every voxel has weight, 256^3 with 640x480 rays, 0.50 and 0.70.) */
+static bool bricks_pay(int W, int H, int D, int dwidth, int dheight) {
+    const double rays = (double)dwidth * dheight, extent = ((double)W + H + D) / 3, voxels = (double)W * H * D;
+    return extent >= 64 && rays * extent >= 27e6 && voxels <= 2 * (rays + 100000) * extent;
+}
 
 /* bricks of 1 << sh voxels along an extent */
 static int tsdf_bricks(int extent, int sh) { return (extent + (1 << sh) - 1) >> sh; }
@@ -484,6 +516,10 @@ cvtpm_status cvtpm_tsdf_add_depthmap(cvtpm_tsdf* v, const float* proj, const flo
     return e == cudaSuccess ? CVTPM_OK : fail(CVTPM_ERR_CUDA, std::string("tsdf add: ") + cudaGetErrorString(e));
 }
 
+int cvtpm_tool_tsdf_bricks(int width, int height, int depth, int dwidth, int dheight) {
+    return bricks_pay(width, height, depth, dwidth, dheight) ? 1 : 0;
+}
+
 cvtpm_status cvtpm_tsdf_raycast(cvtpm_tsdf* v, const float* proj, float* depthmap, int dwidth, int dheight,
                                 size_t dpitch, float scale, void* stream) {
     if (!v || !proj || !depthmap) return fail(CVTPM_ERR_INVALID_ARGUMENT, "tsdf raycast: NULL argument");
@@ -498,22 +534,17 @@ cvtpm_status cvtpm_tsdf_raycast(cvtpm_tsdf* v, const float* proj, float* depthma
     cudaSetDevice(v->device);
     BrickGrid g = {nullptr, nullptr, tsdf_bricks(v->W, TSDF_FINE), tsdf_bricks(v->H, TSDF_FINE),
                    tsdf_bricks(v->W, TSDF_COARSE), tsdf_bricks(v->H, TSDF_COARSE)};
-    /* The bricks cost a pass over the volume and two launches, and save the
-     * evaluations of empty samples, which count where there are many rays: 256^3
-     * with 640x480 rays 0.30 -> 0.24 ms, 128^3 0.17 -> 0.15, 512^3 0.66 -> 0.53;
-     * but 256^3 with 320x240 0.19 -> 0.22 and 48^3 with 640x480 0.09 -> 0.12. */
-    const size_t samples = (size_t)dwidth * dheight * (size_t)(max_steps / 2);
-    if (v->bricks && samples >= 30000000) {
+    if (v->bricks && bricks_pay(v->W, v->H, v->D, dwidth, dheight)) {
         /* formed anew for each cast: the caller may write the volume (cvtpm_tsdf_info) */
         const int fd = tsdf_bricks(v->D, TSDF_FINE), cd = tsdf_bricks(v->D, TSDF_COARSE);
         unsigned char *fine = v->bricks, *coarse = fine + (size_t)g.fw * g.fh * fd;
-        k_tsdf_bricks<<<dim3((v->W + 255) / 256, g.fh, fd), 256, 0, (cudaStream_t)stream>>>(v->vol, v->W, v->H, v->D, fine, g);
-        const size_t nc = (size_t)g.cw * g.ch * cd;
-        k_tsdf_coarse<<<(unsigned)((nc + 127) / 128), 128, 0, (cudaStream_t)stream>>>(fine, coarse, g, fd, cd);
+        const int threads = v->W < 256 ? (v->W + 31) / 32 * 32 : 256;
+        k_tsdf_bricks<<<dim3((v->W + threads - 1) / threads, g.fh, fd), threads, 0, (cudaStream_t)stream>>>(v->vol, v->W, v->H, v->D, fine, g);
+        k_tsdf_coarse<<<(g.cw * g.ch * cd + 7) / 8, 256, 0, (cudaStream_t)stream>>>(fine, coarse, g, fd, cd);
         g.fine = fine;
         g.coarse = coarse;
     }
-    k_tsdf_raycast<<<dim3((dwidth + 31) / 32, (dheight + 7) / 8), dim3(32, 8), 0, (cudaStream_t)stream>>>(
+    (g.fine ? k_tsdf_raycast<true> : k_tsdf_raycast<false>)<<<dim3((dwidth + 31) / 32, (dheight + 7) / 8), dim3(32, 8), 0, (cudaStream_t)stream>>>(
         depthmap, dpitch / 4, dwidth, dheight, v->vol, v->W, v->H, v->D, g, Ti, T, scale, max_steps);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? CVTPM_OK : fail(CVTPM_ERR_CUDA, std::string("tsdf raycast: ") + cudaGetErrorString(e));

@@ -34,6 +34,10 @@ cvtpm_status cvtpm_tool_pd_time(cvtpm_ctx* ctx, int steps, void* stream, float* 
 #define CVTPM_ROUTE_TAP_ADJOINT 8   /* cvtpm_cost_adjoint with image gradients */
 int cvtpm_tool_routes(const cvtpm_params* params, int width, int height);
 
+/* Whether a ray cast of dwidth x dheight rays steps over the empty bricks of a
+ * volume of this size (1) or marches plainly (0).  No device is needed. */
+int cvtpm_tool_tsdf_bricks(int width, int height, int depth, int dwidth, int dheight);
+
 #ifdef __cplusplus
 }
 #endif
