@@ -546,7 +546,8 @@ cvtpm_status run_depthmap(cvtpm_ctx* ctx, const cvtpm_params& p, float* dmap, si
      * view's smoother and pass: the launches of the two chains fill the SMs
      * that the other's last waves leave idle (321x243 51.0 -> 44.5 ms, 1242x375
      * 339.3 -> 335.5).  The right view's pass then takes the left view's planes
-     * and refines on `st`. */
+     * and refines on `st`.  Not while the phases are timed, on `st`. */
+    overlap = overlap && !ctx->timing;
     auto right_own = [&](int iter, float th) -> cvtpm_status {
         const int sw = iter & 1;
         aR.iter = iter;
@@ -565,17 +566,22 @@ cvtpm_status run_depthmap(cvtpm_ctx* ctx, const cvtpm_params& p, float* dmap, si
         const int sw = iter & 1;
         const bool redblack = p.schedule == CVTPM_SCHEDULE_REDBLACK;
         const float next = iter >= 5 ? smoothstep01(((float)iter - 5.0f) / ((float)N - 5.0f)) * 1.0f : theta;
+        aL.iter = iter;
+        aL.theta = theta;
+        aL.old = ctx->S[0][sw]; aL.out = ctx->S[0][1 - sw]; aL.smooth = ctx->smooth[0];
+        aL.viewin = ctx->list[1]; aL.viewsrc = ctx->S[1][sw];
         {
-            NvtxRange r("propagate left and right");
+            NvtxRange r("propagate left");
             PhaseTimer tm(ctx, st, ctx->ev_prop);
-            aL.iter = iter;
-            aL.theta = theta;
-            aL.old = ctx->S[0][sw]; aL.out = ctx->S[0][1 - sw]; aL.smooth = ctx->smooth[0];
-            aL.viewin = ctx->list[1]; aL.viewsrc = ctx->S[1][sw];
             if ((s = propagate_view(ctx, aL, exact, redblack, n, st)) != CVTPM_OK) return s;
-            LK(pm_launch_view_list(ctx->S[0][1 - sw], W, H, ctx->list[0], st), "view list");
-            if (overlap || iter > first) CK(cudaStreamWaitEvent(st, ctx->side_join, 0), "join");   /* smooth[1] */
-            aR.viewin = ctx->list[0]; aR.viewsrc = ctx->S[0][1 - sw];
+            tm.stop();
+        }
+        LK(pm_launch_view_list(ctx->S[0][1 - sw], W, H, ctx->list[0], st), "view list");
+        if (overlap || iter > first) CK(cudaStreamWaitEvent(st, ctx->side_join, 0), "join");   /* smooth[1] */
+        aR.viewin = ctx->list[0]; aR.viewsrc = ctx->S[0][1 - sw];
+        {
+            NvtxRange r("propagate right");
+            PhaseTimer tm(ctx, st, ctx->ev_prop);
             if (overlap) {
                 LK(pm_launch_pass_rest(aR, exact, st), "propagate");
             } else {
