@@ -1947,6 +1947,20 @@ cvtpm_status cvtpm_tool_fp32_peak(int device, void* stream, float* tflops) {
     return CVTPM_OK;
 }
 
+cvtpm_status cvtpm_tool_pd_math_check(int device, void* stream, unsigned long long* bad) {
+    if (!bad) return CVTPM_ERR_INVALID_ARGUMENT;
+    if (cudaSetDevice(device) != cudaSuccess) return CVTPM_ERR_CUDA;
+    cudaStream_t st = (cudaStream_t)stream;
+    unsigned long long* d = nullptr;
+    if (cudaMalloc(&d, 4 * sizeof(*d)) != cudaSuccess) { cudaGetLastError(); return CVTPM_ERR_ALLOC; }
+    cudaError_t e = cudaMemsetAsync(d, 0, 4 * sizeof(*d), st);
+    if (e == cudaSuccess) e = pm_launch_pd_math_check(d, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(bad, d, 4 * sizeof(*d), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(d);
+    return e == cudaSuccess ? CVTPM_OK : CVTPM_ERR_CUDA;
+}
+
 int cvtpm_tool_routes(const cvtpm_params* params, int width, int height) {
     if (!params || width < 1 || height < 1 || params->patchsize < 1) return -1;
     PmCostConsts k;

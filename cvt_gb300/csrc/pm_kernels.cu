@@ -1537,8 +1537,9 @@ PM_DEV float2 neg_div2_any(float2 x, float2 b, float2 ny) {
 /* s = RN(sqrt(v)) and ny = -RN(1 / s) for both halves, 1 <= v <= PDS_VMAX:
  * Newton's iteration for 1 / sqrt(v) from rsqrt.approx and one fused residual
  * step each for the root and its reciprocal (Markstein, as above).  Compared
- * with __fsqrt_rn and __frcp_rn for every float in [1, 2^100]: the roots are
- * all equal, and so are the reciprocals but those of significands of ones.
+ * with __fsqrt_rn and __frcp_rn for every float in [1, 2^100], and in
+ * k_pd_math_check for those of two binades and a stride of the rest: the roots
+ * are all equal, and so are the reciprocals but those of significands of ones.
  * Those, and they alone, leave a residual of 2^-24 before the last step: the
  * return value is the larger residual. */
 #define PDS_VMAX 1.0995116e12f                       /* 2^40: s <= 2^20 */
@@ -2231,6 +2232,68 @@ cudaError_t pm_launch_occmap(const float4* L, const float4* R, int W, int H, flo
 cudaError_t pm_launch_normal_depth(const float4* in, int W, int H, float depthmax, int lr, float4* out,
                                    cudaStream_t st) {
     k_normal_depth<<<pix_grid(W, H), dim3(32, 8), 0, st>>>(in, W, H, depthmax, lr, out);
+    PM_LAUNCH_CHECK();
+    return cudaSuccess;
+}
+
+/* ------------------------------------- the smoother's divisions, checked -- */
+PM_DEV uint32_t check_hash(uint32_t v) {                  /* Wang's integer hash */
+    v = (v ^ 61u) ^ (v >> 16);
+    v *= 9u;
+    v ^= v >> 4;
+    v *= 0x27d4eb2du;
+    return v ^ (v >> 15);
+}
+/* bad[0]: roots or reciprocals of norm2 that are not RN(sqrt v), -RN(1 / s) and
+ * not flagged by the residual; bad[1]: flagged ones that are right; bad[2]: quotients
+ * of neg_div2_any that are not -RN(x / b); bad[3]: of neg_div2, 2^-100 <= |x| <
+ * 2^60.  norm2: every float of [1, 4), then every 251st of [1, 2^40].  neg_div2_any:
+ * quotients around every kind of subnormal tie (half-way points k + 1/2 units,
+ * exact ones and the floats beside them), and x of any size. */
+__global__ void __launch_bounds__(256) k_pd_math_check(unsigned long long* bad) {
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;        /* 2^24 threads */
+    unsigned wrong = 0, idle = 0;
+    for (int part = 0; part < 2; ++part) {
+        const uint32_t bits = part ? 0x3f800000u + i % 1336935u * 251u : 0x3f800000u + i;
+        const float v = fminf(__uint_as_float(bits), PDS_VMAX);
+        float2 s, ny;
+        const float e = norm2(make_float2(v, v), s, ny);
+        const float sr = __fsqrt_rn(v);
+        const bool ok = s.x == sr && s.y == sr && ny.x == -__frcp_rn(sr) && ny.y == ny.x;
+        wrong += !ok && e < PDS_RESID;
+        idle += ok && !(e < PDS_RESID);
+    }
+    if (wrong) atomicAdd(&bad[0], wrong);
+    if (idle) atomicAdd(&bad[1], idle);
+    unsigned any = 0, plain = 0;
+    for (int part = 0; part < 4; ++part) {
+        const uint32_t h = check_hash(4 * i + part), g = check_hash(h ^ 0x9e3779b9u);
+        /* b in [1, 2^20]: a power of two, one of few bits, any */
+        const int eb = (int)(g % 20u);
+        const uint32_t mb = part == 0 ? 0u : part == 1 ? (g >> 8) & 0x700000u : (g >> 8) & 0x7fffffu;
+        const float b = __uint_as_float(((uint32_t)(127 + eb) << 23) | mb);
+        float x;
+        if (part < 3) {                                       /* near (k + 1/2) 2^-149 b */
+            const float k = (float)(h % (part == 2 ? 8388607u : 4096u));
+            x = (float)(((double)k + 0.5) * (double)b * exp2(-149.0));
+            x = __uint_as_float(__float_as_uint(x) + (h >> 29) % 5u - 2u + (__float_as_uint(x) < 2u ? 2u : 0u));
+        } else {
+            x = __uint_as_float((h & 0x007fffffu) | (h % 187u) << 23);      /* below 2^60 */
+        }
+        if (h & 0x10000000u) x = -x;
+        const float2 xx = make_float2(x, 0.5f * b), bb = make_float2(b, b), nn = make_float2(-__frcp_rn(b), -__frcp_rn(b));
+        const float2 q = neg_div2_any(xx, bb, nn);
+        const float want = x == 0.0f ? -x : -__fdiv_rn(x, b);
+        any += __float_as_uint(q.x) != __float_as_uint(want) || q.y != -0.5f;
+        if (part == 3 && fabsf(x) >= 7.8886091e-31f)
+            plain += __float_as_uint(neg_div2(xx, bb, nn).x) != __float_as_uint(want);
+    }
+    if (any) atomicAdd(&bad[2], any);
+    if (plain) atomicAdd(&bad[3], plain);
+}
+
+cudaError_t pm_launch_pd_math_check(unsigned long long* bad, cudaStream_t st) {
+    k_pd_math_check<<<65536, 256, 0, st>>>(bad);
     PM_LAUNCH_CHECK();
     return cudaSuccess;
 }

@@ -160,6 +160,9 @@ size_t pm_pd_dual_bytes(int W, int H);
 cudaError_t pm_launch_pd_block(float4* uout, float* pout, const float4* uin, const float* pin, int pzero,
                                const float4* f, const float* wgt, const float* mask, float lambda, int nsteps, int W,
                                int H, cudaStream_t st);
+/* Compares the smoother's divisions, roots and reciprocals with the IEEE ones
+ * (k_pd_math_check); bad: four counts, cleared before. */
+cudaError_t pm_launch_pd_math_check(unsigned long long* bad, cudaStream_t st);
 cudaError_t pm_launch_ffma_peak(float* out, int blocks, int iters, cudaStream_t st);
 
 /* pm_adjoint.cu */

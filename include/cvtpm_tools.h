@@ -24,6 +24,12 @@ cvtpm_status cvtpm_tool_fp32_peak(int device, void* stream, float* tflops);
  * smoothers concurrently, so its per-phase timings cannot give this. */
 cvtpm_status cvtpm_tool_pd_time(cvtpm_ctx* ctx, int steps, void* stream, float* us_per_step);
 
+/* The smoother's square roots, reciprocals and divisions against the correctly
+ * rounded ones, on `device`; waits.  bad (4 counts): wrong roots or reciprocals
+ * that the residual does not flag, right ones that it flags, wrong quotients of
+ * the form for any size, of the form for moderate sizes. */
+cvtpm_status cvtpm_tool_pd_math_check(int device, void* stream, unsigned long long* bad);
+
 /* The routes that calls of these parameters (patchsize, arith) take for an image
  * size; -1 for a bad argument.  No device is needed.  Routes never change
  * results. */
