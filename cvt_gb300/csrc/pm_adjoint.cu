@@ -159,10 +159,10 @@ __device__ __forceinline__ void add_image(float4* dI, float4* dG, size_t o, cons
     atomicAdd(&dI[o], make_float4(t.v0.x, t.v0.y, t.v1.x, 0.0f));
     atomicAdd(&dG[o], make_float4(t.v1.y, t.v2.x, t.v2.y, t.v3));
 }
-/* w with the sign of e, 0 for e == 0 (w sgn(e)); with a cap, also 0 where |e| is not below it */
+/* w sgn(e), a NaN where w is not finite and e is 0; with a cap, for a finite w, also 0 where |e| is not below it */
 __device__ __forceinline__ float wsgn(float w, float e) {
     const float s = __int_as_float(__float_as_int(w) ^ (__float_as_int(e) & 0x80000000));
-    return e > 0.0f || e < 0.0f ? s : 0.0f;
+    return e > 0.0f || e < 0.0f ? s : w * 0.0f;
 }
 __device__ __forceinline__ float wsgn(float w, float e, float cap) {
     const float s = __int_as_float(__float_as_int(w) ^ (__float_as_int(e) & 0x80000000));
