@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(256) k_cost_adjoint(PmAdjArgs a) {
     float gs0 = 0.0f, gs1 = 0.0f, gs2 = 0.0f;
     float centre[3] = {0.0f, 0.0f, 0.0f};               /* terms of the centre colour */
     if (__any_sync(0xffffffffu, act)) {
-        const float u = act ? g / ws : 0.0f;
+        const float u = act ? g / ws + a.k.alpha * 0.0f : 0.0f;   /* a share that is not finite leaves a NaN, also beside zero slopes */
         const float al = a.k.alpha, oma = a.k.oma;
         const int qy0 = max(y - P, 0), qy1 = min(y + P, H - 1);
         /* inside the image for some lane, which the shuffles and uniform reads of the profile want, or for this one */

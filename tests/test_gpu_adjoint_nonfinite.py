@@ -30,3 +30,22 @@ def test_infinite_gradient(cuda, g, sx, sy, W, H):
     d1 = d1.cpu().numpy()[..., :3]
     assert np.isnan(d1[3:6, 5:8]).all()
     assert (d1[:2] == 0).all() and (d1[7:] == 0).all()
+
+
+@pytest.mark.parametrize("alpha", [np.nan, np.inf])
+def test_alpha_not_finite(cuda, alpha):
+    """A colour share that is not finite leaves NaN gradients at every pixel with
+    support (a cost that is not 1e5), also where residuals are 0 or truncated."""
+    from cvt_gb300.stereo import PMHuberStereo
+    H, W = 9, 40
+    rng = np.random.default_rng(3)
+    left = rng.random((H, W, 4), np.float32)
+    planes = np.zeros((H, W, 4), np.float32)
+    p = default_params(PRESET_BASELINE, patchsize=1, color_alpha=float(alpha))
+    st = PMHuberStereo(0, p)
+    L = torch.from_numpy(left).cuda()
+    C, dpl, d1, d2 = st.cost_adjoint(L, L, torch.from_numpy(planes).cuda(), 1, dcost=torch.ones((H, W), device="cuda"))
+    m = C != 1e5
+    assert m.any()
+    for t in (dpl, d1, d2):
+        assert torch.isnan(t[..., :3][m]).all()
