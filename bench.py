@@ -40,11 +40,15 @@ WORKLOAD = "plain PatchMatch depthMap, 1 pair 1242x375 RGBA f32, 16 planes, dmax
 METRIC = "PatchMatch Mpix-iter/s (plain depthMap, 1242x375, 8 iterations)"
 FLOPS_PER_TAP = 55.0          # per (pixel, candidate) window tap: plane, lerp, truncated L1, accumulate
 FLOPS_PER_WEIGHT_TAP = 20.0   # bilateral weight of a tap, once per pixel and launch
-RECORD_BYTES_PER_TAP = 56.0   # the other view's value/difference records one evaluated tap reads (FAST)
+FLOPS_PER_FOLD = 5.0          # a shared tap's terms into one candidate's sums
+SHARED = 14                   # candidates of a pass that share plane windows (1-8, 10-15)
+SHARED_REACH = 4              # half of the 8 columns or rows by which the pixels testing a plane differ
+RECORD_BYTES_PER_TAP = 56.0   # the other view's value/difference records one tap reads (FAST, shared windows)
+COLUMN_BYTES_PER_TAP = 28.0   # the one new column a tap of a sweep reads (FAST)
 L1_BYTES_PER_CLK_SM = 128.0   # L1/shared data path of one SM
 FP32_LANES_PER_SM = 128       # FP32 CUDA cores per SM (FMA = 2 flops)
 QUALITY_PAIRS = 8
-PD_BYTES_PER_PX = 116.0       # u 16 + p 32 + f 16 + w 4 read; u 16 + p 32 written
+PD_BYTES_PER_PX = 100.0       # a launch: u 16 + p 24 + f 16 + w 4 read; u 16 + p 24 written
 
 
 def params_for(impl: str):
@@ -303,7 +307,12 @@ def run_ours(args, rank, world, local_rank):
     # ---- roofline of the dominant kernel (propagation: FP32 CUDA cores)
     nprop = max(1, stats["propagate_launches"])
     prop_ms = stats["propagate_ms"] / nprop
-    flops_launch = (stats["cost_taps"] * FLOPS_PER_TAP) / nprop + in_image_taps(W, H, PATCH) * FLOPS_PER_WEIGHT_TAP
+    # the work a pass cannot do without: the other candidates' windows, one window
+    # per plane for all pixels that test it, their folds, one set of weights
+    taps, plane_taps = in_image_taps(W, H, PATCH), in_image_taps(W, H, PATCH + SHARED_REACH)
+    own_taps = stats["cost_taps"] / nprop - SHARED * taps
+    flops_launch = ((own_taps + plane_taps) * FLOPS_PER_TAP + SHARED * taps * FLOPS_PER_FOLD + taps * FLOPS_PER_WEIGHT_TAP)
+    all_windows = stats["cost_taps"] / nprop * FLOPS_PER_TAP + taps * FLOPS_PER_WEIGHT_TAP
     achieved = flops_launch / (prop_ms * 1e-3) / 1e12
     traffic = read_traffic()
     roofline = {"kernel": "k_sweep + k_share + k_views + k_propagate (the propagation pass, fast)", "bound": "fp32", "achieved": achieved,
@@ -312,6 +321,8 @@ def run_ours(args, rank, world, local_rank):
                 "traffic": traffic.get("k_propagate_bytes_per_launch"),
                 "peak_source": "FFMA-chain probe run in this process (cvtpm_tool_fp32_peak), FMA = 2 flops",
                 "flops_per_launch": flops_launch, "launch_ms": prop_ms,
+                "work": "each plane's tap terms once for all candidates that share them",
+                "tflops_if_every_candidate_swept_its_window": all_windows / (prop_ms * 1e-3) / 1e12,
                 "share_of_step": stats["propagate_ms"] / max(1e-9, phase_ms),
                 "timed": f"{phase_steps} steps of their own after the timed region, all propagation launches on one stream"}
     hbm_peak, hbm_src = peaks()
@@ -320,18 +331,19 @@ def run_ours(args, rank, world, local_rank):
     pd_us = _lib.ctypes.c_float()
     rc = _lib.lib().cvtpm_tool_pd_time(st._h, 248, _lib.ctypes.c_void_p(stream.cuda_stream), _lib.ctypes.byref(pd_us))
     pd_ms = float(pd_us.value) * 1e-3 if rc == 0 else float("nan")   # per PD step (a launch runs up to 4)
-    pd_bytes = PD_BYTES_PER_PX * W * H
+    pd_steps = stats["pd_steps"] / max(1, stats["pd_launches"])
+    pd_bytes = PD_BYTES_PER_PX * W * H / pd_steps
     roofline_pd = {"kernel": "k_pd_block", "bound": "hbm", "achieved": pd_bytes / (pd_ms * 1e-3) / 1e9,
                    "peak": hbm_peak, "unit": "GB/s", "frac": pd_bytes / (pd_ms * 1e-3) / 1e9 / hbm_peak,
                    "traffic": (traffic["k_pd_block_bytes_per_launch"] / traffic.get("k_pd_block_steps_per_launch", 4)
                                if "k_pd_block_bytes_per_launch" in traffic else None),
                    "traffic_per": "PD step (DRAM bytes of one 4-step launch / 4)", "peak_source": hbm_src,
-                   "per": "PD step (algorithmic bytes of one step / time of one step)",
-                   "steps_per_launch": stats["pd_steps"] / max(1, stats["pd_launches"]),
+                   "per": "PD step (a launch's bytes, each read and written once, and its time, over its steps)",
+                   "steps_per_launch": pd_steps,
                    "timed": "the blocked PD kernel alone, 248 steps on the bench pair's left smoother input "
                             "(cvtpm_tool_pd_time); inside depthMap the two views' smoothers run concurrently",
-                   "note": "the blocked kernel keeps 4 steps in registers, so it moves fewer bytes than one step's algorithmic count"}
-    # the propagation's L1 rate: the algorithm's record bytes against
+                   "note": "what bounds the kernel is the latency of its dependent steps, not these bytes"}
+    # the propagation's L1 rate: the other view's bytes of those taps against
     # 128 B per clock and SM at the sampled clock
     clocks = clk.summary()
     n_sm = torch.cuda.get_device_properties(dev).multi_processor_count
@@ -341,13 +353,12 @@ def run_ours(args, rank, world, local_rank):
     roofline["frac_of_derived"] = (achieved / fp32_derived) if fp32_derived else None
     roofline["peak_derived_source"] = (f"{n_sm} SMs x {FP32_LANES_PER_SM} FP32 lanes x 2 flops x the median SM clock "
                                        "sampled during the timed region")
-    l1_achieved = stats["cost_taps"] / nprop * RECORD_BYTES_PER_TAP / (prop_ms * 1e-3) / 1e9
+    l1_achieved = (own_taps * COLUMN_BYTES_PER_TAP + plane_taps * RECORD_BYTES_PER_TAP) / (prop_ms * 1e-3) / 1e9
     roofline_l1 = {"kernel": "k_sweep + k_share + k_views + k_propagate (the propagation pass, fast)", "bound": "l1",
                    "achieved": l1_achieved, "peak": l1_peak, "unit": "GB/s",
                    "frac": (l1_achieved / l1_peak) if l1_peak else None,
-                   "per": "pass: device-counted evaluated taps x 56 record bytes, as if every candidate read its own "
-                          "window (k_share reads a plane's window once for all candidates that test it, and the "
-                          "sweeps 28 bytes a tap, so the rate can pass the peak) / pass time",
+                   "per": "pass: 28 bytes (one column) per tap of the sweeps, 56 (a record) per tap of a plane's shared "
+                          "window / pass time; image-1 reads and shared memory come on top",
                    "peak_source": f"{n_sm} SMs (from the device) x 128 B/clk x the median SM clock sampled during "
                                   "the timed region"}
     cpu = None

@@ -105,8 +105,10 @@ typedef struct cvtpm_stats {
     uint64_t calls;              /* depthmap calls                              */
     uint64_t launches;           /* kernels this library launched               */
     uint64_t propagate_launches;
-    uint64_t cost_evals;         /* (pixel, candidate) cost evaluations of the
-                                    propagation passes, counted on the device   */
+    uint64_t cost_evals;         /* (pixel, candidate) pairs the propagation passes
+                                    tested, counted on the device (a refinement that
+                                    repeats a rejected one among them, though its
+                                    cost is not formed again)                   */
     uint64_t cost_taps;          /* in-image window taps of those evaluations   */
     uint64_t pd_launches;
     uint64_t pd_steps;           /* PD smoother steps (several per launch)      */
