@@ -24,15 +24,15 @@
  * OpenCL) reads the texel.  dot sums left to right.
  *
  * The disparities run in batches (the grid's z index is the disparity in
- * the batch): per batch one pass forms the cost and block-scans its two
- * integral images, three launches finish them, one pass forms the guided
- * filter's (a, b) from their box means and block-scans a and b, three launches
- * finish those, and one pass per pixel walks the batch's disparities in order
- * through the box means of a and b, the filter output and the running
- * minimum: 9 launches per batch, where the reference launches 24 kernels per
- * disparity.  Measured on the 1242x375 x 128 workload: the cost and (a, b)
- * passes are issue- and L1-bound (bilinear taps, divisions, block-scan
- * barriers), the block fix-up streams its read-modify-write at 3.3 TB/s, the
+ * the batch): per batch one pass forms the cost and block-scans the integral
+ * images of guide * cost and cost, which share one RGBA image, three launches
+ * finish it, one pass forms the guided filter's (a, b) from its box means and
+ * block-scans them, one image again, three launches finish that, and one pass
+ * per pixel walks the batch's disparities in order through the box means of a
+ * and b, the filter output and the running minimum: 9 launches per batch, where
+ * the reference launches 24 kernels per disparity.  On the 1242x375 x 128
+ * workload the cost and (a, b) passes are bound by issue and L1 (bilinear taps,
+ * divisions, shuffles), the block fix-up runs at a copy's rate, the
  * boundary-column scans are latency-bound chains.
  */
 #include <math.h>

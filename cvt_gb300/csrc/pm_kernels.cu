@@ -8,7 +8,7 @@
  *  k_sweep, k_share<EXACT>, k_propagate<EXACT, 2>  pmhstereo_propagate_view (:286-404) without the
  *                       scatter: candidates 9, 16 (k_sweep) and 17-20 (k_views) by pixel; 1-8, 10-15 by plane and the
  *                       acceptance; the refinements 21, 22
- *  k_propagate<EXACT, *>  the same with every candidate by pixel
+ *  k_propagate<EXACT, *>  the same with every candidate by pixel (red/black, small windows, narrow images)
  *  k_taps_*<EXACT>      init and propagate for small images, the taps of a window in parallel
  *  k_view_list          the scatter of :391-400, made deterministic (smallest source x first)
  *  k_consistency        pmhstereo_consistency (:428-464)
@@ -498,12 +498,12 @@ PM_DEV float4 smooth_state(float4 smooth, float cx, float cy, int lr) {
  * An invalid tap (outside either image) is marked in its first term (no_term).
  * The sums take eval_costs' operations in its order, so the costs have its bits.
  *
- * Measured at 1242x375 per view pass (ncu): 9.7 ms for the 14 candidates and
- * the acceptance, where the neighbours by plane (5.9 ms, weights in a table
- * per block) and the random neighbours by pixel (12.1 of the 16.2 ms of a
- * sweep of 8) took 18; depthMap 484.7 -> 363.7 ms, 640x480 x 3 iterations
- * 132 -> 96.3, EXACT 450x375 102 -> 73.4 ms.  With a thread's slots in one
- * column, sharing their image-1 reads: 9.2 ms.
+ * Measured at 1242x375 per view pass (ncu, mean over 8 iterations): 8.9 ms for
+ * the 14 candidates and the acceptance (9.7 at first, 9.2 with a thread's slots in one column, sharing
+ * their image-1 reads), where the neighbours by plane (5.9 ms, weights in a
+ * table per block) and the random neighbours by pixel (12.1 of the 16.2 ms of a
+ * sweep of 8) took 18; depthMap 484.7 -> 363.7 ms, 640x480 x 3 iterations 132 ->
+ * 96.3, EXACT 450x375 102 -> 73.4 ms.
  */
 #define SH_TY 16
 #define SH_NX 40
@@ -1809,7 +1809,7 @@ PM_DEV void pds_tile(float4* __restrict__ uout, float* __restrict__ pout, const 
 }
 
 /* The plain path's region: 8 warps of 3 rows, 4 steps (a 56 x 16 tile), two
- * blocks per SM (108 registers). */
+ * blocks per SM (118 registers). */
 #define PDS_NW 8
 #define PDS_R 3
 #define PDS_K 4
